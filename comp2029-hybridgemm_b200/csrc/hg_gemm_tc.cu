@@ -21,9 +21,10 @@
 //   tcgen05.cp 32x128b.warpx4; the byte of the current K32 block is selected
 //   with the a_sf_id/b_sf_id descriptor fields.
 // * Issue: up to four MMA-issuing threads in separate warps (two by default),
-//   each with its own accumulator: a tcgen05 instruction costs its issuing
-//   thread 50-430 cycles whatever its shape (MMA 90, scale copy 51, commit 432)
-//   and threads issue in parallel.  Up to 64-token tiles issuer q owns every
+//   each with its own accumulator.  A whole warp walks the issue loop and an
+//   elected lane issues: 45 cycles per MMA, against 80 behind a lane == 0 branch
+//   (the tensor core itself needs 40 at 16 tokens, 64 at 128: reading a 4 KiB
+//   slice of the weight tile from shared memory).  Up to 64-token tiles issuer q owns every
 //   I-th pipeline stage; wider tiles have a three-stage ring, and there both
 //   issuers read every stage, issuer q its K128 block q.
 // * Decode sizes (at most 16 tokens) can quantise their activations in the
@@ -178,6 +179,23 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
       if (clock64() - start > kWaitLimitCycles) return false;
     }
   }
+}
+
+// The same wait by a whole warp, with one verdict for all lanes.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)) != 0;
+}
+// True in one lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}"
+      : "=r"(r));
+  return r != 0;
 }
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
@@ -551,77 +569,92 @@ hybrid_gemm_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant_
     }
   } else if (warp == 1 || (warp >= 10 && warp < 13)) {
     // ------------------------------------------------------------------ MMA issuers (warps 1, 10, 11, 12)
-    // A tcgen05 instruction costs its issuing thread on the order of a hundred cycles (descriptor set-up
-    // through the uniform datapath) whatever its shape, far more than a 128 x n_tile x 32 MMA occupies the
-    // tensor core.  So up to four threads in four warps issue independent streams: issuer q takes every I-th
-    // pipeline stage (or, with split_blocks, its K128 block of every stage) and accumulates into its own TMEM
-    // accumulator; the epilogue adds the accumulators in a fixed order, which keeps the result deterministic.
-    const int q = warp == 1 ? 0 : warp - 9;
-    if (lane == 0 && q < p.issuers) {
+    // Up to four warps issue independent streams: issuer q takes every I-th pipeline stage (or, with
+    // split_blocks, its K128 block of every stage) and accumulates into its own TMEM accumulator; the epilogue
+    // adds the accumulators in a fixed order, which keeps the result deterministic.
+    // The whole warp walks the loop and ONE elected lane issues: with the control flow warp-uniform and the issue
+    // behind elect.sync, the operands of a tcgen05 instruction go straight to uniform registers (45 cycles per MMA);
+    // behind a `lane == 0` branch they are handed over lane by lane (80 cycles per MMA, 180 against 329 per K128 block).
+    const int q = __shfl_sync(0xffffffffu, warp == 1 ? 0 : warp - 9, 0);
+    if (q < p.issuers) {
       uint32_t issued = 0;
       int acc_it = 0;
       uint32_t ring = 0;                                   // pipeline stages consumed by earlier units
       const uint32_t issuer_mask = uint32_t(p.issuers) - 1u;
       int ring_slot = 0;
       uint32_t ring_round = 0;
-      const uint32_t sf_base = sf_cols + uint32_t(q) * (8u * kScaleSets);
+      const uint32_t tmem0 = __shfl_sync(0xffffffffu, tmem_base, 0), smem0 = __shfl_sync(0xffffffffu, base, 0);
+      const uint32_t sf_base = tmem0 + uint32_t(p.acc_slots) * acc_stride + uint32_t(q) * (8u * kScaleSets);
       uint32_t sf_flip = 0;
-      for (int u = unit_begin; u < unit_end && !error; ++u, ++acc_it) {
+      const int u_end = __shfl_sync(0xffffffffu, unit_end, 0);
+      for (int u = __shfl_sync(0xffffffffu, unit_begin, 0); u < u_end && !error; ++u, ++acc_it) {
         const WorkUnit wu = u == unit_begin ? first_unit : p.units[u];
-        const int part = wu.tile >= p.tiles[0];
+        const int kb_begin = __shfl_sync(0xffffffffu, wu.kb_begin, 0), kb_end = __shfl_sync(0xffffffffu, wu.kb_end, 0);
+        const int part = __shfl_sync(0xffffffffu, int(wu.tile >= p.tiles[0]), 0);
         const int slot = acc_it % p.acc_slots;
-        const uint32_t unit_stages = uint32_t(wu.kb_end - wu.kb_begin + 1) >> 1;
-        if (!mbar_wait(acc_empty_bar(slot), (uint32_t(acc_it / p.acc_slots) & 1u) ^ 1u, abort_flag)) { error = kErrMmaAcc; break; }
+        const uint32_t unit_stages = uint32_t(kb_end - kb_begin + 1) >> 1;
+        if (!warp_wait(acc_empty_bar(slot), (uint32_t(acc_it / p.acc_slots) & 1u) ^ 1u, abort_flag)) { error = kErrMmaAcc; break; }
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + uint32_t(slot) * acc_stride + uint32_t(q) * acc_cols;
+        const uint32_t tmem_d = tmem0 + uint32_t(slot) * acc_stride + uint32_t(q) * acc_cols;
         const uint32_t idesc = instr_desc(part == 0, p.n_tile);
         // SFB of token tile t0 sits in column (t0 % 128) / 32 of its 128-token atom.
-        const uint32_t sfb_col = uint32_t((wu.token_tile * p.n_tile) % 128) / 32u;
+        const uint32_t sfb_col = uint32_t((__shfl_sync(0xffffffffu, wu.token_tile, 0) * p.n_tile) % 128) / 32u;
         // Ownership follows the ring SLOT of the global stage number g: issuer (g % stages) % issuers.  Each
         // ring slot, and with it each full/empty barrier, then has exactly one consumer that sees every round
         // in turn, so parity waits stay unambiguous however short units are.
         // The ring depth is a multiple of the issuer count (1, 2 or 4), so (g % stages) % issuers is g % issuers.
-        bool fresh = true;   // this issuer's accumulator has not been written in this unit yet
+        uint32_t accumulate = 0;   // 0 until this issuer's accumulator has been written in this unit
         for (uint32_t l = 0; l < unit_stages && !error; ++l, ring_slot = ring_slot + 1 == p.stages ? (ring_round ^= 1u, 0) : ring_slot + 1) {
           if (!p.split_blocks && ((ring + l) & issuer_mask) != uint32_t(q)) continue;
-          const int kb = wu.kb_begin + 2 * int(l);
-          const int nkb = min(2, wu.kb_end - kb);
+          const int kb = kb_begin + 2 * int(l);
+          const int nkb = min(2, kb_end - kb);
           const int stage = ring_slot;   // (ring + l) % stages, kept incrementally with its round parity
-          if (!mbar_wait(full_bar(stage), ring_round, abort_flag)) { error = kErrMmaFull; break; }
-          if (q == 0 && issued == 0) HG_STAMP(3);
+          if (!warp_wait(full_bar(stage), ring_round, abort_flag)) { error = kErrMmaFull; break; }
+#ifdef HG_TRACE
+          if (lane == 0 && q == 0 && issued == 0) HG_STAMP(3);
+#endif
           // The MXFP4 rows were written through the generic proxy (cp.async); the tensor core reads
           // shared memory through the async proxy.
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           tc_fence_after();
-          for (int i = 0; i < nkb; ++i) {
-            if (p.split_blocks && i != q) continue;
-            const uint32_t sf_set = sf_base + (sf_flip ^= 1u) * 8u;
-            tc_cp_scales(sf_set, smem_desc(base + lay.sfa + uint32_t(stage) * 1024u + uint32_t(i) * 512u, 0, 128, kSwizzleNone));
-            tc_cp_scales(sf_set + 4, smem_desc(base + lay.sfb + uint32_t(stage) * 1024u + uint32_t(i) * 512u, 0, 128, kSwizzleNone));
-            const uint64_t desc_a = smem_desc(base + lay.a + uint32_t(stage) * 32768u + uint32_t(i) * 16384u, 0, 1024, kSwizzle128B);
-            const uint64_t desc_b = smem_desc(base + lay.b + (uint32_t(stage) * 2u + uint32_t(i)) * lay.b_tile, 0, 1024, kSwizzle128B);
+          if (elect_one()) {
+            for (int i = 0; i < nkb; ++i) {
+              if (p.split_blocks && i != q) continue;
+              const uint32_t sf_set = sf_base + ((sf_flip ^ uint32_t(i)) & 1u) * 8u;
+              tc_cp_scales(sf_set, smem_desc(smem0 + lay.sfa + uint32_t(stage) * 1024u + uint32_t(i) * 512u, 0, 128, kSwizzleNone));
+              tc_cp_scales(sf_set + 4, smem_desc(smem0 + lay.sfb + uint32_t(stage) * 1024u + uint32_t(i) * 512u, 0, 128, kSwizzleNone));
+              const uint64_t desc_a = smem_desc(smem0 + lay.a + uint32_t(stage) * 32768u + uint32_t(i) * 16384u, 0, 1024, kSwizzle128B);
+              const uint64_t desc_b = smem_desc(smem0 + lay.b + (uint32_t(stage) * 2u + uint32_t(i)) * lay.b_tile, 0, 1024, kSwizzle128B);
 #pragma unroll
-            for (uint32_t j = 0; j < 4; ++j) {
-              // 32 K-elements = 32 bytes further along the swizzled row: start address field += 2.
-              tc_mma(tmem_d, desc_a + 2 * j, desc_b + 2 * j, idesc | (j << 29) | (j << 4),
-                     (!fresh || j > 0) ? 1u : 0u, sf_set, sf_set + 4 + sfb_col);
+              for (uint32_t j = 0; j < 4; ++j) {
+                // 32 K-elements = 32 bytes further along the swizzled row: start address field += 2.
+                tc_mma(tmem_d, desc_a + 2 * j, desc_b + 2 * j, idesc | (j << 29) | (j << 4),
+                       j > 0 ? 1u : (p.split_blocks || i == 0 ? accumulate : 1u), sf_set, sf_set + 4 + sfb_col);
+              }
             }
-            fresh = false;
-            ++issued;
+            // A stage whose second block lies beyond the unit gives the second issuer nothing to read.
+            if (p.split_blocks && q >= nkb) mbar_arrive(empty_bar(stage));
+            else tc_commit(empty_bar(stage));
           }
-          // A stage whose second block lies beyond the unit gives the second issuer nothing to read.
-          if (p.split_blocks && q >= nkb) mbar_arrive(empty_bar(stage));
-          else tc_commit(empty_bar(stage));
+          __syncwarp();
+          const int blocks = p.split_blocks ? int(q < nkb) : nkb;
+          if (blocks) accumulate = 1;
+          issued += uint32_t(blocks);
+          sf_flip += p.split_blocks ? 1u : uint32_t(nkb);
         }
         ring += unit_stages;
         // Every issuer reports, also one that had no stage in this unit (its accumulator is then skipped).
-        if (!error) tc_commit(acc_full_bar(slot));
-        if (q == 0 && acc_it < 4) HG_STAMP(4 + acc_it);
+        if (!error && elect_one()) tc_commit(acc_full_bar(slot));
+        __syncwarp();
+#ifdef HG_TRACE
+        if (lane == 0 && q == 0 && acc_it < 4) HG_STAMP(4 + acc_it);
+#endif
       }
       // Let every MMA issued by this thread retire before TMEM is released.
-      tc_commit(drain_bar);
-      if (q == 0 && !mbar_wait(drain_bar, 0, abort_flag) && !error) error = kErrDrain;
-      if (issued) atomicAdd(p.status + 1, int(issued));
+      if (elect_one()) tc_commit(drain_bar);
+      __syncwarp();
+      if (q == 0 && !warp_wait(drain_bar, 0, abort_flag) && !error) error = kErrDrain;
+      if (lane == 0 && issued) atomicAdd(p.status + 1, int(issued));
     }
   } else {
     // ------------------------------------------------------------------ epilogue (warps 2..5)
