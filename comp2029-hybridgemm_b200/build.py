@@ -9,7 +9,7 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 LIBRARY = HERE / "lib" / "libhygemm_b200.so"
 TRACE_LIBRARY = HERE / "lib" / "libhygemm_b200_trace.so"   # same sources with -DHG_TRACE (per-CTA time stamps)
-SOURCES = ["hg_quant.cu", "hg_gemm_simt.cu", "hg_gemm_tc.cu", "hg_runtime.cu", "hg_tp.cu", "hg_clip.cu"]
+SOURCES = ["hg_quant.cu", "hg_gemm_simt.cu", "hg_gemm_tc.cu", "hg_gemm_cluster.cu", "hg_runtime.cu", "hg_tp.cu", "hg_clip.cu"]
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
          "-Xcompiler", "-fPIC", "-shared", "-cudart", "static"]
 
@@ -29,7 +29,7 @@ def build_library(force: bool = False, verbose: bool = False, trace: bool = Fals
     if not force and not stale(library):
         return library
     library.parent.mkdir(exist_ok=True)
-    cmd = ["nvcc", *FLAGS, *(["-DHG_TRACE=1"] if trace else []), *(["-Xptxas", "-v"] if verbose else []),
+    cmd = ["nvcc", *FLAGS, "-t", "0", *(["-DHG_TRACE=1"] if trace else []), *(["-Xptxas", "-v"] if verbose else []),
            *[str(CSRC / s) for s in SOURCES], "-o", str(library)]
     result = subprocess.run(cmd, capture_output=True, text=True)
     if verbose or result.returncode:

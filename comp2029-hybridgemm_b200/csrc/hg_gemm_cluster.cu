@@ -1,0 +1,865 @@
+// Hybrid MXFP4xMXFP8 + MXFP8xMXFP8 GEMM on clusters of CTAs (sm_100a): what HG_SCHEDULE_AUTO runs.
+//
+//   out[t, ids[r]] = sum_g 2^(sw[r,g]+sx[t,g]-254) * sum_{k in g} W[r,k] * X[t,k]
+//
+// Differences from the single-CTA kernel of hg_gemm_tc.cu, which serves the explicit tile schedules:
+// * Split K inside a cluster.  A tile's K range is cut over the CTAs (or CTA pairs) of one cluster; each pushes its
+//   fp32 partials to the shared memory of the CTAs that own the columns, and the owners add them in K order.
+//   No workspace, no ticket, no second launch: the chain store -> ticket -> load through global memory that ended
+//   a cut tile cost 3.5 us, the exchange between neighbours about one.
+// * Row tiles of any height up to 128.  Weights, their scales and the channel map are addressed by row, so tile
+//   heights are chosen such that every CTA gets the same number of weight bytes (an MXFP8 tile has half the rows
+//   of an MXFP4 tile while weights stream from HBM).
+// * cta_group::2 above 64 tokens.  Two CTAs form one 256-row tile; each stages its own 128 weight rows and HALF of the
+//   activation tile.  At 128 tokens the shared-memory traffic per K128 block falls from 448 to 320 cycles, and
+//   256-token tiles (prefill) run at 512 cycles, the tensor core's own time.
+// * 256-token accumulators overlap.  TMEM holds two of them only if they share 32 columns; the epilogue drains
+//   those first and hands them over, so the main loop of the next tile starts about 0.3 us after the last one ended.
+//
+// Roles per CTA: warp 0 activations and their scales (TMA), warp 1 MMA issue (in the second CTA of a pair: tells the
+// first that a stage is full), warps 2-9 epilogue (two per TMEM quarter, on alternate groups of sixteen columns),
+// warps 10-17 (FUSED 10-13) weights and weight scales (cp.async: MXFP4 codes go in 8-byte granules into the first half of each
+// swizzled 16-byte chunk, the 8-bit container the f8f6f4 kinds read; MXFP8 codes as 16-byte chunks; scales as the 4-byte
+// words of the row), warps 14-17 (FUSED) activation quantisers.
+// One warp per scheduler runs most of these roles alone, so a dependent instruction costs about five cycles and nothing
+// hides it: loops here carry no divisions, addresses are independent of each other, and descriptors are sums.
+// Every mbarrier wait is bounded; on expiry the CTA records a code, drains and leaves.
+#include <algorithm>
+#include <cstdlib>
+#include <cstring>
+#include <mutex>
+#include <vector>
+
+#include "hg_gemm_cluster.cuh"
+
+namespace hg {
+
+namespace {
+
+constexpr int kFirstLoader = 10;                // warps 0-9: see above
+constexpr int kLoaderTeams = 4;                 // each brings in a whole K256 stage
+__host__ __device__ constexpr int team_warps(bool fused) { return fused ? 1 : 2; }   // 18 warps leave 113 registers a thread, with quantisers as well
+__host__ __device__ constexpr int first_quantiser(bool fused) { return kFirstLoader + kLoaderTeams * team_warps(fused); }
+__host__ __device__ constexpr int cluster_threads(bool fused) { return first_quantiser(fused) * 32 + (fused ? kQuantThreads : 0); }
+constexpr int kClusterMaxStages = 6;
+constexpr int kMaxSmem = 232448;
+constexpr uint32_t kScaleStride = 16;                           // TMEM columns per scale set: weights 4, activations up to 8
+
+struct ClusterParams {
+  int rows[2], tile_rows[2], tiles[2];
+  const uint8_t* weight[2];
+  const uint8_t* sfa[2];
+  const int32_t* ids[2];
+  const uint8_t* sfb;
+  OutTargets out;
+  int outputs, tokens, k, kblocks;
+  int n_tile, n_tail, token_tiles, stages, split, split_log, share_log, clusters;
+  int acc_shift, overlap;
+  uint64_t by_token_tiles, by_tiles;   // see fast_div
+  uint32_t tmem_cols;
+  const uint16_t* x;
+  int x_bf16;
+  int audit_tokens;
+  int* status;
+#ifdef HG_TRACE
+  unsigned long long* trace;
+#endif
+};
+
+// Partial tiles are exchanged in groups of four columns, [group][row][4] fp32; every slice owns a power of two of them.
+__host__ __device__ inline int share_log_of(int n_tile, int split) {
+  int log = 0;
+  while ((split << log) * 4 < n_tile) ++log;
+  return log;
+}
+
+// A pipeline stage covers two K128 blocks (K256): 2 x 16 KiB of weights in the 8-bit container, two activation tiles,
+// two scale atoms of the weights and two per 128 tokens of the activations.
+struct ClusterSmem {
+  uint32_t b, sfa, sfb, red, bars;  // byte offsets from the 1024-aligned base; the weight stages start at 0
+  uint32_t b_tile;                  // bytes of one K128 activation tile
+  uint32_t sfb_stage;               // bytes of the activation scales of a stage: per 128 tokens two atoms
+};
+__host__ __device__ inline ClusterSmem cluster_smem(int stages, int n_tile, int pair, int split) {
+  ClusterSmem s;
+  s.b_tile = uint32_t(n_tile / pair) * 128u;
+  s.sfb_stage = uint32_t((n_tile + 127) / 128) * 1024u;
+  s.b = uint32_t(stages) * 32768u;
+  s.sfa = s.b + uint32_t(stages) * 2u * s.b_tile;
+  s.sfb = s.sfa + uint32_t(stages) * 1024u;
+  s.red = s.sfb + uint32_t(stages) * s.sfb_stage;
+  s.bars = s.red + (split > 1 ? uint32_t(split << share_log_of(n_tile, split)) * 2048u : 0u);
+  return s;
+}
+constexpr int kClusterBarBytes = (3 * kClusterMaxStages + 8) * 8 + 32;
+
+template <int PAIR> __device__ __forceinline__ void cg_alloc(uint32_t slot, uint32_t cols) {
+  if constexpr (PAIR == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  } else {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+}
+template <int PAIR> __device__ __forceinline__ void cg_dealloc(uint32_t addr, uint32_t cols) {
+  if constexpr (PAIR == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
+  else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
+}
+// Arrives on the barrier at this offset in every CTA of the tile when all MMAs issued so far have retired.
+template <int PAIR> __device__ __forceinline__ void cg_commit(uint32_t bar, uint16_t cta_mask) {
+  if constexpr (PAIR == 1) tc_commit(bar);
+  else
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(bar), "h"(cta_mask) : "memory");
+}
+template <int PAIR> __device__ __forceinline__ void cg_cp_scales(uint32_t tmem, uint64_t desc) {
+  if constexpr (PAIR == 1) tc_cp_scales(tmem, desc);
+  else asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem), "l"(desc) : "memory");
+}
+template <int PAIR>
+__device__ __forceinline__ void cg_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate, uint32_t sfa, uint32_t sfb) {
+  if constexpr (PAIR == 1) tc_mma(d, a, b, idesc, accumulate, sfa, sfb);
+  else
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n"
+        "}"
+        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb) : "memory");
+}
+
+// Shared-memory descriptors by words: the high one holds the stride of eight rows, version 1 and the swizzle.
+constexpr uint32_t kDescTile = (1024u >> 4) | (1u << 14) | (kSwizzle128B << 29), kDescScales = (128u >> 4) | (1u << 14);
+__device__ __forceinline__ uint64_t desc_of(uint32_t low, uint32_t high) { return uint64_t(low) | (uint64_t(high) << 32); }
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void arrive_remote(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void store_remote(uint32_t cluster_addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// n / d with inverse = ceil(2^40 / d), exact while n d < 2^40; the host passes 0 where that or the product does not fit.
+__device__ __forceinline__ int fast_div(int64_t n, int d, uint64_t inverse) {
+  return inverse ? int((uint64_t(n) * inverse) >> 40) : int(n / d);
+}
+
+// One work unit: a row tile and a token tile, token tiles innermost.  Decode runs its MXFP8 tiles first: their stores
+// scatter over the whole output row, and all but the last epilogue of a CTA run under the next main loop.  With several
+// token tiles they are spread evenly among the MXFP4 tiles, so that the two partitions of a channel range (both sorted)
+// are stored at about the same time and meet in L2: an MXFP8 tile writes one or two channels of nearly every sector.
+struct Unit {
+  int part, tile, token0, n;
+};
+__device__ __forceinline__ Unit unit_at(const ClusterParams& p, int u) {
+  Unit w;
+  if (p.token_tiles == 1) {
+    w.part = u < p.tiles[1];
+    w.tile = w.part ? u : u - p.tiles[1];
+    w.token0 = 0;
+    w.n = p.n_tail;
+  } else {
+    const int t = fast_div(u, p.token_tiles, p.by_token_tiles), tt = u - t * p.token_tiles, total = p.tiles[0] + p.tiles[1];
+    const int high_before = fast_div(int64_t(t) * p.tiles[1], total, p.by_tiles);
+    const int high_after = fast_div(int64_t(t + 1) * p.tiles[1], total, p.by_tiles);
+    w.part = high_after > high_before;
+    w.tile = w.part ? high_before : t - high_before;
+    w.token0 = tt * p.n_tile;
+    w.n = tt == p.token_tiles - 1 ? p.n_tail : p.n_tile;
+  }
+  return w;
+}
+
+template <typename T, int PAIR, bool FUSED>
+__global__ void __launch_bounds__(cluster_threads(FUSED), 1)
+cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_constant__ CUtensorMap map_act,
+                    const __grid_constant__ CUtensorMap map_tail) {
+  pdl_trigger();
+  if (threadIdx.x == 0) HG_STAMP(0);
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
+  const ClusterSmem lay = cluster_smem(p.stages, p.n_tile, PAIR, p.split);
+  const uint32_t bars = base + lay.bars;
+  auto full_bar = [&](int s) { return bars + uint32_t(s) * 8u; };
+  auto empty_bar = [&](int s) { return bars + uint32_t(kClusterMaxStages + s) * 8u; };
+  auto peer_bar = [&](int s) { return bars + uint32_t(2 * kClusterMaxStages + s) * 8u; };   // pair: the second CTA's stage is full
+  auto acc_full_bar = [&](int s) { return bars + uint32_t(3 * kClusterMaxStages + s) * 8u; };
+  auto acc_empty_bar = [&](int s) { return bars + uint32_t(3 * kClusterMaxStages + 2 + s) * 8u; };
+  const uint32_t red_full = bars + uint32_t(3 * kClusterMaxStages + 4) * 8u;    // every slice's partials of this share are here
+  const uint32_t red_empty = bars + uint32_t(3 * kClusterMaxStages + 5) * 8u;   // every slice has summed its share
+  const uint32_t drain_bar = bars + uint32_t(3 * kClusterMaxStages + 6) * 8u;
+  volatile int* words = reinterpret_cast<volatile int*>(base_ptr + lay.bars + (3 * kClusterMaxStages + 8) * 8);
+  volatile int* abort_flag = words + 1;
+
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int cluster_ctas = PAIR * p.split;
+  const int rank = cluster_ctas == 1 ? 0 : int(cluster_rank());
+  const int cluster = cluster_ctas == 1 ? int(blockIdx.x) : int(blockIdx.x) / cluster_ctas;
+  const int half = PAIR == 2 ? rank & 1 : 0;
+  const int slice = PAIR == 2 ? rank >> 1 : rank;
+
+  if (threadIdx.x == 0) {
+    if (!FUSED) {
+      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_act)) : "memory");
+      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_tail)) : "memory");
+    }
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(full_bar(s), 32 * team_warps(FUSED) + (FUSED ? kQuantThreads / 32 : 1));   // the lanes of one loader team; quantiser warps or the TMA thread
+      mbar_init(empty_bar(s), 1);
+      mbar_init(peer_bar(s), 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(acc_full_bar(s), 1);
+      mbar_init(acc_empty_bar(s), 8 * PAIR);
+    }
+    mbar_init(red_full, uint32_t(8 * p.split));
+    mbar_init(red_empty, uint32_t(8 * p.split));
+    mbar_init(drain_bar, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) cg_alloc<PAIR>(smem_u32(const_cast<int*>(words)), p.tmem_cols);
+  tc_fence_before();
+  __syncwarp();
+  if (cluster_ctas > 1) cluster_sync();   // barriers of every CTA are initialised before anyone arrives remotely
+  else __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = uint32_t(*words);
+  if (threadIdx.x == 0) HG_STAMP(1);
+
+  const uint32_t sf_cols = tmem_base + p.tmem_cols - 2u * kScaleStride;
+  const int units = (p.tiles[0] + p.tiles[1]) * p.token_tiles;
+  const int steps = (p.kblocks + 1) >> 1;                        // K256 steps of a tile ...
+  const int step_begin = (steps * slice) >> p.split_log, step_end = (steps * (slice + 1)) >> p.split_log;   // ... and of this slice
+  int error = 0;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ activations and their scales (TMA)
+    // The warp walks the loop together and an elected lane issues: behind a `lane == 0` branch the four copies of a stage
+    // took 300 cycles to issue.  One copy brings both K128 blocks (the map's third dimension counts them).
+    if (!FUSED) {
+      pdl_wait();   // they are the previous kernel's output; the weight stream below is not and already runs
+      if (lane == 0) HG_STAMP(2);
+      const uint32_t smem0 = __shfl_sync(0xffffffffu, base, 0), bars0 = smem0 + lay.bars;
+      const int atoms = (p.tokens + 127) >> 7;
+      int stage = 0;
+      uint32_t phase = 1;
+      for (int u = cluster; u < units && !error; u += p.clusters) {
+        const Unit w = unit_at(p, u);
+        const int first_atom = w.token0 >> 7, n_atoms = min((w.n + 127) >> 7, atoms - first_atom);
+        const int row = w.token0 + half * (w.n / PAIR);
+        const bool whole = w.n == p.n_tile;
+        const uint8_t* sfb_src = p.sfb + int64_t(first_atom) * p.kblocks * 512;
+        for (int step = step_begin; step < step_end; ++step) {
+          const int kb = 2 * step, nkb = min(2, p.kblocks - kb);
+          if (!warp_wait(empty_bar(stage), phase, abort_flag)) { error = kErrProducer; break; }
+          if (elect_one()) {
+            const uint32_t bar = bars0 + uint32_t(stage) * 8u, dst = smem0 + lay.b + uint32_t(2 * stage) * lay.b_tile;
+            mbar_expect_tx(bar, uint32_t(w.n / PAIR) * 256u + uint32_t(n_atoms * nkb) * 512u);   // a block beyond K arrives as zeros
+            // a short last token tile has a box of its own: its second block follows the first directly
+            if (whole) tma_load_3d(dst, &map_act, bar, 0, row, kb);
+            else tma_load_3d(dst, &map_tail, bar, 0, row, kb);
+            for (int a = 0; a < n_atoms; ++a)
+              bulk_load(smem0 + lay.sfb + uint32_t(stage) * lay.sfb_stage + uint32_t(a) * 1024u,
+                        sfb_src + (int64_t(a) * p.kblocks + kb) * 512, uint32_t(nkb) * 512u, bar);
+          }
+          __syncwarp();
+          if (++stage == p.stages) { stage = 0; phase ^= 1u; }
+        }
+      }
+    }
+  } else if (warp >= kFirstLoader && warp < first_quantiser(FUSED)) {
+    // ------------------------------------------------------------------ weights and their scales (cp.async)
+    // Loader team t of L (two warps that share the rows) brings in every L-th K256 step, whole.  Sixteen lanes cover a full 128- or 256-byte run of a row,
+    // so lane l owns granule l % 16 (8 bytes of MXFP4 or 16 bytes of MXFP8 codes) of rows l / 16 + 2 i; for the scales
+    // it owns rows l + 32 j.  A team per step keeps the arrivals on a stage barrier at 64: they serialise there, and
+    // 128 threads that each arrived for both blocks of a step cost more than the copies.  One warp per team was too
+    // slow to refill a three-stage ring: a stage is 72 copies, and their issue counts against the ring's round trip.
+    // L is at most the ring depth S.  The warp of step s + 2 S has seen step s + S - L consumed (its previous wait), so
+    // with L <= S step s has been consumed too and the stage's barrier is past the phase whose parity that wait
+    // would mistake for its own.
+    constexpr int kTeam = team_warps(FUSED);
+    const int lw = (warp - kFirstLoader) / kTeam, sub = (warp - kFirstLoader) % kTeam, m = lane & 15, rsub = lane >> 4, blk = m >> 3;
+    uint32_t swz[4];   // swizzled chunk of rows rsub + 2 i, by i % 4
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      swz[i] = uint32_t(blk) * 16384u + uint32_t(rsub + 2 * i) * 128u + (uint32_t((m & 7) ^ (rsub + 2 * i)) << 4);
+    const int loaders = min(kLoaderTeams, p.stages);
+    int stage = lw, ahead = lw;   // ahead: steps from here to this warp's next one
+    uint32_t phase = 1;
+    for (int u = cluster; u < units && !error && lw < loaders; u += p.clusters) {
+      const Unit w = unit_at(p, u);
+      const int row0 = (w.tile * PAIR + half) * p.tile_rows[w.part];
+      const int rows = min(p.tile_rows[w.part], p.rows[w.part] - row0);   // may be <= 0: nothing to load, the stages still turn
+      const int pitch = w.part ? p.k : p.k >> 1;
+      const uint8_t* src0 = p.weight[w.part] + int64_t(row0 + rsub) * pitch + m * (w.part ? 16 : 8);
+      const uint8_t* sf_part = p.sfa[w.part];
+      int step = step_begin + ahead;
+      for (; step < step_end; step += loaders) {
+        const int kb = 2 * step, nkb = min(2, p.kblocks - kb);
+        if (!warp_wait(empty_bar(stage), phase, abort_flag)) { error = kErrLoader; break; }
+        const uint32_t dst = base + uint32_t(stage) * 32768u;
+        if (blk < nkb) {
+          const uint8_t* src = src0 + int64_t(kb) * (w.part ? 128 : 64);
+          if (w.part) {
+#pragma unroll 4
+            for (int i = sub; i < 16; i += kTeam)
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                if (rsub + 8 * i + 2 * j < rows) cp_async_16(dst + uint32_t(i) * 1024u + swz[j], src + int64_t(pitch) * (8 * i + 2 * j));
+          } else {
+#pragma unroll 4
+            for (int i = sub; i < 16; i += kTeam)
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                if (rsub + 8 * i + 2 * j < rows) cp_async_8(dst + uint32_t(i) * 1024u + swz[j], src + int64_t(pitch) * (8 * i + 2 * j), 8u);
+          }
+        }
+#pragma unroll
+        for (int j = sub; j < 4; j += kTeam) {
+          const int row = row0 + lane + 32 * j;
+          if (lane + 32 * j < rows)
+            for (int i = 0; i < nkb; ++i)
+              cp_async_4(base + lay.sfa + uint32_t(2 * stage + i) * 512u + uint32_t(lane) * 16u + uint32_t(j) * 4u,
+                         sf_part + (int64_t(row >> 7) * p.kblocks + kb + i) * 512 + (row & 31) * 16 + ((row & 127) >> 5) * 4);
+        }
+        cp_async_arrive(full_bar(stage));
+        if ((stage += loaders) >= p.stages) { stage -= p.stages; phase ^= 1u; }
+      }
+      ahead = step - step_end;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");   // copies in flight must land before shared memory is released
+  } else if (FUSED && warp >= first_quantiser(FUSED)) {
+    // ------------------------------------------------------------------ activation quantisers
+    // Thread tq owns one K32 group (tq % 8) of token tq / 8 in each K256 step, with the arithmetic of mx_quant_kernel:
+    // codes and scales are the bytes hg_pack would have produced.  The next step's 64 bytes are requested before the
+    // current ones are converted.
+    if constexpr (FUSED) {
+      const int tq = threadIdx.x - first_quantiser(FUSED) * 32;
+      const int token = tq >> 3, blk = (tq & 7) >> 2, g = tq & 3;
+      const uint16_t* x_row = p.x + int64_t(token) * p.k + blk * 128 + g * 32;
+      auto load_x = [&](int kb, uint4 (&r)[4]) {
+        if (kb + blk < p.kblocks && token < p.tokens) {
+          const uint4* src = reinterpret_cast<const uint4*>(x_row + int64_t(kb) * 128);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) r[c] = src[c];
+        } else {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) r[c] = make_uint4(0u, 0u, 0u, 0u);
+        }
+      };
+      uint4 cur[4], nxt[4];
+      int stage = 0;
+      uint32_t phase = 1;
+      pdl_wait();   // x is the previous kernel's output
+      if (cluster < units) load_x(2 * step_begin, cur);
+      for (int u = cluster; u < units && !error; u += p.clusters) {
+        for (int step = step_begin; step < step_end; ++step) {
+          load_x(step + 1 < step_end ? 2 * step + 2 : 2 * step_begin, nxt);
+          if (!warp_wait(empty_bar(stage), phase, abort_flag)) { error = kErrLoader; break; }
+          if (2 * step + blk < p.kblocks) {
+            const uint32_t row_base = base + lay.b + uint32_t(2 * stage + blk) * lay.b_tile + uint32_t(token) * 128u;
+            const uint32_t sw = uint32_t(token & 7);
+            float v[32];
+            float amax = 0.f;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const uint32_t word[4] = {cur[c].x, cur[c].y, cur[c].z, cur[c].w};
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const uint16_t bits = uint16_t(word[i >> 1] >> ((i & 1) * 16));
+                v[c * 8 + i] = p.x_bf16 ? to_float<__nv_bfloat16>(bits) : to_float<__half>(bits);
+                amax = fmaxf(amax, fabsf(v[c * 8 + i]));
+              }
+            }
+            const int e = mx_exponent<false>(amax);
+            const float inv = mx_inverse_scale(e);
+            uint32_t codes[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              codes[i] = cvt_e4m3x2(v[4 * i] * inv, v[4 * i + 1] * inv) | (cvt_e4m3x2(v[4 * i + 2] * inv, v[4 * i + 3] * inv) << 16);
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_base + ((uint32_t(2 * g) ^ sw) << 4)),
+                         "r"(codes[0]), "r"(codes[1]), "r"(codes[2]), "r"(codes[3]) : "memory");
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_base + ((uint32_t(2 * g + 1) ^ sw) << 4)),
+                         "r"(codes[4]), "r"(codes[5]), "r"(codes[6]), "r"(codes[7]) : "memory");
+            asm volatile("st.shared.u8 [%0], %1;" ::"r"(base + lay.sfb + uint32_t(stage) * lay.sfb_stage + uint32_t(blk) * 512u + uint32_t(token & 31) * 16u + uint32_t(g)),
+                         "r"(uint32_t(e + 127)) : "memory");
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(full_bar(stage));
+#pragma unroll
+          for (int c = 0; c < 4; ++c) cur[c] = nxt[c];
+          if (++stage == p.stages) { stage = 0; phase ^= 1u; }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (half == 0) {
+      // ---------------------------------------------------------------- MMA issue
+      const uint32_t smem0 = __shfl_sync(0xffffffffu, base, 0), tmem0 = __shfl_sync(0xffffffffu, tmem_base, 0);
+      const uint32_t sf0 = __shfl_sync(0xffffffffu, sf_cols, 0);
+      const uint16_t pair_mask = uint16_t(3u << (rank & ~1));
+      // low words of the shared-memory descriptors of stage 0; a stage is a constant number of 16-byte units further on
+      const uint32_t a_desc = smem0 >> 4, b_desc = (smem0 + lay.b) >> 4, b_stage = lay.b_tile >> 3;
+      const uint32_t sfa_desc = (smem0 + lay.sfa) >> 4, sfb_desc = (smem0 + lay.sfb) >> 4, sfb_stage = lay.sfb_stage >> 4;
+      int stage = 0, it = 0, issued = 0;
+      uint32_t phase = 0;
+      for (int u = cluster; u < units && !error; u += p.clusters, ++it) {
+        const Unit w = unit_at(p, u);
+        const int acc = it & 1;
+        // Overlapping accumulators: an accumulator becomes free when the epilogue of the OTHER one has drained the
+        // shared columns, so accumulator 1 waits for an arrival on its first use as well.
+        const uint32_t acc_parity = (uint32_t(it >> 1) & 1u) ^ (p.overlap && acc ? 0u : 1u);
+        if (!(PAIR == 2 ? warp_wait_cluster(acc_empty_bar(acc), acc_parity, abort_flag) : warp_wait(acc_empty_bar(acc), acc_parity, abort_flag))) { error = kErrMmaAcc; break; }
+        tc_fence_after();
+        const uint32_t tmem_d = tmem0 + uint32_t(acc * p.acc_shift);
+        const uint32_t b_block = uint32_t(w.n / PAIR) * 8u;   // descriptor units (16 bytes) between the stage's activation tiles
+        const uint32_t idesc = (w.part ? 0u : 5u << 7) | (uint32_t(w.n >> 3) << 17) | (1u << 23) | (uint32_t(PAIR * kTileRows >> 4) << 24);
+        const bool two_atoms = w.n > 128;
+        uint32_t accumulate = 0;
+        for (int step = step_begin; step < step_end; ++step) {
+          const int nkb = min(2, p.kblocks - 2 * step);
+          if (!warp_wait(full_bar(stage), phase, abort_flag)) { error = kErrMmaFull; break; }
+          if (PAIR == 2 && !warp_wait_cluster(peer_bar(stage), phase, abort_flag)) { error = kErrMmaFull; break; }
+          // codes and scales were written through the generic proxy (cp.async); the tensor core reads through the async proxy
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          tc_fence_after();
+#ifdef HG_TRACE
+          if (lane == 0 && it == 0 && step == step_begin) HG_STAMP(3);
+#endif
+          if (elect_one()) {
+            const uint32_t a_lo = a_desc + uint32_t(stage) * 2048u, b_lo = b_desc + uint32_t(stage) * b_stage;
+            const uint32_t sfa_lo = sfa_desc + uint32_t(stage) * 64u, sfb_lo = sfb_desc + uint32_t(stage) * sfb_stage;
+#pragma unroll
+            for (uint32_t i = 0; i < 2; ++i) {
+              if (i == 1 && nkb == 1) break;
+              const uint32_t sf = sf0 + i * kScaleStride;
+              cg_cp_scales<PAIR>(sf, desc_of(sfa_lo + i * 32u, kDescScales));
+              cg_cp_scales<PAIR>(sf + 4, desc_of(sfb_lo + i * 32u, kDescScales));
+              if (two_atoms) cg_cp_scales<PAIR>(sf + 8, desc_of(sfb_lo + i * 32u + 64u, kDescScales));
+#pragma unroll
+              for (uint32_t j = 0; j < 4; ++j)
+                cg_mma<PAIR>(tmem_d, desc_of(a_lo + i * 1024u + 2 * j, kDescTile), desc_of(b_lo + i * b_block + 2 * j, kDescTile),
+                             idesc | (j << 29) | (j << 4), i + j > 0 ? 1u : accumulate, sf, sf + 4);
+            }
+            cg_commit<PAIR>(empty_bar(stage), pair_mask);
+          }
+          __syncwarp();
+          accumulate = 1;
+          if (++stage == p.stages) { stage = 0; phase ^= 1u; }
+        }
+        if (error) break;
+        if (elect_one()) cg_commit<PAIR>(acc_full_bar(acc), pair_mask);
+        __syncwarp();
+#ifdef HG_TRACE
+        if (lane == 0 && it < 4) HG_STAMP(4 + it);
+#endif
+        // Audit, in tiles of 128 rows x audit_tokens: the tiles whose first row this unit covers.
+        const int first_row = w.tile * PAIR * p.tile_rows[w.part];
+        const int last_row = min(first_row + PAIR * p.tile_rows[w.part], p.rows[w.part]);
+        issued += (((last_row + 127) >> 7) - ((first_row + 127) >> 7)) * (min(2 * step_end, p.kblocks) - 2 * step_begin) *
+                  ((min(w.n, p.tokens - w.token0) + p.audit_tokens - 1) / p.audit_tokens);
+      }
+      // Every MMA of this CTA (pair) retires before TMEM is released.
+      if (elect_one()) cg_commit<PAIR>(drain_bar, pair_mask);
+      __syncwarp();
+      if (!warp_wait(drain_bar, 0, abort_flag) && !error) error = kErrDrain;
+      if (lane == 0 && issued) atomicAdd(p.status + 1, issued);
+    } else if (PAIR == 2) {
+      // ---------------------------------------------------------------- second CTA of a pair: report full stages
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int u = cluster; u < units && !error; u += p.clusters)
+        for (int step = step_begin; step < step_end; ++step) {
+          if (!warp_wait(full_bar(stage), phase, abort_flag)) { error = kErrMmaFull; break; }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          if (lane == 0) arrive_remote(map_to_rank(peer_bar(stage), uint32_t(rank - 1)));
+          __syncwarp();
+          if (++stage == p.stages) { stage = 0; phase ^= 1u; }
+        }
+      if (!warp_wait(drain_bar, 0, abort_flag) && !error) error = kErrDrain;
+    }
+  } else {
+    // ------------------------------------------------------------------ epilogue (warps 2..9)
+    const int quarter = warp & 3, side = (warp - 2) >> 2;   // TMEM lanes this warp may read; which of the two warps of the quarter
+    const int row_in_tile = quarter * 32 + lane;
+    const uint32_t lane_addr = uint32_t(quarter * 32) << 16;
+    int it = 0, stored = 0;
+    pdl_wait();   // nothing is written to global memory before every earlier kernel has finished
+    char* const out = out_base(p.out);
+    const bool out_f32 = p.out.f32 != 0;
+    const int row_bytes = p.outputs * (out_f32 ? 4 : 2);
+    const uint32_t leader = uint32_t(rank & ~(PAIR - 1));
+    for (int u = cluster; u < units; u += p.clusters, ++it) {
+      const Unit w = unit_at(p, u);
+      const int acc = it & 1;
+      const int row0 = (w.tile * PAIR + half) * p.tile_rows[w.part];
+      const int row = row0 + row_in_tile;
+      const bool row_ok = row_in_tile < p.tile_rows[w.part] && row < p.rows[w.part];
+      const int channel = row_ok ? p.ids[w.part][row] : 0;   // fetched while the main loop runs
+      const int valid = min(w.n, p.tokens - w.token0);
+      char* const out_row = out + int64_t(channel) * (out_f32 ? 4 : 2) + int64_t(w.token0) * row_bytes;
+      if (!warp_wait(acc_full_bar(acc), uint32_t(it >> 1) & 1u, abort_flag)) { error = kErrEpilogue; break; }
+      tc_fence_after();
+      if (threadIdx.x == 64 && it < 3) HG_STAMP(8 + 2 * it);
+      const uint32_t taddr = tmem_base + lane_addr + uint32_t(acc * p.acc_shift);
+      auto release = [&](int which) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (PAIR == 1) mbar_arrive(acc_empty_bar(which));
+          else arrive_remote(map_to_rank(acc_empty_bar(which), leader));
+        }
+      };
+      // N columns of this thread's row from column c on.
+      auto store = [&](int c, const auto& v) {
+        constexpr int N = sizeof(v) / sizeof(float);
+        char* at = out_row + int64_t(row_bytes) * c;
+        const int left = valid - c;
+        if (!row_ok) return;
+        if (!out_f32 && left >= N) {
+#pragma unroll
+          for (int i = 0; i < N; ++i) *reinterpret_cast<uint16_t*>(at + int64_t(row_bytes) * i) = from_float<T>(v[i]);
+        } else if (!out_f32) {
+#pragma unroll
+          for (int i = 0; i < N; ++i)
+            if (i < left) *reinterpret_cast<uint16_t*>(at + int64_t(row_bytes) * i) = from_float<T>(v[i]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < N; ++i)
+            if (i < left) *reinterpret_cast<float*>(at + int64_t(row_bytes) * i) = v[i];
+        }
+      };
+
+      if (p.split > 1) {
+        // Every slice owns 2^share_log groups of four columns.  A partial goes straight to the shared memory of the slice
+        // that owns its group (lanes write 512 contiguous bytes), one hop; the owner adds the pieces in K order.
+        if (it > 0 && !warp_wait_cluster(red_empty, uint32_t(it - 1) & 1u, abort_flag)) { error = kErrEpilogue; break; }
+        const uint32_t share = 1u << p.share_log;
+        const uint32_t my_piece = base + lay.red + (uint32_t(slice) << (p.share_log + 11)) + uint32_t(row_in_tile) * 16u;
+        const int groups = (valid + 3) >> 2;
+        for (int g0 = 4 * side; g0 < groups; g0 += 8) {
+          uint32_t r[16];
+          tc_load16(taddr + uint32_t(g0) * 4u, r);
+          tc_wait_ld();
+#pragma unroll
+          for (uint32_t i = 0; i < 4; ++i) {
+            const uint32_t g = uint32_t(g0) + i;
+            const uint32_t to = map_to_rank(my_piece + ((g & (share - 1u)) << 11), (g >> p.share_log) * PAIR + uint32_t(half));
+            store_remote(to, tc_loaded(r[4 * i]), tc_loaded(r[4 * i + 1]), tc_loaded(r[4 * i + 2]), tc_loaded(r[4 * i + 3]));
+          }
+        }
+        release(acc);
+        if (lane < p.split) arrive_remote(map_to_rank(red_full, uint32_t(lane * PAIR + half)));
+        if (!warp_wait_cluster(red_full, uint32_t(it) & 1u, abort_flag)) { error = kErrEpilogue; break; }
+        const uint32_t pieces = base + lay.red + uint32_t(row_in_tile) * 16u;
+        const int g_begin = slice << p.share_log, g_end = min(groups, (slice + 1) << p.share_log);
+        for (int g = g_begin + side; g < g_end; g += 2) {
+          const uint32_t from = pieces + (uint32_t(g - g_begin) << 11);
+          float v[8][4];
+#pragma unroll
+          for (int s = 0; s < 8; ++s)
+            if (s < p.split)
+              asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[s][0]), "=f"(v[s][1]), "=f"(v[s][2]), "=f"(v[s][3])
+                           : "r"(from + (uint32_t(s) << (p.share_log + 11))) : "memory");
+#pragma unroll
+          for (int s = 1; s < 8; ++s)
+            if (s < p.split) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) v[0][i] += v[s][i];
+            }
+          store(4 * g, v[0]);
+        }
+        __syncwarp();
+        if (lane < p.split) arrive_remote(map_to_rank(red_empty, uint32_t(lane * PAIR + half)));
+      } else {
+        // This warp's groups of sixteen columns, the TMEM read of the next one in flight while the current one is stored.
+        // The columns two accumulators share are drained first and handed to the next main loop.
+        const int chunks = (w.n + 15) >> 4;
+        const int begin = p.overlap && acc == 0 && 14 + side < chunks ? 14 + side : side;   // column 224 of accumulator 0 is column 0 of accumulator 1
+        bool hand_over = p.overlap;
+        if (hand_over && acc == 0 && begin != 14 + side) { release(1); hand_over = false; }
+        uint32_t a[16];
+        int c = begin;
+        if (c < chunks) tc_load16(taddr + uint32_t(c) * 16u, a);
+        while (c < chunks) {
+          tc_wait_ld();
+          float r[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) r[i] = __uint_as_float(tc_loaded(a[i]));
+          if (hand_over) { release(acc ^ 1); hand_over = false; }
+          // 14 + side comes first where it is shared, then side, side + 2, ...
+          int next = begin > side ? (c == begin ? side : c + 2) : c + 2;
+          if (begin > side && next == begin) next = chunks;
+          if (next < chunks) tc_load16(taddr + uint32_t(next) * 16u, a);
+          store(16 * c, r);
+          c = next;
+        }
+        if (hand_over) release(acc ^ 1);
+        if (!p.overlap) release(acc);
+      }
+      if (threadIdx.x == 64 && it < 3) HG_STAMP(9 + 2 * it);
+      if (slice == 0 && half == 0 && threadIdx.x == 64) {
+        const int first_row = w.tile * PAIR * p.tile_rows[w.part];
+        const int last_row = min(first_row + PAIR * p.tile_rows[w.part], p.rows[w.part]);
+        stored += (((last_row + 127) >> 7) - ((first_row + 127) >> 7)) * ((valid + p.audit_tokens - 1) / p.audit_tokens);
+      }
+    }
+    if (threadIdx.x == 64 && stored) atomicAdd(p.status + 2, stored);
+  }
+
+  if (error) {
+    *abort_flag = 1;
+    atomicCAS(p.status, 0, error * 1000000 + int(blockIdx.x));
+    // Copies and MMAs in flight get time to land before shared memory and TMEM are released.
+    const long long start = clock64();
+    while (clock64() - start < 400000ll) __nanosleep(1000);
+  }
+  tc_fence_before();
+  __syncwarp();
+  if (cluster_ctas > 1) cluster_sync();   // no CTA leaves while another may still write its shared memory or arrive on its barriers
+  else __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    cg_dealloc<PAIR>(tmem_base, p.tmem_cols);
+  }
+}
+
+}  // namespace
+
+// ---------------------------------------------------------------------------------------------
+// Host side
+// ---------------------------------------------------------------------------------------------
+
+static int tuning(const char* name, int value) {
+  const char* text = std::getenv(name);
+  return text ? std::atoi(text) : value;
+}
+
+// Ring, TMEM and shared-memory figures that follow from pair, split, n_tile.  False when the ring would be too shallow.
+static bool finish_plan(ClusterPlan& plan) {
+  const int n_cols = (plan.n_tile + 31) & ~31;
+  plan.overlap = plan.n_tile > 224 ? 1 : 0;
+  plan.acc_shift = plan.overlap ? 224 : n_cols;
+  const int cols = plan.acc_shift + n_cols + int(2 * kScaleStride);
+  plan.tmem_cols = 64;
+  while (plan.tmem_cols < cols) plan.tmem_cols *= 2;
+  const ClusterSmem one = cluster_smem(1, plan.n_tile, plan.pair, plan.split), none = cluster_smem(0, plan.n_tile, plan.pair, plan.split);
+  const int stage_bytes = int(one.bars - none.bars);
+  plan.stages = std::min((kMaxSmem - 1024 - kClusterBarBytes - int(none.bars)) / stage_bytes,
+                         std::min(kClusterMaxStages, tuning("HYGEMM_CL_STAGES", kClusterMaxStages)));
+  if (plan.stages < 2) return false;
+  plan.smem_bytes = 1024 + int(none.bars) + plan.stages * stage_bytes + kClusterBarBytes;
+  return plan.tmem_cols <= 512;
+}
+
+// Cycles of one K128 block of a CTA: the tensor core's shared-memory traffic and time, the copies into the ring,
+// and the CTA's share of HBM (23 bytes per cycle and SM at the measured copy rate).
+static double block_cycles(const ClusterPlan& plan, int n, double weight_bytes, double hbm_share) {
+  const double b = double(n) / plan.pair;
+  const double mma = plan.pair == 2 ? std::max(2.0 * n, 128 + b) : std::max(4.0 * 40, 128 + b + (n > 64 ? n - 64 : 0));
+  return std::max({mma, 128 + b + 96 + b, weight_bytes / hbm_share});
+}
+
+ClusterPlan make_cluster_plan(int lo, int hi, int tokens, int k, const int max_clusters[4]) {
+  const int kblocks = k / kTileK, steps = (kblocks + 1) / 2;
+  ClusterPlan best;
+  best.cost = 1e30;
+  const int force_split = tuning("HYGEMM_CL_SPLIT", 0), force_pair = tuning("HYGEMM_CL_PAIR", 0), force_n = tuning("HYGEMM_CL_N", 0);
+  auto consider = [&](ClusterPlan plan) {
+    if (force_split && plan.split != force_split) return;
+    if (force_pair && plan.pair != force_pair) return;
+    if (force_n && plan.n_tile != force_n) return;
+    if (!finish_plan(plan)) return;
+    if (plan.cost < best.cost) best = plan;
+  };
+  for (int pair = 1; pair <= 2; ++pair)
+    for (int log = pair - 1; log < 4; ++log) {
+      ClusterPlan plan;
+      plan.pair = pair;
+      plan.split = (1 << log) / pair;
+      if (plan.split > steps) continue;
+      const int capacity = max_clusters[log];
+      if (capacity < 1) continue;
+      const double slice = double(kblocks) / plan.split;
+      const double fixed = plan.split > 1 ? 2500 : 0;
+      if (tokens <= 128) {
+        if ((pair == 2) != (tokens > 64)) continue;
+        // Weights stream from HBM once: every CTA gets the same number of bytes, an MXFP8 row counting two rows.
+        plan.n_tile = plan.n_tail = (tokens + 16 * pair - 1) / (16 * pair) * (16 * pair);
+        plan.token_tiles = 1;
+        const double total = lo + 2.0 * hi;
+        for (int waves = 1; waves <= 64; ++waves) {
+          const double rows = total / (double(waves) * capacity * pair);
+          int height = std::max(8, int(rows) + 1);
+          bool fits = false;
+          for (; height <= 128 && !fits; ++height) {
+            plan.tile_rows[0] = height;
+            plan.tile_rows[1] = (height + 1) / 2;
+            plan.tiles[0] = (lo + pair * plan.tile_rows[0] - 1) / (pair * plan.tile_rows[0]);
+            plan.tiles[1] = (hi + pair * plan.tile_rows[1] - 1) / (pair * plan.tile_rows[1]);
+            fits = plan.tiles[0] + plan.tiles[1] <= waves * capacity;
+          }
+          if (!fits) continue;
+          plan.clusters = std::min(capacity, plan.tiles[0] + plan.tiles[1]);
+          const double share = 23.0 * 148.0 / (plan.clusters << log);
+          plan.cost = waves * (slice * block_cycles(plan, plan.n_tile, plan.tile_rows[0] * 68.0, std::min(share, 40.0)) + 300) + fixed;
+          consider(plan);
+          if (waves > 1 && rows < 32) break;
+        }
+      } else {
+        if (pair == 1) continue;
+        plan.tile_rows[0] = plan.tile_rows[1] = 128;
+        plan.tiles[0] = (lo + 255) / 256;
+        plan.tiles[1] = (hi + 255) / 256;
+        for (int n : {128, 256}) {
+          if (n == 256 && plan.split > 1) continue;   // the partial tiles would not fit beside the ring
+          plan.n_tile = n;
+          plan.token_tiles = (tokens + n - 1) / n;
+          const int tail = tokens - (plan.token_tiles - 1) * n;
+          plan.n_tail = (tail + 31) / 32 * 32;
+          const int64_t units = int64_t(plan.tiles[0] + plan.tiles[1]) * plan.token_tiles;
+          plan.clusters = int(std::min<int64_t>(capacity, units));
+          // Units go round the clusters in order; the busiest cluster decides.
+          std::vector<double> load(size_t(plan.clusters), 0.0);
+          const double whole = slice * block_cycles(plan, n, 0, 1) + 600 + fixed, last = slice * block_cycles(plan, plan.n_tail, 0, 1) + 600 + fixed;
+          for (int64_t u = 0; u < units; ++u)
+            load[size_t(u % plan.clusters)] += (u % plan.token_tiles) == plan.token_tiles - 1 ? last : whole;
+          plan.cost = *std::max_element(load.begin(), load.end());
+          consider(plan);
+        }
+      }
+    }
+  if (best.cost >= 1e30) throw std::runtime_error("No cluster schedule for this shape");
+  return best;
+}
+
+template <typename T, int PAIR, bool FUSED>
+static void set_limits() {
+  check(cudaFuncSetAttribute(cluster_gemm_kernel<T, PAIR, FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem), "cudaFuncSetAttribute");
+}
+
+void configure_cluster_kernels() {
+  set_limits<__nv_bfloat16, 1, false>(); set_limits<__nv_bfloat16, 1, true>(); set_limits<__nv_bfloat16, 2, false>();
+  set_limits<__half, 1, false>(); set_limits<__half, 1, true>(); set_limits<__half, 2, false>();
+}
+
+const int* cluster_capacity() {
+  static int capacity[64][4];
+  static std::once_flag once[64];
+  int device = 0;
+  check(cudaGetDevice(&device), "cudaGetDevice");
+  if (device < 0 || device >= 64) throw std::runtime_error("Device ordinals 0..63 are supported");
+  std::call_once(once[device], [&] {
+    configure_cluster_kernels();
+    int sms = 0;
+    check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "SM count");
+    capacity[device][0] = sms;
+    for (int log = 1; log < 4; ++log) {
+      cudaLaunchConfig_t config{};
+      config.gridDim = dim3(unsigned(sms >> log << log));
+      config.blockDim = dim3(cluster_threads(false));
+      config.dynamicSmemBytes = kMaxSmem;
+      cudaLaunchAttribute attribute[1];
+      attribute[0].id = cudaLaunchAttributeClusterDimension;
+      attribute[0].val.clusterDim = {1u << log, 1u, 1u};
+      config.attrs = attribute;
+      config.numAttrs = 1;
+      int clusters = 0;
+      check(cudaOccupancyMaxActiveClusters(&clusters, cluster_gemm_kernel<__nv_bfloat16, 2, false>, &config), "cluster occupancy");
+      capacity[device][log] = std::min(clusters, sms >> log);
+    }
+  });
+  return capacity[device];
+}
+
+template <typename T, int PAIR, bool FUSED>
+static cudaError_t launch(const ClusterPlan& plan, const ClusterParams& p, const CUtensorMap& map_act, const CUtensorMap& map_tail,
+                          cudaStream_t stream, bool pdl) {
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(unsigned(plan.clusters * plan.pair * plan.split));
+  config.blockDim = dim3(cluster_threads(FUSED));
+  config.dynamicSmemBytes = size_t(plan.smem_bytes);
+  config.stream = stream;
+  cudaLaunchAttribute attribute[2];
+  int count = 0;
+  if (plan.pair * plan.split > 1) {
+    attribute[count].id = cudaLaunchAttributeClusterDimension;
+    attribute[count++].val.clusterDim = {unsigned(plan.pair * plan.split), 1u, 1u};
+  }
+  if (pdl && pdl_enabled()) {
+    attribute[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute[count++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  config.attrs = attribute;
+  config.numAttrs = unsigned(count);
+  return cudaLaunchKernelEx(&config, cluster_gemm_kernel<T, PAIR, FUSED>, p, map_act, map_tail);
+}
+
+void launch_cluster(const ClusterPlan& plan, const ClusterCall& call, const CUtensorMap& map_act, const CUtensorMap& map_tail,
+                    cudaStream_t stream, bool pdl) {
+  const hg_problem &l = *call.low, &h = *call.high, &any = l.rows ? l : h;
+  ClusterParams p{};
+  const hg_problem* parts[2] = {&l, &h};
+  for (int i = 0; i < 2; ++i) {
+    p.rows[i] = parts[i]->rows; p.tile_rows[i] = plan.tile_rows[i]; p.tiles[i] = plan.tiles[i];
+    p.weight[i] = static_cast<const uint8_t*>(parts[i]->weight);
+    p.sfa[i] = static_cast<const uint8_t*>(parts[i]->weight_scales);
+    p.ids[i] = static_cast<const int32_t*>(parts[i]->ids);
+  }
+  p.sfb = static_cast<const uint8_t*>(any.activation_scales);
+  p.out = call.out;
+  p.outputs = any.outputs; p.tokens = any.tokens; p.k = any.k; p.kblocks = any.k / kTileK;
+  p.n_tile = plan.n_tile; p.n_tail = plan.n_tail; p.token_tiles = plan.token_tiles; p.stages = plan.stages;
+  p.split = plan.split; p.clusters = plan.clusters;
+  while ((1 << p.split_log) < plan.split) ++p.split_log;
+  p.share_log = share_log_of(plan.n_tile, plan.split);
+  const uint64_t tiles = uint64_t(plan.tiles[0]) + uint64_t(plan.tiles[1]), most = uint64_t(1) << 40;
+  auto inverse = [&](uint64_t n_max, uint64_t d) {
+    const uint64_t inv = (most + d - 1) / d;
+    return n_max < most / d && n_max < (uint64_t(1) << 63) / inv ? inv : uint64_t(0);
+  };
+  p.by_token_tiles = inverse(tiles * plan.token_tiles, uint64_t(plan.token_tiles));
+  p.by_tiles = inverse((tiles + 1) * uint64_t(plan.tiles[1]), tiles);
+  p.acc_shift = plan.acc_shift; p.overlap = plan.overlap;
+  p.tmem_cols = uint32_t(plan.tmem_cols);
+  p.x = static_cast<const uint16_t*>(call.x);
+  p.x_bf16 = call.x_dtype == HG_DTYPE_BF16;
+  p.audit_tokens = call.audit_tokens;
+  p.status = call.status;
+#ifdef HG_TRACE
+  p.trace = call.trace;
+#endif
+  const bool bf16 = call.dtype == HG_DTYPE_BF16;
+  cudaError_t e;
+  if (call.x) e = bf16 ? launch<__nv_bfloat16, 1, true>(plan, p, map_act, map_tail, stream, pdl) : launch<__half, 1, true>(plan, p, map_act, map_tail, stream, pdl);
+  else if (plan.pair == 1) e = bf16 ? launch<__nv_bfloat16, 1, false>(plan, p, map_act, map_tail, stream, pdl) : launch<__half, 1, false>(plan, p, map_act, map_tail, stream, pdl);
+  else e = bf16 ? launch<__nv_bfloat16, 2, false>(plan, p, map_act, map_tail, stream, pdl) : launch<__half, 2, false>(plan, p, map_act, map_tail, stream, pdl);
+  check(e, "hybrid GEMM launch");
+}
+
+}  // namespace hg

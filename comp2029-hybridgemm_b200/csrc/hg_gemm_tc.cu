@@ -56,24 +56,15 @@
 #include <memory>
 #include <mutex>
 
+#include "hg_gemm_cluster.cuh"
 #include "hg_gemm_tc.cuh"
+#include "hg_tcgen05.cuh"
 
 namespace hg {
 
 // ---------------------------------------------------------------------------------------------
 // Device side
 // ---------------------------------------------------------------------------------------------
-
-// Where the epilogue stores: `ptr` is [tokens, outputs] of 16-bit elements, or of fp32 when `f32` is set.
-// For a row-parallel partial (hg_run_partial) `ptr` is this rank's exchange buffer, `epoch` the device word
-// that counts finished exchanges and `parity_bytes` the distance between the two halves of the buffer; the
-// half written is the one of exchange `*epoch + 1`.
-struct OutTargets {
-  void* ptr;
-  int f32;
-  const int* epoch;
-  int64_t parity_bytes;
-};
 
 // Per-CTA start of the schedule, passed BY VALUE as a kernel parameter: a CTA learns its first work unit
 // from the constant bank instead of from two dependent global loads (about a microsecond before the first
@@ -113,184 +104,6 @@ struct TcParams {
 #endif
 };
 
-enum : int { kErrProducer = 1, kErrMmaFull = 2, kErrMmaAcc = 3, kErrEpilogue = 4, kErrDrain = 5, kErrLoader = 6 };
-// Builds with -DHG_TRACE record, per CTA, the global timer at sixteen points of the kernel (hg_trace reads them
-// back; `bench.py --timeline` prints their distribution over the grid).  Slots: 0 entry, 1 set-up done, 2 dependency
-// wait released (TMA thread), 3 first full stage seen by issuer 0, 4-7 issuer 0's commit of its first four units,
-// 8/9, 10/11, 12/13 start and end of the first three epilogues (thread 64).  Ordinary builds compile none of it.
-#ifdef HG_TRACE
-__device__ __forceinline__ unsigned long long global_timer_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-#define HG_STAMP(slot) do { if (p.trace) p.trace[blockIdx.x * 16 + (slot)] = global_timer_ns(); } while (0)
-#else
-#define HG_STAMP(slot) do { } while (0)
-#endif
-
-constexpr long long kWaitLimitCycles = 4000000000ll;  // about 2 s at the boost clock, per wait
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
-
-__device__ __forceinline__ unsigned long long global_timer() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Bounded wait.  Returns false when the limit expired or another role of this
-// CTA already gave up (abort flag in shared memory).  The clock is only read on
-// the slow path, every 256 failed polls (each poll itself blocks in hardware for
-// a short, implementation-defined time).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-#pragma unroll 1
-  for (int burst = 0; burst < 256; ++burst)
-    if (mbar_try_wait(bar, parity)) return true;
-  const long long start = clock64();
-#pragma unroll 1
-  for (uint32_t spin = 1;; ++spin) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((spin & 255u) == 0) {
-      if (*abort_flag) return false;
-      if (clock64() - start > kWaitLimitCycles) return false;
-    }
-  }
-}
-
-// The same wait by a whole warp, with one verdict for all lanes.
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)) != 0;
-}
-// True in one lane of a converged warp.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t r;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "elect.sync _|p, 0xffffffff;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}"
-      : "=r"(r));
-  return r != 0;
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
-      : "memory");
-}
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tc_cp_scales(uint32_t tmem_addr, uint64_t smem_desc) {
-  asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem_addr), "l"(smem_desc) : "memory");
-}
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                       uint32_t accumulate, uint32_t tmem_sfa, uint32_t tmem_sfb) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n"
-      "}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb)
-      : "memory");
-}
-__device__ __forceinline__ void tc_load16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                 "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-               : "r"(taddr));
-}
-// A register filled by a tcgen05.ld issued before the last tc_wait_ld(): passing it through this (empty)
-// volatile statement keeps every use behind that wait, however far ahead the load was issued.
-__device__ __forceinline__ uint32_t tc_loaded(uint32_t v) {
-  asm volatile("" : "+r"(v));
-  return v;
-}
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// Shared-memory matrix descriptor (tcgen05 format, version 1).
-//   bits [0,14) start address >> 4, [16,30) leading byte offset >> 4,
-//   [32,46) stride byte offset >> 4, [46,48) version = 1, [61,64) swizzle mode.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo, uint32_t layout) {
-  return uint64_t((addr & 0x3ffffu) >> 4) | (uint64_t(lbo >> 4) << 16) | (uint64_t(sbo >> 4) << 32) |
-         (uint64_t(1) << 46) | (uint64_t(layout) << 61);
-}
-constexpr uint32_t kSwizzle128B = 2, kSwizzleNone = 0;
-
-// Instruction descriptor of kind::mxf8f6f4.block_scale:
-//   [4,6) B scale id, [7,10) A format (0 E4M3, 5 E2M1), [10,13) B format, [15] A major, [16] B major
-//   (0 = K-major), [17,23) N>>3, [23] scale format (1 = UE8M0), [24,29) M>>4, [29,31) A scale id.
-__device__ __forceinline__ uint32_t instr_desc(bool a_is_fp4, int n_tile) {
-  return (a_is_fp4 ? 5u << 7 : 0u) | (0u << 10) | (uint32_t(n_tile >> 3) << 17) | (1u << 23) |
-         (uint32_t(kTileRows >> 4) << 24);
-}
-
-__device__ __forceinline__ bool epilogue_all(bool ok) {
-  uint32_t r;
-  asm volatile(
-      "{\n"
-      ".reg .pred p, q;\n"
-      "setp.ne.b32 p, %1, 0;\n"
-      "barrier.cta.red.and.pred q, 1, 128, p;\n"
-      "selp.u32 %0, 1, 0, q;\n"
-      "}"
-      : "=r"(r)
-      : "r"(uint32_t(ok))
-      : "memory");
-  return r != 0;
-}
-__device__ __forceinline__ void epilogue_sync() { asm volatile("barrier.cta.sync 1, 128;" ::: "memory"); }
-
-template <typename T>
-__device__ __forceinline__ void scatter_store(const OutTargets& out, char* base, int64_t index, float v) {
-  if (out.f32) reinterpret_cast<float*>(base)[index] = v;
-  else reinterpret_cast<uint16_t*>(base)[index] = from_float<T>(v);
-}
-
-// Start of the output this launch writes: the plain output, or the half of the exchange buffer that belongs
-// to the coming exchange.  Read after pdl_wait(): the word is advanced by the kernel that ends the previous exchange.
-__device__ __forceinline__ char* out_base(const OutTargets& out) {
-  char* base = static_cast<char*>(out.ptr);
-  if (!out.epoch) return base;
-  const int e = *reinterpret_cast<const volatile int*>(out.epoch) + 1;
-  return base + int64_t(e & 1) * out.parity_bytes;
-}
-
 // Shared-memory plan.  One pipeline stage covers up to two K128 blocks (K256):
 //   A   2 x 16 KiB  weight tiles, 128 rows x 128 B each, 128B-swizzled, K-major
 //   B   2 x n_tile x 128 B activation tiles, same layout
@@ -311,17 +124,6 @@ __host__ __device__ inline SmemLayout smem_layout(int stages, int n_tile) {
 }
 constexpr int kScaleSets = 2;  // TMEM scale-factor buffers, alternated per K128 block
 constexpr int kBarrierBytes = (2 * kMaxStages + 5) * 8 + 32;
-constexpr int kLoaderThreads = 128;  // warps 6..9
-constexpr int kQuantThreads = 128;   // warps 13..16 (fused activation quantisation)
-
-// 8-byte asynchronous copy global -> shared; src_bytes = 0 writes zeros instead.
-__device__ __forceinline__ void cp_async_8(uint32_t dst, const void* src, uint32_t src_bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
-}
-// One arrival on `bar` once every cp.async this thread issued so far has landed.
-__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-}
 
 // FUSED = true adds the activation-quantiser warps (hg_run_x); the plain instantiation has none, so the
 // decode GEMMs on prepacked activations do not carry their threads and registers.
@@ -400,7 +202,6 @@ hybrid_gemm_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant_
   // sets of (SFA, SFB), 4 columns each.
   const uint32_t acc_cols = uint32_t((p.n_tile + 31) & ~31);
   const uint32_t acc_stride = acc_cols * uint32_t(p.issuers);
-  const uint32_t sf_cols = tmem_base + uint32_t(p.acc_slots) * acc_stride;
 
   int error = 0;
 
@@ -937,6 +738,14 @@ static bool staged_fixup() {
 }
 constexpr int kMaxDynamicSmem = 232448;  // 227 KiB, the per-CTA limit of sm_100
 
+// Shapes AUTO hands to the cluster kernel.  Prefill: 256-row pair tiles (gate_up at 2048 tokens 401 -> 279 us).  Up to 64
+// tokens: layers with fewer than about 1.5 tiles per SM, whose tiles are cut along K and exchanged inside a cluster (o_proj
+// at 16 tokens 10.5 -> 7.6 us, down 16.4 -> 15.5).  In between, and for wide layers at decode sizes, the ring of this
+// file's kernel turns faster.
+static bool cluster_serves(int tiles, int tokens, int sms) {
+  return tokens > 128 || (tokens <= 64 && 2 * tiles < 3 * sms);
+}
+
 Plan make_plan(int rows_low, int rows_high, int tokens, int k, int sms, int schedule) {
   Plan plan;
   const int tiles_low = (rows_low + kTileRows - 1) / kTileRows, tiles_high = (rows_high + kTileRows - 1) / kTileRows;
@@ -1098,13 +907,14 @@ Plan make_plan(int rows_low, int rows_high, int tokens, int k, int sms, int sche
   };
 
   if (schedule == HG_SCHEDULE_AUTO) {
-    // Measured on B200 (Qwen2.5-7B layer shapes, M = 1..128): whole tiles win once there are about
+    // The cluster kernel (hg_gemm_cluster.cu) never cuts a tile over units: its unit list is the data-parallel one.
+    // This kernel, measured on B200 (Qwen2.5-7B layer shapes, M = 1..128): whole tiles win once there are about
     // 1.5 tiles per SM, and also for wide token tiles unless K is long, because the fix-up traffic of a
     // cut tile grows with n_tile (n_tile x 128 fp32 partials written and read per piece); otherwise
     // stream-K, which keeps every SM streaming.
     const bool many_tiles = 2 * items >= 3 * sms;
     const bool wide_short = plan.n_tile >= 64 && kblocks < 64;
-    schedule = (many_tiles || wide_short) ? HG_SCHEDULE_DATA_PARALLEL : HG_SCHEDULE_STREAM_K;
+    schedule = (cluster_serves(tiles, tokens, sms) || many_tiles || wide_short) ? HG_SCHEDULE_DATA_PARALLEL : HG_SCHEDULE_STREAM_K;
   }
   plan.ws_slots = 0;
   plan.counters = 0;
@@ -1174,6 +984,21 @@ static CUtensorMap make_map(const void* ptr, int rows, int k, int box_rows) {
   return map;
 }
 
+// The same bytes as [K128 block][row][128]: one copy of a box of 2 blocks x box_rows fills a K256 stage.
+static CUtensorMap make_block_map(const void* ptr, int rows, int k, int box_rows) {
+  CUtensorMap map;
+  std::memset(&map, 0, sizeof(map));
+  const cuuint64_t dims[3] = {128u, cuuint64_t(rows), cuuint64_t(k / 128)};
+  const cuuint64_t strides[2] = {cuuint64_t(k), 128u};
+  const cuuint32_t box[3] = {128u, cuuint32_t(box_rows), 2u};
+  const cuuint32_t elem[3] = {1u, 1u, 1u};
+  const CUresult r = encode_tiled()(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(ptr), dims, strides, box,
+                                    elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled failed with code " + std::to_string(int(r)));
+  return map;
+}
+
 static CtaHeads make_heads(const Plan& plan) {
   CtaHeads heads{};
   static const bool enabled = [] { const char* t = std::getenv("HYGEMM_TC_HEADS"); return !t || std::atoi(t) != 0; }();
@@ -1187,6 +1012,8 @@ static CtaHeads make_heads(const Plan& plan) {
 
 struct TcGemm {
   Plan plan;
+  bool clustered = false;      // HG_SCHEDULE_AUTO: hg_gemm_cluster.cu
+  ClusterPlan cluster;
   CtaHeads heads{};
   int rows[2] = {0, 0}, tokens = 0, k = 0, outputs = 0, dtype = HG_DTYPE_BF16;
   WorkUnit* d_units = nullptr;
@@ -1200,7 +1027,7 @@ struct TcGemm {
 #endif
   // Tensor maps of recent operand pointers (the shape is fixed per handle): a serving loop alternates among
   // a few activation buffers and one weight pointer, so the driver call is paid once per pointer.
-  struct CachedMap { const void* ptr = nullptr; CUtensorMap map; };
+  struct CachedMap { const void* ptr = nullptr; CUtensorMap map, tail; };
   CachedMap act_maps[4], high_map;
   int act_next = 0;
 };
@@ -1245,13 +1072,26 @@ TcGemm* tc_create(const hg_problem& l, const hg_problem& h, int schedule, int dt
   g->rows[0] = l.rows; g->rows[1] = h.rows;
   g->tokens = any.tokens; g->k = any.k; g->outputs = any.outputs; g->dtype = dtype;
   g->plan = make_plan(l.rows, h.rows, any.tokens, any.k, sms, schedule);
-  g->heads = make_heads(g->plan);
   const Plan& plan = g->plan;
+  const int row_tiles = (l.rows + kTileRows - 1) / kTileRows + (h.rows + kTileRows - 1) / kTileRows;
+  if (schedule == HG_SCHEDULE_AUTO && cluster_serves(row_tiles, any.tokens, sms)) {
+    g->clustered = true;
+    g->cluster = make_cluster_plan(l.rows, h.rows, any.tokens, any.k, cluster_capacity());
+    check(cudaMalloc(&g->d_status, sizeof(int) * 4), "cudaMalloc status");
+    check(cudaMemsetAsync(g->d_status, 0, sizeof(int) * 4, stream), "clear status");
+#ifdef HG_TRACE
+    check(cudaMalloc(&g->d_trace, sizeof(unsigned long long) * 16 * size_t(sms)), "trace buffer");
+    check(cudaMemsetAsync(g->d_trace, 0, sizeof(unsigned long long) * 16 * size_t(sms), stream), "trace buffer");
+    g->plan.grid = g->cluster.clusters * g->cluster.pair * g->cluster.split;
+#endif
+    return g.release();
+  }
+  g->heads = make_heads(g->plan);
   check(cudaMalloc(&g->d_units, sizeof(WorkUnit) * std::max<size_t>(1, plan.units.size())), "cudaMalloc units");
   check(cudaMalloc(&g->d_cta_begin, sizeof(int) * plan.cta_begin.size()), "cudaMalloc schedule");
   check(cudaMalloc(&g->d_workspace, sizeof(float) * std::max<int64_t>(1, int64_t(plan.ws_slots) * plan.n_tile * kTileRows)), "cudaMalloc workspace");
   check(cudaMalloc(&g->d_counters, sizeof(int) * std::max(1, plan.counters)), "cudaMalloc counters");
-    check(cudaMalloc(&g->d_status, sizeof(int) * 4), "cudaMalloc status");
+  check(cudaMalloc(&g->d_status, sizeof(int) * 4), "cudaMalloc status");
   check(cudaMalloc(&g->d_cut, sizeof(int) * std::max<size_t>(4, plan.cut_tiles.size())), "cudaMalloc cut list");
 #ifdef HG_TRACE
   check(cudaMalloc(&g->d_trace, sizeof(unsigned long long) * 16 * size_t(plan.grid)), "trace buffer");
@@ -1323,31 +1163,24 @@ void tc_run(TcGemm* g, const hg_problem& l, const hg_problem& h, cudaStream_t st
   if (l.rows != g->rows[0] || h.rows != g->rows[1] || any.tokens != g->tokens || any.k != g->k || any.outputs != g->outputs)
     throw std::runtime_error("Hybrid GEMM handle was created for a different shape");
   const Plan& plan = g->plan;
-  TcParams p = base_params(plan, l, h, g->dtype);
+  OutTargets out{};
   if (partial) {
     // This rank's exchange buffer (two halves); decode sizes travel as fp32 so the sum is rounded once.
     if (!partial->buffer || !partial->state) throw std::runtime_error("Null exchange buffer or state");
     if (reinterpret_cast<uintptr_t>(partial->buffer) & 15 || partial->half_bytes % 16) throw std::runtime_error("Exchange buffer halves must be 16-byte aligned");
     if (partial->half_bytes < int64_t(any.tokens) * any.outputs * (partial->f32 ? 4 : 2))
       throw std::runtime_error("Exchange buffer half smaller than tokens x outputs");
-    p.out.ptr = partial->buffer;
-    p.out.f32 = partial->f32 ? 1 : 0;
-    p.out.epoch = partial->state;
-    p.out.parity_bytes = partial->half_bytes;
+    out.ptr = partial->buffer;
+    out.f32 = partial->f32 ? 1 : 0;
+    out.epoch = partial->state;
+    out.parity_bytes = partial->half_bytes;
   } else {
-    p.out.ptr = any.output;
+    out.ptr = any.output;
   }
-  p.x = static_cast<const uint16_t*>(x);
-  p.x_bf16 = x_dtype == HG_DTYPE_BF16;
-  p.units = g->d_units; p.cta_begin = g->d_cta_begin;
-  p.workspace = g->d_workspace; p.counters = g->d_counters; p.status = g->d_status;
-#ifdef HG_TRACE
-  p.trace = g->d_trace;
-#endif
   // Tensor maps by operand pointer.  A map that the launch does not use (no MXFP8 rows; activations
   // quantised in the kernel) is passed as zeros and never touched by the kernel.
   static const CUtensorMap no_map{};
-  const CUtensorMap* map_act = &no_map;
+  const TcGemm::CachedMap* act = nullptr;
   if (!fused) {
     TcGemm::CachedMap* hit = nullptr;
     for (auto& entry : g->act_maps)
@@ -1355,11 +1188,35 @@ void tc_run(TcGemm* g, const hg_problem& l, const hg_problem& h, cudaStream_t st
     if (!hit) {
       hit = &g->act_maps[g->act_next];
       g->act_next = (g->act_next + 1) % 4;
-      hit->map = make_map(any.activation, any.tokens, any.k, plan.n_tile);
+      hit->ptr = nullptr;
+      if (g->clustered) {
+        hit->map = make_block_map(any.activation, any.tokens, any.k, g->cluster.n_tile / g->cluster.pair);
+        hit->tail = make_block_map(any.activation, any.tokens, any.k, g->cluster.n_tail / g->cluster.pair);
+      } else {
+        hit->map = make_map(any.activation, any.tokens, any.k, plan.n_tile);
+      }
       hit->ptr = any.activation;
     }
-    map_act = &hit->map;
+    act = hit;
   }
+  if (g->clustered) {
+    ClusterCall call{&l, &h, x, x_dtype, out, g->dtype, plan.n_tile, g->d_status, nullptr};
+#ifdef HG_TRACE
+    call.trace = g->d_trace;
+#endif
+    launch_cluster(g->cluster, call, act ? act->map : no_map, act ? act->tail : no_map, stream, true);
+    return;
+  }
+  TcParams p = base_params(plan, l, h, g->dtype);
+  p.out = out;
+  p.x = static_cast<const uint16_t*>(x);
+  p.x_bf16 = x_dtype == HG_DTYPE_BF16;
+  p.units = g->d_units; p.cta_begin = g->d_cta_begin;
+  p.workspace = g->d_workspace; p.counters = g->d_counters; p.status = g->d_status;
+#ifdef HG_TRACE
+  p.trace = g->d_trace;
+#endif
+  const CUtensorMap* map_act = act ? &act->map : &no_map;
   const CUtensorMap* map_high = &no_map;
   if (h.rows) {
     if (g->high_map.ptr != h.weight) {
@@ -1453,6 +1310,8 @@ struct StaticPlan {
   int key[6] = {0, 0, 0, 0, 0, 0};
   uint64_t used = 0;             // 0 = empty
   Plan plan;
+  bool clustered = false;        // the cluster kernel serves this shape
+  ClusterPlan cluster;
   CtaHeads heads{};
 };
 
@@ -1520,11 +1379,22 @@ void tc_run_static(int schedule, const hg_problem& l, const hg_problem& h, int d
     for (auto& resident : st.resident)
       if (resident == entry) resident = nullptr;   // the array of that device holds a schedule that is going away
     entry->plan = make_plan(l.rows, h.rows, any.tokens, any.k, st.sms[device], schedule);
-    entry->heads = make_heads(entry->plan);
+    entry->clustered = schedule == HG_SCHEDULE_AUTO && cluster_serves((l.rows + kTileRows - 1) / kTileRows + (h.rows + kTileRows - 1) / kTileRows, any.tokens, st.sms[device]);
+    if (entry->clustered) entry->cluster = make_cluster_plan(l.rows, h.rows, any.tokens, any.k, cluster_capacity());
+    else entry->heads = make_heads(entry->plan);
     std::memcpy(entry->key, key, sizeof(key));
   }
   entry->used = ++st.clock;
   const Plan& plan = entry->plan;
+  if (entry->clustered) {
+    // The cluster kernel keeps its partial sums on chip: of the array it needs the status words only.
+    const ClusterPlan& cluster = entry->cluster;
+    ClusterCall call{&l, &h, nullptr, HG_DTYPE_BF16, OutTargets{}, dtype, plan.n_tile, reinterpret_cast<int*>(base + kStaticStatusOffset), nullptr};
+    call.out.ptr = any.output;
+    launch_cluster(cluster, call, make_block_map(any.activation, any.tokens, any.k, cluster.n_tile / cluster.pair),
+                   make_block_map(any.activation, any.tokens, any.k, cluster.n_tail / cluster.pair), stream, false);
+    return;
+  }
 
   // Carve the array: status | counters | cta_begin | units | cut list | workspace.
   const size_t off_cta = align_up(kStaticCountersOffset + sizeof(int) * size_t(std::max(1, plan.counters)), 256);
