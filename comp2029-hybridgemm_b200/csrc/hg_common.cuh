@@ -39,6 +39,11 @@ __host__ __device__ inline int64_t scale_word_offset(int row, int kb, int k) {
   return (int64_t(row / 128) * (k / 128) + kb) * 512 + (row % 32) * 16 + ((row % 128) / 32) * 4;
 }
 
+// A small pinned buffer of the calling thread that kernels can write, for calls that end with a host-side result: a
+// copy from device memory (through a pageable buffer above all) costs more than the wait itself.
+constexpr size_t kPinnedResultBytes = 256;
+void* pinned_result();
+
 #ifdef __CUDACC__
 // Programmatic dependent launch.  Every kernel of the library is launched with the
 // programmatic-stream-serialization attribute (unless HYGEMM_PDL=0): it may start while its

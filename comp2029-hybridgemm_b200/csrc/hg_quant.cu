@@ -20,12 +20,51 @@ std::string& last_error() {
   return message;
 }
 
+void* pinned_result() {
+  struct Pinned {
+    void* ptr = nullptr;
+    ~Pinned() { if (ptr) cudaFreeHost(ptr); }
+  };
+  static thread_local Pinned pinned;   // one small buffer per thread, given back with it
+  if (!pinned.ptr) check(cudaHostAlloc(&pinned.ptr, kPinnedResultBytes, cudaHostAllocPortable | cudaHostAllocMapped), "pinned buffer");
+  return pinned.ptr;
+}
+
 bool pdl_enabled() {
   static const bool enabled = [] {
     const char* v = std::getenv("HYGEMM_PDL");
     return !(v && v[0] == '0');
   }();
   return enabled;
+}
+
+template <typename T>
+__device__ __forceinline__ void widen8(const uint4& raw, float (&v)[8]) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = to_float<T>(uint16_t(w[i >> 1] >> ((i & 1) * 16)));
+}
+
+// SwiGLU of eight (gate, up) pairs with the roundings of SiluAndMul; `product` receives the 16-bit products.
+template <typename T, int MATH>
+__device__ __forceinline__ void silu8(const uint4& g4, const uint4& u4, float (&v)[8], uint4& product) {
+  float g[8], u[8];
+  widen8<T>(g4, g);
+  widen8<T>(u4, u);
+  uint32_t dw[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float e = MATH == 0 ? expf(-g[i]) : __expf(-g[i]);
+    const float act = MATH == 1 ? __fdividef(g[i], 1.f + e) : g[i] / (1.f + e);
+    // The consumer this replaces adds a zero beta to `up` before multiplying;
+    // keeping the addition preserves +0 + -0 -> +0 and with it the sign bit
+    // of a zero product (integrations/vllm/native/producer.cu:30-32).
+    const float up = __fadd_rn(u[i], 0.f);
+    const uint16_t p16 = from_float<T>(to_float<T>(from_float<T>(act)) * up);
+    v[i] = to_float<T>(p16);
+    dw[i >> 1] |= uint32_t(p16) << ((i & 1) * 16);
+  }
+  product = make_uint4(dw[0], dw[1], dw[2], dw[3]);
 }
 
 template <typename T, bool FP4, bool SILU, int MATH>
@@ -57,24 +96,9 @@ mx_quant_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint
   if constexpr (SILU) {
     const uint4 g4 = *reinterpret_cast<const uint4*>(in + int64_t(row) * 2 * k + col);
     const uint4 u4 = *reinterpret_cast<const uint4*>(in + int64_t(row) * 2 * k + k + col);
-    const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w}, uw[4] = {u4.x, u4.y, u4.z, u4.w};
-    uint32_t dw[4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float g = to_float<T>(uint16_t(gw[i >> 1] >> ((i & 1) * 16)));
-      const float u = to_float<T>(uint16_t(uw[i >> 1] >> ((i & 1) * 16)));
-      const float e = MATH == 0 ? expf(-g) : __expf(-g);
-      const float act = MATH == 1 ? __fdividef(g, 1.f + e) : g / (1.f + e);
-      // The consumer this replaces adds a zero beta to `up` before multiplying;
-      // keeping the addition preserves +0 + -0 -> +0 and with it the sign bit
-      // of a zero product (integrations/vllm/native/producer.cu:30-32).
-      const float up = __fadd_rn(u, 0.f);
-      const uint16_t a16 = from_float<T>(act);
-      const uint16_t p16 = from_float<T>(to_float<T>(a16) * up);
-      v[i] = to_float<T>(p16);
-      if (i & 1) dw[i >> 1] |= uint32_t(p16) << 16; else dw[i >> 1] = p16;
-    }
-    if (debug) *reinterpret_cast<uint4*>(debug + int64_t(row) * k + col) = make_uint4(dw[0], dw[1], dw[2], dw[3]);
+    uint4 product;
+    silu8<T, MATH>(g4, u4, v, product);
+    if (debug) *reinterpret_cast<uint4*>(debug + int64_t(row) * k + col) = product;
   } else {
     const uint4 x4 = *reinterpret_cast<const uint4*>(in + int64_t(row) * k + col);
     const uint32_t xw[4] = {x4.x, x4.y, x4.z, x4.w};
@@ -109,8 +133,250 @@ mx_quant_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint
   if (sub == 0) *reinterpret_cast<uint32_t*>(sf + scale_word_offset(row, kb, k)) = word;
 }
 
+// ---- Many rows: weights at load time, prefill activations -----------------------------------------------------------
+//
+// A warp owns rows r, r+32, r+64, r+96 of a 128-row scale block x 512 columns, sixteen consecutive values per lane and row,
+// and has its four 32-byte loads (SwiGLU: eight) in flight before it converts the first.  Sixteen values per lane halve the
+// instructions per value against eight (one shuffle, one exponent and one scale byte per sixteen, maxima in packed 16-bit
+// form): the kernel above is bound by them, 3.8 TB/s on a 272 MB weight matrix.  The four rows share the 16-byte
+// entries of the scale atoms, so scales leave as whole entries instead of single words, each a partial write of a
+// sector.  With row lists the rows are gathered: a layer's two partitions are packed from the 16-bit matrix in one
+// launch, without copies of the partitions in between.
+struct QuantPart {
+  const int32_t* ids;   // source row of each packed row; null = the same
+  uint8_t* codes;
+  uint8_t* sf;
+  int rows;
+};
+
+struct Raw16 { uint32_t w[8]; };   // sixteen 16-bit values
+
+__device__ __forceinline__ Raw16 load16(const uint16_t* p) {
+  Raw16 r;
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]), "=r"(r.w[5]), "=r"(r.w[6]), "=r"(r.w[7])
+               : "l"(p));
+  return r;
+}
+template <typename T> struct Packed;
+template <> struct Packed<__half> {
+  static __device__ __forceinline__ uint32_t max_abs(uint32_t a, uint32_t b) {   // a is a maximum already
+    const __half2 m = __hmax2(*reinterpret_cast<const __half2*>(&a), __habs2(*reinterpret_cast<const __half2*>(&b)));
+    return *reinterpret_cast<const uint32_t*>(&m);
+  }
+  static __device__ __forceinline__ float2 widen(uint32_t v) { return __half22float2(*reinterpret_cast<const __half2*>(&v)); }
+};
+template <> struct Packed<__nv_bfloat16> {
+  static __device__ __forceinline__ uint32_t max_abs(uint32_t a, uint32_t b) {
+    const __nv_bfloat162 m = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a), __habs2(*reinterpret_cast<const __nv_bfloat162*>(&b)));
+    return *reinterpret_cast<const uint32_t*>(&m);
+  }
+  static __device__ __forceinline__ float2 widen(uint32_t v) { return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
+};
+
+// Sixteen values of a lane; two lanes make a K32 group, eight a K128 block.  Codes and scales as mx_quant_kernel's (a maximum
+// that skips NaNs, exact scaling by a power of two).  Returns the scale word of the block; `codes` null: beyond the row.
+template <typename T, bool FP4>
+__device__ __forceinline__ uint32_t quantise16(const Raw16& x, uint8_t* codes, int lane) {
+  uint32_t top = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) top = Packed<T>::max_abs(top, x.w[i]);
+  top = Packed<T>::max_abs(top, __shfl_xor_sync(0xffffffffu, top, 1));
+  const float2 ends = Packed<T>::widen(top);
+  const int e = mx_exponent<FP4>(fmaxf(fmaxf(0.f, ends.x), ends.y));
+  const float inv = mx_inverse_scale(e);
+  if (codes) {
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float2 pair = Packed<T>::widen(x.w[i]);
+      v[2 * i] = pair.x * inv;
+      v[2 * i + 1] = pair.y * inv;
+    }
+    if constexpr (FP4) {
+      const float (&low)[8] = *reinterpret_cast<const float (*)[8]>(v), (&high)[8] = *reinterpret_cast<const float (*)[8]>(v + 8);
+      *reinterpret_cast<uint2*>(codes) = make_uint2(cvt_e2m1x8(low), cvt_e2m1x8(high));
+    } else {
+      uint32_t c[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) c[i] = cvt_e4m3x2(v[4 * i], v[4 * i + 1]) | (cvt_e4m3x2(v[4 * i + 2], v[4 * i + 3]) << 16);
+      *reinterpret_cast<uint4*>(codes) = make_uint4(c[0], c[1], c[2], c[3]);
+    }
+  }
+  uint32_t word = uint32_t(e + 127) << (8 * ((lane >> 1) & 3));
+  word |= __shfl_xor_sync(0xffffffffu, word, 2);
+  return word | __shfl_xor_sync(0xffffffffu, word, 4);
+}
+
+// Rows 128 (group / 32) + group % 32 + 32 i of a partition, columns col0 .. col0 + 511.
+template <typename T, bool FP4>
+__device__ __forceinline__ void quantise_rows(const uint16_t* __restrict__ in, const QuantPart& part, int group, int col0, int k, int lane) {
+  const int row0 = (group >> 5) * 128 + (group & 31), col = col0 + 16 * lane;
+  Raw16 raw[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int row = row0 + 32 * r;
+    raw[r] = Raw16{};
+    if (row < part.rows && col < k) raw[r] = load16(in + int64_t(part.ids ? part.ids[row] : row) * k + col);
+  }
+  uint32_t word[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int row = row0 + 32 * r;
+    word[r] = 0x7f7f7f7fu;   // padding rows of the last 128-row scale block
+    if (row < part.rows) {
+      const int64_t at = int64_t(row) * k + col;
+      word[r] = quantise16<T, FP4>(raw[r], col < k ? part.codes + (FP4 ? at >> 1 : at) : nullptr, lane);
+    }
+  }
+  if (col < k && (lane & 7) == 0)
+    *reinterpret_cast<uint4*>(part.sf + scale_word_offset(row0, col >> 7, k)) = make_uint4(word[0], word[1], word[2], word[3]);
+}
+
+// Packs `low` to MXFP4 and `high` to MXFP8 (either may be empty).
+template <typename T>
+__global__ void __launch_bounds__(256)
+mx_rows_kernel(const uint16_t* __restrict__ in, const QuantPart low, const QuantPart high, int k) {
+  pdl_trigger();
+  pdl_wait();   // input and row lists come from the kernels before
+  const int lane = threadIdx.x & 31, chunks = (k + 511) >> 9;
+  const int item = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int group = item / chunks, col0 = (item - group * chunks) << 9;
+  const int low_groups = ((low.rows + 127) & ~127) >> 2, high_groups = ((high.rows + 127) & ~127) >> 2;
+  if (group < low_groups) quantise_rows<T, true>(in, low, group, col0, k, lane);
+  else if (group < low_groups + high_groups) quantise_rows<T, false>(in, high, group - low_groups, col0, k, lane);
+}
+
+// SwiGLU + MXFP8 for many rows; bound by the exponentials and divisions (IEEE, as SiluAndMul's) rather than by memory.
+template <typename T, int MATH>
+__global__ void __launch_bounds__(256)
+mx_silu_rows_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint8_t* __restrict__ sf, uint16_t* __restrict__ debug, int rows, int k) {
+  pdl_trigger();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, chunks = (k + 511) >> 9;
+  const int item = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int group = item / chunks, col = ((item - group * chunks) << 9) + 16 * lane;
+  if (group >= ((rows + 127) & ~127) >> 2) return;
+  const int row0 = (group >> 5) * 128 + (group & 31);
+  uint32_t word[4];
+#pragma unroll
+  for (int half = 0; half < 4; half += 2) {   // two rows in flight at a time: four would not fit the registers
+    Raw16 gate[2], up[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int row = row0 + 32 * (half + r);
+      gate[r] = up[r] = Raw16{};
+      if (row < rows && col < k) {
+        const uint16_t* at = in + int64_t(row) * 2 * k + col;
+        gate[r] = load16(at);
+        up[r] = load16(at + k);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int row = row0 + 32 * (half + r);
+      word[half + r] = 0x7f7f7f7fu;
+      if (row < rows) {
+        Raw16 product;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float v[8];
+          uint4 p;
+          silu8<T, MATH>(make_uint4(gate[r].w[4 * j], gate[r].w[4 * j + 1], gate[r].w[4 * j + 2], gate[r].w[4 * j + 3]),
+                         make_uint4(up[r].w[4 * j], up[r].w[4 * j + 1], up[r].w[4 * j + 2], up[r].w[4 * j + 3]), v, p);
+          product.w[4 * j] = p.x; product.w[4 * j + 1] = p.y; product.w[4 * j + 2] = p.z; product.w[4 * j + 3] = p.w;
+          if (debug && col < k) *reinterpret_cast<uint4*>(debug + int64_t(row) * k + col + 8 * j) = p;
+        }
+        word[half + r] = quantise16<T, false>(product, col < k ? out + int64_t(row) * k + col : nullptr, lane);
+      }
+    }
+  }
+  if (col < k && (lane & 7) == 0)
+    *reinterpret_cast<uint4*>(sf + scale_word_offset(row0, col >> 7, k)) = make_uint4(word[0], word[1], word[2], word[3]);
+}
+
+// From this many elements on the many-rows kernels are faster (K = 3584: 777 rows 3.2 us against 3.8, 2048 rows 6.5 against
+// 5.4; SwiGLU, K = 18944: 128 rows 5.7 against 7.3, 256 rows level, 2048 rows 70 against 59); below, one load per thread has
+// the shorter chain.  gate_up's 37888 x 3584 weights: 107 us against 67.
+constexpr int64_t kManyRowsElements = 4 << 20;
+
+static unsigned row_blocks(int64_t groups, int k) { return unsigned((groups * ((k + 511) / 512) + 7) / 8); }
+
+template <typename T>
+static cudaError_t launch_rows(const void* in, const QuantPart& low, const QuantPart& high, int k, cudaStream_t s) {
+  const int64_t groups = (int64_t((low.rows + 127) & ~127) + ((high.rows + 127) & ~127)) / 4;
+  return launch_kernel(mx_rows_kernel<T>, dim3(row_blocks(groups, k)), dim3(256), 0, s, static_cast<const uint16_t*>(in), low, high, k);
+}
+
+// The row lists of a layer from the ids of its MXFP8 channels: one block, a bitmap of the rows in shared memory, and a
+// scan of its words.  result = {distinct ids, an id was out of range}; lists are only complete when ids are distinct.
+constexpr int kPartitionThreads = 1024;
+__global__ void __launch_bounds__(kPartitionThreads)
+partition_rows_kernel(const int64_t* __restrict__ ids, int n_ids, int rows, int32_t* __restrict__ lo, int32_t* __restrict__ hi, int* __restrict__ result) {
+  extern __shared__ uint32_t bitmap[];
+  __shared__ int warp_sum[32];
+  pdl_trigger();
+  pdl_wait();
+  const int words = (rows + 31) >> 5, tid = threadIdx.x;
+  for (int w = tid; w < words; w += kPartitionThreads) bitmap[w] = 0;
+  __syncthreads();
+  int bad = 0;
+  for (int i = tid; i < n_ids; i += kPartitionThreads) {
+    const int64_t id = ids[i];
+    if (id < 0 || id >= rows) bad = 1;
+    else atomicOr(bitmap + (id >> 5), 1u << (id & 31));
+  }
+  bad = __syncthreads_or(bad);
+  const int per = (words + kPartitionThreads - 1) / kPartitionThreads, begin = min(words, tid * per), end = min(words, begin + per);
+  int mine = 0;
+  for (int w = begin; w < end; ++w) mine += __popc(bitmap[w]);
+  int sum = mine;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int other = __shfl_up_sync(0xffffffffu, sum, d);
+    if ((tid & 31) >= d) sum += other;
+  }
+  if ((tid & 31) == 31) warp_sum[tid >> 5] = sum;
+  __syncthreads();
+  if (tid < 32) {
+    int total = warp_sum[tid];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int other = __shfl_up_sync(0xffffffffu, total, d);
+      if (tid >= d) total += other;
+    }
+    warp_sum[tid] = total;
+  }
+  __syncthreads();
+  int high = sum - mine + (tid >= 32 ? warp_sum[(tid >> 5) - 1] : 0);   // MXFP8 rows before this thread's first row
+  for (int w = begin; w < end; ++w) {
+    const uint32_t bits = bitmap[w];
+    for (int b = 0; b < 32; ++b) {
+      const int row = w * 32 + b;
+      if (row >= rows) break;
+      if ((bits >> b) & 1u) {
+        if (high < n_ids) hi[high] = row;
+        ++high;
+      } else if (row - high < rows - n_ids) {
+        lo[row - high] = row;
+      }
+    }
+  }
+  if (tid == 0) { result[0] = warp_sum[31]; result[1] = bad; }
+}
+
 template <typename T, bool FP4, bool SILU, int MATH>
 static cudaError_t launch_quant(const void* in, void* out, void* sf, void* debug, int rows, int k, cudaStream_t s) {
+  if (int64_t(rows) * k >= kManyRowsElements && (reinterpret_cast<uintptr_t>(in) & 31) == 0) {   // 32-byte loads
+    if constexpr (SILU) {
+      const int64_t groups = ((int64_t(rows) + 127) & ~int64_t(127)) / 4;
+      return launch_kernel(mx_silu_rows_kernel<T, MATH>, dim3(row_blocks(groups, k)), dim3(256), 0, s, static_cast<const uint16_t*>(in),
+                           static_cast<uint8_t*>(out), static_cast<uint8_t*>(sf), static_cast<uint16_t*>(debug), rows, k);
+    } else {
+      const QuantPart part{nullptr, static_cast<uint8_t*>(out), static_cast<uint8_t*>(sf), rows}, none{};
+      return launch_rows<T>(in, FP4 ? part : none, FP4 ? none : part, k, s);
+    }
+  }
   const int kblocks = k / 128;
   const int64_t pad_rows = ((rows + 127) & ~127) - rows;
   const int64_t threads = int64_t(rows) * kblocks * 16 + pad_rows * kblocks;
@@ -136,6 +402,10 @@ static void pack_any(const void* in, void* out, void* sf, int rows, int k, int f
   check(e, "MX pack launch");
 }
 
+void pack_activations(const void* x, void* codes, void* scales, int tokens, int k, int dtype, cudaStream_t stream) {
+  pack_any(x, codes, scales, tokens, k, 0, stream, dtype == HG_DTYPE_BF16);
+}
+
 static int silu_any(const void* in, void* q, void* sf, void* debug, int rows, int k, void* stream, int math, bool bf16) {
   // Argument rule and return convention of integrations/vllm/native/producer.cu:46-54.
   if (!in || !q || !sf || rows <= 0 || k <= 0 || k % 128 || math < 0 || math > 2) return int(cudaErrorInvalidValue);
@@ -147,6 +417,23 @@ static int silu_any(const void* in, void* q, void* sf, void* debug, int rows, in
                : launch_quant<T, false, true, 2>(in, q, sf, debug, rows, k, s))
   return int(bf16 ? HG_SILU(__nv_bfloat16) : HG_SILU(__half));
 #undef HG_SILU
+}
+
+static void split_pack(const void* weight, const int64_t* ids, int n_ids, int rows, int k, int32_t* lo, int32_t* hi, void* w4, void* sf4,
+                       void* w8, void* sf8, int host_result[2], int dtype, cudaStream_t s) {
+  if (rows <= 0 || k <= 0 || k % 128 || n_ids < 0 || n_ids > rows || !weight || (n_ids && !ids)) throw std::runtime_error("Invalid split-pack arguments");
+  if (dtype != HG_DTYPE_F16 && dtype != HG_DTYPE_BF16) throw std::runtime_error("Unknown weight dtype");
+  if (reinterpret_cast<uintptr_t>(weight) & 31) throw std::runtime_error("Split-pack weights must be 32-byte aligned");
+  if (!aligned16(w4) || !aligned16(sf4) || !aligned16(w8) || !aligned16(sf8)) throw std::runtime_error("MX pack pointers must be 16-byte aligned");
+  const size_t bitmap = size_t((rows + 31) / 32) * 4;
+  if (bitmap > 47 * 1024) throw std::runtime_error("Too many rows for one split-pack");
+  int* const result = static_cast<int*>(pinned_result());   // written by the kernel itself, over the bus: no copy afterwards
+  check(launch_kernel(partition_rows_kernel, dim3(1), dim3(kPartitionThreads), bitmap, s, ids, n_ids, rows, lo, hi, result), "partition launch");
+  const QuantPart low{lo, static_cast<uint8_t*>(w4), static_cast<uint8_t*>(sf4), rows - n_ids}, high{hi, static_cast<uint8_t*>(w8), static_cast<uint8_t*>(sf8), n_ids};
+  check(dtype == HG_DTYPE_BF16 ? launch_rows<__nv_bfloat16>(weight, low, high, k, s) : launch_rows<__half>(weight, low, high, k, s), "split-pack launch");
+  check(cudaStreamSynchronize(s), "split-pack");
+  host_result[0] = result[0];
+  host_result[1] = result[1];
 }
 
 }  // namespace hg
@@ -172,6 +459,13 @@ int hg_pack_bf16(const void* in, void* out, void* sf, int rows, int k, int fp4, 
 int hg_pack_mode_bf16(const void* in, void* out, void* sf, int rows, int k, int fp4, void* stream, int mode) {
   (void)mode;
   HG_TRY hg::pack_any(in, out, sf, rows, k, fp4, stream, true); HG_CATCH
+}
+
+int hg_split_pack(const void* weight, const int64_t* ids, int n_ids, int rows, int k, int32_t* lo, int32_t* hi, void* w4, void* sf4,
+                  void* w8, void* sf8, int* host_result, int dtype, void* stream) {
+  HG_TRY
+  if (!host_result) throw std::runtime_error("Invalid split-pack arguments");
+  hg::split_pack(weight, ids, n_ids, rows, k, lo, hi, w4, sf4, w8, sf8, host_result, dtype, static_cast<cudaStream_t>(stream)); HG_CATCH
 }
 
 int hg_silu_pack(const void* in, void* q, void* sf, void* debug, int rows, int k, void* stream, int math) {

@@ -15,7 +15,6 @@ import ctypes as C
 import torch
 
 from . import native
-from .offline_weights import logical_scales
 
 # Midpoints between neighbouring E2M1 magnitudes 0, .5, 1, 1.5, 2, 3, 4, 6.
 _MIDPOINTS = (0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5.0)
@@ -59,40 +58,32 @@ def quantize(w: torch.Tensor, importance: torch.Tensor | None = None, offsets=(0
     """
     if w.ndim != 2 or w.dtype not in native.DTYPES or not w.is_cuda or w.shape[1] % 128:
         raise ValueError("quantize needs a CUDA FP16/BF16 [rows, K] matrix with K % 128 == 0")
-    if not torch.isfinite(w).all():
-        raise ValueError("weights must be finite")
     rows, k = w.shape
     w = w.contiguous()
     weight = None
     if importance is not None:
         weight = importance.to(device=w.device, dtype=torch.float32).contiguous()
-        if weight.shape != (k,) or not torch.isfinite(weight).all() or (weight < 0).any():
+        if weight.shape != (k,):
             raise ValueError("importance must be k finite non-negative values")
     q4 = torch.empty((rows, k // 2), dtype=torch.uint8, device=w.device)
     scales = torch.empty((rows, k // 32), dtype=torch.uint8, device=w.device)
-    shifts = (C.c_int * len(offsets))(*[int(o) for o in offsets])
-    lib = native.library()
-    lib.hg_clip_pack.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int,
-                                 C.POINTER(C.c_int), C.c_int, C.c_int, C.c_void_p]
-    native.check(lib.hg_clip_pack(w.data_ptr(), weight.data_ptr() if weight is not None else None, q4.data_ptr(),
-                                  scales.data_ptr(), rows, k, shifts, len(offsets), native.DTYPES[w.dtype],
-                                  torch.cuda.current_stream(w.device).cuda_stream))
-
-    # Statistics against the round-to-nearest baseline (the same kernel with no offsets is hg_pack's result).
-    base_q, base_sf = native.pack(w, True)
-    base_scales = logical_scales(base_sf, rows, k)
-    source = w.float().reshape(rows, k // 32, 32)
-    per_k = (torch.ones(k, device=w.device) if weight is None else weight).reshape(1, k // 32, 32)
-    before = (decode_logical(base_q, base_scales, k).reshape_as(source) - source).square()
-    after = (decode_logical(q4, scales, k).reshape_as(source) - source).square()
-    weighted_before, weighted_after = (before * per_k).sum(-1), (after * per_k).sum(-1)
-    if not torch.all(weighted_after <= weighted_before * (1 + 1e-6) + 1e-25):
+    gathered = torch.empty(16, dtype=torch.float64, device=w.device)
+    shifts, found = (C.c_int * len(offsets))(*[int(o) for o in offsets]), (C.c_double * 16)()
+    native.check(native.library().hg_clip_pack_stats(
+        w.data_ptr(), weight.data_ptr() if weight is not None else None, q4.data_ptr(), scales.data_ptr(), rows, k, shifts,
+        len(offsets), native.DTYPES[w.dtype], gathered.data_ptr(), found, torch.cuda.current_stream(w.device).cuda_stream))
+    # One read of sixteen numbers tells whether the inputs were valid and what the search did.
+    weighted_before, weighted_after, before, after, not_finite, bad_importance, grew, _, *moved = found
+    if not_finite:
+        raise ValueError("weights must be finite")
+    if bad_importance:
+        raise ValueError("importance must be k finite non-negative values")
+    if grew:
         raise AssertionError("exponent search increased a group's weighted error")
-    moved = base_scales.int() - scales.int()
     stats = {"groups": rows * (k // 32),
-             "shift_groups": {str(-s): int((moved == -s).sum()) for s in offsets},
-             "weighted_error_before": weighted_before.double().sum().item(),
-             "weighted_error_after": weighted_after.double().sum().item(),
-             "weight_error_before": before.double().sum().item(),
-             "weight_error_after": after.double().sum().item()}
+             "shift_groups": {str(-s): int(count) for s, count in zip(offsets, moved)},
+             "weighted_error_before": weighted_before,
+             "weighted_error_after": weighted_after,
+             "weight_error_before": before,
+             "weight_error_after": after}
     return q4, scales, stats

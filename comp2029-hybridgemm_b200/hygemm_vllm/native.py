@@ -42,6 +42,8 @@ POLICIES = {"serial": 0, "concurrent": 1, "high_first": 2, "high_main": 3,
             "gemv_pair1": 4, "gemv_pair2": 5, "gemv_pair4": 6}
 DTYPES = {torch.float16: 0, torch.bfloat16: 1}
 
+SPLIT_PACK_ROWS = 385024   # most rows hg_split_pack takes (its bitmap of the rows lives in shared memory)
+
 _DEFAULT_LIBRARY = Path(__file__).resolve().parent.parent / "lib" / "libhygemm_b200.so"
 _lib = None
 
@@ -68,12 +70,14 @@ def library():
         getattr(lib, name).argtypes = [vp, vp, vp, ci, ci, ci, vp]
     for name in ("hg_pack_mode", "hg_pack_mode_bf16"):
         getattr(lib, name).argtypes = [vp, vp, vp, ci, ci, ci, vp, ci]
+    lib.hg_split_pack.argtypes = [vp, vp, ci, ci, ci] + [vp] * 6 + [C.POINTER(ci), ci, vp]
     for name in ("hg_silu_pack", "hg_silu_pack_bf16"):
         getattr(lib, name).argtypes = [vp, vp, vp, vp, ci, ci, vp, ci]
     lib.hg_create.argtypes = [ci, ci, pp, pp, vp, C.POINTER(vp)]
     lib.hg_create_dtype.argtypes = [ci, ci, pp, pp, vp, ci, C.POINTER(vp)]
     lib.hg_run.argtypes = [vp, pp, pp, vp, ci]
     lib.hg_run_x.argtypes = [vp, pp, pp, vp, ci, vp]
+    lib.hg_linear.argtypes = [vp, pp, pp, vp, ci, vp, vp, vp]
     lib.hg_info.argtypes = [vp, C.POINTER(ci)]
     lib.hg_status.argtypes = [vp, vp, C.POINTER(ci)]
     lib.hg_destroy.argtypes, lib.hg_destroy.restype = [vp], None
@@ -84,6 +88,9 @@ def library():
     lib.hg_run_partial.argtypes = [vp, pp, pp, vp, ci, vp, C.c_int64, ci, vp, vp]
     lib.hg_tp_allreduce.argtypes = [C.POINTER(vp), vp, C.c_int64, C.c_int64, ci, ci, ci, C.POINTER(vp), vp, ci, vp]
     lib.hg_tp_status.argtypes = [vp, vp, C.POINTER(ci)]
+    clip = [vp, vp, vp, vp, ci, ci, C.POINTER(ci), ci, ci]
+    lib.hg_clip_pack.argtypes = clip + [vp]
+    lib.hg_clip_pack_stats.argtypes = clip + [vp, C.POINTER(C.c_double), vp]
     lib.hg_fused_error.restype = C.c_char_p
     lib.hg_fused_create.argtypes = [ci, pp, pp, vp, C.POINTER(vp)]
     lib.hg_fused_create_dtype.argtypes = [ci, pp, pp, vp, ci, C.POINTER(vp)]
@@ -107,7 +114,7 @@ def scale_size(rows: int, k: int) -> int:
 
 
 def _stream(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(device.index)
 
 
 def pack(x: torch.Tensor, fp4: bool = False):
@@ -150,16 +157,18 @@ class DualLinear:
             raise ValueError("HyGEMM weights must be a CUDA FP16/BF16 [N,K] matrix")
         self.outputs, self.k = weight.shape
         self.dtype = weight.dtype
-        selected = torch.zeros(self.outputs, dtype=torch.bool, device=weight.device)
-        selected[high_ids] = True
-        rows = torch.arange(self.outputs, device=weight.device)
-        self.hi = rows[selected].to(torch.int32)
-        self.lo = rows[~selected].to(torch.int32)
-        self.w4, self.sf4 = pack(weight.index_select(0, self.lo.long()).contiguous(), True)
-        self.w8, self.sf8 = pack(weight.index_select(0, self.hi.long()).contiguous(), False)
-        # The GEMM starts reading weights before it waits for the kernel in front of it (programmatic
-        # dependent launch), so the packed weights must be complete before the first call: load time only.
-        torch.cuda.current_stream(weight.device).synchronize()
+        if not self._pack_split(weight, high_ids):
+            # Any other selection torch can index with (a mask, a list, negative or repeated ids).
+            selected = torch.zeros(self.outputs, dtype=torch.bool, device=weight.device)
+            selected[high_ids] = True
+            rows = torch.arange(self.outputs, device=weight.device)
+            self.hi = rows[selected].to(torch.int32)
+            self.lo = rows[~selected].to(torch.int32)
+            self.w4, self.sf4 = pack(weight.index_select(0, self.lo.long()).contiguous(), True)
+            self.w8, self.sf8 = pack(weight.index_select(0, self.hi.long()).contiguous(), False)
+            # The GEMM starts reading weights before it waits for the kernel in front of it (programmatic
+            # dependent launch), so the packed weights must be complete before the first call: load time only.
+            torch.cuda.current_stream(weight.device).synchronize()
         self.low_id, self.high_id, self.concurrent = low_id, high_id, concurrent
         self.handles = {}
         self.fused_handles = {}
@@ -167,28 +176,63 @@ class DualLinear:
         self.plans = plans
         self.plans_used = {}
         self._problems = {}
+        self._ready = {}   # token count -> what a plain call needs, see _prepare
+
+    def _pack_split(self, weight, high_ids) -> bool:
+        """Both partitions from one pass over the 16-bit matrix (`hg_split_pack`).  True when the selection was a CUDA
+        tensor of distinct row numbers, the form every loader of this package passes; the call waits for the packing
+        (the GEMM reads weights before it waits for the kernel in front of it) and tells whether it was."""
+        n, k = weight.shape
+        if not (torch.is_tensor(high_ids) and high_ids.dtype == torch.int64 and high_ids.ndim == 1 and weight.is_cuda
+                and high_ids.device == weight.device and high_ids.is_contiguous() and weight.is_contiguous()
+                and weight.data_ptr() % 32 == 0
+                and k % 128 == 0 and k and 0 < n <= SPLIT_PACK_ROWS and high_ids.numel() <= n):
+            return False
+        high = high_ids.numel()
+        low = n - high
+
+        def empty(*shape, dtype=torch.uint8):
+            return torch.empty(shape, dtype=dtype, device=weight.device)
+        self.hi, self.lo = empty(high, dtype=torch.int32), empty(low, dtype=torch.int32)
+        self.w4, self.sf4 = empty(low, k // 2), empty(scale_size(low, k))
+        self.w8, self.sf8 = empty(high, k), empty(scale_size(high, k))
+        found = (C.c_int * 2)()
+        check(library().hg_split_pack(weight.data_ptr(), high_ids.data_ptr(), high, n, k, self.lo.data_ptr(), self.hi.data_ptr(),
+                                      self.w4.data_ptr(), self.sf4.data_ptr(), self.w8.data_ptr(), self.sf8.data_ptr(),
+                                      found, DTYPES[weight.dtype], _stream(weight.device)))
+        return tuple(found) == (high, 0)
 
     def __call__(self, x):
-        if x.ndim != 2 or x.shape[1] != self.k or x.device != self.w4.device:
+        shape = x.shape
+        if len(shape) != 2 or shape[1] != self.k or x.device != self.w4.device:
             raise ValueError("HyGEMM input shape/device does not match its weights")
-        if 0 < x.shape[0] <= FUSED_QUANT_TOKENS and x.dtype in DTYPES and x.is_contiguous() and not self.plans \
-                and not 28 <= self.low_id <= 34 and self.outputs <= FUSED_QUANT_MAX_OUTPUTS:
-            return self._run_fused(x)
-        q, sf = pack(x)
-        return self.run_packed(q, sf)
-
-    def _run_fused(self, x):
-        """Decode path: activation quantisation inside the GEMM launch (`hg_run_x`)."""
-        tokens = x.shape[0]
-        y = torch.empty((tokens, self.outputs), dtype=self.dtype, device=x.device)
-        low, high, _, low_ref, high_ref = self._rebound(tokens, x, x, y)
-        stream = _stream(x.device)
-        handle = self._handle(tokens, self.low_id, self.high_id, low_ref, high_ref, stream)
-        status = _lib.hg_run_x(handle, low_ref, high_ref, x.data_ptr(), DTYPES[x.dtype], stream)
+        tokens = shape[0]
+        dtype = DTYPES.get(x.dtype)
+        if not tokens or dtype is None or self.plans or PACK_MODE or not x.is_contiguous() or 28 <= self.low_id <= 34:
+            return self.run_packed(*pack(x))
+        # One foreign call for the whole layer: decode sizes quantise inside the GEMM launch, others into a workspace.
+        # (Fresh tensors per call: under CUDA-graph capture the graph's pool owns them.)
+        ready = self._ready.get(tokens)
+        if ready is None or ready[0] is not self.w4 or ready[1] is not self.sf4 or ready[2] != (self.low_id, self.high_id):
+            ready = self._prepare(tokens, x)
+        y = ready[7].new_empty((tokens, self.outputs))
+        workspace = self.w4.new_empty(ready[6]) if ready[6] else None
+        status = _lib.hg_linear(ready[3], ready[4], ready[5], x.data_ptr(), dtype, workspace.data_ptr() if ready[6] else None,
+                                y.data_ptr(), torch._C._cuda_getCurrentRawStream(x.device.index))
         if status:
             check(status)
         self.calls[tokens] = self.calls.get(tokens, 0) + 1
         return y
+
+    def _prepare(self, tokens, x):
+        """Handle, operand structs and workspace size of plain calls with this token count, kept between calls."""
+        y = torch.empty((tokens, self.outputs), dtype=self.dtype, device=x.device)
+        low, high, _, low_ref, high_ref = self._rebound(tokens, x, x, y)
+        handle = self._handle(tokens, self.low_id, self.high_id, low_ref, high_ref, _stream(x.device))
+        fused = tokens <= FUSED_QUANT_TOKENS and self.outputs <= FUSED_QUANT_MAX_OUTPUTS
+        ready = self._ready[tokens] = (self.w4, self.sf4, (self.low_id, self.high_id), handle, low_ref, high_ref,
+                                       0 if fused else tokens * self.k + scale_size(tokens, self.k), y.new_empty(0))
+        return ready
 
     def _handle(self, tokens, low_id, high_id, low_ref, high_ref, stream):
         """GEMM handle of one (token count, schedule ids) pair, created on first use: never during stream
@@ -314,6 +358,7 @@ class DualLinear:
         for handle in self.handles.values():
             library().hg_destroy(handle)
         self.handles.clear()
+        self._ready.clear()
         for handle in self.fused_handles.values():
             library().hg_fused_destroy(handle)
         self.fused_handles.clear()
