@@ -4,6 +4,10 @@
 schemas (quantization.py:18-25, producer.py:27-40 of the reference): the layer
 runtime is looked up by an integer handle in `_runtimes`, nothing is mutated,
 and the fake implementations give shape/dtype for tracing.
+
+The ops are registered with the dispatcher directly, and the functions `linear` and `linear_silu` of this module only go
+through it where something may be watching (tracing, dispatch modes, tensor subclasses, autograd): an eager call
+of an op registered with `torch.library.custom_op` costs about as much host time as the layer itself.
 """
 from __future__ import annotations
 
@@ -18,18 +22,15 @@ def register_runtime(runtime) -> int:
     return handle
 
 
-@torch.library.custom_op("hygemm_vllm::linear", mutates_args=())
-def linear(x: torch.Tensor, handle: int, outputs: int) -> torch.Tensor:
+def _linear(x: torch.Tensor, handle: int, outputs: int) -> torch.Tensor:
     return _runtimes[handle](x)
 
 
-@linear.register_fake
 def _linear_fake(x, handle, outputs):
     return x.new_empty((x.shape[0], outputs))
 
 
-@torch.library.custom_op("hygemm_vllm::linear_silu", mutates_args=())
-def linear_silu(x: torch.Tensor, handle: int, outputs: int, math: int) -> torch.Tensor:
+def _linear_silu(x: torch.Tensor, handle: int, outputs: int, math: int) -> torch.Tensor:
     from .producer import silu_pack
     runtime = _runtimes[handle]
     if hasattr(runtime, "profile_name") and torch.cuda.is_current_stream_capturing():
@@ -41,6 +42,26 @@ def linear_silu(x: torch.Tensor, handle: int, outputs: int, math: int) -> torch.
     return runtime.run_packed(*silu_pack(x, math))
 
 
-@linear_silu.register_fake
 def _linear_silu_fake(x, handle, outputs, math):
     return x.new_empty((x.shape[0], outputs))
+
+
+_library = torch.library.Library("hygemm_vllm", "DEF")
+for _name, _function, _fake in (("linear", _linear, _linear_fake), ("linear_silu", _linear_silu, _linear_silu_fake)):
+    _library.define(_name + torch.library.infer_schema(_function, mutates_args=()))
+    _library.impl(_name, _function, "CompositeExplicitAutograd")
+    torch.library.register_fake(f"hygemm_vllm::{_name}", _fake, lib=_library)
+
+
+def _plain(x) -> bool:
+    """An eager call on an ordinary tensor that nothing traces, intercepts or differentiates."""
+    return (not torch.compiler.is_compiling() and type(x) is torch.Tensor and not x.requires_grad
+            and not torch._C._len_torch_dispatch_stack())
+
+
+def linear(x: torch.Tensor, handle: int, outputs: int) -> torch.Tensor:
+    return _runtimes[handle](x) if _plain(x) else torch.ops.hygemm_vllm.linear(x, handle, outputs)
+
+
+def linear_silu(x: torch.Tensor, handle: int, outputs: int, math: int) -> torch.Tensor:
+    return _linear_silu(x, handle, outputs, math) if _plain(x) else torch.ops.hygemm_vllm.linear_silu(x, handle, outputs, math)
