@@ -7,24 +7,23 @@
 //   fp32 partials to the shared memory of the CTAs that own the columns, and the owners add them in K order.
 //   No workspace, no ticket, no second launch: the chain store -> ticket -> load through global memory that ended
 //   a cut tile cost 3.5 us, the exchange between neighbours about one.
-// * Row tiles of any height up to 128.  Weights, their scales and the channel map are addressed by row, so tile
-//   heights are chosen such that every CTA gets the same number of weight bytes (an MXFP8 tile has half the rows
-//   of an MXFP4 tile while weights stream from HBM).
-// * cta_group::2 above 64 tokens.  Two CTAs form one 256-row tile; each stages its own 128 weight rows and HALF of the
-//   activation tile.  At 128 tokens the shared-memory traffic per K128 block falls from 448 to 320 cycles, and
-//   256-token tiles (prefill) run at 512 cycles, the tensor core's own time.
-// * 256-token accumulators overlap.  TMEM holds two of them only if they share 32 columns; the epilogue drains
-//   those first and hands them over, so the main loop of the next tile starts about 0.3 us after the last one ended.
+// * Weights by TMA.  MXFP4 rows through the tensor map type 16U4_ALIGN16B, which unpacks sixteen codes into the first half of
+//   each swizzled 16-byte chunk, the 8-bit container the f8f6f4 kinds read: one instruction brings a K256 slice of a tile, no
+//   thread touches the weights and nothing passes through L1.  Alone it streams at 6.3 TB/s (61 MB, 148 SMs).  8-byte
+//   cp.async from loader warps needs a line of L1 for every line in flight, and beside 228 KB of shared memory only 28 KB
+//   of L1 are left: the same loop was 3 us slower on gate_up with the larger carve-out.
+// * Row tiles of 128, 64 or 32 rows, always inside one 128-row scale atom.  The ring holds only the rows a tile loads; the MMA
+//   still reads 128, from the address at which the atom's first row would lie, and the accumulator lanes of rows
+//   that were not loaded are never read.
 //
-// Roles per CTA: warp 0 activations and their scales (TMA), warp 1 MMA issue (in the second CTA of a pair: tells the
-// first that a stage is full), warps 2-9 epilogue (two per TMEM quarter, on alternate groups of sixteen columns),
-// warps 10-17 (FUSED 10-13) weights and weight scales (cp.async: MXFP4 codes go in 8-byte granules into the first half of each
-// swizzled 16-byte chunk, the 8-bit container the f8f6f4 kinds read; MXFP8 codes as 16-byte chunks; scales as the 4-byte
-// words of the row), warps 14-17 (FUSED) activation quantisers.
+// Roles per CTA: warp 0 weights and their scales (TMA), warp 1 MMA issue (idle in the second CTA of a pair, whose copies
+// complete on the first CTA's barriers: reporting every stage with a remote arrive cost 750 cycles each), then epilogue warps (four; in pairs eight, two per TMEM quarter on alternate groups of sixteen columns),
+// then one warp for the activations and their scales (TMA) or, FUSED, four warps that quantise the activations.
 // One warp per scheduler runs most of these roles alone, so a dependent instruction costs about five cycles and nothing
 // hides it: loops here carry no divisions, addresses are independent of each other, and descriptors are sums.
 // Every mbarrier wait is bounded; on expiry the CTA records a code, drains and leaves.
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -36,24 +35,24 @@ namespace hg {
 
 namespace {
 
-constexpr int kFirstLoader = 10;                // warps 0-9: see above
-constexpr int kLoaderTeams = 4;                 // each brings in a whole K256 stage
-__host__ __device__ constexpr int team_warps(bool fused) { return fused ? 1 : 2; }   // 18 warps leave 113 registers a thread, with quantisers as well
-__host__ __device__ constexpr int first_quantiser(bool fused) { return kFirstLoader + kLoaderTeams * team_warps(fused); }
-__host__ __device__ constexpr int cluster_threads(bool fused) { return first_quantiser(fused) * 32 + (fused ? kQuantThreads : 0); }
-constexpr int kClusterMaxStages = 6;
+__host__ __device__ constexpr int epilogue_sides(int pair) { return pair == 2 ? 2 : 1; }
+__host__ __device__ constexpr int first_act_warp(int pair) { return 2 + 4 * epilogue_sides(pair); }
+__host__ __device__ constexpr int cluster_threads(int pair, bool fused) { return first_act_warp(pair) * 32 + (fused ? kQuantThreads : 32); }
+constexpr int kClusterMaxStages = 12;
 constexpr int kMaxSmem = 232448;
 constexpr uint32_t kScaleStride = 16;                           // TMEM columns per scale set: weights 4, activations up to 8
 
 struct ClusterParams {
-  int rows[2], tile_rows[2], tiles[2];
-  const uint8_t* weight[2];
+  int rows[2], cut_log[2], tiles[2];   // a 128-row atom (PAIR: two) is cut into 2^cut_log tiles
+  int slot_rows, least_rows;           // height of the taller and of the shorter tiles
   const uint8_t* sfa[2];
   const int32_t* ids[2];
   const uint8_t* sfb;
   OutTargets out;
   int outputs, tokens, k, kblocks;
   int n_tile, n_tail, token_tiles, stages, split, split_log, share_log, clusters;
+  int async_push;      // partials travel by st.async
+  int ring_exchange;   // partials are exchanged in the ring, which is idle by then (a cluster that splits K has one unit)
   int acc_shift, overlap;
   uint64_t by_token_tiles, by_tiles;   // see fast_div
   uint32_t tmem_cols;
@@ -73,25 +72,39 @@ __host__ __device__ inline int share_log_of(int n_tile, int split) {
   return log;
 }
 
-// A pipeline stage covers two K128 blocks (K256): 2 x 16 KiB of weights in the 8-bit container, two activation tiles,
-// two scale atoms of the weights and two per 128 tokens of the activations.
+// A pipeline stage covers two K128 blocks (K256): two weight tiles of slot_rows x 128 B in the 8-bit container, two
+// activation tiles, two scale atoms of the weights and two per 128 tokens of the activations.
 struct ClusterSmem {
-  uint32_t b, sfa, sfb, red, bars;  // byte offsets from the 1024-aligned base; the weight stages start at 0
-  uint32_t b_tile;                  // bytes of one K128 activation tile
-  uint32_t sfb_stage;               // bytes of the activation scales of a stage: per 128 tokens two atoms
+  uint32_t b, sfa, sfb, a, red, bars, end;  // byte offsets from the 1024-aligned base; activations start at 0
+  uint32_t a_tile, b_tile;                  // bytes of one K128 block
+  uint32_t sfb_stage;                       // bytes of the activation scales of a stage: per 128 tokens two atoms
 };
-__host__ __device__ inline ClusterSmem cluster_smem(int stages, int n_tile, int pair, int split) {
+__host__ __device__ inline ClusterSmem cluster_smem(int stages, int n_tile, int pair, int split, int slot_rows, int least_rows, int ring_exchange) {
   ClusterSmem s;
+  s.a_tile = uint32_t(slot_rows) * 128u;
   s.b_tile = uint32_t(n_tile / pair) * 128u;
   s.sfb_stage = uint32_t((n_tile + 127) / 128) * 1024u;
-  s.b = uint32_t(stages) * 32768u;
-  s.sfa = s.b + uint32_t(stages) * 2u * s.b_tile;
+  s.b = 0;
+  s.sfa = uint32_t(stages) * 2u * s.b_tile;
   s.sfb = s.sfa + uint32_t(stages) * 1024u;
-  s.red = s.sfb + uint32_t(stages) * s.sfb_stage;
-  s.bars = s.red + (split > 1 ? uint32_t(split << share_log_of(n_tile, split)) * 2048u : 0u);
+  s.a = s.sfb + uint32_t(stages) * s.sfb_stage;
+  // An MMA reads the 128 rows of the whole atom: up to 128 - least_rows before the ring, up to 128 - slot_rows behind it.
+  const uint32_t before = uint32_t(128 - least_rows) * 128u, behind = uint32_t(128 - slot_rows) * 128u;
+  if (s.a < before) s.a = before;
+  s.a = (s.a + 1023u) & ~1023u;
+  s.red = s.a + uint32_t(stages) * 2u * s.a_tile;
+  const uint32_t exchange = split > 1 ? uint32_t(split << share_log_of(n_tile, split)) * 2048u : 0u;
+  s.bars = s.red + exchange;
+  if (ring_exchange) {
+    s.bars = s.a + exchange > s.red ? s.a + exchange : s.red;
+    s.red = s.a;
+  }
+  s.end = s.bars + uint32_t((2 * 12 + 8) * 8 + 32);
+  const uint32_t read_end = s.a + uint32_t(stages) * 2u * s.a_tile + behind;
+  if (s.end < read_end) s.end = read_end;
   return s;
 }
-constexpr int kClusterBarBytes = (3 * kClusterMaxStages + 8) * 8 + 32;
+static_assert(kClusterMaxStages == 12, "the barrier block of cluster_smem holds twelve stages");
 
 template <int PAIR> __device__ __forceinline__ void cg_alloc(uint32_t slot, uint32_t cols) {
   if constexpr (PAIR == 1) {
@@ -134,6 +147,22 @@ __device__ __forceinline__ void cg_mma(uint32_t d, uint64_t a, uint64_t b, uint3
 constexpr uint32_t kDescTile = (1024u >> 4) | (1u << 14) | (kSwizzle128B << 29), kDescScales = (128u >> 4) | (1u << 14);
 __device__ __forceinline__ uint64_t desc_of(uint32_t low, uint32_t high) { return uint64_t(low) | (uint64_t(high) << 32); }
 
+// Copies into this CTA's shared memory; in a pair `bar` is a cluster address and may lie in either CTA.
+template <int PAIR>
+__device__ __forceinline__ void cg_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
+  if constexpr (PAIR == 1) tma_load_3d(dst, map, bar, x, y, z);
+  else
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
+}
+// Two consecutive 512-byte scale atoms, `row` counted in atoms from the start of the buffer.
+__device__ __forceinline__ void load_scales_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int row) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(0), "r"(row) : "memory");
+}
+
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -150,17 +179,15 @@ __device__ __forceinline__ void arrive_remote(uint32_t cluster_addr) {
 __device__ __forceinline__ void store_remote(uint32_t cluster_addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
   asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
+// 16 bytes to another CTA's shared memory; their arrival counts on a barrier there, so no fence and no second message.
+__device__ __forceinline__ void store_async(uint32_t cluster_addr, uint32_t cluster_bar, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%2, %3, %4, %5}, [%1];"
+               ::"r"(cluster_addr), "r"(cluster_bar), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
-
 // n / d with inverse = ceil(2^40 / d), exact while n d < 2^40; the host passes 0 where that or the product does not fit.
 __device__ __forceinline__ int fast_div(int64_t n, int d, uint64_t inverse) {
   return inverse ? int((uint64_t(n) * inverse) >> 40) : int(n / d);
@@ -171,13 +198,14 @@ __device__ __forceinline__ int fast_div(int64_t n, int d, uint64_t inverse) {
 // token tiles they are spread evenly among the MXFP4 tiles, so that the two partitions of a channel range (both sorted)
 // are stored at about the same time and meet in L2: an MXFP8 tile writes one or two channels of nearly every sector.
 struct Unit {
-  int part, tile, token0, n;
+  int part, atom, first, last, token0, n;   // rows first .. last - 1 of the 128-row atom (PAIR: of atoms 2 atom and 2 atom + 1)
 };
 __device__ __forceinline__ Unit unit_at(const ClusterParams& p, int u) {
   Unit w;
+  int tile;
   if (p.token_tiles == 1) {
     w.part = u < p.tiles[1];
-    w.tile = w.part ? u : u - p.tiles[1];
+    tile = w.part ? u : u - p.tiles[1];
     w.token0 = 0;
     w.n = p.n_tail;
   } else {
@@ -185,35 +213,43 @@ __device__ __forceinline__ Unit unit_at(const ClusterParams& p, int u) {
     const int high_before = fast_div(int64_t(t) * p.tiles[1], total, p.by_tiles);
     const int high_after = fast_div(int64_t(t + 1) * p.tiles[1], total, p.by_tiles);
     w.part = high_after > high_before;
-    w.tile = w.part ? high_before : t - high_before;
+    tile = w.part ? high_before : t - high_before;
     w.token0 = tt * p.n_tile;
     w.n = tt == p.token_tiles - 1 ? p.n_tail : p.n_tile;
   }
+  const int log = p.cut_log[w.part], height = kTileRows >> log;
+  w.atom = tile >> log;
+  w.first = (tile & ((1 << log) - 1)) * height;
+  w.last = w.first + height;
   return w;
 }
 
+// 128-row atoms a unit starts: what the audit counters count.
+template <int PAIR>
+__device__ __forceinline__ int atoms_started(const ClusterParams& p, const Unit& w) {
+  return w.first ? 0 : min(PAIR, ((p.rows[w.part] + kTileRows - 1) >> 7) - w.atom * PAIR);
+}
+
 template <typename T, int PAIR, bool FUSED>
-__global__ void __launch_bounds__(cluster_threads(FUSED), 1)
-cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_constant__ CUtensorMap map_act,
-                    const __grid_constant__ CUtensorMap map_tail) {
-  pdl_trigger();
+__global__ void __launch_bounds__(cluster_threads(PAIR, FUSED), 1)
+cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_constant__ ClusterMaps maps) {
   if (threadIdx.x == 0) HG_STAMP(0);
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
-  const ClusterSmem lay = cluster_smem(p.stages, p.n_tile, PAIR, p.split);
+  const ClusterSmem lay = cluster_smem(p.stages, p.n_tile, PAIR, p.split, p.slot_rows, p.least_rows, p.ring_exchange);
   const uint32_t bars = base + lay.bars;
   auto full_bar = [&](int s) { return bars + uint32_t(s) * 8u; };
   auto empty_bar = [&](int s) { return bars + uint32_t(kClusterMaxStages + s) * 8u; };
-  auto peer_bar = [&](int s) { return bars + uint32_t(2 * kClusterMaxStages + s) * 8u; };   // pair: the second CTA's stage is full
-  auto acc_full_bar = [&](int s) { return bars + uint32_t(3 * kClusterMaxStages + s) * 8u; };
-  auto acc_empty_bar = [&](int s) { return bars + uint32_t(3 * kClusterMaxStages + 2 + s) * 8u; };
-  const uint32_t red_full = bars + uint32_t(3 * kClusterMaxStages + 4) * 8u;    // every slice's partials of this share are here
-  const uint32_t red_empty = bars + uint32_t(3 * kClusterMaxStages + 5) * 8u;   // every slice has summed its share
-  const uint32_t drain_bar = bars + uint32_t(3 * kClusterMaxStages + 6) * 8u;
-  volatile int* words = reinterpret_cast<volatile int*>(base_ptr + lay.bars + (3 * kClusterMaxStages + 8) * 8);
+  auto acc_full_bar = [&](int s) { return bars + uint32_t(2 * kClusterMaxStages + s) * 8u; };
+  auto acc_empty_bar = [&](int s) { return bars + uint32_t(2 * kClusterMaxStages + 2 + s) * 8u; };
+  const uint32_t red_full = bars + uint32_t(2 * kClusterMaxStages + 4) * 8u;    // every slice's partials of this share are here
+  const uint32_t red_empty = bars + uint32_t(2 * kClusterMaxStages + 5) * 8u;   // every slice's ring is idle
+  const uint32_t drain_bar = bars + uint32_t(2 * kClusterMaxStages + 6) * 8u;
+  volatile int* words = reinterpret_cast<volatile int*>(base_ptr + lay.bars + (2 * kClusterMaxStages + 8) * 8);
   volatile int* abort_flag = words + 1;
 
+  constexpr int kSides = epilogue_sides(PAIR), kActWarp = first_act_warp(PAIR);
   const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int cluster_ctas = PAIR * p.split;
   const int rank = cluster_ctas == 1 ? 0 : int(cluster_rank());
@@ -222,21 +258,23 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
   const int slice = PAIR == 2 ? rank >> 1 : rank;
 
   if (threadIdx.x == 0) {
+    if (p.tiles[0]) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.low)) : "memory");
+    if (p.tiles[1]) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.high)) : "memory");
     if (!FUSED) {
-      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_act)) : "memory");
-      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_tail)) : "memory");
+      if (PAIR == 2) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.act_scales)) : "memory");
+      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.act)) : "memory");
+      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.tail)) : "memory");
     }
     for (int s = 0; s < p.stages; ++s) {
-      mbar_init(full_bar(s), 32 * team_warps(FUSED) + (FUSED ? kQuantThreads / 32 : 1));   // the lanes of one loader team; quantiser warps or the TMA thread
+      mbar_init(full_bar(s), 1 + (FUSED ? kQuantThreads / 32 : 1));   // weights; activations or the quantiser warps
       mbar_init(empty_bar(s), 1);
-      mbar_init(peer_bar(s), 1);
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(acc_full_bar(s), 1);
-      mbar_init(acc_empty_bar(s), 8 * PAIR);
+      mbar_init(acc_empty_bar(s), 4 * kSides * PAIR);
     }
-    mbar_init(red_full, uint32_t(8 * p.split));
-    mbar_init(red_empty, uint32_t(8 * p.split));
+    mbar_init(red_full, p.async_push ? 1u : uint32_t(4 * kSides * p.split));   // one thread, with the bytes to come; or every warp
+    mbar_init(red_empty, uint32_t(4 * kSides * p.split));
     mbar_init(drain_bar, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -248,6 +286,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
   if (cluster_ctas > 1) cluster_sync();   // barriers of every CTA are initialised before anyone arrives remotely
   else __syncthreads();
   tc_fence_after();
+  pdl_trigger();
   const uint32_t tmem_base = uint32_t(*words);
   if (threadIdx.x == 0) HG_STAMP(1);
 
@@ -258,13 +297,45 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
   int error = 0;
 
   if (warp == 0) {
+    // ------------------------------------------------------------------ weights and their scales (TMA)
+    // They were complete before the first launch (hg_run), so this stream does not wait for the kernel in front.  The warp
+    // walks the loop together and an elected lane issues: behind a `lane == 0` branch every copy took 80 cycles to issue.
+    const uint32_t smem0 = __shfl_sync(0xffffffffu, base, 0);
+    const uint32_t bars0 = PAIR == 1 ? smem0 + lay.bars : __shfl_sync(0xffffffffu, map_to_rank(bars, uint32_t(rank & ~1)), 0);
+    int stage = 0;
+    uint32_t phase = 1;
+    for (int u = cluster; u < units && !error; u += p.clusters) {
+      const Unit w = unit_at(p, u);
+      const int atom = w.atom * PAIR + half;
+      const uint8_t* sfa_src = p.sfa[w.part] + int64_t(atom) * p.kblocks * 512;
+      const int row = atom * kTileRows + w.first;
+      const uint32_t weight_bytes = uint32_t(w.last - w.first) * (w.part ? 256u : 128u);
+      for (int step = step_begin; step < step_end; ++step) {
+        const int kb = 2 * step, nkb = min(2, p.kblocks - kb);
+        if (!warp_wait(empty_bar(stage), phase, abort_flag)) { error = kErrLoader; break; }
+        if (elect_one()) {
+          const uint32_t bar = bars0 + uint32_t(stage) * 8u, dst = smem0 + lay.a + uint32_t(2 * stage) * lay.a_tile;
+          const uint32_t scales = smem0 + lay.sfa + uint32_t(stage) * 1024u;
+          // Rows and blocks beyond the matrix arrive as zeros.  In a pair the first CTA expects both CTAs' bytes.
+          if (PAIR == 1) mbar_expect_tx(bar, weight_bytes + uint32_t(nkb) * 512u);
+          else if (half == 0) mbar_expect_tx(full_bar(stage), 2u * (weight_bytes + 1024u));
+          if (w.part) cg_load_3d<PAIR>(dst, &maps.high, bar, 0, row, kb);
+          else cg_load_3d<PAIR>(dst, &maps.low, bar, 0, row, kb);
+          if (PAIR == 1) bulk_load(scales, sfa_src + int64_t(kb) * 512, uint32_t(nkb) * 512u, bar);
+          else load_scales_pair(scales, w.part ? &maps.high_scales : &maps.low_scales, bar, atom * p.kblocks + kb);
+        }
+        __syncwarp();
+        if (++stage == p.stages) { stage = 0; phase ^= 1u; }
+      }
+    }
+  } else if (!FUSED && warp == kActWarp) {
     // ------------------------------------------------------------------ activations and their scales (TMA)
-    // The warp walks the loop together and an elected lane issues: behind a `lane == 0` branch the four copies of a stage
-    // took 300 cycles to issue.  One copy brings both K128 blocks (the map's third dimension counts them).
+    // One copy brings both K128 blocks (the map's third dimension counts them).
     if (!FUSED) {
-      pdl_wait();   // they are the previous kernel's output; the weight stream below is not and already runs
+      pdl_wait();   // they are the previous kernel's output; the weight stream is not and already runs
       if (lane == 0) HG_STAMP(2);
-      const uint32_t smem0 = __shfl_sync(0xffffffffu, base, 0), bars0 = smem0 + lay.bars;
+      const uint32_t smem0 = __shfl_sync(0xffffffffu, base, 0);
+      const uint32_t bars0 = PAIR == 1 ? smem0 + lay.bars : __shfl_sync(0xffffffffu, map_to_rank(bars, uint32_t(rank & ~1)), 0);
       const int atoms = (p.tokens + 127) >> 7;
       int stage = 0;
       uint32_t phase = 1;
@@ -279,87 +350,29 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
           if (!warp_wait(empty_bar(stage), phase, abort_flag)) { error = kErrProducer; break; }
           if (elect_one()) {
             const uint32_t bar = bars0 + uint32_t(stage) * 8u, dst = smem0 + lay.b + uint32_t(2 * stage) * lay.b_tile;
-            mbar_expect_tx(bar, uint32_t(w.n / PAIR) * 256u + uint32_t(n_atoms * nkb) * 512u);   // a block beyond K arrives as zeros
+            if (PAIR == 1) mbar_expect_tx(bar, uint32_t(w.n) * 256u + uint32_t(n_atoms * nkb) * 512u);   // a block beyond K arrives as zeros
+            else if (half == 0) mbar_expect_tx(full_bar(stage), 2u * (uint32_t(w.n / 2) * 256u + uint32_t(n_atoms) * 1024u));
             // a short last token tile has a box of its own: its second block follows the first directly
-            if (whole) tma_load_3d(dst, &map_act, bar, 0, row, kb);
-            else tma_load_3d(dst, &map_tail, bar, 0, row, kb);
-            for (int a = 0; a < n_atoms; ++a)
-              bulk_load(smem0 + lay.sfb + uint32_t(stage) * lay.sfb_stage + uint32_t(a) * 1024u,
-                        sfb_src + (int64_t(a) * p.kblocks + kb) * 512, uint32_t(nkb) * 512u, bar);
+            if (whole) cg_load_3d<PAIR>(dst, &maps.act, bar, 0, row, kb);
+            else cg_load_3d<PAIR>(dst, &maps.tail, bar, 0, row, kb);
+            for (int a = 0; a < n_atoms; ++a) {
+              const uint32_t scales = smem0 + lay.sfb + uint32_t(stage) * lay.sfb_stage + uint32_t(a) * 1024u;
+              if (PAIR == 1) bulk_load(scales, sfb_src + (int64_t(a) * p.kblocks + kb) * 512, uint32_t(nkb) * 512u, bar);
+              else load_scales_pair(scales, &maps.act_scales, bar, (first_atom + a) * p.kblocks + kb);
+            }
           }
           __syncwarp();
           if (++stage == p.stages) { stage = 0; phase ^= 1u; }
         }
       }
     }
-  } else if (warp >= kFirstLoader && warp < first_quantiser(FUSED)) {
-    // ------------------------------------------------------------------ weights and their scales (cp.async)
-    // Loader team t of L (two warps that share the rows) brings in every L-th K256 step, whole.  Sixteen lanes cover a full 128- or 256-byte run of a row,
-    // so lane l owns granule l % 16 (8 bytes of MXFP4 or 16 bytes of MXFP8 codes) of rows l / 16 + 2 i; for the scales
-    // it owns rows l + 32 j.  A team per step keeps the arrivals on a stage barrier at 64: they serialise there, and
-    // 128 threads that each arrived for both blocks of a step cost more than the copies.  One warp per team was too
-    // slow to refill a three-stage ring: a stage is 72 copies, and their issue counts against the ring's round trip.
-    // L is at most the ring depth S.  The warp of step s + 2 S has seen step s + S - L consumed (its previous wait), so
-    // with L <= S step s has been consumed too and the stage's barrier is past the phase whose parity that wait
-    // would mistake for its own.
-    constexpr int kTeam = team_warps(FUSED);
-    const int lw = (warp - kFirstLoader) / kTeam, sub = (warp - kFirstLoader) % kTeam, m = lane & 15, rsub = lane >> 4, blk = m >> 3;
-    uint32_t swz[4];   // swizzled chunk of rows rsub + 2 i, by i % 4
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      swz[i] = uint32_t(blk) * 16384u + uint32_t(rsub + 2 * i) * 128u + (uint32_t((m & 7) ^ (rsub + 2 * i)) << 4);
-    const int loaders = min(kLoaderTeams, p.stages);
-    int stage = lw, ahead = lw;   // ahead: steps from here to this warp's next one
-    uint32_t phase = 1;
-    for (int u = cluster; u < units && !error && lw < loaders; u += p.clusters) {
-      const Unit w = unit_at(p, u);
-      const int row0 = (w.tile * PAIR + half) * p.tile_rows[w.part];
-      const int rows = min(p.tile_rows[w.part], p.rows[w.part] - row0);   // may be <= 0: nothing to load, the stages still turn
-      const int pitch = w.part ? p.k : p.k >> 1;
-      const uint8_t* src0 = p.weight[w.part] + int64_t(row0 + rsub) * pitch + m * (w.part ? 16 : 8);
-      const uint8_t* sf_part = p.sfa[w.part];
-      int step = step_begin + ahead;
-      for (; step < step_end; step += loaders) {
-        const int kb = 2 * step, nkb = min(2, p.kblocks - kb);
-        if (!warp_wait(empty_bar(stage), phase, abort_flag)) { error = kErrLoader; break; }
-        const uint32_t dst = base + uint32_t(stage) * 32768u;
-        if (blk < nkb) {
-          const uint8_t* src = src0 + int64_t(kb) * (w.part ? 128 : 64);
-          if (w.part) {
-#pragma unroll 4
-            for (int i = sub; i < 16; i += kTeam)
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                if (rsub + 8 * i + 2 * j < rows) cp_async_16(dst + uint32_t(i) * 1024u + swz[j], src + int64_t(pitch) * (8 * i + 2 * j));
-          } else {
-#pragma unroll 4
-            for (int i = sub; i < 16; i += kTeam)
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                if (rsub + 8 * i + 2 * j < rows) cp_async_8(dst + uint32_t(i) * 1024u + swz[j], src + int64_t(pitch) * (8 * i + 2 * j), 8u);
-          }
-        }
-#pragma unroll
-        for (int j = sub; j < 4; j += kTeam) {
-          const int row = row0 + lane + 32 * j;
-          if (lane + 32 * j < rows)
-            for (int i = 0; i < nkb; ++i)
-              cp_async_4(base + lay.sfa + uint32_t(2 * stage + i) * 512u + uint32_t(lane) * 16u + uint32_t(j) * 4u,
-                         sf_part + (int64_t(row >> 7) * p.kblocks + kb + i) * 512 + (row & 31) * 16 + ((row & 127) >> 5) * 4);
-        }
-        cp_async_arrive(full_bar(stage));
-        if ((stage += loaders) >= p.stages) { stage -= p.stages; phase ^= 1u; }
-      }
-      ahead = step - step_end;
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");   // copies in flight must land before shared memory is released
-  } else if (FUSED && warp >= first_quantiser(FUSED)) {
+  } else if (FUSED && warp >= kActWarp) {
     // ------------------------------------------------------------------ activation quantisers
     // Thread tq owns one K32 group (tq % 8) of token tq / 8 in each K256 step, with the arithmetic of mx_quant_kernel:
     // codes and scales are the bytes hg_pack would have produced.  The next step's 64 bytes are requested before the
     // current ones are converted.
     if constexpr (FUSED) {
-      const int tq = threadIdx.x - first_quantiser(FUSED) * 32;
+      const int tq = threadIdx.x - kActWarp * 32;
       const int token = tq >> 3, blk = (tq & 7) >> 2, g = tq & 3;
       const uint16_t* x_row = p.x + int64_t(token) * p.k + blk * 128 + g * 32;
       auto load_x = [&](int kb, uint4 (&r)[4]) {
@@ -381,7 +394,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
         for (int step = step_begin; step < step_end; ++step) {
           load_x(step + 1 < step_end ? 2 * step + 2 : 2 * step_begin, nxt);
           if (!warp_wait(empty_bar(stage), phase, abort_flag)) { error = kErrLoader; break; }
-          if (2 * step + blk < p.kblocks) {
+          if (2 * step + blk < p.kblocks && token < p.tokens) {   // columns of tokens that are not there are never stored
             const uint32_t row_base = base + lay.b + uint32_t(2 * stage + blk) * lay.b_tile + uint32_t(token) * 128u;
             const uint32_t sw = uint32_t(token & 7);
             float v[32];
@@ -424,7 +437,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
       const uint32_t sf0 = __shfl_sync(0xffffffffu, sf_cols, 0);
       const uint16_t pair_mask = uint16_t(3u << (rank & ~1));
       // low words of the shared-memory descriptors of stage 0; a stage is a constant number of 16-byte units further on
-      const uint32_t a_desc = smem0 >> 4, b_desc = (smem0 + lay.b) >> 4, b_stage = lay.b_tile >> 3;
+      const uint32_t a_desc = (smem0 + lay.a) >> 4, a_stage = lay.a_tile >> 3, b_desc = smem0 >> 4, b_stage = lay.b_tile >> 3;
       const uint32_t sfa_desc = (smem0 + lay.sfa) >> 4, sfb_desc = (smem0 + lay.sfb) >> 4, sfb_stage = lay.sfb_stage >> 4;
       int stage = 0, it = 0, issued = 0;
       uint32_t phase = 0;
@@ -437,6 +450,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
         if (!(PAIR == 2 ? warp_wait_cluster(acc_empty_bar(acc), acc_parity, abort_flag) : warp_wait(acc_empty_bar(acc), acc_parity, abort_flag))) { error = kErrMmaAcc; break; }
         tc_fence_after();
         const uint32_t tmem_d = tmem0 + uint32_t(acc * p.acc_shift);
+        const uint32_t a_block = uint32_t(w.last - w.first) * 8u;
         const uint32_t b_block = uint32_t(w.n / PAIR) * 8u;   // descriptor units (16 bytes) between the stage's activation tiles
         const uint32_t idesc = (w.part ? 0u : 5u << 7) | (uint32_t(w.n >> 3) << 17) | (1u << 23) | (uint32_t(PAIR * kTileRows >> 4) << 24);
         const bool two_atoms = w.n > 128;
@@ -444,15 +458,14 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
         for (int step = step_begin; step < step_end; ++step) {
           const int nkb = min(2, p.kblocks - 2 * step);
           if (!warp_wait(full_bar(stage), phase, abort_flag)) { error = kErrMmaFull; break; }
-          if (PAIR == 2 && !warp_wait_cluster(peer_bar(stage), phase, abort_flag)) { error = kErrMmaFull; break; }
-          // codes and scales were written through the generic proxy (cp.async); the tensor core reads through the async proxy
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          // the quantisers write codes and scales through the generic proxy; the tensor core reads through the async proxy
+          if (FUSED) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           tc_fence_after();
 #ifdef HG_TRACE
           if (lane == 0 && it == 0 && step == step_begin) HG_STAMP(3);
 #endif
           if (elect_one()) {
-            const uint32_t a_lo = a_desc + uint32_t(stage) * 2048u, b_lo = b_desc + uint32_t(stage) * b_stage;
+            const uint32_t a_lo = a_desc + uint32_t(stage) * a_stage - uint32_t(w.first) * 8u, b_lo = b_desc + uint32_t(stage) * b_stage;
             const uint32_t sfa_lo = sfa_desc + uint32_t(stage) * 64u, sfb_lo = sfb_desc + uint32_t(stage) * sfb_stage;
 #pragma unroll
             for (uint32_t i = 0; i < 2; ++i) {
@@ -463,7 +476,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
               if (two_atoms) cg_cp_scales<PAIR>(sf + 8, desc_of(sfb_lo + i * 32u + 64u, kDescScales));
 #pragma unroll
               for (uint32_t j = 0; j < 4; ++j)
-                cg_mma<PAIR>(tmem_d, desc_of(a_lo + i * 1024u + 2 * j, kDescTile), desc_of(b_lo + i * b_block + 2 * j, kDescTile),
+                cg_mma<PAIR>(tmem_d, desc_of(a_lo + i * a_block + 2 * j, kDescTile), desc_of(b_lo + i * b_block + 2 * j, kDescTile),
                              idesc | (j << 29) | (j << 4), i + j > 0 ? 1u : accumulate, sf, sf + 4);
             }
             cg_commit<PAIR>(empty_bar(stage), pair_mask);
@@ -478,10 +491,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
 #ifdef HG_TRACE
         if (lane == 0 && it < 4) HG_STAMP(4 + it);
 #endif
-        // Audit, in tiles of 128 rows x audit_tokens: the tiles whose first row this unit covers.
-        const int first_row = w.tile * PAIR * p.tile_rows[w.part];
-        const int last_row = min(first_row + PAIR * p.tile_rows[w.part], p.rows[w.part]);
-        issued += (((last_row + 127) >> 7) - ((first_row + 127) >> 7)) * (min(2 * step_end, p.kblocks) - 2 * step_begin) *
+        issued += atoms_started<PAIR>(p, w) * (min(2 * step_end, p.kblocks) - 2 * step_begin) *
                   ((min(w.n, p.tokens - w.token0) + p.audit_tokens - 1) / p.audit_tokens);
       }
       // Every MMA of this CTA (pair) retires before TMEM is released.
@@ -490,21 +500,11 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
       if (!warp_wait(drain_bar, 0, abort_flag) && !error) error = kErrDrain;
       if (lane == 0 && issued) atomicAdd(p.status + 1, issued);
     } else if (PAIR == 2) {
-      // ---------------------------------------------------------------- second CTA of a pair: report full stages
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int u = cluster; u < units && !error; u += p.clusters)
-        for (int step = step_begin; step < step_end; ++step) {
-          if (!warp_wait(full_bar(stage), phase, abort_flag)) { error = kErrMmaFull; break; }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          if (lane == 0) arrive_remote(map_to_rank(peer_bar(stage), uint32_t(rank - 1)));
-          __syncwarp();
-          if (++stage == p.stages) { stage = 0; phase ^= 1u; }
-        }
+      // ---------------------------------------------------------------- second CTA of a pair: wait for the last MMA
       if (!warp_wait(drain_bar, 0, abort_flag) && !error) error = kErrDrain;
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..9)
+    // ------------------------------------------------------------------ epilogue
     const int quarter = warp & 3, side = (warp - 2) >> 2;   // TMEM lanes this warp may read; which of the two warps of the quarter
     const int row_in_tile = quarter * 32 + lane;
     const uint32_t lane_addr = uint32_t(quarter * 32) << 16;
@@ -517,9 +517,9 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
     for (int u = cluster; u < units; u += p.clusters, ++it) {
       const Unit w = unit_at(p, u);
       const int acc = it & 1;
-      const int row0 = (w.tile * PAIR + half) * p.tile_rows[w.part];
-      const int row = row0 + row_in_tile;
-      const bool row_ok = row_in_tile < p.tile_rows[w.part] && row < p.rows[w.part];
+      const int row = (w.atom * PAIR + half) * kTileRows + row_in_tile;
+      const bool active = quarter * 32 >= w.first && quarter * 32 < w.last;   // this quarter's rows belong to the tile
+      const bool row_ok = active && row < p.rows[w.part];
       const int channel = row_ok ? p.ids[w.part][row] : 0;   // fetched while the main loop runs
       const int valid = min(w.n, p.tokens - w.token0);
       char* const out_row = out + int64_t(channel) * (out_f32 ? 4 : 2) + int64_t(w.token0) * row_bytes;
@@ -558,27 +558,36 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
       if (p.split > 1) {
         // Every slice owns 2^share_log groups of four columns.  A partial goes straight to the shared memory of the slice
         // that owns its group (lanes write 512 contiguous bytes), one hop; the owner adds the pieces in K order.
-        if (it > 0 && !warp_wait_cluster(red_empty, uint32_t(it - 1) & 1u, abort_flag)) { error = kErrEpilogue; break; }
+        // In the ring: every slice first tells the others that its own MMAs, and with them its ring, are done.
+        if (p.ring_exchange && lane < p.split) arrive_remote(map_to_rank(red_empty, uint32_t(lane * PAIR + half)));
+        if (p.ring_exchange && !warp_wait_cluster(red_empty, 0, abort_flag)) { error = kErrEpilogue; break; }
         const uint32_t share = 1u << p.share_log;
         const uint32_t my_piece = base + lay.red + (uint32_t(slice) << (p.share_log + 11)) + uint32_t(row_in_tile) * 16u;
         const int groups = (valid + 3) >> 2;
-        for (int g0 = 4 * side; g0 < groups; g0 += 8) {
+        const int g_begin = slice << p.share_log, g_end = min(groups, (slice + 1) << p.share_log);
+        // st.async saves a round trip (the release of the stores before an arrival; 0.5 us), but counts every 16 bytes on the
+        // barrier one after the other: beyond 32 columns plain stores and one arrival per warp are faster (o_proj at 128
+        // tokens, K in two: 8.5 us against 10.4).
+        if (p.async_push && threadIdx.x == 64) mbar_expect_tx(red_full, uint32_t(max(0, g_end - g_begin) * p.split * (w.last - w.first)) * 16u);
+        for (int g0 = 4 * side; g0 < groups && active; g0 += 4 * kSides) {
           uint32_t r[16];
           tc_load16(taddr + uint32_t(g0) * 4u, r);
           tc_wait_ld();
 #pragma unroll
           for (uint32_t i = 0; i < 4; ++i) {
             const uint32_t g = uint32_t(g0) + i;
-            const uint32_t to = map_to_rank(my_piece + ((g & (share - 1u)) << 11), (g >> p.share_log) * PAIR + uint32_t(half));
-            store_remote(to, tc_loaded(r[4 * i]), tc_loaded(r[4 * i + 1]), tc_loaded(r[4 * i + 2]), tc_loaded(r[4 * i + 3]));
+            const uint32_t owner = (g >> p.share_log) * PAIR + uint32_t(half);
+            const uint32_t to = map_to_rank(my_piece + ((g & (share - 1u)) << 11), owner);
+            if (!p.async_push) store_remote(to, tc_loaded(r[4 * i]), tc_loaded(r[4 * i + 1]), tc_loaded(r[4 * i + 2]), tc_loaded(r[4 * i + 3]));
+            else if (int(g) < groups)
+              store_async(to, map_to_rank(red_full, owner), tc_loaded(r[4 * i]), tc_loaded(r[4 * i + 1]), tc_loaded(r[4 * i + 2]), tc_loaded(r[4 * i + 3]));
           }
         }
         release(acc);
-        if (lane < p.split) arrive_remote(map_to_rank(red_full, uint32_t(lane * PAIR + half)));
-        if (!warp_wait_cluster(red_full, uint32_t(it) & 1u, abort_flag)) { error = kErrEpilogue; break; }
+        if (!p.async_push && lane < p.split) arrive_remote(map_to_rank(red_full, uint32_t(lane * PAIR + half)));
+        if (!warp_wait_cluster(red_full, 0, abort_flag)) { error = kErrEpilogue; break; }
         const uint32_t pieces = base + lay.red + uint32_t(row_in_tile) * 16u;
-        const int g_begin = slice << p.share_log, g_end = min(groups, (slice + 1) << p.share_log);
-        for (int g = g_begin + side; g < g_end; g += 2) {
+        for (int g = g_begin + side; g < g_end && active; g += kSides) {
           const uint32_t from = pieces + (uint32_t(g - g_begin) << 11);
           float v[8][4];
 #pragma unroll
@@ -594,12 +603,10 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
             }
           store(4 * g, v[0]);
         }
-        __syncwarp();
-        if (lane < p.split) arrive_remote(map_to_rank(red_empty, uint32_t(lane * PAIR + half)));
       } else {
         // This warp's groups of sixteen columns, the TMEM read of the next one in flight while the current one is stored.
         // The columns two accumulators share are drained first and handed to the next main loop.
-        const int chunks = (w.n + 15) >> 4;
+        const int chunks = active ? (w.n + 15) >> 4 : 0;
         const int begin = p.overlap && acc == 0 && 14 + side < chunks ? 14 + side : side;   // column 224 of accumulator 0 is column 0 of accumulator 1
         bool hand_over = p.overlap;
         if (hand_over && acc == 0 && begin != 14 + side) { release(1); hand_over = false; }
@@ -613,7 +620,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
           for (int i = 0; i < 16; ++i) r[i] = __uint_as_float(tc_loaded(a[i]));
           if (hand_over) { release(acc ^ 1); hand_over = false; }
           // 14 + side comes first where it is shared, then side, side + 2, ...
-          int next = begin > side ? (c == begin ? side : c + 2) : c + 2;
+          int next = begin > side && c == begin ? side : c + kSides;
           if (begin > side && next == begin) next = chunks;
           if (next < chunks) tc_load16(taddr + uint32_t(next) * 16u, a);
           store(16 * c, r);
@@ -623,11 +630,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
         if (!p.overlap) release(acc);
       }
       if (threadIdx.x == 64 && it < 3) HG_STAMP(9 + 2 * it);
-      if (slice == 0 && half == 0 && threadIdx.x == 64) {
-        const int first_row = w.tile * PAIR * p.tile_rows[w.part];
-        const int last_row = min(first_row + PAIR * p.tile_rows[w.part], p.rows[w.part]);
-        stored += (((last_row + 127) >> 7) - ((first_row + 127) >> 7)) * ((valid + p.audit_tokens - 1) / p.audit_tokens);
-      }
+      if (slice == 0 && half == 0 && threadIdx.x == 64) stored += atoms_started<PAIR>(p, w) * ((valid + p.audit_tokens - 1) / p.audit_tokens);
     }
     if (threadIdx.x == 64 && stored) atomicAdd(p.status + 2, stored);
   }
@@ -660,7 +663,41 @@ static int tuning(const char* name, int value) {
   return text ? std::atoi(text) : value;
 }
 
-// Ring, TMEM and shared-memory figures that follow from pair, split, n_tile.  False when the ring would be too shallow.
+// Estimated microseconds of a launch.  A K256 step of a CTA takes the longest of: the tensor core with its operand reads from
+// shared memory; a turn of the ring (from commit to the next full stage); the CTA's part of what L2 delivers (11 TB/s over
+// all SMs).  The launch takes the busiest cluster's steps or its weights' time from HBM (6.3 TB/s), whichever is longer,
+// plus a constant, a little per CTA, the last epilogue and the exchange of partials.  A ring's worth of weights is in shared
+// memory before the kernel in front has ended.  The constants are a fit to 130 measured launches (Qwen2.5-7B and
+// Mistral-7B / 4 shapes, 16 to 128 tokens; 10 % rms); the plan it prefers is 2 % slower than the best one on average.
+static double plan_cost(const ClusterPlan& plan, int64_t units, int kblocks, double weight_megabytes) {
+  const double steps = double((kblocks + 1) / 2) / plan.split;
+  const int cluster_ctas = plan.pair * plan.split, ctas = plan.clusters * cluster_ctas;
+  double prefetched = 0;
+  auto unit = [&](int n, bool high) {
+    const double b = double(n) / plan.pair;
+    const double mma = 2 * (plan.pair == 2 ? std::max(2.0 * n, 200.0 + b) : std::max(171.0, 128.0 + 1.3 * b)) / 1900;
+    const double kilobytes = double(kTileRows >> plan.cut_log[high]) * (high ? 0.25 : 0.125) + b * 0.25 + 2;
+    const double step = std::max({mma, 1.42 / plan.stages, kilobytes * ctas / 11000});
+    prefetched = std::max(prefetched, std::min(steps, double(plan.stages)) * (step - mma));
+    return steps * step + (plan.split > 1 ? 0.5 + 0.011 * n : 0.15);
+  };
+  const double whole = unit(plan.n_tile, false), last = unit(plan.n_tail, false);
+  double busiest;
+  if (plan.token_tiles == 1) {   // MXFP8 tiles first, round the clusters
+    const double high = unit(plan.n_tail, true);
+    const int64_t turns = (units + plan.clusters - 1) / plan.clusters, high_turns = (plan.tiles[1] + plan.clusters - 1) / plan.clusters;
+    busiest = double(high_turns) * high + double(turns - high_turns) * last;
+  } else {
+    std::vector<double> load(size_t(plan.clusters), 0.0);
+    for (int64_t u = 0; u < units; ++u) load[size_t(u % plan.clusters)] += u % plan.token_tiles == plan.token_tiles - 1 ? last : whole;
+    busiest = *std::max_element(load.begin(), load.end());
+  }
+  const double epilogue = 0.35 + 0.0185 * plan.n_tail / plan.split;
+  const double exchange = plan.split > 1 ? 0.14 * std::log2(double(cluster_ctas)) - 0.17 : 0.0;
+  return 2.2 + 0.012 * ctas + std::max(busiest - prefetched, weight_megabytes / 6.3) + epilogue + exchange;
+}
+
+// Ring, TMEM and shared-memory figures that follow from the other choices.  False when the ring would be too shallow.
 static bool finish_plan(ClusterPlan& plan) {
   const int n_cols = (plan.n_tile + 31) & ~31;
   plan.overlap = plan.n_tile > 224 ? 1 : 0;
@@ -668,92 +705,60 @@ static bool finish_plan(ClusterPlan& plan) {
   const int cols = plan.acc_shift + n_cols + int(2 * kScaleStride);
   plan.tmem_cols = 64;
   while (plan.tmem_cols < cols) plan.tmem_cols *= 2;
-  const ClusterSmem one = cluster_smem(1, plan.n_tile, plan.pair, plan.split), none = cluster_smem(0, plan.n_tile, plan.pair, plan.split);
-  const int stage_bytes = int(one.bars - none.bars);
-  plan.stages = std::min((kMaxSmem - 1024 - kClusterBarBytes - int(none.bars)) / stage_bytes,
-                         std::min(kClusterMaxStages, tuning("HYGEMM_CL_STAGES", kClusterMaxStages)));
-  if (plan.stages < 2) return false;
-  plan.smem_bytes = 1024 + int(none.bars) + plan.stages * stage_bytes + kClusterBarBytes;
-  return plan.tmem_cols <= 512;
-}
-
-// Cycles of one K128 block of a CTA: the tensor core's shared-memory traffic and time, the copies into the ring,
-// and the CTA's share of HBM (23 bytes per cycle and SM at the measured copy rate).
-static double block_cycles(const ClusterPlan& plan, int n, double weight_bytes, double hbm_share) {
-  const double b = double(n) / plan.pair;
-  const double mma = plan.pair == 2 ? std::max(2.0 * n, 128 + b) : std::max(4.0 * 40, 128 + b + (n > 64 ? n - 64 : 0));
-  return std::max({mma, 128 + b + 96 + b, weight_bytes / hbm_share});
+  plan.slot_rows = kTileRows >> std::min(plan.cut_log[0], plan.cut_log[1]);
+  plan.least_rows = kTileRows >> std::max(plan.cut_log[0], plan.cut_log[1]);
+  const int most = std::min(kClusterMaxStages, tuning("HYGEMM_CL_STAGES", kClusterMaxStages));
+  for (plan.stages = most; plan.stages >= 2; --plan.stages) {
+    plan.smem_bytes = 1024 + int(cluster_smem(plan.stages, plan.n_tile, plan.pair, plan.split, plan.slot_rows, plan.least_rows, plan.ring_exchange).end);
+    if (plan.smem_bytes <= kMaxSmem) return true;
+  }
+  return false;
 }
 
 ClusterPlan make_cluster_plan(int lo, int hi, int tokens, int k, const int max_clusters[4]) {
   const int kblocks = k / kTileK, steps = (kblocks + 1) / 2;
+  const int atoms[2] = {(lo + kTileRows - 1) / kTileRows, (hi + kTileRows - 1) / kTileRows};
   ClusterPlan best;
   best.cost = 1e30;
   const int force_split = tuning("HYGEMM_CL_SPLIT", 0), force_pair = tuning("HYGEMM_CL_PAIR", 0), force_n = tuning("HYGEMM_CL_N", 0);
-  auto consider = [&](ClusterPlan plan) {
-    if (force_split && plan.split != force_split) return;
-    if (force_pair && plan.pair != force_pair) return;
-    if (force_n && plan.n_tile != force_n) return;
-    if (!finish_plan(plan)) return;
-    if (plan.cost < best.cost) best = plan;
-  };
+  const int force_cut = tuning("HYGEMM_CL_CUT", -1), force_cut_high = tuning("HYGEMM_CL_CUT_HIGH", -1);
   for (int pair = 1; pair <= 2; ++pair)
-    for (int log = pair - 1; log < 4; ++log) {
-      ClusterPlan plan;
-      plan.pair = pair;
-      plan.split = (1 << log) / pair;
-      if (plan.split > steps) continue;
-      const int capacity = max_clusters[log];
-      if (capacity < 1) continue;
-      const double slice = double(kblocks) / plan.split;
-      const double fixed = plan.split > 1 ? 2500 : 0;
-      if (tokens <= 128) {
-        if ((pair == 2) != (tokens > 64)) continue;
-        // Weights stream from HBM once: every CTA gets the same number of bytes, an MXFP8 row counting two rows.
-        plan.n_tile = plan.n_tail = (tokens + 16 * pair - 1) / (16 * pair) * (16 * pair);
-        plan.token_tiles = 1;
-        const double total = lo + 2.0 * hi;
-        for (int waves = 1; waves <= 64; ++waves) {
-          const double rows = total / (double(waves) * capacity * pair);
-          int height = std::max(8, int(rows) + 1);
-          bool fits = false;
-          for (; height <= 128 && !fits; ++height) {
-            plan.tile_rows[0] = height;
-            plan.tile_rows[1] = (height + 1) / 2;
-            plan.tiles[0] = (lo + pair * plan.tile_rows[0] - 1) / (pair * plan.tile_rows[0]);
-            plan.tiles[1] = (hi + pair * plan.tile_rows[1] - 1) / (pair * plan.tile_rows[1]);
-            fits = plan.tiles[0] + plan.tiles[1] <= waves * capacity;
-          }
-          if (!fits) continue;
-          plan.clusters = std::min(capacity, plan.tiles[0] + plan.tiles[1]);
-          const double share = 23.0 * 148.0 / (plan.clusters << log);
-          plan.cost = waves * (slice * block_cycles(plan, plan.n_tile, plan.tile_rows[0] * 68.0, std::min(share, 40.0)) + 300) + fixed;
-          consider(plan);
-          if (waves > 1 && rows < 32) break;
-        }
-      } else {
-        if (pair == 1) continue;
-        plan.tile_rows[0] = plan.tile_rows[1] = 128;
-        plan.tiles[0] = (lo + 255) / 256;
-        plan.tiles[1] = (hi + 255) / 256;
-        for (int n : {128, 256}) {
-          if (n == 256 && plan.split > 1) continue;   // the partial tiles would not fit beside the ring
-          plan.n_tile = n;
-          plan.token_tiles = (tokens + n - 1) / n;
-          const int tail = tokens - (plan.token_tiles - 1) * n;
-          plan.n_tail = (tail + 31) / 32 * 32;
-          const int64_t units = int64_t(plan.tiles[0] + plan.tiles[1]) * plan.token_tiles;
-          plan.clusters = int(std::min<int64_t>(capacity, units));
-          // Units go round the clusters in order; the busiest cluster decides.
-          std::vector<double> load(size_t(plan.clusters), 0.0);
-          const double whole = slice * block_cycles(plan, n, 0, 1) + 600 + fixed, last = slice * block_cycles(plan, plan.n_tail, 0, 1) + 600 + fixed;
-          for (int64_t u = 0; u < units; ++u)
-            load[size_t(u % plan.clusters)] += (u % plan.token_tiles) == plan.token_tiles - 1 ? last : whole;
-          plan.cost = *std::max_element(load.begin(), load.end());
-          consider(plan);
-        }
-      }
-    }
+    for (int log = pair - 1; log < 4; ++log)
+      for (int cut = 0; cut < 3; ++cut)
+        for (int more = 0; more < 2; ++more)
+          for (int n : {0, 128, 256}) {
+              ClusterPlan plan;
+              plan.pair = pair;
+              plan.split = (1 << log) / pair;
+              plan.cut_log[0] = cut;
+              plan.cut_log[1] = cut + more;
+              if (plan.split > steps || cut + more > 2 || max_clusters[log] < 1) continue;
+              if (tokens <= 128) {
+                if (n || (tokens > 64 && pair == 1) || (tokens <= 32 && pair == 2)) continue;   // (fused quantisation: single CTAs)
+                plan.n_tile = plan.n_tail = (tokens + 16 * pair - 1) / (16 * pair) * (16 * pair);
+                plan.token_tiles = 1;
+              } else {
+                if (!n || pair == 1 || cut || more || (n == 256 && plan.split > 1)) continue;
+                plan.n_tile = n;
+                plan.token_tiles = (tokens + n - 1) / n;
+                plan.n_tail = (tokens - (plan.token_tiles - 1) * n + 31) / 32 * 32;
+              }
+              if ((force_split && plan.split != force_split) || (force_pair && pair != force_pair) || (force_n && plan.n_tile != force_n) ||
+                  (force_cut >= 0 && cut != force_cut) || (force_cut_high >= 0 && cut + more != force_cut_high))
+                continue;
+              for (int i = 0; i < 2; ++i) plan.tiles[i] = ((atoms[i] + pair - 1) / pair) << plan.cut_log[i];
+              const int64_t units = int64_t(plan.tiles[0] + plan.tiles[1]) * plan.token_tiles;
+              plan.clusters = int(std::min<int64_t>(max_clusters[log], units));
+              // With several units to a cluster every exchange would stall the next main loop (gate_up at 16 tokens, K in
+              // two: 19.8 us against 15.4).
+              if (plan.split > 1 && units > plan.clusters) continue;
+              // Worth its extra hop (about 0.4 us) where the exchange buffer would take a stage from the ring (down_proj at 128
+              // tokens 17.1 -> 16.0 us).
+              plan.ring_exchange = plan.split > 1 && plan.n_tile > 32;
+              if (!finish_plan(plan)) continue;
+              plan.cost = plan_cost(plan, units, kblocks, (lo * 0.53125 + hi * 1.03125) * k * 1e-6);
+              if (plan.cost < best.cost) best = plan;
+            }
   if (best.cost >= 1e30) throw std::runtime_error("No cluster schedule for this shape");
   return best;
 }
@@ -782,7 +787,7 @@ const int* cluster_capacity() {
     for (int log = 1; log < 4; ++log) {
       cudaLaunchConfig_t config{};
       config.gridDim = dim3(unsigned(sms >> log << log));
-      config.blockDim = dim3(cluster_threads(false));
+      config.blockDim = dim3(cluster_threads(2, false));
       config.dynamicSmemBytes = kMaxSmem;
       cudaLaunchAttribute attribute[1];
       attribute[0].id = cudaLaunchAttributeClusterDimension;
@@ -798,11 +803,10 @@ const int* cluster_capacity() {
 }
 
 template <typename T, int PAIR, bool FUSED>
-static cudaError_t launch(const ClusterPlan& plan, const ClusterParams& p, const CUtensorMap& map_act, const CUtensorMap& map_tail,
-                          cudaStream_t stream, bool pdl) {
+static cudaError_t launch(const ClusterPlan& plan, const ClusterParams& p, const ClusterMaps& maps, cudaStream_t stream, bool pdl) {
   cudaLaunchConfig_t config{};
   config.gridDim = dim3(unsigned(plan.clusters * plan.pair * plan.split));
-  config.blockDim = dim3(cluster_threads(FUSED));
+  config.blockDim = dim3(cluster_threads(PAIR, FUSED));
   config.dynamicSmemBytes = size_t(plan.smem_bytes);
   config.stream = stream;
   cudaLaunchAttribute attribute[2];
@@ -817,25 +821,25 @@ static cudaError_t launch(const ClusterPlan& plan, const ClusterParams& p, const
   }
   config.attrs = attribute;
   config.numAttrs = unsigned(count);
-  return cudaLaunchKernelEx(&config, cluster_gemm_kernel<T, PAIR, FUSED>, p, map_act, map_tail);
+  return cudaLaunchKernelEx(&config, cluster_gemm_kernel<T, PAIR, FUSED>, p, maps);
 }
 
-void launch_cluster(const ClusterPlan& plan, const ClusterCall& call, const CUtensorMap& map_act, const CUtensorMap& map_tail,
-                    cudaStream_t stream, bool pdl) {
+void launch_cluster(const ClusterPlan& plan, const ClusterCall& call, const ClusterMaps& maps, cudaStream_t stream, bool pdl) {
   const hg_problem &l = *call.low, &h = *call.high, &any = l.rows ? l : h;
   ClusterParams p{};
   const hg_problem* parts[2] = {&l, &h};
   for (int i = 0; i < 2; ++i) {
-    p.rows[i] = parts[i]->rows; p.tile_rows[i] = plan.tile_rows[i]; p.tiles[i] = plan.tiles[i];
-    p.weight[i] = static_cast<const uint8_t*>(parts[i]->weight);
+    p.rows[i] = parts[i]->rows; p.cut_log[i] = plan.cut_log[i]; p.tiles[i] = plan.tiles[i];
     p.sfa[i] = static_cast<const uint8_t*>(parts[i]->weight_scales);
     p.ids[i] = static_cast<const int32_t*>(parts[i]->ids);
   }
+  p.slot_rows = plan.slot_rows; p.least_rows = plan.least_rows;
   p.sfb = static_cast<const uint8_t*>(any.activation_scales);
   p.out = call.out;
   p.outputs = any.outputs; p.tokens = any.tokens; p.k = any.k; p.kblocks = any.k / kTileK;
   p.n_tile = plan.n_tile; p.n_tail = plan.n_tail; p.token_tiles = plan.token_tiles; p.stages = plan.stages;
-  p.split = plan.split; p.clusters = plan.clusters;
+  p.async_push = plan.n_tile <= 32;
+  p.ring_exchange = plan.ring_exchange; p.split = plan.split; p.clusters = plan.clusters;
   while ((1 << p.split_log) < plan.split) ++p.split_log;
   p.share_log = share_log_of(plan.n_tile, plan.split);
   const uint64_t tiles = uint64_t(plan.tiles[0]) + uint64_t(plan.tiles[1]), most = uint64_t(1) << 40;
@@ -856,9 +860,9 @@ void launch_cluster(const ClusterPlan& plan, const ClusterCall& call, const CUte
 #endif
   const bool bf16 = call.dtype == HG_DTYPE_BF16;
   cudaError_t e;
-  if (call.x) e = bf16 ? launch<__nv_bfloat16, 1, true>(plan, p, map_act, map_tail, stream, pdl) : launch<__half, 1, true>(plan, p, map_act, map_tail, stream, pdl);
-  else if (plan.pair == 1) e = bf16 ? launch<__nv_bfloat16, 1, false>(plan, p, map_act, map_tail, stream, pdl) : launch<__half, 1, false>(plan, p, map_act, map_tail, stream, pdl);
-  else e = bf16 ? launch<__nv_bfloat16, 2, false>(plan, p, map_act, map_tail, stream, pdl) : launch<__half, 2, false>(plan, p, map_act, map_tail, stream, pdl);
+  if (call.x) e = bf16 ? launch<__nv_bfloat16, 1, true>(plan, p, maps, stream, pdl) : launch<__half, 1, true>(plan, p, maps, stream, pdl);
+  else if (plan.pair == 1) e = bf16 ? launch<__nv_bfloat16, 1, false>(plan, p, maps, stream, pdl) : launch<__half, 1, false>(plan, p, maps, stream, pdl);
+  else e = bf16 ? launch<__nv_bfloat16, 2, false>(plan, p, maps, stream, pdl) : launch<__half, 2, false>(plan, p, maps, stream, pdl);
   check(e, "hybrid GEMM launch");
 }
 

@@ -13,14 +13,16 @@ struct ClusterPlan {
   int n_tile = 0;          // tokens per tile
   int n_tail = 0;          // MMA columns of the last token tile
   int token_tiles = 0;
-  int tile_rows[2] = {0, 0};   // weight rows per CTA tile of each partition, at most 128
-  int tiles[2] = {0, 0};       // tiles (pair * tile_rows rows) of each partition
+  int cut_log[2] = {0, 0};     // each partition's 128-row atoms (pairs of atoms) are cut into 2^cut_log tiles
+  int tiles[2] = {0, 0};       // tiles of each partition
+  int slot_rows = 0, least_rows = 0;   // the taller and the shorter tile height; a ring slot holds the taller
+  int ring_exchange = 0;       // partials are exchanged in the ring, idle by then
   int stages = 0;          // K256 stages of the ring
   int acc_shift = 0;       // TMEM columns between the two accumulators
   int overlap = 0;         // the accumulators share 32 columns (256-token tiles)
   int tmem_cols = 0;
   int smem_bytes = 0;
-  double cost = 0;         // estimated cycles
+  double cost = 0;         // estimated microseconds
 };
 
 // Plan for one shape; `max_clusters[i]` is the number of clusters of 2^i CTAs the device holds at once.
@@ -40,9 +42,11 @@ struct ClusterCall {
   int* status;
   unsigned long long* trace;
 };
-// `map_act`, `map_tail`: activation maps of boxes n_tile / pair and n_tail / pair rows (unused when `x` is set).
-void launch_cluster(const ClusterPlan& plan, const ClusterCall& call, const CUtensorMap& map_act, const CUtensorMap& map_tail,
-                    cudaStream_t stream, bool pdl);
+// Boxes: weights 128 >> cut_log rows x 2 K128 blocks; activations n_tile / pair and, for the last token tile, n_tail / pair rows;
+// scales (pairs only) 2 atoms.  Maps a launch does not use (an absent partition; activations quantised in the kernel) may
+// be zeros.
+struct ClusterMaps { CUtensorMap low, high, act, tail, low_scales, high_scales, act_scales; };
+void launch_cluster(const ClusterPlan& plan, const ClusterCall& call, const ClusterMaps& maps, cudaStream_t stream, bool pdl);
 void configure_cluster_kernels();
 
 }  // namespace hg

@@ -738,14 +738,6 @@ static bool staged_fixup() {
 }
 constexpr int kMaxDynamicSmem = 232448;  // 227 KiB, the per-CTA limit of sm_100
 
-// Shapes AUTO hands to the cluster kernel.  Prefill: 256-row pair tiles (gate_up at 2048 tokens 401 -> 279 us).  Up to 64
-// tokens: layers with fewer than about 1.5 tiles per SM, whose tiles are cut along K and exchanged inside a cluster (o_proj
-// at 16 tokens 10.5 -> 7.6 us, down 16.4 -> 15.5).  In between, and for wide layers at decode sizes, the ring of this
-// file's kernel turns faster.
-static bool cluster_serves(int tiles, int tokens, int sms) {
-  return tokens > 128 || (tokens <= 64 && 2 * tiles < 3 * sms);
-}
-
 Plan make_plan(int rows_low, int rows_high, int tokens, int k, int sms, int schedule) {
   Plan plan;
   const int tiles_low = (rows_low + kTileRows - 1) / kTileRows, tiles_high = (rows_high + kTileRows - 1) / kTileRows;
@@ -906,16 +898,9 @@ Plan make_plan(int rows_low, int rows_high, int tokens, int k, int sms, int sche
     plan.counters = counters;
   };
 
-  if (schedule == HG_SCHEDULE_AUTO) {
-    // The cluster kernel (hg_gemm_cluster.cu) never cuts a tile over units: its unit list is the data-parallel one.
-    // This kernel, measured on B200 (Qwen2.5-7B layer shapes, M = 1..128): whole tiles win once there are about
-    // 1.5 tiles per SM, and also for wide token tiles unless K is long, because the fix-up traffic of a
-    // cut tile grows with n_tile (n_tile x 128 fp32 partials written and read per piece); otherwise
-    // stream-K, which keeps every SM streaming.
-    const bool many_tiles = 2 * items >= 3 * sms;
-    const bool wide_short = plan.n_tile >= 64 && kblocks < 64;
-    schedule = (cluster_serves(tiles, tokens, sms) || many_tiles || wide_short) ? HG_SCHEDULE_DATA_PARALLEL : HG_SCHEDULE_STREAM_K;
-  }
+  // AUTO runs the cluster kernel (hg_gemm_cluster.cu), which never cuts a tile over units: its unit list is the
+  // data-parallel one.
+  if (schedule == HG_SCHEDULE_AUTO) schedule = HG_SCHEDULE_DATA_PARALLEL;
   plan.ws_slots = 0;
   plan.counters = 0;
   if (schedule == HG_SCHEDULE_DATA_PARALLEL) {
@@ -984,19 +969,46 @@ static CUtensorMap make_map(const void* ptr, int rows, int k, int box_rows) {
   return map;
 }
 
-// The same bytes as [K128 block][row][128]: one copy of a box of 2 blocks x box_rows fills a K256 stage.
-static CUtensorMap make_block_map(const void* ptr, int rows, int k, int box_rows) {
+// The same matrix as [K128 block][row][128 elements]: one copy of a box of 2 blocks x box_rows fills a K256 stage.  Packed
+// E2M1 codes are unpacked by the copy, eight bytes of codes and eight of padding in every 16-byte chunk.
+static CUtensorMap make_block_map(const void* ptr, int rows, int k, int box_rows, bool fp4 = false) {
   CUtensorMap map;
   std::memset(&map, 0, sizeof(map));
   const cuuint64_t dims[3] = {128u, cuuint64_t(rows), cuuint64_t(k / 128)};
-  const cuuint64_t strides[2] = {cuuint64_t(k), 128u};
+  const cuuint64_t strides[2] = {cuuint64_t(fp4 ? k / 2 : k), fp4 ? 64u : 128u};
   const cuuint32_t box[3] = {128u, cuuint32_t(box_rows), 2u};
   const cuuint32_t elem[3] = {1u, 1u, 1u};
-  const CUresult r = encode_tiled()(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(ptr), dims, strides, box,
-                                    elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const CUresult r = encode_tiled()(&map, fp4 ? CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B : CU_TENSOR_MAP_DATA_TYPE_UINT8, 3,
+                                    const_cast<void*>(ptr), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled failed with code " + std::to_string(int(r)));
   return map;
+}
+
+// Scale atoms of 512 bytes, two to a box; `atoms` in the buffer.
+static CUtensorMap make_scale_map(const void* ptr, int64_t atoms) {
+  CUtensorMap map;
+  std::memset(&map, 0, sizeof(map));
+  const cuuint64_t dims[2] = {128u, cuuint64_t(atoms)};
+  const cuuint64_t strides[1] = {512u};
+  const cuuint32_t box[2] = {128u, 2u};
+  const cuuint32_t elem[2] = {1u, 1u};
+  const CUresult r = encode_tiled()(&map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(ptr), dims, strides, box, elem,
+                                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled failed with code " + std::to_string(int(r)));
+  return map;
+}
+
+// The maps of a cluster launch that belong to one partition's weights, and to the activations.
+static void set_weight_maps(ClusterMaps& maps, const ClusterPlan& plan, const hg_problem& q, int part) {
+  (part ? maps.high : maps.low) = make_block_map(q.weight, q.rows, q.k, kTileRows >> plan.cut_log[part], part == 0);
+  if (plan.pair == 2) (part ? maps.high_scales : maps.low_scales) = make_scale_map(q.weight_scales, scale_size(q.rows, q.k) / 512);
+}
+static void set_activation_maps(ClusterMaps& maps, const ClusterPlan& plan, const hg_problem& q) {
+  maps.act = make_block_map(q.activation, q.tokens, q.k, plan.n_tile / plan.pair);
+  maps.tail = plan.n_tail == plan.n_tile ? maps.act : make_block_map(q.activation, q.tokens, q.k, plan.n_tail / plan.pair);
+  if (plan.pair == 2) maps.act_scales = make_scale_map(q.activation_scales, scale_size(q.tokens, q.k) / 512);
 }
 
 static CtaHeads make_heads(const Plan& plan) {
@@ -1027,9 +1039,13 @@ struct TcGemm {
 #endif
   // Tensor maps of recent operand pointers (the shape is fixed per handle): a serving loop alternates among
   // a few activation buffers and one weight pointer, so the driver call is paid once per pointer.
-  struct CachedMap { const void* ptr = nullptr; CUtensorMap map, tail; };
+  struct CachedMap { const void* ptr = nullptr; CUtensorMap map; };
   CachedMap act_maps[4], high_map;
   int act_next = 0;
+  // Cluster kernel: the same for all maps of a launch, by activation and scale pointer; the weights' by weight pointer.
+  struct CachedMaps { const void* codes = nullptr; const void* scales = nullptr; ClusterMaps maps{}; };
+  CachedMaps cluster_maps[4];
+  const void* cluster_weights[2][2] = {};
 };
 
 void validate(const hg_problem& l, const hg_problem& h, bool fused) {
@@ -1073,16 +1089,15 @@ TcGemm* tc_create(const hg_problem& l, const hg_problem& h, int schedule, int dt
   g->tokens = any.tokens; g->k = any.k; g->outputs = any.outputs; g->dtype = dtype;
   g->plan = make_plan(l.rows, h.rows, any.tokens, any.k, sms, schedule);
   const Plan& plan = g->plan;
-  const int row_tiles = (l.rows + kTileRows - 1) / kTileRows + (h.rows + kTileRows - 1) / kTileRows;
-  if (schedule == HG_SCHEDULE_AUTO && cluster_serves(row_tiles, any.tokens, sms)) {
+  if (schedule == HG_SCHEDULE_AUTO) {
     g->clustered = true;
     g->cluster = make_cluster_plan(l.rows, h.rows, any.tokens, any.k, cluster_capacity());
     check(cudaMalloc(&g->d_status, sizeof(int) * 4), "cudaMalloc status");
     check(cudaMemsetAsync(g->d_status, 0, sizeof(int) * 4, stream), "clear status");
 #ifdef HG_TRACE
-    check(cudaMalloc(&g->d_trace, sizeof(unsigned long long) * 16 * size_t(sms)), "trace buffer");
-    check(cudaMemsetAsync(g->d_trace, 0, sizeof(unsigned long long) * 16 * size_t(sms), stream), "trace buffer");
     g->plan.grid = g->cluster.clusters * g->cluster.pair * g->cluster.split;
+    check(cudaMalloc(&g->d_trace, sizeof(unsigned long long) * 16 * size_t(g->plan.grid)), "trace buffer");
+    check(cudaMemsetAsync(g->d_trace, 0, sizeof(unsigned long long) * 16 * size_t(g->plan.grid), stream), "trace buffer");
 #endif
     return g.release();
   }
@@ -1177,10 +1192,44 @@ void tc_run(TcGemm* g, const hg_problem& l, const hg_problem& h, cudaStream_t st
   } else {
     out.ptr = any.output;
   }
+  if (g->clustered) {
+    const hg_problem* parts[2] = {&l, &h};
+    bool stale = false;
+    for (int i = 0; i < 2; ++i)
+      if (parts[i]->rows && (g->cluster_weights[i][0] != parts[i]->weight || g->cluster_weights[i][1] != parts[i]->weight_scales)) stale = true;
+    if (stale) {
+      g->cluster_weights[0][0] = g->cluster_weights[1][0] = nullptr;
+      for (auto& entry : g->cluster_maps) entry.codes = entry.scales = nullptr;
+      for (int i = 0; i < 2; ++i)
+        if (parts[i]->rows) set_weight_maps(g->cluster_maps[0].maps, g->cluster, *parts[i], i);
+      for (int c = 1; c < 4; ++c) g->cluster_maps[c].maps = g->cluster_maps[0].maps;
+      for (int i = 0; i < 2; ++i)
+        if (parts[i]->rows) { g->cluster_weights[i][0] = parts[i]->weight; g->cluster_weights[i][1] = parts[i]->weight_scales; }
+    }
+    TcGemm::CachedMaps* hit = nullptr;
+    if (fused) hit = &g->cluster_maps[0];   // the activation maps are not used
+    else
+      for (auto& entry : g->cluster_maps)
+        if (entry.codes == any.activation && entry.scales == any.activation_scales) hit = &entry;
+    if (!hit) {
+      hit = &g->cluster_maps[g->act_next];
+      g->act_next = (g->act_next + 1) % 4;
+      hit->codes = hit->scales = nullptr;
+      set_activation_maps(hit->maps, g->cluster, any);
+      hit->codes = any.activation;
+      hit->scales = any.activation_scales;
+    }
+    ClusterCall call{&l, &h, x, x_dtype, out, g->dtype, plan.n_tile, g->d_status, nullptr};
+#ifdef HG_TRACE
+    call.trace = g->d_trace;
+#endif
+    launch_cluster(g->cluster, call, hit->maps, stream, true);
+    return;
+  }
   // Tensor maps by operand pointer.  A map that the launch does not use (no MXFP8 rows; activations
   // quantised in the kernel) is passed as zeros and never touched by the kernel.
   static const CUtensorMap no_map{};
-  const TcGemm::CachedMap* act = nullptr;
+  const CUtensorMap* map_act = &no_map;
   if (!fused) {
     TcGemm::CachedMap* hit = nullptr;
     for (auto& entry : g->act_maps)
@@ -1189,23 +1238,10 @@ void tc_run(TcGemm* g, const hg_problem& l, const hg_problem& h, cudaStream_t st
       hit = &g->act_maps[g->act_next];
       g->act_next = (g->act_next + 1) % 4;
       hit->ptr = nullptr;
-      if (g->clustered) {
-        hit->map = make_block_map(any.activation, any.tokens, any.k, g->cluster.n_tile / g->cluster.pair);
-        hit->tail = make_block_map(any.activation, any.tokens, any.k, g->cluster.n_tail / g->cluster.pair);
-      } else {
-        hit->map = make_map(any.activation, any.tokens, any.k, plan.n_tile);
-      }
+      hit->map = make_map(any.activation, any.tokens, any.k, plan.n_tile);
       hit->ptr = any.activation;
     }
-    act = hit;
-  }
-  if (g->clustered) {
-    ClusterCall call{&l, &h, x, x_dtype, out, g->dtype, plan.n_tile, g->d_status, nullptr};
-#ifdef HG_TRACE
-    call.trace = g->d_trace;
-#endif
-    launch_cluster(g->cluster, call, act ? act->map : no_map, act ? act->tail : no_map, stream, true);
-    return;
+    map_act = &hit->map;
   }
   TcParams p = base_params(plan, l, h, g->dtype);
   p.out = out;
@@ -1216,7 +1252,6 @@ void tc_run(TcGemm* g, const hg_problem& l, const hg_problem& h, cudaStream_t st
 #ifdef HG_TRACE
   p.trace = g->d_trace;
 #endif
-  const CUtensorMap* map_act = act ? &act->map : &no_map;
   const CUtensorMap* map_high = &no_map;
   if (h.rows) {
     if (g->high_map.ptr != h.weight) {
@@ -1379,7 +1414,7 @@ void tc_run_static(int schedule, const hg_problem& l, const hg_problem& h, int d
     for (auto& resident : st.resident)
       if (resident == entry) resident = nullptr;   // the array of that device holds a schedule that is going away
     entry->plan = make_plan(l.rows, h.rows, any.tokens, any.k, st.sms[device], schedule);
-    entry->clustered = schedule == HG_SCHEDULE_AUTO && cluster_serves((l.rows + kTileRows - 1) / kTileRows + (h.rows + kTileRows - 1) / kTileRows, any.tokens, st.sms[device]);
+    entry->clustered = schedule == HG_SCHEDULE_AUTO;
     if (entry->clustered) entry->cluster = make_cluster_plan(l.rows, h.rows, any.tokens, any.k, cluster_capacity());
     else entry->heads = make_heads(entry->plan);
     std::memcpy(entry->key, key, sizeof(key));
@@ -1391,8 +1426,11 @@ void tc_run_static(int schedule, const hg_problem& l, const hg_problem& h, int d
     const ClusterPlan& cluster = entry->cluster;
     ClusterCall call{&l, &h, nullptr, HG_DTYPE_BF16, OutTargets{}, dtype, plan.n_tile, reinterpret_cast<int*>(base + kStaticStatusOffset), nullptr};
     call.out.ptr = any.output;
-    launch_cluster(cluster, call, make_block_map(any.activation, any.tokens, any.k, cluster.n_tile / cluster.pair),
-                   make_block_map(any.activation, any.tokens, any.k, cluster.n_tail / cluster.pair), stream, false);
+    ClusterMaps maps{};
+    if (l.rows) set_weight_maps(maps, cluster, l, 0);
+    if (h.rows) set_weight_maps(maps, cluster, h, 1);
+    set_activation_maps(maps, cluster, any);
+    launch_cluster(cluster, call, maps, stream, false);
     return;
   }
 
