@@ -14,7 +14,9 @@
 //
 // The statistics of the search (errors before and after, how far the scales moved) and the checks on its inputs are
 // gathered in the same pass: the values, codes and both scales are in registers here, and as torch ops they were a
-// dozen passes over full-size fp32 tensors and ten host synchronisations (4096 x 3584: 1660 us, 60 us now).
+// dozen passes over full-size fp32 tensors and ten host synchronisations (4096 x 3584: 1660 us, 67 us now, half of them host work).  The
+// kernel is bound by its arithmetic, so only the winning candidate is encoded, a
+// thread's sums over its dozen items are kept in fp32 (one conversion to fp64 at the end) and the offsets are read from the constant bank.
 #include <algorithm>
 
 #include "hg_common.cuh"
@@ -27,39 +29,38 @@ struct ClipOffsets {
   int value[kMaxClipOffsets];
 };
 
-// Two E2M1 codes -> their values (exact in half precision).
-__device__ __forceinline__ float2 e2m1_values(uint32_t byte) {
+// A pair of values rounded to E2M1 (nearest, ties to the even code, saturating) and back; exact in half precision.
+__device__ __forceinline__ float2 e2m1_round(float x, float y) {
   uint32_t halves;
   asm("{\n"
-      ".reg .b8 b0, b1, b2, b3;\n"
-      "mov.b32 {b0, b1, b2, b3}, %1;\n"
-      "cvt.rn.f16x2.e2m1x2 %0, b0;\n"
+      ".reg .b8 b;\n"
+      "cvt.rn.satfinite.e2m1x2.f32 b, %2, %1;\n"
+      "cvt.rn.f16x2.e2m1x2 %0, b;\n"
       "}"
-      : "=r"(halves) : "r"(byte));
+      : "=r"(halves) : "f"(x), "f"(y));
   return __half22float2(*reinterpret_cast<const __half2*>(&halves));
 }
 
-// Codes of eight values at scale 2^e and the thread's part of the squared error, weighted and plain.
-__device__ __forceinline__ uint32_t clip_candidate(const float (&v)[8], const float (&weight)[8], int e, float& error, float& plain_error) {
+// The thread's part of the squared error of eight values at scale 2^e, weighted and plain.  (A code's value times a power of
+// two is exact, so the fused multiply-add rounds once where a product and a difference would.)
+__device__ __forceinline__ float clip_candidate(const float (&v)[8], const float (&weight)[8], int e, float& plain_error) {
   const float inv = mx_inverse_scale(e);
   // 2^e as a factor: e in [-127,127]; 2^-127 is the subnormal 0x00400000.
   const float scale = e == -127 ? __uint_as_float(0x00400000u) : __uint_as_float(uint32_t(e + 127) << 23);
-  float scaled[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) scaled[i] = v[i] * inv;
-  const uint32_t codes = cvt_e2m1x8(scaled);
   float sum = 0.f, plain = 0.f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float2 pair = e2m1_values(codes >> (8 * (i >> 1)));
-    const float diff = __fsub_rn(__fmul_rn(i & 1 ? pair.y : pair.x, scale), v[i]);
-    const float square = __fmul_rn(diff, diff);
-    plain = __fadd_rn(plain, square);
-    sum = __fadd_rn(sum, __fmul_rn(square, weight[i]));
+  for (int i = 0; i < 8; i += 2) {
+    const float2 q = e2m1_round(v[i] * inv, v[i + 1] * inv);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float diff = __fmaf_rn(j ? q.y : q.x, scale, -v[i + j]);
+      const float square = __fmul_rn(diff, diff);
+      plain = __fadd_rn(plain, square);
+      sum = __fadd_rn(sum, __fmul_rn(square, weight[i + j]));
+    }
   }
-  error = sum;
   plain_error = plain;
-  return codes;
+  return sum;
 }
 
 // Slots of the statistics (doubles, added to): squared errors, flags, then one count per offset.
@@ -69,11 +70,11 @@ enum : int { kWeightedBefore = 0, kWeightedAfter = 1, kPlainBefore = 2, kPlainAf
 template <typename T, bool STATS>
 __global__ void __launch_bounds__(256, 4)
 mx_clip_search_kernel(const uint16_t* __restrict__ in, const float* __restrict__ importance, uint8_t* __restrict__ q4,
-                      uint8_t* __restrict__ scales, int rows, int k, ClipOffsets offsets, double* stats, double* __restrict__ host_stats) {
+                      uint8_t* __restrict__ scales, int rows, int k, const __grid_constant__ ClipOffsets offsets, double* stats, double* __restrict__ host_stats) {
   const int per_row = k >> 3;
   const int64_t threads = int64_t(rows) * per_row, stride = int64_t(gridDim.x) * blockDim.x;
   const uint32_t mask = 0xfu << (threadIdx.x & 28);   // the four threads of this K32 group (groups never straddle the tail)
-  double sums[4] = {0., 0., 0., 0.};
+  float sums[4] = {0.f, 0.f, 0.f, 0.f};
   int moved[kMaxClipOffsets] = {}, flags = 0;
   for (int64_t thread = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; thread < threads; thread += stride) {   // whole groups leave together
     const int row = threads < (int64_t(1) << 31) ? int(uint32_t(thread) / uint32_t(per_row)) : int(thread / per_row);
@@ -88,7 +89,10 @@ mx_clip_search_kernel(const uint16_t* __restrict__ in, const float* __restrict__
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) weight[i] = 1.f;
-    if (importance) {   // 16-byte aligned, see clip_pack
+    if (importance && (reinterpret_cast<uintptr_t>(importance) & 15)) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) weight[i] = importance[col + i];
+    } else if (importance) {
       const float4 a = __ldg(reinterpret_cast<const float4*>(importance + col)), b = __ldg(reinterpret_cast<const float4*>(importance + col) + 1);
       weight[0] = a.x; weight[1] = a.y; weight[2] = a.z; weight[3] = a.w;
       weight[4] = b.x; weight[5] = b.y; weight[6] = b.z; weight[7] = b.w;
@@ -104,8 +108,7 @@ mx_clip_search_kernel(const uint16_t* __restrict__ in, const float* __restrict__
       part = __fadd_rn(part, __shfl_xor_sync(mask, part, 1));
       return __fadd_rn(part, __shfl_xor_sync(mask, part, 2));
     };
-    float part, plain;
-    uint32_t best_codes = clip_candidate(v, weight, base, part, plain);
+    float plain, part = clip_candidate(v, weight, base, plain);
     float best = group_error(part), best_part = part, best_plain = plain;
     const float first = best;
     if constexpr (STATS) {
@@ -116,11 +119,14 @@ mx_clip_search_kernel(const uint16_t* __restrict__ in, const float* __restrict__
     for (int o = 0; o < offsets.count; ++o) {
       if (offsets.value[o] == 0) continue;
       const int e = max(-127, min(127, base + offsets.value[o]));
-      const uint32_t codes = clip_candidate(v, weight, e, part, plain);
+      part = clip_candidate(v, weight, e, plain);
       const float error = group_error(part);
-      if (error < best) { best = error; best_e = e; best_codes = codes; best_part = part; best_plain = plain; }
+      if (error < best) { best = error; best_e = e; best_part = part; best_plain = plain; }
     }
-    *reinterpret_cast<uint32_t*>(q4 + (int64_t(row) * k + col) / 2) = best_codes;
+    float scaled[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) scaled[i] = v[i] * mx_inverse_scale(best_e);
+    *reinterpret_cast<uint32_t*>(q4 + (int64_t(row) * k + col) / 2) = cvt_e2m1x8(scaled);
     if ((col & 31) == 0) scales[int64_t(row) * (k >> 5) + (col >> 5)] = uint8_t(best_e + 127);
     if constexpr (STATS) {
       sums[kWeightedAfter] += best_part;
@@ -151,7 +157,7 @@ mx_clip_search_kernel(const uint16_t* __restrict__ in, const float* __restrict__
       if (lane == 0) block_sum[warp][slot] = value;
     };
 #pragma unroll
-    for (int i = 0; i < 4; ++i) over_warp(sums[i], i);
+    for (int i = 0; i < 4; ++i) over_warp(double(sums[i]), i);
 #pragma unroll
     for (int i = 0; i < 3; ++i) over_warp(double((flags >> i) & 1), kNotFinite + i);
     if (lane == 0) block_sum[warp][7] = 0.;
@@ -170,6 +176,8 @@ mx_clip_search_kernel(const uint16_t* __restrict__ in, const float* __restrict__
       if (arrived == double(gridDim.x)) {
         __threadfence();
         host_stats[threadIdx.x] = threadIdx.x == kTicket ? 0. : __ldcg(stats + threadIdx.x);
+        __syncwarp(0xffffu);
+        stats[threadIdx.x] = 0.;   // ready for the next call
       }
     }
   }
@@ -180,8 +188,7 @@ static void clip_pack(const void* in, const float* importance, void* q4, void* s
   if (!in || !q4 || !scales || rows <= 0 || k <= 0 || k % 128) throw std::runtime_error("Invalid MX clip-pack arguments");
   if (n_offsets < 0 || n_offsets > kMaxClipOffsets || (n_offsets && !offsets)) throw std::runtime_error("At most 8 exponent offsets");
   if (dtype != HG_DTYPE_F16 && dtype != HG_DTYPE_BF16) throw std::runtime_error("Unknown input dtype");
-  if ((reinterpret_cast<uintptr_t>(in) & 15) || (reinterpret_cast<uintptr_t>(q4) & 3) || (reinterpret_cast<uintptr_t>(importance) & 15))
-    throw std::runtime_error("Weights and importance must be 16-byte aligned");
+  if ((reinterpret_cast<uintptr_t>(in) & 15) || (reinterpret_cast<uintptr_t>(q4) & 3)) throw std::runtime_error("Weights must be 16-byte aligned");
   ClipOffsets list{};
   list.count = n_offsets;
   for (int i = 0; i < n_offsets; ++i) {
@@ -214,14 +221,13 @@ extern "C" int hg_clip_pack(const void* in, const float* importance, void* q4, v
 }
 
 extern "C" int hg_clip_pack_stats(const void* in, const float* importance, void* q4, void* scales, int rows, int k,
-                                  const int* offsets, int n_offsets, int dtype, double* stats, double* host_stats, void* stream) {
+                                  const int* offsets, int n_offsets, int dtype, double* host_stats, void* stream) {
   HG_TRY
-  if (!stats || !host_stats || (reinterpret_cast<uintptr_t>(stats) & 7)) throw std::runtime_error("Invalid MX clip-pack arguments");
+  if (!host_stats) throw std::runtime_error("Invalid MX clip-pack arguments");
   const auto s = static_cast<cudaStream_t>(stream);
-  hg::check(cudaMemsetAsync(stats, 0, sizeof(double) * hg::kClipStats, s), "clear statistics");
-  auto* const totals = static_cast<double*>(hg::pinned_result());
-  hg::clip_pack(in, importance, q4, scales, rows, k, offsets, n_offsets, dtype, stats, totals, s);
+  const hg::HostResult result = hg::host_result();
+  hg::clip_pack(in, importance, q4, scales, rows, k, offsets, n_offsets, dtype, static_cast<double*>(result.device), static_cast<double*>(result.host), s);
   hg::check(cudaStreamSynchronize(s), "clip-pack");
-  std::copy(totals, totals + hg::kClipStats, host_stats);
+  std::copy(static_cast<double*>(result.host), static_cast<double*>(result.host) + hg::kClipStats, host_stats);
   HG_CATCH
 }

@@ -39,10 +39,12 @@ __host__ __device__ inline int64_t scale_word_offset(int row, int kb, int k) {
   return (int64_t(row / 128) * (k / 128) + kb) * 512 + (row % 32) * 16 + ((row % 128) / 32) * 4;
 }
 
-// A small pinned buffer of the calling thread that kernels can write, for calls that end with a host-side result: a
-// copy from device memory (through a pageable buffer above all) costs more than the wait itself.
-constexpr size_t kPinnedResultBytes = 256;
-void* pinned_result();
+// For calls that end with a host-side result, 256 bytes each of pinned memory that kernels can write (a copy from device
+// memory, through a pageable buffer above all, costs more than the wait itself) and of zeroed device memory that a kernel
+// leaves zeroed.  They belong to the calling thread and device and are given back with the thread; such a call waits for
+// its stream, so one at a time uses them.
+struct HostResult { void* host; void* device; };
+HostResult host_result();
 
 #ifdef __CUDACC__
 // Programmatic dependent launch.  Every kernel of the library is launched with the

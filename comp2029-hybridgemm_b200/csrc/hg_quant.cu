@@ -9,6 +9,7 @@
 // word of the 512-byte scale atom.  Threads past the real work write the 0x7f
 // padding words of the last 128-row scale block, so no memset node precedes
 // the kernel and every byte of the scale buffer is rewritten on every call.
+#include <algorithm>
 #include <cstdlib>
 
 #include "hg_common.cuh"
@@ -20,14 +21,32 @@ std::string& last_error() {
   return message;
 }
 
-void* pinned_result() {
-  struct Pinned {
-    void* ptr = nullptr;
-    ~Pinned() { if (ptr) cudaFreeHost(ptr); }
+HostResult host_result() {
+  constexpr size_t kBytes = 256;
+  constexpr int kDevices = 64;
+  struct Buffers {
+    HostResult of[kDevices] = {};
+    ~Buffers() {
+      for (HostResult& r : of) {
+        if (r.host) cudaFreeHost(r.host);
+        if (r.device) cudaFree(r.device);
+      }
+    }
   };
-  static thread_local Pinned pinned;   // one small buffer per thread, given back with it
-  if (!pinned.ptr) check(cudaHostAlloc(&pinned.ptr, kPinnedResultBytes, cudaHostAllocPortable | cudaHostAllocMapped), "pinned buffer");
-  return pinned.ptr;
+  static thread_local Buffers buffers;
+  int device = 0;
+  check(cudaGetDevice(&device), "cudaGetDevice");
+  if (device < 0 || device >= kDevices) throw std::runtime_error("Device ordinals 0..63 are supported");
+  HostResult& r = buffers.of[device];
+  if (!r.host) check(cudaHostAlloc(&r.host, kBytes, cudaHostAllocPortable | cudaHostAllocMapped), "pinned buffer");
+  if (!r.device) {
+    void* fresh = nullptr;
+    check(cudaMalloc(&fresh, kBytes), "result buffer");
+    check(cudaMemset(fresh, 0, kBytes), "result buffer");
+    check(cudaDeviceSynchronize(), "result buffer");
+    r.device = fresh;
+  }
+  return r;
 }
 
 bool pdl_enabled() {
@@ -142,11 +161,12 @@ mx_quant_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint
 // entries of the scale atoms, so scales leave as whole entries instead of single words, each a partial write of a
 // sector.  With row lists the rows are gathered: a layer's two partitions are packed from the 16-bit matrix in one
 // launch, without copies of the partitions in between.
+constexpr int kRowsBlocks = 3;   // resident blocks of mx_rows_kernel per SM: 24 warps with 4 KB in flight each
 struct QuantPart {
   const int32_t* ids;   // source row of each packed row; null = the same
   uint8_t* codes;
   uint8_t* sf;
-  int rows;
+  int rows, sources;    // packed rows; rows of the source matrix
 };
 
 struct Raw16 { uint32_t w[8]; };   // sixteen 16-bit values
@@ -208,17 +228,30 @@ __device__ __forceinline__ uint32_t quantise16(const Raw16& x, uint8_t* codes, i
   return word | __shfl_xor_sync(0xffffffffu, word, 4);
 }
 
-// Rows 128 (group / 32) + group % 32 + 32 i of a partition, columns col0 .. col0 + 511.
-template <typename T, bool FP4>
-__device__ __forceinline__ void quantise_rows(const uint16_t* __restrict__ in, const QuantPart& part, int group, int col0, int k, int lane) {
-  const int row0 = (group >> 5) * 128 + (group & 31), col = col0 + 16 * lane;
-  Raw16 raw[4];
+// Source rows of packed rows 128 (group / 32) + group % 32 + 32 r; -1: none.
+__device__ __forceinline__ void find_rows(int (&source)[4], const QuantPart& part, int group) {
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    const int row = row0 + 32 * r;
-    raw[r] = Raw16{};
-    if (row < part.rows && col < k) raw[r] = load16(in + int64_t(part.ids ? part.ids[row] : row) * k + col);
+    const int row = (group >> 5) * 128 + (group & 31) + 32 * r;
+    source[r] = -1;
+    if (row < part.rows) {
+      const int s = part.ids ? __ldg(part.ids + row) : row;
+      // a list is incomplete, its entries undefined, when ids were repeated or out of range
+      if (uint32_t(s) < uint32_t(part.sources)) source[r] = s;
+    }
   }
+}
+// Columns col .. col + 15 of this lane.
+__device__ __forceinline__ void load_rows(Raw16 (&raw)[4], const int (&source)[4], const uint16_t* __restrict__ in, int col, int k) {
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    raw[r] = Raw16{};
+    if (source[r] >= 0 && col < k) raw[r] = load16(in + int64_t(source[r]) * k + col);
+  }
+}
+template <typename T, bool FP4>
+__device__ __forceinline__ void emit_rows(const Raw16 (&raw)[4], const QuantPart& part, int group, int col, int k, int lane) {
+  const int row0 = (group >> 5) * 128 + (group & 31);
   uint32_t word[4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
@@ -233,18 +266,38 @@ __device__ __forceinline__ void quantise_rows(const uint16_t* __restrict__ in, c
     *reinterpret_cast<uint4*>(part.sf + scale_word_offset(row0, col >> 7, k)) = make_uint4(word[0], word[1], word[2], word[3]);
 }
 
-// Packs `low` to MXFP4 and `high` to MXFP8 (either may be empty).
+// Packs `low` to MXFP4 and `high` to MXFP8 (either may be empty).  Every warp walks items of one row group x 512 columns and has
+// the next item's loads in flight while it converts the current one (37888 x 3584 to MXFP4 56 us, 67 without).  Row numbers
+// another item ahead cost more in registers than their latency.
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, kRowsBlocks)
 mx_rows_kernel(const uint16_t* __restrict__ in, const QuantPart low, const QuantPart high, int k) {
   pdl_trigger();
   pdl_wait();   // input and row lists come from the kernels before
   const int lane = threadIdx.x & 31, chunks = (k + 511) >> 9;
-  const int item = blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int group = item / chunks, col0 = (item - group * chunks) << 9;
-  const int low_groups = ((low.rows + 127) & ~127) >> 2, high_groups = ((high.rows + 127) & ~127) >> 2;
-  if (group < low_groups) quantise_rows<T, true>(in, low, group, col0, k, lane);
-  else if (group < low_groups + high_groups) quantise_rows<T, false>(in, high, group - low_groups, col0, k, lane);
+  const int low_groups = ((low.rows + 127) & ~127) >> 2, groups = low_groups + (((high.rows + 127) & ~127) >> 2);
+  const int stride = gridDim.x * 8;
+  int item = blockIdx.x * 8 + (threadIdx.x >> 5);
+  int group = item / chunks, col = ((item - group * chunks) << 9) + 16 * lane;
+  Raw16 raw[4], next[4];
+  auto load = [&](Raw16 (&to)[4]) {
+    int source[4];
+    if (group < low_groups) find_rows(source, low, group);
+    else find_rows(source, high, group - low_groups);
+    load_rows(to, source, in, col, k);
+  };
+  if (group < groups) load(raw);
+  while (group < groups) {
+    const int this_group = group, this_col = col;
+    item += stride;
+    group = item / chunks;
+    col = ((item - group * chunks) << 9) + 16 * lane;
+    if (group < groups) load(next);
+    if (this_group < low_groups) emit_rows<T, true>(raw, low, this_group, this_col, k, lane);
+    else emit_rows<T, false>(raw, high, this_group - low_groups, this_col, k, lane);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) raw[r] = next[r];
+  }
 }
 
 // SwiGLU + MXFP8 for many rows; bound by the exponentials and divisions (IEEE, as SiluAndMul's) rather than by memory.
@@ -297,7 +350,7 @@ mx_silu_rows_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, 
 
 // From this many elements on the many-rows kernels are faster (K = 3584: 777 rows 3.2 us against 3.8, 2048 rows 6.5 against
 // 5.4; SwiGLU, K = 18944: 128 rows 5.7 against 7.3, 256 rows level, 2048 rows 70 against 59); below, one load per thread has
-// the shorter chain.  gate_up's 37888 x 3584 weights: 107 us against 67.
+// the shorter chain.  gate_up's 37888 x 3584 weights to MXFP4: 107 us against 56.
 constexpr int64_t kManyRowsElements = 4 << 20;
 
 static unsigned row_blocks(int64_t groups, int k) { return unsigned((groups * ((k + 511) / 512) + 7) / 8); }
@@ -305,19 +358,21 @@ static unsigned row_blocks(int64_t groups, int k) { return unsigned((groups * ((
 template <typename T>
 static cudaError_t launch_rows(const void* in, const QuantPart& low, const QuantPart& high, int k, cudaStream_t s) {
   const int64_t groups = (int64_t((low.rows + 127) & ~127) + ((high.rows + 127) & ~127)) / 4;
-  return launch_kernel(mx_rows_kernel<T>, dim3(row_blocks(groups, k)), dim3(256), 0, s, static_cast<const uint16_t*>(in), low, high, k);
+  return launch_kernel(mx_rows_kernel<T>, dim3(std::min(row_blocks(groups, k), unsigned(148 * kRowsBlocks))), dim3(256), 0, s, static_cast<const uint16_t*>(in), low, high, k);
 }
 
-// The row lists of a layer from the ids of its MXFP8 channels: one block, a bitmap of the rows in shared memory, and a
-// scan of its words.  result = {distinct ids, an id was out of range}; lists are only complete when ids are distinct.
+// The row lists of a layer from the ids of its MXFP8 channels: one block, a bitmap of the rows in shared memory, a scan of its
+// words, and a warp per word that writes 32 rows at once.  result = {distinct ids, an id was out of range}; the lists are
+// only complete when ids are distinct and in range.
 constexpr int kPartitionThreads = 1024;
 __global__ void __launch_bounds__(kPartitionThreads)
 partition_rows_kernel(const int64_t* __restrict__ ids, int n_ids, int rows, int32_t* __restrict__ lo, int32_t* __restrict__ hi, int* __restrict__ result) {
-  extern __shared__ uint32_t bitmap[];
+  extern __shared__ uint32_t bitmap[];   // words of the bitmap, then the MXFP8 rows before each word
   __shared__ int warp_sum[32];
   pdl_trigger();
   pdl_wait();
-  const int words = (rows + 31) >> 5, tid = threadIdx.x;
+  const int words = (rows + 31) >> 5, tid = threadIdx.x, lane = tid & 31;
+  int* const before = reinterpret_cast<int*>(bitmap + words);
   for (int w = tid; w < words; w += kPartitionThreads) bitmap[w] = 0;
   __syncthreads();
   int bad = 0;
@@ -334,9 +389,9 @@ partition_rows_kernel(const int64_t* __restrict__ ids, int n_ids, int rows, int3
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
     const int other = __shfl_up_sync(0xffffffffu, sum, d);
-    if ((tid & 31) >= d) sum += other;
+    if (lane >= d) sum += other;
   }
-  if ((tid & 31) == 31) warp_sum[tid >> 5] = sum;
+  if (lane == 31) warp_sum[tid >> 5] = sum;
   __syncthreads();
   if (tid < 32) {
     int total = warp_sum[tid];
@@ -348,18 +403,20 @@ partition_rows_kernel(const int64_t* __restrict__ ids, int n_ids, int rows, int3
     warp_sum[tid] = total;
   }
   __syncthreads();
-  int high = sum - mine + (tid >= 32 ? warp_sum[(tid >> 5) - 1] : 0);   // MXFP8 rows before this thread's first row
+  int running = sum - mine + (tid >= 32 ? warp_sum[(tid >> 5) - 1] : 0);
   for (int w = begin; w < end; ++w) {
+    before[w] = running;
+    running += __popc(bitmap[w]);
+  }
+  __syncthreads();
+  for (int w = tid >> 5; w < words; w += kPartitionThreads / 32) {
     const uint32_t bits = bitmap[w];
-    for (int b = 0; b < 32; ++b) {
-      const int row = w * 32 + b;
-      if (row >= rows) break;
-      if ((bits >> b) & 1u) {
-        if (high < n_ids) hi[high] = row;
-        ++high;
-      } else if (row - high < rows - n_ids) {
-        lo[row - high] = row;
-      }
+    const int row = w * 32 + lane, high = before[w] + __popc(bits & ((1u << lane) - 1u));
+    if (row >= rows) break;
+    if ((bits >> lane) & 1u) {
+      if (high < n_ids) hi[high] = row;
+    } else if (row - high < rows - n_ids) {
+      lo[row - high] = row;
     }
   }
   if (tid == 0) { result[0] = warp_sum[31]; result[1] = bad; }
@@ -373,7 +430,7 @@ static cudaError_t launch_quant(const void* in, void* out, void* sf, void* debug
       return launch_kernel(mx_silu_rows_kernel<T, MATH>, dim3(row_blocks(groups, k)), dim3(256), 0, s, static_cast<const uint16_t*>(in),
                            static_cast<uint8_t*>(out), static_cast<uint8_t*>(sf), static_cast<uint16_t*>(debug), rows, k);
     } else {
-      const QuantPart part{nullptr, static_cast<uint8_t*>(out), static_cast<uint8_t*>(sf), rows}, none{};
+      const QuantPart part{nullptr, static_cast<uint8_t*>(out), static_cast<uint8_t*>(sf), rows, rows}, none{};
       return launch_rows<T>(in, FP4 ? part : none, FP4 ? none : part, k, s);
     }
   }
@@ -419,21 +476,26 @@ static int silu_any(const void* in, void* q, void* sf, void* debug, int rows, in
 #undef HG_SILU
 }
 
-static void split_pack(const void* weight, const int64_t* ids, int n_ids, int rows, int k, int32_t* lo, int32_t* hi, void* w4, void* sf4,
-                       void* w8, void* sf8, int host_result[2], int dtype, cudaStream_t s) {
-  if (rows <= 0 || k <= 0 || k % 128 || n_ids < 0 || n_ids > rows || !weight || (n_ids && !ids)) throw std::runtime_error("Invalid split-pack arguments");
+static void split_rows(const int64_t* ids, int n_ids, int rows, int32_t* lo, int32_t* hi, cudaStream_t s) {
+  if (rows <= 0 || n_ids < 0 || n_ids > rows || (n_ids && (!ids || !hi)) || (n_ids < rows && !lo)) throw std::runtime_error("Invalid split-rows arguments");
+  const size_t shared = size_t((rows + 31) / 32) * 8;
+  if (shared > 47 * 1024) throw std::runtime_error("Too many rows for one split");
+  // the verdict goes straight to the host's buffer, over the bus: no copy afterwards
+  check(launch_kernel(partition_rows_kernel, dim3(1), dim3(kPartitionThreads), shared, s, ids, n_ids, rows, lo, hi, static_cast<int*>(host_result().host)), "partition launch");
+}
+
+static void split_pack(const void* weight, int n_ids, int rows, int k, const int32_t* lo, const int32_t* hi, void* w4, void* sf4, void* w8,
+                       void* sf8, int verdict[2], int dtype, cudaStream_t s) {
+  if (rows <= 0 || k <= 0 || k % 128 || n_ids < 0 || n_ids > rows || !weight || !verdict) throw std::runtime_error("Invalid split-pack arguments");
   if (dtype != HG_DTYPE_F16 && dtype != HG_DTYPE_BF16) throw std::runtime_error("Unknown weight dtype");
   if (reinterpret_cast<uintptr_t>(weight) & 31) throw std::runtime_error("Split-pack weights must be 32-byte aligned");
   if (!aligned16(w4) || !aligned16(sf4) || !aligned16(w8) || !aligned16(sf8)) throw std::runtime_error("MX pack pointers must be 16-byte aligned");
-  const size_t bitmap = size_t((rows + 31) / 32) * 4;
-  if (bitmap > 47 * 1024) throw std::runtime_error("Too many rows for one split-pack");
-  int* const result = static_cast<int*>(pinned_result());   // written by the kernel itself, over the bus: no copy afterwards
-  check(launch_kernel(partition_rows_kernel, dim3(1), dim3(kPartitionThreads), bitmap, s, ids, n_ids, rows, lo, hi, result), "partition launch");
-  const QuantPart low{lo, static_cast<uint8_t*>(w4), static_cast<uint8_t*>(sf4), rows - n_ids}, high{hi, static_cast<uint8_t*>(w8), static_cast<uint8_t*>(sf8), n_ids};
+  const QuantPart low{lo, static_cast<uint8_t*>(w4), static_cast<uint8_t*>(sf4), rows - n_ids, rows}, high{hi, static_cast<uint8_t*>(w8), static_cast<uint8_t*>(sf8), n_ids, rows};
   check(dtype == HG_DTYPE_BF16 ? launch_rows<__nv_bfloat16>(weight, low, high, k, s) : launch_rows<__half>(weight, low, high, k, s), "split-pack launch");
   check(cudaStreamSynchronize(s), "split-pack");
-  host_result[0] = result[0];
-  host_result[1] = result[1];
+  const int* result = static_cast<const int*>(host_result().host);
+  verdict[0] = result[0];
+  verdict[1] = result[1];
 }
 
 }  // namespace hg
@@ -461,11 +523,12 @@ int hg_pack_mode_bf16(const void* in, void* out, void* sf, int rows, int k, int 
   HG_TRY hg::pack_any(in, out, sf, rows, k, fp4, stream, true); HG_CATCH
 }
 
-int hg_split_pack(const void* weight, const int64_t* ids, int n_ids, int rows, int k, int32_t* lo, int32_t* hi, void* w4, void* sf4,
-                  void* w8, void* sf8, int* host_result, int dtype, void* stream) {
-  HG_TRY
-  if (!host_result) throw std::runtime_error("Invalid split-pack arguments");
-  hg::split_pack(weight, ids, n_ids, rows, k, lo, hi, w4, sf4, w8, sf8, host_result, dtype, static_cast<cudaStream_t>(stream)); HG_CATCH
+int hg_split_rows(const int64_t* ids, int n_ids, int rows, int32_t* lo, int32_t* hi, void* stream) {
+  HG_TRY hg::split_rows(ids, n_ids, rows, lo, hi, static_cast<cudaStream_t>(stream)); HG_CATCH
+}
+int hg_split_pack(const void* weight, int n_ids, int rows, int k, const int32_t* lo, const int32_t* hi, void* w4, void* sf4, void* w8,
+                  void* sf8, int* verdict, int dtype, void* stream) {
+  HG_TRY hg::split_pack(weight, n_ids, rows, k, lo, hi, w4, sf4, w8, sf8, verdict, dtype, static_cast<cudaStream_t>(stream)); HG_CATCH
 }
 
 int hg_silu_pack(const void* in, void* q, void* sf, void* debug, int rows, int k, void* stream, int math) {

@@ -66,12 +66,11 @@ def quantize(w: torch.Tensor, importance: torch.Tensor | None = None, offsets=(0
         if weight.shape != (k,):
             raise ValueError("importance must be k finite non-negative values")
     q4 = torch.empty((rows, k // 2), dtype=torch.uint8, device=w.device)
-    scales = torch.empty((rows, k // 32), dtype=torch.uint8, device=w.device)
-    gathered = torch.empty(16, dtype=torch.float64, device=w.device)
+    scales = q4.new_empty((rows, k // 32))
     shifts, found = (C.c_int * len(offsets))(*[int(o) for o in offsets]), (C.c_double * 16)()
     native.check(native.library().hg_clip_pack_stats(
         w.data_ptr(), weight.data_ptr() if weight is not None else None, q4.data_ptr(), scales.data_ptr(), rows, k, shifts,
-        len(offsets), native.DTYPES[w.dtype], gathered.data_ptr(), found, torch.cuda.current_stream(w.device).cuda_stream))
+        len(offsets), native.DTYPES[w.dtype], found, native._stream(w.device)))
     # One read of sixteen numbers tells whether the inputs were valid and what the search did.
     weighted_before, weighted_after, before, after, not_finite, bad_importance, grew, _, *moved = found
     if not_finite:

@@ -42,7 +42,7 @@ POLICIES = {"serial": 0, "concurrent": 1, "high_first": 2, "high_main": 3,
             "gemv_pair1": 4, "gemv_pair2": 5, "gemv_pair4": 6}
 DTYPES = {torch.float16: 0, torch.bfloat16: 1}
 
-SPLIT_PACK_ROWS = 385024   # most rows hg_split_pack takes (its bitmap of the rows lives in shared memory)
+SPLIT_PACK_ROWS = 192512   # most rows hg_split_rows takes (its bitmap of the rows lives in shared memory)
 
 _DEFAULT_LIBRARY = Path(__file__).resolve().parent.parent / "lib" / "libhygemm_b200.so"
 _lib = None
@@ -70,7 +70,8 @@ def library():
         getattr(lib, name).argtypes = [vp, vp, vp, ci, ci, ci, vp]
     for name in ("hg_pack_mode", "hg_pack_mode_bf16"):
         getattr(lib, name).argtypes = [vp, vp, vp, ci, ci, ci, vp, ci]
-    lib.hg_split_pack.argtypes = [vp, vp, ci, ci, ci] + [vp] * 6 + [C.POINTER(ci), ci, vp]
+    lib.hg_split_rows.argtypes = [vp, ci, ci, vp, vp, vp]
+    lib.hg_split_pack.argtypes = [vp, ci, ci, ci] + [vp] * 6 + [C.POINTER(ci), ci, vp]
     for name in ("hg_silu_pack", "hg_silu_pack_bf16"):
         getattr(lib, name).argtypes = [vp, vp, vp, vp, ci, ci, vp, ci]
     lib.hg_create.argtypes = [ci, ci, pp, pp, vp, C.POINTER(vp)]
@@ -90,7 +91,7 @@ def library():
     lib.hg_tp_status.argtypes = [vp, vp, C.POINTER(ci)]
     clip = [vp, vp, vp, vp, ci, ci, C.POINTER(ci), ci, ci]
     lib.hg_clip_pack.argtypes = clip + [vp]
-    lib.hg_clip_pack_stats.argtypes = clip + [vp, C.POINTER(C.c_double), vp]
+    lib.hg_clip_pack_stats.argtypes = clip + [C.POINTER(C.c_double), vp]
     lib.hg_fused_error.restype = C.c_char_p
     lib.hg_fused_create.argtypes = [ci, pp, pp, vp, C.POINTER(vp)]
     lib.hg_fused_create_dtype.argtypes = [ci, pp, pp, vp, ci, C.POINTER(vp)]
@@ -179,7 +180,7 @@ class DualLinear:
         self._ready = {}   # token count -> what a plain call needs, see _prepare
 
     def _pack_split(self, weight, high_ids) -> bool:
-        """Both partitions from one pass over the 16-bit matrix (`hg_split_pack`).  True when the selection was a CUDA
+        """Both partitions from one pass over the 16-bit matrix (`hg_split_rows`, `hg_split_pack`).  True when the selection was a CUDA
         tensor of distinct row numbers, the form every loader of this package passes; the call waits for the packing
         (the GEMM reads weights before it waits for the kernel in front of it) and tells whether it was."""
         n, k = weight.shape
@@ -191,15 +192,16 @@ class DualLinear:
         high = high_ids.numel()
         low = n - high
 
-        def empty(*shape, dtype=torch.uint8):
-            return torch.empty(shape, dtype=dtype, device=weight.device)
-        self.hi, self.lo = empty(high, dtype=torch.int32), empty(low, dtype=torch.int32)
-        self.w4, self.sf4 = empty(low, k // 2), empty(scale_size(low, k))
-        self.w8, self.sf8 = empty(high, k), empty(scale_size(high, k))
+        stream, lib = _stream(weight.device), library()
+        self.hi = torch.empty(high, dtype=torch.int32, device=weight.device)
+        self.lo = self.hi.new_empty(low)
+        check(lib.hg_split_rows(high_ids.data_ptr(), high, n, self.lo.data_ptr(), self.hi.data_ptr(), stream))
+        # the larger buffers are allocated while the maps are being written
+        self.w4 = torch.empty((low, k // 2), dtype=torch.uint8, device=weight.device)
+        self.sf4, self.w8, self.sf8 = (self.w4.new_empty(shape) for shape in (scale_size(low, k), (high, k), scale_size(high, k)))
         found = (C.c_int * 2)()
-        check(library().hg_split_pack(weight.data_ptr(), high_ids.data_ptr(), high, n, k, self.lo.data_ptr(), self.hi.data_ptr(),
-                                      self.w4.data_ptr(), self.sf4.data_ptr(), self.w8.data_ptr(), self.sf8.data_ptr(),
-                                      found, DTYPES[weight.dtype], _stream(weight.device)))
+        check(lib.hg_split_pack(weight.data_ptr(), high, n, k, self.lo.data_ptr(), self.hi.data_ptr(), self.w4.data_ptr(),
+                                self.sf4.data_ptr(), self.w8.data_ptr(), self.sf8.data_ptr(), found, DTYPES[weight.dtype], stream))
         return tuple(found) == (high, 0)
 
     def __call__(self, x):

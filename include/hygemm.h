@@ -79,14 +79,16 @@ int hg_pack_mode(const void* in, void* out, void* sf, int rows, int k, int fp4, 
 int hg_pack_bf16(const void* in, void* out, void* sf, int rows, int k, int fp4, void* stream);
 int hg_pack_mode_bf16(const void* in, void* out, void* sf, int rows, int k, int fp4, void* stream, int mode);
 
-/* Load-time packing of a [rows,k] 16-bit weight matrix (HG_DTYPE_*) into both partitions of a hybrid linear: `ids` holds the
- * output channels kept in MXFP8 (n_ids distinct values in [0,rows), any order).  Writes the sorted channel maps `hi`
- * [n_ids] and `lo` [rows-n_ids], and what hg_pack writes for the gathered rows: w4 [rows-n_ids,k/2] and sf4, w8 [n_ids,k] and
- * sf8.  host_result[2] = {distinct ids, 1 if an id was out of range}: with anything but {n_ids, 0} the
- * outputs are not complete and must not be used.  Two launches; waits for the stream.  `weight` is 32-byte aligned.  (The reference gathers and packs per
- * partition, integrations/vllm/hygemm_vllm/native.py:53-68.)  Fails for more than 385024 rows. */
-int hg_split_pack(const void* weight, const int64_t* ids, int n_ids, int rows, int k, int32_t* lo, int32_t* hi, void* w4,
-                  void* sf4, void* w8, void* sf8, int* host_result, int dtype, void* stream);
+/* Load-time packing of a [rows,k] 16-bit weight matrix (HG_DTYPE_*) into both partitions of a hybrid linear, in two calls on one
+ * stream by one thread.  hg_split_rows: `ids` holds the output channels kept in MXFP8 (n_ids distinct values in [0,rows), any
+ * order); enqueues the sorted channel maps `hi` [n_ids] and `lo` [rows-n_ids]; at most 192512 rows.  hg_split_pack: what
+ * hg_pack writes for the rows the maps name, w4 [rows-n_ids,k/2] and sf4, w8 [n_ids,k] and sf8; waits for the stream.
+ * verdict[2] = {distinct ids, 1 if an id was out of range}: with anything but {n_ids, 0} the outputs are not complete and must
+ * not be used.  `weight` is 32-byte aligned.  (The reference gathers and packs per partition,
+ * integrations/vllm/hygemm_vllm/native.py:53-68.) */
+int hg_split_rows(const int64_t* ids, int n_ids, int rows, int32_t* lo, int32_t* hi, void* stream);
+int hg_split_pack(const void* weight, int n_ids, int rows, int k, const int32_t* lo, const int32_t* hi, void* w4, void* sf4,
+                  void* w8, void* sf8, int* verdict, int dtype, void* stream);
 
 /* integrations/vllm/native/producer.cu:46-54 — SwiGLU + MXFP8 quantisation of
  * [rows,2k] gate||up; debug (optional) receives the 16-bit product.  Returns a
@@ -209,12 +211,11 @@ int hg_tp_status(int* state, void* stream, int* status);
  * LOGICAL scale bytes [rows,k/32] (offline_weights.physical_scales lays them out in atoms). */
 int hg_clip_pack(const void* in, const float* importance, void* q4, void* scales, int rows, int k,
                  const int* offsets, int n_offsets, int dtype, void* stream);
-/* The same, with the statistics of fp4_quant.py:45-58 gathered in the pass; waits for the stream.  host_stats[16] (`stats` is
- * device scratch of the same size): weighted squared error before and after, plain squared error before and after, then non-zero if a weight was not
- * finite, an importance was negative or not finite, a group's weighted error grew; [8+i] = groups whose scale byte moved by
- * offsets[i]. */
+/* The same, with the statistics of fp4_quant.py:45-58 gathered in the pass; waits for the stream.  host_stats[16]: weighted
+ * squared error before and after, plain squared error before and after, then non-zero if a weight was not finite, an
+ * importance was negative or not finite, a group's weighted error grew; [8+i] = groups whose scale byte moved by offsets[i]. */
 int hg_clip_pack_stats(const void* in, const float* importance, void* q4, void* scales, int rows, int k,
-                       const int* offsets, int n_offsets, int dtype, double* stats, double* host_stats, void* stream);
+                       const int* offsets, int n_offsets, int dtype, double* host_stats, void* stream);
 
 /* Single-kernel path kept for binding compatibility
  * (integrations/vllm/native/fused_probe.cu:7-28).  The tcgen05 kernel already
