@@ -664,37 +664,50 @@ static int tuning(const char* name, int value) {
 }
 
 // Estimated microseconds of a launch.  A K256 step of a CTA takes the longest of: the tensor core with its operand reads from
-// shared memory; a turn of the ring (from commit to the next full stage); the CTA's part of what L2 delivers (11 TB/s over
-// all SMs).  The launch takes the busiest cluster's steps or its weights' time from HBM (6.3 TB/s), whichever is longer,
-// plus a constant, a little per CTA, the last epilogue and the exchange of partials.  A ring's worth of weights is in shared
-// memory before the kernel in front has ended.  The constants are a fit to 130 measured launches (Qwen2.5-7B and
-// Mistral-7B / 4 shapes, 16 to 128 tokens; 10 % rms); the plan it prefers is 2 % slower than the best one on average.
+// shared memory; a turn of the ring (from commit to the next full stage); what L2 delivers (9 to 11 TB/s over all SMs, 110
+// bytes per nanosecond to one).  An SM stores 1.4 sectors per cycle: 128 rows of an MXFP4 tile touch 13 sectors per token, 128
+// rows of an MXFP8 tile 128, so an MXFP8 tile of 256 tokens is stored for 13 us.  Finer MXFP8 tiles spread that over more
+// CTAs (qkv of Qwen2.5-7B: 24.8 -> 17.5 us at 777 tokens, 46.7 -> 37.5 us at 2048).  Stores run under the next main loop.  The
+// launch takes the busiest cluster's time or its weights' time from HBM (6.3 TB/s), whichever is longer, plus a constant, a
+// little per CTA and the exchange of partials.  A ring's worth of weights is in shared memory before the kernel in front has
+// ended.  The constants are a fit to 200 measured launches (Qwen2.5-7B and Mistral-7B / 4 shapes, 16 to 2048 tokens).
 static double plan_cost(const ClusterPlan& plan, int64_t units, int kblocks, double weight_megabytes) {
   const double steps = double((kblocks + 1) / 2) / plan.split;
   const int cluster_ctas = plan.pair * plan.split, ctas = plan.clusters * cluster_ctas;
   double prefetched = 0;
-  auto unit = [&](int n, bool high) {
+  auto main_loop = [&](int n, bool high) {
     const double b = double(n) / plan.pair;
     const double mma = 2 * (plan.pair == 2 ? std::max(2.0 * n, 200.0 + b) : std::max(171.0, 128.0 + 1.3 * b)) / 1900;
-    const double kilobytes = double(kTileRows >> plan.cut_log[high]) * (high ? 0.25 : 0.125) + b * 0.25 + 2;
-    const double step = std::max({mma, 1.42 / plan.stages, kilobytes * ctas / 11000});
+    auto kilobytes = [&](int part) { return double(kTileRows >> plan.cut_log[part]) * (part ? 0.25 : 0.125) + b * 0.25 + 2; };
+    const double average = (kilobytes(0) * plan.tiles[0] + kilobytes(1) * plan.tiles[1]) / (double(plan.tiles[0]) + plan.tiles[1]);
+    const double step = std::max({mma, 1.42 / plan.stages, average * ctas / (n > 128 ? 9000 : 11000), kilobytes(high) / 110});
     prefetched = std::max(prefetched, std::min(steps, double(plan.stages)) * (step - mma));
     return steps * step + (plan.split > 1 ? 0.5 + 0.011 * n : 0.15);
   };
-  const double whole = unit(plan.n_tile, false), last = unit(plan.n_tail, false);
-  double busiest;
-  if (plan.token_tiles == 1) {   // MXFP8 tiles first, round the clusters
-    const double high = unit(plan.n_tail, true);
-    const int64_t turns = (units + plan.clusters - 1) / plan.clusters, high_turns = (plan.tiles[1] + plan.clusters - 1) / plan.clusters;
-    busiest = double(high_turns) * high + double(turns - high_turns) * last;
-  } else {
-    std::vector<double> load(size_t(plan.clusters), 0.0);
-    for (int64_t u = 0; u < units; ++u) load[size_t(u % plan.clusters)] += u % plan.token_tiles == plan.token_tiles - 1 ? last : whole;
-    busiest = *std::max_element(load.begin(), load.end());
+  auto stores = [&](int n, bool high) {
+    const double rows = double(kTileRows >> plan.cut_log[high]);
+    return 0.35 + std::max(0.0185 * n, n * rows * (high ? 0.72 : 0.1) / 1900) / plan.split;
+  };
+  const double main_of[2][2] = {{main_loop(plan.n_tile, false), main_loop(plan.n_tail, false)},
+                                {plan.tiles[1] ? main_loop(plan.n_tile, true) : 0, plan.tiles[1] ? main_loop(plan.n_tail, true) : 0}};
+  const double store_of[2][2] = {{stores(plan.n_tile, false), stores(plan.n_tail, false)}, {stores(plan.n_tile, true), stores(plan.n_tail, true)}};
+  std::vector<double> load(size_t(plan.clusters), 0.0), storing(size_t(plan.clusters), 0.0);   // end of a cluster's main loops, of its stores
+  const int64_t tiles = int64_t(plan.tiles[0]) + plan.tiles[1];
+  for (int64_t u = 0; u < units; ++u) {
+    const int64_t t = u / plan.token_tiles;
+    const bool tail = u % plan.token_tiles == plan.token_tiles - 1;
+    const bool high = plan.token_tiles == 1 ? t < plan.tiles[1] : (t + 1) * plan.tiles[1] / tiles > t * plan.tiles[1] / tiles;
+    double &main_end = load[size_t(u % plan.clusters)], &store_end = storing[size_t(u % plan.clusters)];
+    // two accumulators: a main loop starts once the stores before the last ones are done
+    main_end += main_of[high][tail];
+    const double begin = std::max(main_end, store_end);
+    main_end = std::max(main_end, store_end);
+    store_end = begin + store_of[high][tail];
   }
-  const double epilogue = 0.35 + 0.0185 * plan.n_tail / plan.split;
+  const double busiest = *std::max_element(storing.begin(), storing.end());
   const double exchange = plan.split > 1 ? 0.14 * std::log2(double(cluster_ctas)) - 0.17 : 0.0;
-  return 2.2 + 0.012 * ctas + std::max(busiest - prefetched, weight_megabytes / 6.3) + epilogue + exchange;
+  const double least = weight_megabytes / 6.3 + store_of[0][1];
+  return 2.2 + 0.012 * ctas + 0.1 * (plan.cut_log[1] - plan.cut_log[0]) + std::max(busiest - prefetched, least) + exchange;
 }
 
 // Ring, TMEM and shared-memory figures that follow from the other choices.  False when the ring would be too shallow.
@@ -725,7 +738,7 @@ ClusterPlan make_cluster_plan(int lo, int hi, int tokens, int k, const int max_c
   for (int pair = 1; pair <= 2; ++pair)
     for (int log = pair - 1; log < 4; ++log)
       for (int cut = 0; cut < 3; ++cut)
-        for (int more = 0; more < 2; ++more)
+        for (int more = 0; more < 3; ++more)
           for (int n : {0, 128, 256}) {
               ClusterPlan plan;
               plan.pair = pair;
@@ -738,7 +751,7 @@ ClusterPlan make_cluster_plan(int lo, int hi, int tokens, int k, const int max_c
                 plan.n_tile = plan.n_tail = (tokens + 16 * pair - 1) / (16 * pair) * (16 * pair);
                 plan.token_tiles = 1;
               } else {
-                if (!n || pair == 1 || cut || more || (n == 256 && plan.split > 1)) continue;
+                if (!n || pair == 1 || cut || (n == 256 && plan.split > 1)) continue;
                 plan.n_tile = n;
                 plan.token_tiles = (tokens + n - 1) / n;
                 plan.n_tail = (tokens - (plan.token_tiles - 1) * n + 31) / 32 * 32;

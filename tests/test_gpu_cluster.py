@@ -1,0 +1,23 @@
+"""The cluster GEMM where its plan changes: token counts on both sides of every tile width and of the single / paired CTA
+switch, K with odd and single K128 blocks (also cut over a cluster), row counts around a tile.
+
+Operands are exactly representable and their sums stay below 2^24 quanta, so every order of summation gives the same fp32
+value: results must be equal bit for bit (tolerance 0).
+"""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from helpers import run_gemm
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("tokens", [1, 16, 17, 32, 33, 64, 65, 96, 127, 129, 255, 257, 290])
+def test_exact_at_the_edges_of_the_plan(tokens):
+    for outputs, k, high in [(129, 128, 1), (640, 896, 128), (385, 2432, 129)]:
+        case = oracle.exact_case(outputs, tokens, k, high, "random")
+        got, guards, status = run_gemm(case, torch.bfloat16, 0)
+        assert status[0] == 0 and guards, (outputs, k, high, status)
+        assert np.array_equal(got, case["expected"]), (outputs, k, high, int((got != case["expected"]).sum()))
