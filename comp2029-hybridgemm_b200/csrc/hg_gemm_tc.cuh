@@ -77,6 +77,8 @@ void validate(const hg_problem& l, const hg_problem& h, bool fused = false);
 
 // hg_pack to E4M3 codes and scales (HG_DTYPE_* input).
 void pack_activations(const void* x, void* codes, void* scales, int tokens, int k, int dtype, cudaStream_t stream);
+// hg_silu_pack of gate||up [tokens,2k].
+void silu_pack_activations(const void* x, void* codes, void* scales, int tokens, int k, int dtype, int math, cudaStream_t stream);
 
 void run_simt_pair(const hg_problem& l, const hg_problem& h, cudaStream_t stream, int tokens_per_pass, int dtype);
 

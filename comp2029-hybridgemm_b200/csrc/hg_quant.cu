@@ -498,6 +498,10 @@ static void split_pack(const void* weight, int n_ids, int rows, int k, const int
   verdict[1] = result[1];
 }
 
+void silu_pack_activations(const void* x, void* codes, void* scales, int tokens, int k, int dtype, int math, cudaStream_t stream) {
+  check(cudaError_t(silu_any(x, codes, scales, nullptr, tokens, k, stream, math, dtype == HG_DTYPE_BF16)), "SwiGLU producer");
+}
+
 }  // namespace hg
 
 extern "C" {

@@ -108,26 +108,35 @@ int hg_run_x(void* handle, const hg_problem* l, const hg_problem* h, const void*
   HG_CATCH
 }
 
-int hg_linear(void* handle, const hg_problem* l, const hg_problem* h, const void* x, int x_dtype, void* workspace, void* output, void* stream) {
-  HG_TRY
-  if (!handle || !l || !h || !x || !output) throw std::runtime_error("Null argument to hg_linear");
+// hg_linear and hg_linear_silu: quantise into the workspace and multiply, or (no workspace) both in one launch.
+static void run_linear(void* handle, const hg_problem* l, const hg_problem* h, const void* x, int x_dtype, bool swiglu, int math,
+                       void* workspace, void* output, cudaStream_t s) {
+  if (!handle || !l || !h || !x || !output || (swiglu && !workspace)) throw std::runtime_error("Null argument to a layer call");
   if (x_dtype != HG_DTYPE_F16 && x_dtype != HG_DTYPE_BF16) throw std::runtime_error("Unknown activation dtype");
   auto* runner = static_cast<hg::Runner*>(handle);
-  const auto s = static_cast<cudaStream_t>(stream);
   hg_problem low = *l, high = *h;
   low.output = high.output = output;
   if (!workspace) {
     low.activation = high.activation = low.activation_scales = high.activation_scales = nullptr;
     runner->run_x(low, high, x, x_dtype, s);
-  } else {
-    const int tokens = l->rows ? l->tokens : h->tokens, k = l->rows ? l->k : h->k;
-    auto* codes = static_cast<unsigned char*>(workspace);
-    low.activation = high.activation = codes;
-    low.activation_scales = high.activation_scales = codes + int64_t(tokens) * k;
-    hg::pack_activations(x, codes, codes + int64_t(tokens) * k, tokens, k, x_dtype, s);
-    runner->run(low, high, s, HG_POLICY_SERIAL);
+    return;
   }
-  HG_CATCH
+  const int tokens = l->rows ? l->tokens : h->tokens, k = l->rows ? l->k : h->k;
+  auto* codes = static_cast<unsigned char*>(workspace);
+  auto* scales = codes + int64_t(tokens) * k;
+  low.activation = high.activation = codes;
+  low.activation_scales = high.activation_scales = scales;
+  if (swiglu) hg::silu_pack_activations(x, codes, scales, tokens, k, x_dtype, math, s);
+  else hg::pack_activations(x, codes, scales, tokens, k, x_dtype, s);
+  runner->run(low, high, s, HG_POLICY_SERIAL);
+}
+
+int hg_linear(void* handle, const hg_problem* l, const hg_problem* h, const void* x, int x_dtype, void* workspace, void* output, void* stream) {
+  HG_TRY run_linear(handle, l, h, x, x_dtype, false, 0, workspace, output, static_cast<cudaStream_t>(stream)); HG_CATCH
+}
+
+int hg_linear_silu(void* handle, const hg_problem* l, const hg_problem* h, const void* x, int x_dtype, int math, void* workspace, void* output, void* stream) {
+  HG_TRY run_linear(handle, l, h, x, x_dtype, true, math, workspace, output, static_cast<cudaStream_t>(stream)); HG_CATCH
 }
 
 int hg_run_partial(void* handle, const hg_problem* l, const hg_problem* h, const void* x, int x_dtype,

@@ -79,6 +79,7 @@ def library():
     lib.hg_run.argtypes = [vp, pp, pp, vp, ci]
     lib.hg_run_x.argtypes = [vp, pp, pp, vp, ci, vp]
     lib.hg_linear.argtypes = [vp, pp, pp, vp, ci, vp, vp, vp]
+    lib.hg_linear_silu.argtypes = [vp, pp, pp, vp, ci, ci, vp, vp, vp]
     lib.hg_info.argtypes = [vp, C.POINTER(ci)]
     lib.hg_status.argtypes = [vp, vp, C.POINTER(ci)]
     lib.hg_destroy.argtypes, lib.hg_destroy.restype = [vp], None
@@ -212,15 +213,33 @@ class DualLinear:
         dtype = DTYPES.get(x.dtype)
         if not tokens or dtype is None or self.plans or PACK_MODE or not x.is_contiguous() or 28 <= self.low_id <= 34:
             return self.run_packed(*pack(x))
+        return self._call(x, tokens, dtype, None)
+
+    def silu_linear(self, x, math):
+        """This layer on SwiGLU of `x` = gate||up `[tokens, 2K]`: `producer.silu_pack` followed by `run_packed`."""
+        shape = x.shape
+        dtype = DTYPES.get(x.dtype)
+        if (len(shape) != 2 or shape[1] != 2 * self.k or not shape[0] or dtype is None or x.device != self.w4.device
+                or self.plans or not x.is_contiguous() or 28 <= self.low_id <= 34):
+            from .producer import silu_pack
+            return self.run_packed(*silu_pack(x, math))
+        return self._call(x, shape[0], dtype, math)
+
+    def _call(self, x, tokens, dtype, math):
         # One foreign call for the whole layer: decode sizes quantise inside the GEMM launch, others into a workspace.
         # (Fresh tensors per call: under CUDA-graph capture the graph's pool owns them.)
         ready = self._ready.get(tokens)
         if ready is None or ready[0] is not self.w4 or ready[1] is not self.sf4 or ready[2] != (self.low_id, self.high_id):
             ready = self._prepare(tokens, x)
         y = ready[7].new_empty((tokens, self.outputs))
-        workspace = self.w4.new_empty(ready[6]) if ready[6] else None
-        status = _lib.hg_linear(ready[3], ready[4], ready[5], x.data_ptr(), dtype, workspace.data_ptr() if ready[6] else None,
-                                y.data_ptr(), torch._C._cuda_getCurrentRawStream(x.device.index))
+        stream = torch._C._cuda_getCurrentRawStream(x.device.index)
+        if math is not None:
+            workspace = self.w4.new_empty(tokens * self.k + scale_size(tokens, self.k))
+            status = _lib.hg_linear_silu(ready[3], ready[4], ready[5], x.data_ptr(), dtype, math, workspace.data_ptr(), y.data_ptr(), stream)
+        else:
+            workspace = self.w4.new_empty(ready[6]) if ready[6] else None
+            status = _lib.hg_linear(ready[3], ready[4], ready[5], x.data_ptr(), dtype, workspace.data_ptr() if ready[6] else None,
+                                    y.data_ptr(), stream)
         if status:
             check(status)
         self.calls[tokens] = self.calls.get(tokens, 0) + 1

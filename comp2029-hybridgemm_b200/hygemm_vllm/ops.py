@@ -30,16 +30,22 @@ def _linear_fake(x, handle, outputs):
     return x.new_empty((x.shape[0], outputs))
 
 
-def _linear_silu(x: torch.Tensor, handle: int, outputs: int, math: int) -> torch.Tensor:
+def _silu_linear(runtime, x, math):
+    if hasattr(runtime, "silu_linear"):
+        return runtime.silu_linear(x, math)
     from .producer import silu_pack
+    return runtime.run_packed(*silu_pack(x, math))
+
+
+def _linear_silu(x: torch.Tensor, handle: int, outputs: int, math: int) -> torch.Tensor:
     runtime = _runtimes[handle]
     if hasattr(runtime, "profile_name") and torch.cuda.is_current_stream_capturing():
         # Same NVTX label as the reference's profiling hook (producer.py:31).
         label = (f"projection|{runtime.profile_name}|O={runtime.outputs}|K={runtime.k}"
                  f"|H={runtime.hi.numel()}|T={x.shape[0]}")
         with torch.cuda.nvtx.range(label):
-            return runtime.run_packed(*silu_pack(x, math))
-    return runtime.run_packed(*silu_pack(x, math))
+            return _silu_linear(runtime, x, math)
+    return _silu_linear(runtime, x, math)
 
 
 def _linear_silu_fake(x, handle, outputs, math):

@@ -119,6 +119,9 @@ int hg_run_x(void* handle, const hg_problem* low, const hg_problem* high, const 
  * hg_pack into it followed by hg_run; without one it is hg_run_x (at most 16 tokens). */
 int hg_linear(void* handle, const hg_problem* low, const hg_problem* high, const void* x, int x_dtype, void* workspace,
               void* output, void* stream);
+/* The same for the SwiGLU of `x` = gate||up [tokens,2k]: hg_silu_pack (`math` as there) into the workspace, then hg_run. */
+int hg_linear_silu(void* handle, const hg_problem* low, const hg_problem* high, const void* x, int x_dtype, int math,
+                   void* workspace, void* output, void* stream);
 /* integrations/vllm/native/runtime.cu:151-161 — 10 ints per partition: id, tile_m,
  * tile_n, tile_k, stages, registers, shared bytes, local bytes, fp8, pingpong (-1 if absent). */
 int hg_info(void* handle, int* out20);

@@ -10,6 +10,7 @@ import torch
 
 import oracle
 from helpers import run_gemm
+from hygemm_vllm import native, producer
 
 pytestmark = pytest.mark.gpu
 
@@ -21,3 +22,20 @@ def test_exact_at_the_edges_of_the_plan(tokens):
         got, guards, status = run_gemm(case, torch.bfloat16, 0)
         assert status[0] == 0 and guards, (outputs, k, high, status)
         assert np.array_equal(got, case["expected"]), (outputs, k, high, int((got != case["expected"]).sum()))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_swiglu_layer_call_equals_producer_then_gemm(dtype):
+    """One foreign call for SwiGLU and down_proj: the same bytes as the producer followed by the GEMM on its codes."""
+    g = torch.Generator().manual_seed(3)
+    for outputs, k, high in [(257, 128, 26), (300, 896, 0), (640, 2432, 128), (384, 256, 384)]:
+        layer = native.DualLinear((torch.randn(outputs, k, generator=g) * 0.04).to(dtype).cuda(), torch.randperm(outputs, generator=g)[:high].cuda())
+        for tokens in (1, 8, 17, 130):
+            x = torch.randn(tokens, 2 * k, generator=g) * 2
+            x[0, :64] = 0
+            x = x.to(dtype).cuda()
+            got = layer.silu_linear(x, 0)
+            want = layer.run_packed(*producer.silu_pack(x, 0))
+            assert torch.equal(got.view(torch.int16), want.view(torch.int16)), (outputs, k, high, tokens)
+        assert layer.status()[0] == 0
+        layer.close()
