@@ -1,0 +1,224 @@
+// Host path of one layer call (`DualLinear.__call__`, `DualLinear.silu_linear`) as a CPython extension.
+//
+// A call at decode sizes is bounded by the host: 3.4 us of GPU time at 8 tokens of 896 -> 4864.  Through ctypes and
+// torch's Python bindings the host needed 7.3 us a call, of which 2.4 us are the launch itself; the rest was the output
+// allocation (1.9 us), the foreign call (0.9 us) and Python bytecode.  Here one C call checks the argument, finds the
+// prepared state of the token count, allocates and launches: 4.4 us.
+//
+// The module holds no state of its own but the addresses of the library's entry points.  It is built against the torch
+// that loads it and knows nothing of CUDA beyond the current stream.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/core/Tensor.h>
+#include <ATen/ops/empty.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <exception>
+
+#include "../../include/hygemm.h"
+
+namespace {
+
+decltype(&hg_linear) run_linear = nullptr;
+decltype(&hg_linear_silu) run_linear_silu = nullptr;
+decltype(&hg_last_error) last_error = nullptr;
+
+PyObject *s_ready, *s_w4, *s_sf4, *s_low_id, *s_high_id, *s_plans, *s_calls;
+
+const char kName[] = "hygemm.ready";
+
+// What calls of one layer with one token count share.  Valid while the layer still has the same weights and schedule ids.
+struct Ready {
+  PyObject *w4, *sf4, *low_id, *high_id, *problems;   // owned
+  void* handle;
+  const hg_problem *low, *high;                       // inside `problems`
+  int64_t tokens, k, outputs, packed;                 // packed: bytes of the quantised activations
+  bool fused;                                         // eager calls quantise inside the GEMM launch
+  at::TensorOptions output, bytes;
+  c10::Device device = c10::Device(c10::kCPU);
+};
+
+Ready* ready_of(PyObject* capsule) { return static_cast<Ready*>(PyCapsule_GetPointer(capsule, kName)); }
+
+void destroy(PyObject* capsule) {
+  Ready* r = ready_of(capsule);
+  if (!r) return;
+  for (PyObject* o : {r->w4, r->sf4, r->low_id, r->high_id, r->problems}) Py_XDECREF(o);
+  delete r;
+}
+
+// True when attribute `name` of `layer` is `wanted` (the same object, or an equal int).
+bool unchanged(PyObject* layer, PyObject* name, PyObject* wanted) {
+  PyObject* now = PyObject_GetAttr(layer, name);
+  if (!now) { PyErr_Clear(); return false; }
+  bool same = now == wanted;
+  if (!same && PyLong_Check(now)) {
+    const int equal = PyObject_RichCompareBool(now, wanted, Py_EQ);
+    if (equal < 0) PyErr_Clear();
+    same = equal == 1;
+  }
+  Py_DECREF(now);
+  return same;
+}
+
+// The prepared state of a call, a new reference; null without an error when the call is not a prepared, ordinary one.
+PyObject* find(PyObject* layer, int64_t tokens) {
+  PyObject* plans = PyObject_GetAttr(layer, s_plans);
+  if (!plans) return nullptr;
+  const int planned = PyObject_IsTrue(plans);
+  Py_DECREF(plans);
+  if (planned) return nullptr;
+  PyObject* all = PyObject_GetAttr(layer, s_ready);
+  if (!all) return nullptr;
+  PyObject* capsule = nullptr;
+  PyObject* key = PyLong_FromLongLong(tokens);
+  if (key && PyDict_Check(all)) {
+    capsule = PyDict_GetItemWithError(all, key);
+    Py_XINCREF(capsule);
+  }
+  Py_XDECREF(key);
+  Py_DECREF(all);
+  return capsule;
+}
+
+bool count_call(PyObject* layer, int64_t tokens) {
+  PyObject* calls = PyObject_GetAttr(layer, s_calls);
+  if (!calls) return false;
+  bool ok = false;
+  PyObject* key = PyLong_FromLongLong(tokens);
+  if (key && PyDict_Check(calls)) {
+    PyObject* old = PyDict_GetItemWithError(calls, key);
+    if (old || !PyErr_Occurred()) {
+      PyObject* sum = PyLong_FromLongLong((old ? PyLong_AsLongLong(old) : 0) + 1);
+      ok = sum && !PyErr_Occurred() && PyDict_SetItem(calls, key, sum) == 0;
+      Py_XDECREF(sum);
+    }
+  }
+  Py_XDECREF(key);
+  Py_DECREF(calls);
+  return ok;
+}
+
+PyObject* forward_checked(PyObject* layer, const at::Tensor& x, long math) {
+  const bool swiglu = math >= 0;
+  if (x.dim() != 2) Py_RETURN_NONE;
+  const auto type = x.scalar_type();
+  if (type != at::kHalf && type != at::kBFloat16) Py_RETURN_NONE;
+  const int64_t tokens = x.size(0);
+  PyObject* capsule = find(layer, tokens);
+  if (!capsule) {
+    if (PyErr_Occurred()) return nullptr;
+    Py_RETURN_NONE;
+  }
+  struct Release { PyObject* o; ~Release() { Py_DECREF(o); } } release{capsule};
+  const Ready* r = ready_of(capsule);
+  if (!r) return nullptr;
+  if (x.size(1) != (swiglu ? 2 * r->k : r->k) || x.device() != r->device || !x.is_contiguous() ||
+      !unchanged(layer, s_w4, r->w4) || !unchanged(layer, s_sf4, r->sf4) || !unchanged(layer, s_low_id, r->low_id) ||
+      !unchanged(layer, s_high_id, r->high_id))
+    Py_RETURN_NONE;
+  // Fresh tensors per call: under CUDA-graph capture the graph's pool owns them.
+  at::Tensor y = at::empty({r->tokens, r->outputs}, r->output);
+  at::Tensor workspace;
+  // Quantising inside the GEMM saves an eager call 2.5 us of host time for the second launch.  A replayed graph does not pay
+  // that, and there the separate quantiser runs under the end of the kernel in front: a decoder block of Qwen2.5-7B takes 43.2
+  // against 44.8 us at 8 tokens, 44.6 against 45.2 us at 16; one token is level or better in one launch.
+  const bool in_gemm = !swiglu && r->fused &&
+                       (tokens == 1 || c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None);
+  const int64_t bytes = in_gemm ? 0 : r->packed;
+  if (bytes) workspace = at::empty({bytes}, r->bytes);
+  const void* in = x.const_data_ptr();
+  void* out = y.mutable_data_ptr();
+  void* scratch = bytes ? workspace.mutable_data_ptr() : nullptr;
+  void* stream = c10::cuda::getCurrentCUDAStream(r->device.index()).stream();
+  const int dtype = type == at::kBFloat16 ? HG_DTYPE_BF16 : HG_DTYPE_F16;
+  int status;
+  Py_BEGIN_ALLOW_THREADS
+  status = swiglu ? run_linear_silu(r->handle, r->low, r->high, in, dtype, int(math), scratch, out, stream)
+                  : run_linear(r->handle, r->low, r->high, in, dtype, scratch, out, stream);
+  Py_END_ALLOW_THREADS
+  if (status) return PyErr_SetString(PyExc_RuntimeError, last_error()), nullptr;
+  if (!count_call(layer, tokens)) return nullptr;
+  return THPVariable_Wrap(std::move(y));
+}
+
+// forward(layer, x, math): the layer on `x`, of SwiGLU of `x` when math >= 0.  None: not an ordinary call, or the first one.
+PyObject* forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 3) return PyErr_SetString(PyExc_TypeError, "forward(layer, x, math)"), nullptr;
+  if (!run_linear || !THPVariable_Check(args[1])) Py_RETURN_NONE;
+  const long math = PyLong_AsLong(args[2]);
+  if (math == -1 && PyErr_Occurred()) return nullptr;
+  try {
+    return forward_checked(args[0], THPVariable_Unpack(args[1]), math);
+  } catch (const c10::OutOfMemoryError& e) {
+    PyObject* type = PyObject_GetAttrString(PyImport_AddModule("torch"), "OutOfMemoryError");
+    PyErr_SetString(type ? type : PyExc_RuntimeError, e.what_without_backtrace());
+    Py_XDECREF(type);
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+  }
+  return nullptr;
+}
+
+// prepare(layer, tokens, handle, low, high, problems, y, packed, fused): the state `forward` looks up.
+// `low` and `high` are addresses of the two structs that `problems` keeps alive, `y` is a tensor like the output.
+PyObject* prepare(PyObject*, PyObject* args) {
+  PyObject *layer, *problems, *y;
+  long long tokens, packed;
+  int fused;
+  unsigned long long handle, low, high;
+  if (!PyArg_ParseTuple(args, "OLKKKOOLp", &layer, &tokens, &handle, &low, &high, &problems, &y, &packed, &fused)) return nullptr;
+  if (!THPVariable_Check(y)) return PyErr_SetString(PyExc_TypeError, "prepare: y must be a tensor"), nullptr;
+  auto* r = new Ready{};
+  PyObject** slots[4] = {&r->w4, &r->sf4, &r->low_id, &r->high_id};
+  PyObject* names[4] = {s_w4, s_sf4, s_low_id, s_high_id};
+  r->problems = Py_NewRef(problems);
+  PyObject* capsule = PyCapsule_New(r, kName, destroy);
+  if (!capsule) return nullptr;
+  for (int i = 0; i < 4; ++i)
+    if (!(*slots[i] = PyObject_GetAttr(layer, names[i]))) return Py_DECREF(capsule), nullptr;
+  const at::Tensor& like = THPVariable_Unpack(y);
+  r->handle = reinterpret_cast<void*>(uintptr_t(handle));
+  r->low = reinterpret_cast<const hg_problem*>(uintptr_t(low));
+  r->high = reinterpret_cast<const hg_problem*>(uintptr_t(high));
+  r->tokens = tokens;
+  r->outputs = like.size(1);
+  r->k = r->low->k;
+  r->packed = packed;
+  r->fused = fused;
+  r->device = like.device();
+  r->output = at::TensorOptions().dtype(like.scalar_type()).device(like.device());
+  r->bytes = r->output.dtype(at::kByte);
+  return capsule;
+}
+
+// bind(hg_linear, hg_linear_silu, hg_last_error): addresses in the loaded library.
+PyObject* bind(PyObject*, PyObject* args) {
+  unsigned long long linear, silu, error;
+  if (!PyArg_ParseTuple(args, "KKK", &linear, &silu, &error)) return nullptr;
+  run_linear = reinterpret_cast<decltype(run_linear)>(uintptr_t(linear));
+  run_linear_silu = reinterpret_cast<decltype(run_linear_silu)>(uintptr_t(silu));
+  last_error = reinterpret_cast<decltype(last_error)>(uintptr_t(error));
+  Py_RETURN_NONE;
+}
+
+PyMethodDef methods[] = {
+    {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(forward)), METH_FASTCALL, nullptr},
+    {"prepare", prepare, METH_VARARGS, nullptr},
+    {"bind", bind, METH_VARARGS, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_hygemm_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__hygemm_host() {
+  PyObject** names[] = {&s_ready, &s_w4, &s_sf4, &s_low_id, &s_high_id, &s_plans, &s_calls};
+  const char* text[] = {"_ready", "w4", "sf4", "low_id", "high_id", "plans", "calls"};
+  for (int i = 0; i < 7; ++i)
+    if (!(*names[i] = PyUnicode_InternFromString(text[i]))) return nullptr;
+  return PyModule_Create(&module);
+}

@@ -1,4 +1,4 @@
-"""ctypes binding of the CUDA library and the per-layer runtime (`DualLinear`).
+"""Binding of the CUDA library (ctypes; the layer call itself goes through csrc/hg_host.cpp) and the per-layer runtime (`DualLinear`).
 
 Host-side mirror of the reference's `integrations/vllm/hygemm_vllm/native.py`:
 same names (`Problem`, `library`, `check`, `pack`, `DualLinear`, `POLICIES`),
@@ -14,6 +14,8 @@ from), and both precision partitions run in ONE persistent tcgen05 launch.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 from pathlib import Path
 
@@ -28,12 +30,12 @@ class Problem(C.Structure):
 
 
 PACK_MODE = int(os.environ.get("HYGEMM_PACK_MODE", "0"))
-# Decode sizes (at most FUSED_QUANT_TOKENS tokens) quantise the activations inside the GEMM kernel
-# (`hg_run_x`: one launch instead of two, identical bytes); HYGEMM_FUSED_QUANT=0 turns it off.
+# Eager calls at decode sizes (at most FUSED_QUANT_TOKENS tokens; one token in captured calls) quantise the activations inside
+# the GEMM kernel (`hg_run_x`: one launch instead of two, identical bytes); HYGEMM_FUSED_QUANT=0 turns it off.
 FUSED_QUANT_TOKENS = 16 if os.environ.get("HYGEMM_FUSED_QUANT", "1") != "0" else 0
 # Every CTA quantises the K slice it multiplies, so the work repeats once per row tile; layers wider than this
-# many output channels keep the separate quantiser launch (gate_up, 37888 wide, measured 30.8 us with its own
-# quantiser launch against 36.3 us fused at 16 tokens; the narrow layers gain from the missing launch).
+# many output channels keep the separate quantiser launch (a decoder block with gate_up, 37888 wide, measured 45.2 us with its
+# own quantiser launch against 51.0 us fused at 16 tokens; narrow eager layers gain the host time of the launch).
 FUSED_QUANT_MAX_OUTPUTS = int(os.environ.get("HYGEMM_FUSED_QUANT_MAX_OUTPUTS", "8192"))
 # Row-parallel exchange: up to this many tokens the partial sums cross NVLink as fp32 (rounded once after the sum).
 FUSED_QUANT_TOKENS_F32 = 16
@@ -45,7 +47,9 @@ DTYPES = {torch.float16: 0, torch.bfloat16: 1}
 SPLIT_PACK_ROWS = 192512   # most rows hg_split_rows takes (its bitmap of the rows lives in shared memory)
 
 _DEFAULT_LIBRARY = Path(__file__).resolve().parent.parent / "lib" / "libhygemm_b200.so"
+_HOST_EXTENSION = _DEFAULT_LIBRARY.with_name("_hygemm_host.so")
 _lib = None
+_host = None   # the layer call's host path (csrc/hg_host.cpp), loaded with the library
 
 
 def library_path() -> Path:
@@ -54,13 +58,16 @@ def library_path() -> Path:
 
 def library():
     """Load the shared library once and declare its prototypes (reference: native.py:19-32)."""
-    global _lib
+    global _lib, _host
     if _lib is not None:
         return _lib
     path = library_path()
     if not path.exists():
         raise FileNotFoundError(f"HyGEMM CUDA library not found at {path}; build it with "
                                 f"`python {_DEFAULT_LIBRARY.parent.parent / 'build.py'}` or set HYGEMM_LIBRARY")
+    if not _HOST_EXTENSION.exists():
+        raise FileNotFoundError(f"HyGEMM host extension not found at {_HOST_EXTENSION}; build it with "
+                                f"`python {_DEFAULT_LIBRARY.parent.parent / 'build.py'}`")
     lib = C.CDLL(str(path))
     vp, ci = C.c_void_p, C.c_int
     pp = C.POINTER(Problem)
@@ -100,7 +107,10 @@ def library():
     lib.hg_fused_run.argtypes = [vp, vp]
     lib.hg_fused_info.argtypes = [vp, C.POINTER(ci)]
     lib.hg_fused_destroy.argtypes, lib.hg_fused_destroy.restype = [vp], None
-    _lib = lib
+    loader = importlib.machinery.ExtensionFileLoader("_hygemm_host", str(_HOST_EXTENSION))
+    host = importlib.util.module_from_spec(importlib.util.spec_from_loader("_hygemm_host", loader))
+    host.bind(*(C.cast(f, vp).value for f in (lib.hg_linear, lib.hg_linear_silu, lib.hg_last_error)))
+    _lib, _host = lib, host
     return lib
 
 
@@ -171,6 +181,7 @@ class DualLinear:
             # The GEMM starts reading weights before it waits for the kernel in front of it (programmatic
             # dependent launch), so the packed weights must be complete before the first call: load time only.
             torch.cuda.current_stream(weight.device).synchronize()
+        library()
         self.low_id, self.high_id, self.concurrent = low_id, high_id, concurrent
         self.handles = {}
         self.fused_handles = {}
@@ -178,7 +189,7 @@ class DualLinear:
         self.plans = plans
         self.plans_used = {}
         self._problems = {}
-        self._ready = {}   # token count -> what a plain call needs, see _prepare
+        self._ready = {}   # token count -> what a plain call needs, see _prepared
 
     def _pack_split(self, weight, high_ids) -> bool:
         """Both partitions from one pass over the 16-bit matrix (`hg_split_rows`, `hg_split_pack`).  True when the selection was a CUDA
@@ -206,54 +217,43 @@ class DualLinear:
         return tuple(found) == (high, 0)
 
     def __call__(self, x):
+        y = None if PACK_MODE else _host.forward(self, x, -1)
+        return self._unprepared(x) if y is None else y
+
+    def _unprepared(self, x):
+        """A call that the native path did not take: the first one with this token count, or an unusual one."""
         shape = x.shape
         if len(shape) != 2 or shape[1] != self.k or x.device != self.w4.device:
             raise ValueError("HyGEMM input shape/device does not match its weights")
-        tokens = shape[0]
-        dtype = DTYPES.get(x.dtype)
-        if not tokens or dtype is None or self.plans or PACK_MODE or not x.is_contiguous() or 28 <= self.low_id <= 34:
+        if not shape[0] or x.dtype not in DTYPES or self.plans or PACK_MODE or not x.is_contiguous() or 28 <= self.low_id <= 34:
             return self.run_packed(*pack(x))
-        return self._call(x, tokens, dtype, None)
+        return self._prepared(x, -1)
 
     def silu_linear(self, x, math):
         """This layer on SwiGLU of `x` = gate||up `[tokens, 2K]`: `producer.silu_pack` followed by `run_packed`."""
+        y = _host.forward(self, x, math)
+        if y is not None:
+            return y
         shape = x.shape
-        dtype = DTYPES.get(x.dtype)
-        if (len(shape) != 2 or shape[1] != 2 * self.k or not shape[0] or dtype is None or x.device != self.w4.device
+        if (len(shape) != 2 or shape[1] != 2 * self.k or not shape[0] or x.dtype not in DTYPES or x.device != self.w4.device
                 or self.plans or not x.is_contiguous() or 28 <= self.low_id <= 34):
             from .producer import silu_pack
             return self.run_packed(*silu_pack(x, math))
-        return self._call(x, shape[0], dtype, math)
+        return self._prepared(x, math)
 
-    def _call(self, x, tokens, dtype, math):
-        # One foreign call for the whole layer: decode sizes quantise inside the GEMM launch, others into a workspace.
-        # (Fresh tensors per call: under CUDA-graph capture the graph's pool owns them.)
-        ready = self._ready.get(tokens)
-        if ready is None or ready[0] is not self.w4 or ready[1] is not self.sf4 or ready[2] != (self.low_id, self.high_id):
-            ready = self._prepare(tokens, x)
-        y = ready[7].new_empty((tokens, self.outputs))
-        stream = torch._C._cuda_getCurrentRawStream(x.device.index)
-        if math is not None:
-            workspace = self.w4.new_empty(tokens * self.k + scale_size(tokens, self.k))
-            status = _lib.hg_linear_silu(ready[3], ready[4], ready[5], x.data_ptr(), dtype, math, workspace.data_ptr(), y.data_ptr(), stream)
-        else:
-            workspace = self.w4.new_empty(ready[6]) if ready[6] else None
-            status = _lib.hg_linear(ready[3], ready[4], ready[5], x.data_ptr(), dtype, workspace.data_ptr() if ready[6] else None,
-                                    y.data_ptr(), stream)
-        if status:
-            check(status)
-        self.calls[tokens] = self.calls.get(tokens, 0) + 1
-        return y
-
-    def _prepare(self, tokens, x):
-        """Handle, operand structs and workspace size of plain calls with this token count, kept between calls."""
+    def _prepared(self, x, math):
+        """Prepares plain calls with this token count (handle, operand structs, workspace sizes; kept between calls) and makes one."""
+        tokens = x.shape[0]
         y = torch.empty((tokens, self.outputs), dtype=self.dtype, device=x.device)
-        low, high, _, low_ref, high_ref = self._rebound(tokens, x, x, y)
-        handle = self._handle(tokens, self.low_id, self.high_id, low_ref, high_ref, _stream(x.device))
+        low, high = self.problems(x, x, y)
+        handle = self._handle(tokens, self.low_id, self.high_id, C.byref(low), C.byref(high), _stream(x.device))
         fused = tokens <= FUSED_QUANT_TOKENS and self.outputs <= FUSED_QUANT_MAX_OUTPUTS
-        ready = self._ready[tokens] = (self.w4, self.sf4, (self.low_id, self.high_id), handle, low_ref, high_ref,
-                                       0 if fused else tokens * self.k + scale_size(tokens, self.k), y.new_empty(0))
-        return ready
+        self._ready[tokens] = _host.prepare(self, tokens, handle.value, C.addressof(low), C.addressof(high), (low, high), y,
+                                            tokens * self.k + scale_size(tokens, self.k), fused)
+        result = _host.forward(self, x, math)
+        if result is None:
+            raise RuntimeError("HyGEMM layer call was not prepared")
+        return result
 
     def _handle(self, tokens, low_id, high_id, low_ref, high_ref, stream):
         """GEMM handle of one (token count, schedule ids) pair, created on first use: never during stream

@@ -39,3 +39,34 @@ def test_swiglu_layer_call_equals_producer_then_gemm(dtype):
             assert torch.equal(got.view(torch.int16), want.view(torch.int16)), (outputs, k, high, tokens)
         assert layer.status()[0] == 0
         layer.close()
+
+
+@pytest.mark.parametrize("tokens", [1, 16, 17, 130])
+def test_layer_call_by_every_route(tokens):
+    """Prepared calls, the first call, the other input dtype, tensor subclasses, replaced weights and a changed
+    schedule id: always the bytes of the quantiser followed by the GEMM on its codes, and one count per call."""
+    g = torch.Generator().manual_seed(tokens)
+    outputs, k, high = 300, 384, 40
+    layer = native.DualLinear((torch.randn(outputs, k, generator=g) * 0.04).half().cuda(), torch.arange(high).cuda())
+    wide = torch.randn(tokens, 2 * k, generator=g).half().cuda()
+    x = wide[:, :k].contiguous()
+
+    def check(x):
+        before = layer.calls.get(tokens, 0)
+        got = layer(x)
+        assert layer.calls[tokens] == before + 1 and got.dtype == torch.float16 and type(got) is torch.Tensor
+        assert torch.equal(got.view(torch.int16), layer.run_packed(*native.pack(x.contiguous())).view(torch.int16))
+        return got
+
+    check(x), check(x)
+    check(x.bfloat16())
+    check(torch.nn.Parameter(x, requires_grad=False))
+    layer.w4, layer.sf4 = layer.w4.flip(0).contiguous(), layer.sf4.clone()
+    torch.cuda.synchronize()
+    check(x), check(x)
+    layer.low_id = layer.high_id = 1
+    check(x), check(x)
+    for bad in (wide, x.cpu(), x[0], wide[:, ::2]):
+        with pytest.raises(ValueError):
+            layer(bad)
+    layer.close()
