@@ -663,30 +663,46 @@ static int tuning(const char* name, int value) {
   return text ? std::atoi(text) : value;
 }
 
-// Estimated microseconds of a launch.  A K256 step of a CTA takes the longest of: the tensor core with its operand reads from
-// shared memory; a turn of the ring (from commit to the next full stage); what L2 delivers (9 to 11 TB/s over all SMs, 110
-// bytes per nanosecond to one).  An SM stores 1.4 sectors per cycle: 128 rows of an MXFP4 tile touch 13 sectors per token, 128
-// rows of an MXFP8 tile 128, so an MXFP8 tile of 256 tokens is stored for 13 us.  Finer MXFP8 tiles spread that over more
+// Estimated microseconds of a launch, up to what all plans of a shape share.  A K256 step of a CTA takes the longest of: the
+// tensor core with its operand reads from shared memory; a turn of the ring (from commit to the next full stage); what L2
+// delivers, over all SMs and to one.  An SM stores 1.4 sectors per cycle: 128 rows of an MXFP4 tile touch 13 sectors per token,
+// 128 rows of an MXFP8 tile 128, so an MXFP8 tile of 256 tokens is stored for 13 us.  Finer MXFP8 tiles spread that over more
 // CTAs (qkv of Qwen2.5-7B: 24.8 -> 17.5 us at 777 tokens, 46.7 -> 37.5 us at 2048).  Stores run under the next main loop.  The
-// launch takes the busiest cluster's time or its weights' time from HBM (6.3 TB/s), whichever is longer, plus a constant, a
-// little per CTA and the exchange of partials.  A ring's worth of weights is in shared memory before the kernel in front has
-// ended.  The constants are a fit to 200 measured launches (Qwen2.5-7B and Mistral-7B / 4 shapes, 16 to 2048 tokens).
-static double plan_cost(const ClusterPlan& plan, int64_t units, int kblocks, double weight_megabytes) {
+// launch takes the busiest cluster's time or its weights' time from HBM, whichever is longer, plus a little per CTA and the
+// exchange of partials.
+//
+// The constants are a fit to the order of 5500 measured launches: 425 shapes drawn from 640 to 37888 channels, K 512 to 18944
+// and 1 to 2048 tokens, each with every plan it can have.  The plan it prefers is 1.4 % slower than the best one of the shape
+// on average up to 128 tokens (5.7 % with the constants of fewer and longer shapes before; 7003 x 2432 at 77 tokens 8.8 -> 7.0
+// us, 1920 x 1280 at 66 tokens 6.5 -> 4.4 us) and 0.6 % above (1.7 % before).
+struct PlanFit {
+  double mma_floor;                                  // cycles of a single CTA's narrow MMA with its operand reads
+  double turn, l2, l2_wide, to_one;                  // us per turn of the ring; bytes per ns from L2 to all SMs, tiles of 129 tokens and more, to one
+  double unit, split_unit, split_token;              // after a unit's main loop, whole or one of several parts of K; per token
+  double store, store_token, low_row, high_row;      // stores: start; per token; cycles per token and row
+  double hops, exchange, part, part_token;           // exchange: per doubling of the cluster, constant, per part, per part and token
+  double cta, pair, cut, finer, hbm;                 // per CTA of the grid, paired CTAs, cut of all tiles, further cut of MXFP8 tiles; bytes per ns
+};
+constexpr PlanFit kDecodeFit{234, 1.34, 13100, 13100, 250, 0.147, 0.579, 0.0147, 0.374, 0.0146, 0.0221, 0.866, -0.379, 0.238, 0.0614, 0.00225,
+                             0.0199, 0.587, -0.0142, 0.268, 7200};
+constexpr PlanFit kPrefillFit{234, 1.28, 18800, 12300, 380, 0.397, 1.75, 0.0159, 0.632, 0.0142, 0.0146, 0.648, -0.67, 0.09, 0.0186, 0.00254,
+                              0.00225, 2.55, 0.0711, -0.221, 3120};
+
+static double plan_cost(const ClusterPlan& plan, int64_t units, int kblocks, double weight_kilobytes) {
+  const PlanFit& fit = plan.token_tiles == 1 && plan.n_tile <= 128 ? kDecodeFit : kPrefillFit;
   const double steps = double((kblocks + 1) / 2) / plan.split;
   const int cluster_ctas = plan.pair * plan.split, ctas = plan.clusters * cluster_ctas;
-  double prefetched = 0;
   auto main_loop = [&](int n, bool high) {
     const double b = double(n) / plan.pair;
-    const double mma = 2 * (plan.pair == 2 ? std::max(2.0 * n, 200.0 + b) : std::max(171.0, 128.0 + 1.3 * b)) / 1900;
-    auto kilobytes = [&](int part) { return double(kTileRows >> plan.cut_log[part]) * (part ? 0.25 : 0.125) + b * 0.25 + 2; };
-    const double average = (kilobytes(0) * plan.tiles[0] + kilobytes(1) * plan.tiles[1]) / (double(plan.tiles[0]) + plan.tiles[1]);
-    const double step = std::max({mma, 1.42 / plan.stages, average * ctas / (n > 128 ? 9000 : 11000), kilobytes(high) / 110});
-    prefetched = std::max(prefetched, std::min(steps, double(plan.stages)) * (step - mma));
-    return steps * step + (plan.split > 1 ? 0.5 + 0.011 * n : 0.15);
+    const double mma = 2 * (plan.pair == 2 ? std::max(2.0 * n, 200.0 + b) : std::max(171.0, fit.mma_floor + 1.3 * b)) / 1900;
+    auto bytes = [&](int part) { return 1000 * (double(kTileRows >> plan.cut_log[part]) * (part ? 0.25 : 0.125) + b * 0.25 + 2); };
+    const double average = (bytes(0) * plan.tiles[0] + bytes(1) * plan.tiles[1]) / (double(plan.tiles[0]) + plan.tiles[1]);
+    const double step = std::max({mma, fit.turn / plan.stages, average * ctas / (1000 * (n > 128 ? fit.l2_wide : fit.l2)), bytes(high) / (1000 * fit.to_one)});
+    return steps * step + (plan.split > 1 ? fit.split_unit + fit.split_token * n : fit.unit);
   };
   auto stores = [&](int n, bool high) {
     const double rows = double(kTileRows >> plan.cut_log[high]);
-    return 0.35 + std::max(0.0185 * n, n * rows * (high ? 0.72 : 0.1) / 1900) / plan.split;
+    return fit.store + std::max(fit.store_token * n, n * rows * (high ? fit.high_row : fit.low_row) / 1900) / plan.split;
   };
   const double main_of[2][2] = {{main_loop(plan.n_tile, false), main_loop(plan.n_tail, false)},
                                 {plan.tiles[1] ? main_loop(plan.n_tile, true) : 0, plan.tiles[1] ? main_loop(plan.n_tail, true) : 0}};
@@ -699,15 +715,16 @@ static double plan_cost(const ClusterPlan& plan, int64_t units, int kblocks, dou
     const bool high = plan.token_tiles == 1 ? t < plan.tiles[1] : (t + 1) * plan.tiles[1] / tiles > t * plan.tiles[1] / tiles;
     double &main_end = load[size_t(u % plan.clusters)], &store_end = storing[size_t(u % plan.clusters)];
     // two accumulators: a main loop starts once the stores before the last ones are done
-    main_end += main_of[high][tail];
-    const double begin = std::max(main_end, store_end);
-    main_end = std::max(main_end, store_end);
-    store_end = begin + store_of[high][tail];
+    main_end = std::max(main_end + main_of[high][tail], store_end);
+    store_end = main_end + store_of[high][tail];
   }
   const double busiest = *std::max_element(storing.begin(), storing.end());
-  const double exchange = plan.split > 1 ? 0.14 * std::log2(double(cluster_ctas)) - 0.17 : 0.0;
-  const double least = weight_megabytes / 6.3 + store_of[0][1];
-  return 2.2 + 0.012 * ctas + 0.1 * (plan.cut_log[1] - plan.cut_log[0]) + std::max(busiest - prefetched, least) + exchange;
+  double exchange = 0;
+  if (plan.split > 1)
+    exchange = fit.hops * std::log2(double(cluster_ctas)) + fit.exchange + (fit.part + fit.part_token * plan.n_tile) * plan.split;
+  const double least = weight_kilobytes / fit.hbm + store_of[0][1];
+  return fit.cta * ctas + (plan.pair == 2 ? fit.pair : 0) + fit.cut * plan.cut_log[0] + fit.finer * (plan.cut_log[1] - plan.cut_log[0]) +
+         std::max(busiest, least) + exchange;
 }
 
 // Ring, TMEM and shared-memory figures that follow from the other choices.  False when the ring would be too shallow.
@@ -769,7 +786,7 @@ ClusterPlan make_cluster_plan(int lo, int hi, int tokens, int k, const int max_c
               // tokens 17.1 -> 16.0 us).
               plan.ring_exchange = plan.split > 1 && plan.n_tile > 32;
               if (!finish_plan(plan)) continue;
-              plan.cost = plan_cost(plan, units, kblocks, (lo * 0.53125 + hi * 1.03125) * k * 1e-6);
+              plan.cost = plan_cost(plan, units, kblocks, (lo * 0.53125 + hi * 1.03125) * k * 1e-3);
               if (plan.cost < best.cost) best = plan;
             }
   if (best.cost >= 1e30) throw std::runtime_error("No cluster schedule for this shape");
