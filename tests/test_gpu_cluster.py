@@ -70,3 +70,20 @@ def test_layer_call_by_every_route(tokens):
         with pytest.raises(ValueError):
             layer(bad)
     layer.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_swiglu_of_every_gate_value(dtype):
+    """Both SwiGLU producers (many rows, few rows) on all 65536 gates of the type, infinities and NaNs too, each with 128 values of
+    up: the bytes of the producer that also returns its products, which keeps to the exact functions."""
+    k = 2048
+    g = torch.Generator(device="cuda").manual_seed(9)
+    gate = torch.arange(65536, device="cuda").repeat(128)[torch.randperm(128 * 65536, device="cuda", generator=g)]
+    up = torch.randint(0, 65536, (128 * 65536,), device="cuda", generator=g)
+    gate, up = (t.to(torch.int16).view(dtype).view(-1, k) for t in (gate, up))
+    up = torch.where(torch.arange(up.shape[0], device="cuda")[:, None] % 4 == 0, up, torch.randn(up.shape, device="cuda", generator=g).to(dtype))
+    x = torch.cat([gate, up], 1).contiguous()
+    for part in (x, *x.split(512)):
+        q, sf = producer.silu_pack(part, 0)
+        exact_q, exact_sf, _ = producer.silu_pack(part, 0, debug=True)
+        assert torch.equal(q, exact_q) and torch.equal(sf, exact_sf)
