@@ -17,8 +17,9 @@
 //   that were not loaded are never read.
 //
 // Roles per CTA: warp 0 weights and their scales (TMA), warp 1 MMA issue (idle in the second CTA of a pair, whose copies
-// complete on the first CTA's barriers: reporting every stage with a remote arrive cost 750 cycles each), then epilogue warps (four; in pairs eight, two per TMEM quarter on alternate groups of sixteen columns),
-// then one warp for the activations and their scales (TMA) or, FUSED, four warps that quantise the activations.
+// complete on the first CTA's barriers: reporting every stage with a remote arrive cost 750 cycles each), then epilogue warps
+// (four; in pairs eight, two per TMEM quarter on alternate groups of sixteen columns), then one warp for the activations and
+// their scales (TMA) or, FUSED, four warps that quantise the activations.
 // One warp per scheduler runs most of these roles alone, so a dependent instruction costs about five cycles and nothing
 // hides it: loops here carry no divisions, addresses are independent of each other, and descriptors are sums.
 // Every mbarrier wait is bounded; on expiry the CTA records a code, drains and leaves.
