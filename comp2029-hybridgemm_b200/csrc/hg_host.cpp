@@ -17,6 +17,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <exception>
+#include <iterator>
 
 #include "../../include/hygemm.h"
 
@@ -26,13 +27,14 @@ decltype(&hg_linear) run_linear = nullptr;
 decltype(&hg_linear_silu) run_linear_silu = nullptr;
 decltype(&hg_last_error) last_error = nullptr;
 
-PyObject *s_ready, *s_w4, *s_sf4, *s_low_id, *s_high_id, *s_plans, *s_calls;
+PyObject *s_ready, *s_w4, *s_sf4, *s_lo, *s_w8, *s_sf8, *s_hi, *s_low_id, *s_high_id, *s_plans, *s_calls;
 
 const char kName[] = "hygemm.ready";
 
-// What calls of one layer with one token count share.  Valid while the layer still has the same weights and schedule ids.
+// What calls of one layer with one token count share.  Valid while the layer's six operand tensors still lie where the
+// structs say (an attribute may be replaced, and so may the storage behind one) and the schedule ids are the same.
 struct Ready {
-  PyObject *w4, *sf4, *low_id, *high_id, *problems;   // owned
+  PyObject *low_id, *high_id, *problems;              // owned
   void* handle;
   const hg_problem *low, *high;                       // inside `problems`
   int64_t tokens, k, outputs, packed;                 // packed: bytes of the quantised activations
@@ -46,13 +48,32 @@ Ready* ready_of(PyObject* capsule) { return static_cast<Ready*>(PyCapsule_GetPoi
 void destroy(PyObject* capsule) {
   Ready* r = ready_of(capsule);
   if (!r) return;
-  for (PyObject* o : {r->w4, r->sf4, r->low_id, r->high_id, r->problems}) Py_XDECREF(o);
+  for (PyObject* o : {r->low_id, r->high_id, r->problems}) Py_XDECREF(o);
   delete r;
 }
 
-// True when attribute `name` of `layer` is `wanted` (the same object, or an equal int).
-bool unchanged(PyObject* layer, PyObject* name, PyObject* wanted) {
-  PyObject* now = PyObject_GetAttr(layer, name);
+// The attributes of a layer.  A call asks for eleven, so they are looked up in the instance's dict directly; one that is
+// not there is asked for in the ordinary way.
+struct Attributes {
+  PyObject *layer, *dict;
+  explicit Attributes(PyObject* of) : layer(of), dict(PyObject_GenericGetDict(of, nullptr)) {
+    if (!dict) PyErr_Clear();
+  }
+  ~Attributes() { Py_XDECREF(dict); }
+  Attributes(const Attributes&) = delete;
+  // A new reference, or null with an error set.
+  PyObject* get(PyObject* name) const {
+    if (dict) {
+      if (PyObject* found = PyDict_GetItemWithError(dict, name)) return Py_NewRef(found);
+      if (PyErr_Occurred()) return nullptr;
+    }
+    return PyObject_GetAttr(layer, name);
+  }
+};
+
+// True when attribute `name` is `wanted` (the same object, or an equal int).
+bool unchanged(const Attributes& layer, PyObject* name, PyObject* wanted) {
+  PyObject* now = layer.get(name);
   if (!now) { PyErr_Clear(); return false; }
   bool same = now == wanted;
   if (!same && PyLong_Check(now)) {
@@ -64,14 +85,29 @@ bool unchanged(PyObject* layer, PyObject* name, PyObject* wanted) {
   return same;
 }
 
+// True when attribute `name` is a tensor whose elements start at `data`, `elements` of them (-1: any number).
+bool still_at(const Attributes& layer, PyObject* name, const void* data, int64_t elements = -1) {
+  PyObject* now = layer.get(name);
+  if (!now) { PyErr_Clear(); return false; }
+  struct Release { PyObject* o; ~Release() { Py_DECREF(o); } } release{now};   // the tensor's accessors may throw
+  if (!THPVariable_Check(now)) return false;
+  const at::Tensor& t = THPVariable_Unpack(now);
+  return t.const_data_ptr() == data && (elements < 0 || t.numel() == elements);
+}
+
+bool operands_unchanged(const Attributes& layer, const hg_problem& low, const hg_problem& high) {
+  return still_at(layer, s_w4, low.weight) && still_at(layer, s_sf4, low.weight_scales) && still_at(layer, s_lo, low.ids, low.rows) &&
+         still_at(layer, s_w8, high.weight) && still_at(layer, s_sf8, high.weight_scales) && still_at(layer, s_hi, high.ids, high.rows);
+}
+
 // The prepared state of a call, a new reference; null without an error when the call is not a prepared, ordinary one.
-PyObject* find(PyObject* layer, int64_t tokens) {
-  PyObject* plans = PyObject_GetAttr(layer, s_plans);
+PyObject* find(const Attributes& layer, int64_t tokens) {
+  PyObject* plans = layer.get(s_plans);
   if (!plans) return nullptr;
   const int planned = PyObject_IsTrue(plans);
   Py_DECREF(plans);
   if (planned) return nullptr;
-  PyObject* all = PyObject_GetAttr(layer, s_ready);
+  PyObject* all = layer.get(s_ready);
   if (!all) return nullptr;
   PyObject* capsule = nullptr;
   PyObject* key = PyLong_FromLongLong(tokens);
@@ -84,8 +120,8 @@ PyObject* find(PyObject* layer, int64_t tokens) {
   return capsule;
 }
 
-bool count_call(PyObject* layer, int64_t tokens) {
-  PyObject* calls = PyObject_GetAttr(layer, s_calls);
+bool count_call(const Attributes& layer, int64_t tokens) {
+  PyObject* calls = layer.get(s_calls);
   if (!calls) return false;
   bool ok = false;
   PyObject* key = PyLong_FromLongLong(tokens);
@@ -102,7 +138,8 @@ bool count_call(PyObject* layer, int64_t tokens) {
   return ok;
 }
 
-PyObject* forward_checked(PyObject* layer, const at::Tensor& x, long math) {
+PyObject* forward_checked(PyObject* self, const at::Tensor& x, long math) {
+  const Attributes layer(self);
   const bool swiglu = math >= 0;
   if (x.dim() != 2) Py_RETURN_NONE;
   const auto type = x.scalar_type();
@@ -117,8 +154,7 @@ PyObject* forward_checked(PyObject* layer, const at::Tensor& x, long math) {
   const Ready* r = ready_of(capsule);
   if (!r) return nullptr;
   if (x.size(1) != (swiglu ? 2 * r->k : r->k) || x.device() != r->device || !x.is_contiguous() ||
-      !unchanged(layer, s_w4, r->w4) || !unchanged(layer, s_sf4, r->sf4) || !unchanged(layer, s_low_id, r->low_id) ||
-      !unchanged(layer, s_high_id, r->high_id))
+      !unchanged(layer, s_low_id, r->low_id) || !unchanged(layer, s_high_id, r->high_id) || !operands_unchanged(layer, *r->low, *r->high))
     Py_RETURN_NONE;
   // Fresh tensors per call: under CUDA-graph capture the graph's pool owns them.
   at::Tensor y = at::empty({r->tokens, r->outputs}, r->output);
@@ -173,13 +209,10 @@ PyObject* prepare(PyObject*, PyObject* args) {
   if (!PyArg_ParseTuple(args, "OLKKKOOLp", &layer, &tokens, &handle, &low, &high, &problems, &y, &packed, &fused)) return nullptr;
   if (!THPVariable_Check(y)) return PyErr_SetString(PyExc_TypeError, "prepare: y must be a tensor"), nullptr;
   auto* r = new Ready{};
-  PyObject** slots[4] = {&r->w4, &r->sf4, &r->low_id, &r->high_id};
-  PyObject* names[4] = {s_w4, s_sf4, s_low_id, s_high_id};
   r->problems = Py_NewRef(problems);
   PyObject* capsule = PyCapsule_New(r, kName, destroy);
   if (!capsule) return nullptr;
-  for (int i = 0; i < 4; ++i)
-    if (!(*slots[i] = PyObject_GetAttr(layer, names[i]))) return Py_DECREF(capsule), nullptr;
+  if (!(r->low_id = PyObject_GetAttr(layer, s_low_id)) || !(r->high_id = PyObject_GetAttr(layer, s_high_id))) return Py_DECREF(capsule), nullptr;
   const at::Tensor& like = THPVariable_Unpack(y);
   r->handle = reinterpret_cast<void*>(uintptr_t(handle));
   r->low = reinterpret_cast<const hg_problem*>(uintptr_t(low));
@@ -216,9 +249,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_hygemm_host", nullptr, -1, method
 }  // namespace
 
 PyMODINIT_FUNC PyInit__hygemm_host() {
-  PyObject** names[] = {&s_ready, &s_w4, &s_sf4, &s_low_id, &s_high_id, &s_plans, &s_calls};
-  const char* text[] = {"_ready", "w4", "sf4", "low_id", "high_id", "plans", "calls"};
-  for (int i = 0; i < 7; ++i)
+  PyObject** names[] = {&s_ready, &s_w4, &s_sf4, &s_lo, &s_w8, &s_sf8, &s_hi, &s_low_id, &s_high_id, &s_plans, &s_calls};
+  const char* text[] = {"_ready", "w4", "sf4", "lo", "w8", "sf8", "hi", "low_id", "high_id", "plans", "calls"};
+  for (size_t i = 0; i < std::size(names); ++i)
     if (!(*names[i] = PyUnicode_InternFromString(text[i]))) return nullptr;
   return PyModule_Create(&module);
 }

@@ -280,10 +280,11 @@ class DualLinear:
     def _rebound(self, tokens, q, sf, y):
         """Per-token-count `Problem` pair kept between calls; only the three per-call pointers change."""
         pair = self._problems.get(tokens)
-        if pair is None or pair[2] != (self.w4.data_ptr(), self.sf4.data_ptr()):
+        operands = (self.w4.data_ptr(), self.sf4.data_ptr(), self.lo.data_ptr(), self.lo.numel(),
+                    self.w8.data_ptr(), self.sf8.data_ptr(), self.hi.data_ptr(), self.hi.numel())
+        if pair is None or pair[2] != operands:
             low, high = self.problems(q, sf, y)
-            pair = self._problems[tokens] = (low, high, (self.w4.data_ptr(), self.sf4.data_ptr()),
-                                             C.byref(low), C.byref(high))
+            pair = self._problems[tokens] = (low, high, operands, C.byref(low), C.byref(high))
             return pair
         qp, sp, yp = q.data_ptr(), sf.data_ptr(), y.data_ptr()
         for prob in pair[:2]:

@@ -72,6 +72,39 @@ def test_layer_call_by_every_route(tokens):
     layer.close()
 
 
+@pytest.mark.parametrize("how", ["attribute", "storage"])
+@pytest.mark.parametrize("name", ["w4", "sf4", "lo", "w8", "sf8", "hi"])
+def test_layer_call_after_an_operand_was_replaced(name, how):
+    """Each operand tensor of a layer exchanged, as an attribute and as the storage behind it, after calls that prepared the layer:
+    the bytes of a layer that had the new operand from the start, by the one-call route and by `run_packed`."""
+    g = torch.Generator().manual_seed(11)
+    outputs, k, high = 300, 384, 40
+
+    def fresh(seed):
+        g.manual_seed(seed)
+        return native.DualLinear((torch.randn(outputs, k, generator=g) * 0.04).bfloat16().cuda(), torch.randperm(outputs, generator=g)[:high].cuda())
+
+    layer, other, wanted = fresh(1), fresh(2), fresh(1)
+    new = getattr(layer, name).flip(0).contiguous() if name in ("lo", "hi") else getattr(other, name)
+    setattr(wanted, name, new)
+    for tokens in (3, 40):
+        x = torch.randn(tokens, k, generator=g).bfloat16().cuda()
+        y, want = layer(x), wanted(x)
+        assert torch.equal(y, layer.run_packed(*native.pack(x))) and not torch.equal(y, want)
+        old = getattr(layer, name).clone()
+        if how == "attribute":
+            setattr(layer, name, new.clone())
+        else:
+            getattr(layer, name).data = new.clone()
+        torch.cuda.synchronize()
+        assert torch.equal(layer(x), want) and torch.equal(layer.run_packed(*native.pack(x)), want)
+        setattr(layer, name, old)
+        torch.cuda.synchronize()
+        assert torch.equal(layer(x), y)
+    for each in (layer, other, wanted):
+        each.close()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_swiglu_of_every_gate_value(dtype):
     """Both SwiGLU producers (many rows, few rows) on all 65536 gates of the type, infinities and NaNs too, each with 128 values of
