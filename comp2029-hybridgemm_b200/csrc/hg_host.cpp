@@ -27,7 +27,7 @@ decltype(&hg_linear) run_linear = nullptr;
 decltype(&hg_linear_silu) run_linear_silu = nullptr;
 decltype(&hg_last_error) last_error = nullptr;
 
-PyObject *s_ready, *s_w4, *s_sf4, *s_lo, *s_w8, *s_sf8, *s_hi, *s_low_id, *s_high_id, *s_plans, *s_calls;
+PyObject *s_ready, *s_w4, *s_sf4, *s_lo, *s_w8, *s_sf8, *s_hi, *s_low_id, *s_high_id, *s_concurrent, *s_plans, *s_calls;
 
 const char kName[] = "hygemm.ready";
 
@@ -95,6 +95,22 @@ bool still_at(const Attributes& layer, PyObject* name, const void* data, int64_t
   return t.const_data_ptr() == data && (elements < 0 || t.numel() == elements);
 }
 
+// True for the launch policies that all enqueue the tensor-core launch: False and True, 0 to 3.
+bool tensor_core_policy(const Attributes& layer) {
+  PyObject* now = layer.get(s_concurrent);
+  if (!now) { PyErr_Clear(); return false; }
+  bool plain = now == Py_True || now == Py_False;
+  if (!plain) {
+    PyObject* number = PyNumber_Long(now);
+    const long policy = number ? PyLong_AsLong(number) : -1;
+    PyErr_Clear();
+    Py_XDECREF(number);
+    plain = policy >= HG_POLICY_SERIAL && policy < HG_POLICY_GEMV_PAIR1;
+  }
+  Py_DECREF(now);
+  return plain;
+}
+
 bool operands_unchanged(const Attributes& layer, const hg_problem& low, const hg_problem& high) {
   return still_at(layer, s_w4, low.weight) && still_at(layer, s_sf4, low.weight_scales) && still_at(layer, s_lo, low.ids, low.rows) &&
          still_at(layer, s_w8, high.weight) && still_at(layer, s_sf8, high.weight_scales) && still_at(layer, s_hi, high.ids, high.rows);
@@ -154,7 +170,8 @@ PyObject* forward_checked(PyObject* self, const at::Tensor& x, long math) {
   const Ready* r = ready_of(capsule);
   if (!r) return nullptr;
   if (x.size(1) != (swiglu ? 2 * r->k : r->k) || x.device() != r->device || !x.is_contiguous() ||
-      !unchanged(layer, s_low_id, r->low_id) || !unchanged(layer, s_high_id, r->high_id) || !operands_unchanged(layer, *r->low, *r->high))
+      !unchanged(layer, s_low_id, r->low_id) || !unchanged(layer, s_high_id, r->high_id) || !tensor_core_policy(layer) ||
+      !operands_unchanged(layer, *r->low, *r->high))
     Py_RETURN_NONE;
   // Fresh tensors per call: under CUDA-graph capture the graph's pool owns them.
   at::Tensor y = at::empty({r->tokens, r->outputs}, r->output);
@@ -249,8 +266,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_hygemm_host", nullptr, -1, method
 }  // namespace
 
 PyMODINIT_FUNC PyInit__hygemm_host() {
-  PyObject** names[] = {&s_ready, &s_w4, &s_sf4, &s_lo, &s_w8, &s_sf8, &s_hi, &s_low_id, &s_high_id, &s_plans, &s_calls};
-  const char* text[] = {"_ready", "w4", "sf4", "lo", "w8", "sf8", "hi", "low_id", "high_id", "plans", "calls"};
+  PyObject** names[] = {&s_ready, &s_w4, &s_sf4, &s_lo, &s_w8, &s_sf8, &s_hi, &s_low_id, &s_high_id, &s_concurrent, &s_plans, &s_calls};
+  const char* text[] = {"_ready", "w4", "sf4", "lo", "w8", "sf8", "hi", "low_id", "high_id", "concurrent", "plans", "calls"};
   for (size_t i = 0; i < std::size(names); ++i)
     if (!(*names[i] = PyUnicode_InternFromString(text[i]))) return nullptr;
   return PyModule_Create(&module);

@@ -225,9 +225,14 @@ class DualLinear:
         shape = x.shape
         if len(shape) != 2 or shape[1] != self.k or x.device != self.w4.device:
             raise ValueError("HyGEMM input shape/device does not match its weights")
-        if not shape[0] or x.dtype not in DTYPES or self.plans or PACK_MODE or not x.is_contiguous() or 28 <= self.low_id <= 34:
+        if not shape[0] or x.dtype not in DTYPES or PACK_MODE or not x.is_contiguous() or not self._tensor_core():
             return self.run_packed(*pack(x))
         return self._prepared(x, -1)
+
+    def _tensor_core(self) -> bool:
+        """Calls go to the tensor-core launch whatever their token count: no plan table, no schedule id of the SIMT kernel
+        (28-34) and, of the launch policies, one of the four that enqueue it (the GEMV pairs and unknown ones are run_packed's)."""
+        return not self.plans and not 28 <= self.low_id <= 34 and int(self.concurrent) in (0, 1, 2, 3)
 
     def silu_linear(self, x, math):
         """This layer on SwiGLU of `x` = gate||up `[tokens, 2K]`: `producer.silu_pack` followed by `run_packed`."""
@@ -236,7 +241,7 @@ class DualLinear:
             return y
         shape = x.shape
         if (len(shape) != 2 or shape[1] != 2 * self.k or not shape[0] or x.dtype not in DTYPES or x.device != self.w4.device
-                or self.plans or not x.is_contiguous() or 28 <= self.low_id <= 34):
+                or not x.is_contiguous() or not self._tensor_core()):
             from .producer import silu_pack
             return self.run_packed(*silu_pack(x, math))
         return self._prepared(x, math)

@@ -105,6 +105,36 @@ def test_layer_call_after_an_operand_was_replaced(name, how):
         each.close()
 
 
+@pytest.mark.parametrize("policy", [False, True, 0, 2, 3, 4, 5, 6, 7, -1])
+def test_layer_calls_keep_the_launch_policy(policy):
+    """`layer(x)` and `silu_linear` under every launch policy, set when the layer is built and changed after calls that prepared it:
+    the bytes of `run_packed`, which the GEMV policies send to the SIMT kernel; unknown policies are refused by both."""
+    g = torch.Generator().manual_seed(4)
+    outputs, k, high = 300, 2432, 40
+    w, ids = (torch.randn(outputs, k, generator=g) * 0.04).bfloat16().cuda(), torch.arange(high).cuda()
+    built, changed = native.DualLinear(w, ids, concurrent=policy), native.DualLinear(w, ids)
+    for tokens in (3, 40):
+        x = torch.randn(tokens, k, generator=g).bfloat16().cuda()
+        pair = torch.randn(tokens, 2 * k, generator=g).bfloat16().cuda()
+        changed.concurrent = True
+        changed(x), changed.silu_linear(pair, 0)
+        changed.concurrent = policy
+        for layer in (built, changed):
+            if policy in (7, -1):
+                for call in (lambda: layer(x), lambda: layer.silu_linear(pair, 0), lambda: layer.run_packed(*native.pack(x))):
+                    with pytest.raises(RuntimeError, match="Unknown launch policy"):
+                        call()
+                continue
+            layer.status()
+            for call, packed in ((lambda: layer(x), native.pack(x)), (lambda: layer.silu_linear(pair, 0), producer.silu_pack(pair, 0))):
+                y = call()
+                assert (layer.status()[1] > 0) == (policy not in (4, 5, 6))   # K128 blocks that the tensor cores were given
+                assert torch.equal(y, layer.run_packed(*packed))
+                layer.status()
+    built.close()
+    changed.close()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_swiglu_of_every_gate_value(dtype):
     """Both SwiGLU producers (many rows, few rows) on all 65536 gates of the type, infinities and NaNs too, each with 128 values of
