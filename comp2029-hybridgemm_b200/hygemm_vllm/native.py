@@ -236,11 +236,12 @@ class DualLinear:
 
     def silu_linear(self, x, math):
         """This layer on SwiGLU of `x` = gate||up `[tokens, 2K]`: `producer.silu_pack` followed by `run_packed`."""
-        y = _host.forward(self, x, math)
+        known = math in (0, 1, 2)   # the native path takes a negative one for a call without SwiGLU
+        y = _host.forward(self, x, math) if known else None
         if y is not None:
             return y
         shape = x.shape
-        if (len(shape) != 2 or shape[1] != 2 * self.k or not shape[0] or x.dtype not in DTYPES or x.device != self.w4.device
+        if (not known or len(shape) != 2 or shape[1] != 2 * self.k or not shape[0] or x.dtype not in DTYPES or x.device != self.w4.device
                 or not x.is_contiguous() or not self._tensor_core()):
             from .producer import silu_pack
             return self.run_packed(*silu_pack(x, math))

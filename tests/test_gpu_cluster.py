@@ -105,6 +105,21 @@ def test_layer_call_after_an_operand_was_replaced(name, how):
         each.close()
 
 
+def test_swiglu_layer_refuses_an_unknown_math():
+    """What the producer refuses stays refused on a prepared layer: not taken for the layer on an input that is as wide as its K."""
+    g = torch.Generator().manual_seed(6)
+    layer = native.DualLinear((torch.randn(300, 256, generator=g) * 0.04).bfloat16().cuda(), torch.arange(40).cuda())
+    x, pair = torch.randn(5, 256, generator=g).bfloat16().cuda(), torch.randn(5, 512, generator=g).bfloat16().cuda()
+    layer(x), layer.silu_linear(pair, 0)
+    calls = dict(layer.calls)
+    for math in (-1, -7, 3):
+        for given in (x, pair):
+            with pytest.raises(RuntimeError, match="producer"):
+                layer.silu_linear(given, math)
+    assert layer.calls == calls
+    layer.close()
+
+
 @pytest.mark.parametrize("policy", [False, True, 0, 2, 3, 4, 5, 6, 7, -1])
 def test_layer_calls_keep_the_launch_policy(policy):
     """`layer(x)` and `silu_linear` under every launch policy, set when the layer is built and changed after calls that prepared it:
