@@ -1100,6 +1100,7 @@ TcGemm* tc_create(const hg_problem& l, const hg_problem& h, int schedule, int dt
     check(cudaMalloc(&g->d_trace, sizeof(unsigned long long) * 16 * size_t(g->plan.grid)), "trace buffer");
     check(cudaMemsetAsync(g->d_trace, 0, sizeof(unsigned long long) * 16 * size_t(g->plan.grid), stream), "trace buffer");
 #endif
+    check(cudaStreamSynchronize(stream), "clear status");   // the first launch may be on another stream
     return g.release();
   }
   g->heads = make_heads(g->plan);

@@ -4,6 +4,8 @@ switch, K with odd and single K128 blocks (also cut over a cluster), row counts 
 Operands are exactly representable and their sums stay below 2^24 quanta, so every order of summation gives the same fp32
 value: results must be equal bit for bit (tolerance 0).
 """
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -103,6 +105,33 @@ def test_layer_call_after_an_operand_was_replaced(name, how):
         assert torch.equal(layer(x), y)
     for each in (layer, other, wanted):
         each.close()
+
+
+@pytest.mark.parametrize("schedule", [0, 1])
+def test_status_of_a_handle_made_on_a_busy_stream(schedule):
+    """A handle made on one stream and run on another: its status words are clear before it is handed out, so the launch's counts
+    are not cleared behind its back."""
+    lib = native.library()
+    g = torch.Generator().manual_seed(8)
+    layer = native.DualLinear((torch.randn(300, 256, generator=g) * 0.04).bfloat16().cuda(), torch.arange(40).cuda())
+    q, sf = native.pack(torch.randn(5, 256, generator=g).bfloat16().cuda())
+    y = torch.empty(5, 300, dtype=torch.bfloat16, device="cuda")
+    low, high = layer.problems(q, sf, y)
+    layer.low_id = layer.high_id = schedule
+    layer.run_packed(q, sf)   # the kernel is loaded
+    busy, other = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(200_000_000)   # about a tenth of a second
+    handle = C.c_void_p()
+    native.check(lib.hg_create_dtype(schedule, schedule, C.byref(low), C.byref(high), busy.cuda_stream, 1, C.byref(handle)))
+    native.check(lib.hg_run(handle, C.byref(low), C.byref(high), other.cuda_stream, 0))
+    torch.cuda.synchronize()
+    status = (C.c_int * 3)()
+    native.check(lib.hg_status(handle, other.cuda_stream, status))
+    lib.hg_destroy(handle)
+    layer.close()
+    assert status[0] == 0 and status[1] > 0 and status[2] > 0, list(status)
 
 
 def test_swiglu_layer_refuses_an_unknown_math():
