@@ -5,9 +5,8 @@ schemas (quantization.py:18-25, producer.py:27-40 of the reference): the layer
 runtime is looked up by an integer handle in `_runtimes`, nothing is mutated,
 and the fake implementations give shape/dtype for tracing.
 
-The ops are registered with the dispatcher directly, and the functions `linear` and `linear_silu` of this module only go
-through it where something may be watching (tracing, dispatch modes, tensor subclasses, autograd): an eager call
-of an op registered with `torch.library.custom_op` costs about as much host time as the layer itself.
+An eager call of a custom op costs about as much host time as the layer itself, so calling `linear` or `linear_silu` goes
+straight to the layer unless something may be watching (tracing, dispatch modes, tensor subclasses, autograd).
 """
 from __future__ import annotations
 
@@ -52,22 +51,28 @@ def _linear_silu_fake(x, handle, outputs, math):
     return x.new_empty((x.shape[0], outputs))
 
 
-_library = torch.library.Library("hygemm_vllm", "DEF")
-for _name, _function, _fake in (("linear", _linear, _linear_fake), ("linear_silu", _linear_silu, _linear_silu_fake)):
-    _library.define(_name + torch.library.infer_schema(_function, mutates_args=()))
-    _library.impl(_name, _function, "CompositeExplicitAutograd")
-    torch.library.register_fake(f"hygemm_vllm::{_name}", _fake, lib=_library)
-
-
 def _plain(x) -> bool:
     """An eager call on an ordinary tensor that nothing traces, intercepts or differentiates."""
     return (not torch.compiler.is_compiling() and type(x) is torch.Tensor and not x.requires_grad
             and not torch._C._len_torch_dispatch_stack())
 
 
-def linear(x: torch.Tensor, handle: int, outputs: int) -> torch.Tensor:
-    return _runtimes[handle](x) if _plain(x) else torch.ops.hygemm_vllm.linear(x, handle, outputs)
+class _Op(torch.library.CustomOpDef):
+    """A custom op with the short way round the dispatcher; `direct` is its function."""
+
+    def __call__(self, x, *args, **kwargs):
+        if _plain(x):
+            return self.direct(x, *args, **kwargs)
+        return super().__call__(x, *args, **kwargs)
 
 
-def linear_silu(x: torch.Tensor, handle: int, outputs: int, math: int) -> torch.Tensor:
-    return _linear_silu(x, handle, outputs, math) if _plain(x) else torch.ops.hygemm_vllm.linear_silu(x, handle, outputs, math)
+def _define(name, function, fake):
+    op = torch.library.custom_op(f"hygemm_vllm::{name}", function, mutates_args=())
+    op.register_fake(fake)
+    op.__class__ = _Op
+    op.direct = function
+    return op
+
+
+linear = _define("linear", _linear, _linear_fake)
+linear_silu = _define("linear_silu", _linear_silu, _linear_silu_fake)
