@@ -5,8 +5,10 @@ schemas (quantization.py:18-25, producer.py:27-40 of the reference): the layer
 runtime is looked up by an integer handle in `_runtimes`, nothing is mutated,
 and the fake implementations give shape/dtype for tracing.
 
-An eager call of a custom op costs about as much host time as the layer itself, so calling `linear` or `linear_silu` goes
-straight to the layer unless something may be watching (tracing, dispatch modes, tensor subclasses, autograd).
+An eager call of a custom op costs about as much host time as the layer itself, so calling `linear` or `linear_silu` on an
+ordinary tensor with nothing watching goes straight to the layer.  Everything else goes through the dispatcher: tracing,
+modes, functorch transforms, profiling, tensor subclasses and wrappers, tensors that require a gradient (the ops have none,
+and say so in the backward pass).
 """
 from __future__ import annotations
 
@@ -52,9 +54,13 @@ def _linear_silu_fake(x, handle, outputs, math):
 
 
 def _plain(x) -> bool:
-    """An eager call on an ordinary tensor that nothing traces, intercepts or differentiates."""
-    return (not torch.compiler.is_compiling() and type(x) is torch.Tensor and not x.requires_grad
-            and not torch._C._len_torch_dispatch_stack())
+    """An eager call on an ordinary tensor that nothing traces, transforms, intercepts, records or differentiates."""
+    return (not torch.compiler.is_compiling()
+            and not torch._C._len_torch_function_stack() and not torch._C._len_torch_dispatch_stack()
+            and torch._C._functorch.peek_interpreter_stack() is None and torch._C._get_tracing_state() is None
+            and not torch.autograd._profiler_enabled()
+            and type(x) is torch.Tensor and not x.requires_grad and not x.is_meta
+            and not torch._C._functorch.is_functorch_wrapped_tensor(x) and not torch._is_functional_tensor(x))
 
 
 class _Op(torch.library.CustomOpDef):

@@ -6,6 +6,7 @@ from pathlib import Path
 
 import pytest
 import torch
+from torch.fx.experimental.proxy_tensor import make_fx
 
 from hygemm_vllm import ops
 
@@ -40,10 +41,50 @@ def test_an_ordinary_call(op):
         assert torch.equal(op(X.clone()), SUM)
 
 
+def test_transforms(op):
+    assert torch.equal(torch.vmap(op)(torch.stack([X, 2 * X])), torch.stack([SUM, 2 * SUM]))
+    assert torch.equal(torch.func.functionalize(op)(X), SUM)
+    assert torch.equal(torch.func.jvp(op, (X,), (X,))[0], SUM)
+
+
 def test_a_gradient_is_refused(op):
     x = X.clone().requires_grad_()
     with pytest.raises(RuntimeError, match="no autograd formula"):
         op(x).sum().backward()
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda x: op(x).sum())(X)
+
+
+def test_tracers_see_one_op(op):
+    for graph in (make_fx(op)(X).graph, make_fx(op, pre_dispatch=True)(X).graph, torch.fx.symbolic_trace(op).graph):
+        names = [str(n.target) for n in graph.nodes if n.op == "call_function"]
+        assert len(names) == 1 and names[0].startswith("hygemm_vllm.linear"), names
+    traced = torch.jit.trace(op, X, check_trace=False)
+    assert [n.kind() for n in traced.graph.nodes() if n.kind() != "prim::Constant"][0].startswith("hygemm_vllm::linear")
+    assert torch.equal(traced(3 * X), 3 * SUM)
+    compiled = torch.compile(lambda x: op(x) + 1, backend="aot_eager", fullgraph=True)
+    assert torch.equal(compiled(X), SUM + 1)
+
+
+def test_modes_and_profiler_see_the_op(op):
+    seen = []
+
+    class Mode(torch.overrides.TorchFunctionMode):
+        def __torch_function__(self, function, types, args=(), kwargs=None):
+            seen.append(str(function))
+            return function(*args, **(kwargs or {}))
+
+    with Mode():
+        op(X)
+    assert any(s.startswith("hygemm_vllm.linear") for s in seen) and not any("data_ptr" in s for s in seen), seen
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as profile:
+        op(X)
+    assert any(e.key.startswith("hygemm_vllm::linear") for e in profile.key_averages())
+
+
+def test_a_meta_tensor_gives_a_meta_tensor(op):
+    y = op(torch.empty(5, 4, device="meta"))
+    assert y.is_meta and y.shape == (5, 3)
 
 
 def test_registration():
