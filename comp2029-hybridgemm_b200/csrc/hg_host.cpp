@@ -154,6 +154,12 @@ bool count_call(const Attributes& layer, int64_t tokens) {
   return ok;
 }
 
+// The interpreter lock given up for a scope, also when it is left by an exception.
+struct Unlocked {
+  PyThreadState* const state = PyEval_SaveThread();
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
+
 PyObject* forward_checked(PyObject* self, const at::Tensor& x, long math) {
   const Attributes layer(self);
   const bool swiglu = math >= 0;
@@ -173,26 +179,29 @@ PyObject* forward_checked(PyObject* self, const at::Tensor& x, long math) {
       !unchanged(layer, s_low_id, r->low_id) || !unchanged(layer, s_high_id, r->high_id) || !tensor_core_policy(layer) ||
       !operands_unchanged(layer, *r->low, *r->high))
     Py_RETURN_NONE;
-  // Fresh tensors per call: under CUDA-graph capture the graph's pool owns them.
-  at::Tensor y = at::empty({r->tokens, r->outputs}, r->output);
-  at::Tensor workspace;
-  // Quantising inside the GEMM saves an eager call 2.5 us of host time for the second launch.  A replayed graph does not pay
-  // that, and there the separate quantiser runs under the end of the kernel in front: a decoder block of Qwen2.5-7B takes 43.2
-  // against 44.8 us at 8 tokens, 44.6 against 45.2 us at 16; one token is level or better in one launch.
-  const bool in_gemm = !swiglu && r->fused &&
-                       (tokens == 1 || c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None);
-  const int64_t bytes = in_gemm ? 0 : r->packed;
-  if (bytes) workspace = at::empty({bytes}, r->bytes);
-  const void* in = x.const_data_ptr();
-  void* out = y.mutable_data_ptr();
-  void* scratch = bytes ? workspace.mutable_data_ptr() : nullptr;
-  void* stream = c10::cuda::getCurrentCUDAStream(r->device.index()).stream();
   const int dtype = type == at::kBFloat16 ? HG_DTYPE_BF16 : HG_DTYPE_F16;
+  at::Tensor y, workspace;
   int status;
-  Py_BEGIN_ALLOW_THREADS
-  status = swiglu ? run_linear_silu(r->handle, r->low, r->high, in, dtype, int(math), scratch, out, stream)
-                  : run_linear(r->handle, r->low, r->high, in, dtype, scratch, out, stream);
-  Py_END_ALLOW_THREADS
+  {
+    // Without the interpreter lock, as torch's own bindings: an allocator may wait for a thread that wants it (one whose
+    // callbacks are Python functions, as of a pool that a serving engine puts to sleep), or for the device.
+    const Unlocked unlocked;
+    // Fresh tensors per call: under CUDA-graph capture the graph's pool owns them.
+    y = at::empty({r->tokens, r->outputs}, r->output);
+    // Quantising inside the GEMM saves an eager call 2.5 us of host time for the second launch.  A replayed graph does not pay
+    // that, and there the separate quantiser runs under the end of the kernel in front: a decoder block of Qwen2.5-7B takes 43.2
+    // against 44.8 us at 8 tokens, 44.6 against 45.2 us at 16; one token is level or better in one launch.
+    const bool in_gemm = !swiglu && r->fused &&
+                         (tokens == 1 || c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None);
+    const int64_t bytes = in_gemm ? 0 : r->packed;
+    if (bytes) workspace = at::empty({bytes}, r->bytes);
+    const void* in = x.const_data_ptr();
+    void* out = y.mutable_data_ptr();
+    void* scratch = bytes ? workspace.mutable_data_ptr() : nullptr;
+    void* stream = c10::cuda::getCurrentCUDAStream(r->device.index()).stream();
+    status = swiglu ? run_linear_silu(r->handle, r->low, r->high, in, dtype, int(math), scratch, out, stream)
+                    : run_linear(r->handle, r->low, r->high, in, dtype, scratch, out, stream);
+  }
   if (status) return PyErr_SetString(PyExc_RuntimeError, last_error()), nullptr;
   if (!count_call(layer, tokens)) return nullptr;
   return THPVariable_Wrap(std::move(y));
