@@ -10,7 +10,6 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 LIBRARY = HERE / "lib" / "libhygemm_b200.so"
 TRACE_LIBRARY = HERE / "lib" / "libhygemm_b200_trace.so"   # same sources with -DHG_TRACE (per-CTA time stamps)
-HOST_EXTENSION = HERE / "lib" / "_hygemm_host.so"          # host path of a layer call, against the installed torch
 HOST_SOURCE = CSRC / "hg_host.cpp"
 SOURCES = ["hg_quant.cu", "hg_gemm_simt.cu", "hg_gemm_tc.cu", "hg_gemm_cluster.cu", "hg_runtime.cu", "hg_tp.cu", "hg_clip.cu"]
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -25,21 +24,29 @@ def stale(library: Path = LIBRARY) -> bool:
     return any(d.stat().st_mtime > built for d in deps)
 
 
+def host_extension() -> Path:
+    """Where the host path of a layer call is built.  It is C++ against torch and CPython, whose binary interfaces change with
+    their versions, so it is named after both: after an upgrade another file is looked for and built."""
+    import torch
+    return HERE / "lib" / f"_hygemm_host.torch-{torch.__version__}.{sys.implementation.cache_tag}.so"
+
+
 def build_host_extension(force: bool = False) -> Path:
-    """Compile ``lib/_hygemm_host.so``; returns its path."""
-    if not force and HOST_EXTENSION.exists() and HOST_EXTENSION.stat().st_mtime >= max(
+    """Compile the host extension; returns its path."""
+    extension = host_extension()
+    if not force and extension.exists() and extension.stat().st_mtime >= max(
             d.stat().st_mtime for d in (HOST_SOURCE, HERE.parent / "include" / "hygemm.h")):
-        return HOST_EXTENSION
+        return extension
     from torch.utils.cpp_extension import include_paths, library_paths
-    HOST_EXTENSION.parent.mkdir(exist_ok=True)
+    extension.parent.mkdir(exist_ok=True)
     cmd = ["g++", "-O2", "-std=c++20", "-fPIC", "-shared", "-Wall", "-I", sysconfig.get_paths()["include"],
-           *[a for p in include_paths("cuda") for a in ("-isystem", p)], str(HOST_SOURCE), "-o", str(HOST_EXTENSION),
+           *[a for p in include_paths("cuda") for a in ("-isystem", p)], str(HOST_SOURCE), "-o", str(extension),
            *["-L" + p for p in library_paths("cuda")], "-lc10", "-lc10_cuda", "-lcudart", "-ltorch_cpu", "-ltorch_python"]
     result = subprocess.run(cmd, capture_output=True, text=True)
     if result.returncode:
         sys.stderr.write(result.stdout + result.stderr)
-        raise RuntimeError(f"g++ failed building {HOST_EXTENSION.name}")
-    return HOST_EXTENSION
+        raise RuntimeError(f"g++ failed building {extension.name}")
+    return extension
 
 
 def build_library(force: bool = False, verbose: bool = False, trace: bool = False) -> Path:

@@ -17,6 +17,7 @@ import ctypes as C
 import importlib.machinery
 import importlib.util
 import os
+import sys
 from pathlib import Path
 
 import torch
@@ -47,7 +48,8 @@ DTYPES = {torch.float16: 0, torch.bfloat16: 1}
 SPLIT_PACK_ROWS = 192512   # most rows hg_split_rows takes (its bitmap of the rows lives in shared memory)
 
 _DEFAULT_LIBRARY = Path(__file__).resolve().parent.parent / "lib" / "libhygemm_b200.so"
-_HOST_EXTENSION = _DEFAULT_LIBRARY.with_name("_hygemm_host.so")
+# Named after the torch and the Python it was built against (build.py).
+_HOST_EXTENSION = _DEFAULT_LIBRARY.with_name(f"_hygemm_host.torch-{torch.__version__}.{sys.implementation.cache_tag}.so")
 _lib = None
 _host = None   # the layer call's host path (csrc/hg_host.cpp), loaded with the library
 

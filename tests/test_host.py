@@ -1,8 +1,10 @@
 """Host-side logic and the C ABI surface (no GPU): exported symbols, tile schedules, plan tables,
 scale-layout helpers, tensor-parallel shard arithmetic."""
 import ctypes as C
+import importlib.util
 import json
 import re
+import sys
 from pathlib import Path
 
 import numpy as np
@@ -271,3 +273,17 @@ def test_tuner_candidates_and_plan_binding(tmp_path):
     path.write_text(json.dumps(tune.bind(rows, other)))
     with pytest.raises(ValueError, match="different binary"):
         plans.PlanTable(path, "hygemm")
+
+
+def test_host_extension_is_named_after_torch_and_python(monkeypatch):
+    """A binary built against another torch or another Python is neither taken for fresh nor loaded."""
+    spec = importlib.util.spec_from_file_location("hygemm_b200_build", ROOT / "comp2029-hybridgemm_b200" / "build.py")
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    here = build.host_extension()
+    assert here == native._HOST_EXTENSION and here.exists()
+    monkeypatch.setattr(torch, "__version__", "2.99.0")
+    assert build.host_extension() != here and not build.host_extension().exists()
+    monkeypatch.undo()
+    monkeypatch.setattr(sys.implementation, "cache_tag", "cpython-399")
+    assert build.host_extension() != here
