@@ -18,6 +18,7 @@ import importlib.machinery
 import importlib.util
 import os
 import sys
+import warnings
 from pathlib import Path
 
 import torch
@@ -51,7 +52,7 @@ _DEFAULT_LIBRARY = Path(__file__).resolve().parent.parent / "lib" / "libhygemm_b
 # Named after the torch and the Python it was built against (build.py).
 _HOST_EXTENSION = _DEFAULT_LIBRARY.with_name(f"_hygemm_host.torch-{torch.__version__}.{sys.implementation.cache_tag}.so")
 _lib = None
-_host = None   # the layer call's host path (csrc/hg_host.cpp), loaded with the library
+_host = None   # the layer call's host path (csrc/hg_host.cpp), loaded with the library where it was built
 
 
 def library_path() -> Path:
@@ -67,9 +68,6 @@ def library():
     if not path.exists():
         raise FileNotFoundError(f"HyGEMM CUDA library not found at {path}; build it with "
                                 f"`python {_DEFAULT_LIBRARY.parent.parent / 'build.py'}` or set HYGEMM_LIBRARY")
-    if not _HOST_EXTENSION.exists():
-        raise FileNotFoundError(f"HyGEMM host extension not found at {_HOST_EXTENSION}; build it with "
-                                f"`python {_DEFAULT_LIBRARY.parent.parent / 'build.py'}`")
     lib = C.CDLL(str(path))
     vp, ci = C.c_void_p, C.c_int
     pp = C.POINTER(Problem)
@@ -109,10 +107,12 @@ def library():
     lib.hg_fused_run.argtypes = [vp, vp]
     lib.hg_fused_info.argtypes = [vp, C.POINTER(ci)]
     lib.hg_fused_destroy.argtypes, lib.hg_fused_destroy.restype = [vp], None
-    loader = importlib.machinery.ExtensionFileLoader("_hygemm_host", str(_HOST_EXTENSION))
-    host = importlib.util.module_from_spec(importlib.util.spec_from_loader("_hygemm_host", loader))
-    host.bind(*(C.cast(f, vp).value for f in (lib.hg_linear, lib.hg_linear_silu, lib.hg_last_error)))
-    _lib, _host = lib, host
+    if _HOST_EXTENSION.exists():
+        loader = importlib.machinery.ExtensionFileLoader("_hygemm_host", str(_HOST_EXTENSION))
+        host = importlib.util.module_from_spec(importlib.util.spec_from_loader("_hygemm_host", loader))
+        host.bind(*(C.cast(f, vp).value for f in (lib.hg_linear, lib.hg_linear_silu, lib.hg_last_error)))
+        _host = host
+    _lib = lib
     return lib
 
 
@@ -184,6 +184,9 @@ class DualLinear:
             # dependent launch), so the packed weights must be complete before the first call: load time only.
             torch.cuda.current_stream(weight.device).synchronize()
         library()
+        if _host is None:
+            warnings.warn(f"HyGEMM host extension not found at {_HOST_EXTENSION}: layer calls take the slower way through ctypes "
+                          f"(`python {_DEFAULT_LIBRARY.parent.parent / 'build.py'}` builds it)", RuntimeWarning, stacklevel=2)
         self.low_id, self.high_id, self.concurrent = low_id, high_id, concurrent
         self.handles = {}
         self.fused_handles = {}
@@ -219,7 +222,7 @@ class DualLinear:
         return tuple(found) == (high, 0)
 
     def __call__(self, x):
-        y = None if PACK_MODE else _host.forward(self, x, -1)
+        y = None if PACK_MODE or _host is None else _host.forward(self, x, -1)
         return self._unprepared(x) if y is None else y
 
     def _unprepared(self, x):
@@ -227,7 +230,7 @@ class DualLinear:
         shape = x.shape
         if len(shape) != 2 or shape[1] != self.k or x.device != self.w4.device:
             raise ValueError("HyGEMM input shape/device does not match its weights")
-        if not shape[0] or x.dtype not in DTYPES or PACK_MODE or not x.is_contiguous() or not self._tensor_core():
+        if not shape[0] or x.dtype not in DTYPES or PACK_MODE or _host is None or not x.is_contiguous() or not self._tensor_core():
             return self.run_packed(*pack(x))
         return self._prepared(x, -1)
 
@@ -238,12 +241,12 @@ class DualLinear:
 
     def silu_linear(self, x, math):
         """This layer on SwiGLU of `x` = gate||up `[tokens, 2K]`: `producer.silu_pack` followed by `run_packed`."""
-        known = math in (0, 1, 2)   # the native path takes a negative one for a call without SwiGLU
-        y = _host.forward(self, x, math) if known else None
+        native_path = _host is not None and math in (0, 1, 2)   # it takes a negative one for a call without SwiGLU
+        y = _host.forward(self, x, math) if native_path else None
         if y is not None:
             return y
         shape = x.shape
-        if (not known or len(shape) != 2 or shape[1] != 2 * self.k or not shape[0] or x.dtype not in DTYPES or x.device != self.w4.device
+        if (not native_path or len(shape) != 2 or shape[1] != 2 * self.k or not shape[0] or x.dtype not in DTYPES or x.device != self.w4.device
                 or not x.is_contiguous() or not self._tensor_core()):
             from .producer import silu_pack
             return self.run_packed(*silu_pack(x, math))

@@ -74,6 +74,21 @@ def test_layer_call_by_every_route(tokens):
     layer.close()
 
 
+def test_layer_calls_without_the_host_extension(monkeypatch):
+    """A library whose host extension was not built: the layer says so once it is made, and its calls give the same bytes."""
+    g = torch.Generator().manual_seed(5)
+    w, ids = (torch.randn(300, 256, generator=g) * 0.04).bfloat16().cuda(), torch.arange(40).cuda()
+    x, pair = torch.randn(5, 256, generator=g).bfloat16().cuda(), torch.randn(5, 512, generator=g).bfloat16().cuda()
+    layer = native.DualLinear(w, ids)
+    want = layer(x), layer.silu_linear(pair, 0)
+    monkeypatch.setattr(native, "_host", None)
+    with pytest.warns(RuntimeWarning, match="host extension not found"):
+        plain = native.DualLinear(w, ids)
+    assert torch.equal(plain(x), want[0]) and torch.equal(plain.silu_linear(pair, 0), want[1])
+    layer.close()
+    plain.close()
+
+
 @pytest.mark.parametrize("how", ["attribute", "storage"])
 @pytest.mark.parametrize("name", ["w4", "sf4", "lo", "w8", "sf8", "hi"])
 def test_layer_call_after_an_operand_was_replaced(name, how):

@@ -3,7 +3,10 @@ scale-layout helpers, tensor-parallel shard arithmetic."""
 import ctypes as C
 import importlib.util
 import json
+import os
 import re
+import shutil
+import subprocess
 import sys
 from pathlib import Path
 
@@ -287,3 +290,14 @@ def test_host_extension_is_named_after_torch_and_python(monkeypatch):
     monkeypatch.undo()
     monkeypatch.setattr(sys.implementation, "cache_tag", "cpython-399")
     assert build.host_extension() != here
+
+
+def test_library_loads_without_the_host_extension(tmp_path):
+    """The CUDA library alone, named by HYGEMM_LIBRARY beside a package that was never built: everything but the native
+    route of a layer call is there."""
+    package = ROOT / "comp2029-hybridgemm_b200"
+    shutil.copytree(package / "hygemm_vllm", tmp_path / "hygemm_vllm")
+    code = "from hygemm_vllm import native; assert native.library().hg_scale_size(129, 256) == 2048 and native._host is None"
+    environment = {**os.environ, "HYGEMM_LIBRARY": str(native._DEFAULT_LIBRARY), "PYTHONPATH": str(tmp_path)}
+    result = subprocess.run([sys.executable, "-c", code], cwd=tmp_path, env=environment, capture_output=True, text=True)
+    assert result.returncode == 0, result.stderr[-2000:]
