@@ -14,9 +14,10 @@
 //
 // The statistics of the search (errors before and after, how far the scales moved) and the checks on its inputs are
 // gathered in the same pass: the values, codes and both scales are in registers here, and as torch ops they were a
-// dozen passes over full-size fp32 tensors and ten host synchronisations (4096 x 3584: 1660 us, 67 us now, half of them host work).  The
-// kernel is bound by its arithmetic, so only the winning candidate is encoded, a
-// thread's sums over its dozen items are kept in fp32 (one conversion to fp64 at the end) and the offsets are read from the constant bank.
+// dozen passes over full-size fp32 tensors and ten host synchronisations (4096 x 3584: 1660 us a call, 65 us now, of which
+// the kernel is 43).  The kernel is bound by its arithmetic, so only the winning candidate is encoded and the offsets are read
+// from the constant bank.  An item's eight terms are added in fp32, everything above that in fp64: a thread has 12 items of a
+// 4096 x 3584 matrix and 590 of a 37888 x 18944 one, over which fp32 sums drift (they took 42.3 us here).
 #include <algorithm>
 
 #include "hg_common.cuh"
@@ -74,7 +75,7 @@ mx_clip_search_kernel(const uint16_t* __restrict__ in, const float* __restrict__
   const int per_row = k >> 3;
   const int64_t threads = int64_t(rows) * per_row, stride = int64_t(gridDim.x) * blockDim.x;
   const uint32_t mask = 0xfu << (threadIdx.x & 28);   // the four threads of this K32 group (groups never straddle the tail)
-  float sums[4] = {0.f, 0.f, 0.f, 0.f};
+  double sums[4] = {0., 0., 0., 0.};
   int moved[kMaxClipOffsets] = {}, flags = 0;
   for (int64_t thread = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; thread < threads; thread += stride) {   // whole groups leave together
     const int row = threads < (int64_t(1) << 31) ? int(uint32_t(thread) / uint32_t(per_row)) : int(thread / per_row);
@@ -157,7 +158,7 @@ mx_clip_search_kernel(const uint16_t* __restrict__ in, const float* __restrict__
       if (lane == 0) block_sum[warp][slot] = value;
     };
 #pragma unroll
-    for (int i = 0; i < 4; ++i) over_warp(double(sums[i]), i);
+    for (int i = 0; i < 4; ++i) over_warp(sums[i], i);
 #pragma unroll
     for (int i = 0; i < 3; ++i) over_warp(double((flags >> i) & 1), kNotFinite + i);
     if (lane == 0) block_sum[warp][7] = 0.;

@@ -44,6 +44,21 @@ def test_random_matrices_match_the_oracle(dtype, rows, k):
         assert stats["shift_groups"]["0"] < scales.numel() or rows == 1
 
 
+@pytest.mark.parametrize("weighted", [False, True])
+def test_statistics_of_a_tall_matrix_do_not_drift(weighted):
+    """One row repeated: the sums are the row's, times the number of rows, to the rounding of fp64 sums.  (20000 x 3584 gives a thread 59
+    items; each item's fp32 part is the same in both calls, and a sum of N doubles is off by at most N 2^-53: 1e-9 for 9e6.)"""
+    g = torch.Generator().manual_seed(SEED)
+    rows, k = 20000, 3584
+    row = (torch.randn(1, k, generator=g) * 0.03).bfloat16().cuda()
+    importance = (torch.rand(k, generator=g) * 3).cuda() if weighted else None
+    _, _, one = fp4_quant.quantize(row, importance)
+    _, _, many = fp4_quant.quantize(row.expand(rows, k).contiguous(), importance)
+    for name in ("weighted_error_before", "weighted_error_after", "weight_error_before", "weight_error_after"):
+        assert abs(many[name] / (rows * one[name]) - 1) <= 1e-9, (name, many[name], rows * one[name])
+    assert many["shift_groups"] == {s: rows * n for s, n in one["shift_groups"].items()}
+
+
 def test_no_offsets_is_round_to_nearest_and_feeds_a_layer():
     """Without offsets the result is hg_pack's; a searched bank installs into a layer and changes only the low rows."""
     g = torch.Generator().manual_seed(SEED)
