@@ -342,14 +342,23 @@ __device__ __forceinline__ void emit_rows(const Raw16 (&raw)[4], const QuantPart
     *reinterpret_cast<uint4*>(part.sf + scale_word_offset(row0, col >> 7, k)) = make_uint4(word[0], word[1], word[2], word[3]);
 }
 
+// How row lists say that they are not complete: see partition_rows_kernel.
+__device__ __forceinline__ int bad_list_mark(int distinct, int out_of_range) { return -1 - (2 * distinct + out_of_range); }
+// {distinct ids, an id was out of range}
+__device__ __forceinline__ int2 list_verdict(const int32_t* hi, int n_ids) {
+  const int last = n_ids ? __ldcg(hi + n_ids - 1) : 0;
+  return last >= 0 ? make_int2(n_ids, 0) : make_int2((-1 - last) >> 1, (-1 - last) & 1);
+}
+
 // Packs `low` to MXFP4 and `high` to MXFP8 (either may be empty).  Every warp walks items of one row group x 512 columns and has
 // the next item's loads in flight while it converts the current one (37888 x 3584 to MXFP4 56 us, 67 without).  Row numbers
-// another item ahead cost more in registers than their latency.
+// another item ahead cost more in registers than their latency.  `verdict`: where to tell the host about the lists, or null.
 template <typename T>
 __global__ void __launch_bounds__(256, kRowsBlocks)
-mx_rows_kernel(const uint16_t* __restrict__ in, const QuantPart low, const QuantPart high, int k) {
+mx_rows_kernel(const uint16_t* __restrict__ in, const QuantPart low, const QuantPart high, int k, int* __restrict__ verdict) {
   pdl_trigger();
   pdl_wait();   // input and row lists come from the kernels before
+  if (verdict && blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<int2*>(verdict) = list_verdict(high.ids, high.rows);
   const int lane = threadIdx.x & 31, chunks = (k + 511) >> 9;
   const int low_groups = ((low.rows + 127) & ~127) >> 2, groups = low_groups + (((high.rows + 127) & ~127) >> 2);
   const int stride = gridDim.x * 8;
@@ -457,17 +466,18 @@ constexpr int64_t kManyRowsElements = 4 << 20;
 static unsigned row_blocks(int64_t groups, int k) { return unsigned((groups * ((k + 511) / 512) + 7) / 8); }
 
 template <typename T>
-static cudaError_t launch_rows(const void* in, const QuantPart& low, const QuantPart& high, int k, cudaStream_t s) {
+static cudaError_t launch_rows(const void* in, const QuantPart& low, const QuantPart& high, int k, cudaStream_t s, int* verdict = nullptr) {
   const int64_t groups = (int64_t((low.rows + 127) & ~127) + ((high.rows + 127) & ~127)) / 4;
-  return launch_kernel(mx_rows_kernel<T>, dim3(std::min(row_blocks(groups, k), unsigned(148 * kRowsBlocks))), dim3(256), 0, s, static_cast<const uint16_t*>(in), low, high, k);
+  return launch_kernel(mx_rows_kernel<T>, dim3(std::min(row_blocks(groups, k), unsigned(148 * kRowsBlocks))), dim3(256), 0, s, static_cast<const uint16_t*>(in), low, high, k, verdict);
 }
 
 // The row lists of a layer from the ids of its MXFP8 channels: one block, a bitmap of the rows in shared memory, a scan of its
-// words, and a warp per word that writes 32 rows at once.  result = {distinct ids, an id was out of range}; the lists are
-// only complete when ids are distinct and in range.
+// words, and a warp per word that writes 32 rows at once.  The lists are only complete when ids are distinct and in range.
+// Otherwise fewer than n_ids rows are set, the last entry of `hi` is left over, and it says so (list_verdict): the verdict
+// belongs to the lists, wherever the packing that reads it is enqueued.
 constexpr int kPartitionThreads = 1024;
 __global__ void __launch_bounds__(kPartitionThreads)
-partition_rows_kernel(const int64_t* __restrict__ ids, int n_ids, int rows, int32_t* __restrict__ lo, int32_t* __restrict__ hi, int* __restrict__ result) {
+partition_rows_kernel(const int64_t* __restrict__ ids, int n_ids, int rows, int32_t* __restrict__ lo, int32_t* __restrict__ hi) {
   extern __shared__ uint32_t bitmap[];   // words of the bitmap, then the MXFP8 rows before each word
   __shared__ int warp_sum[32];
   pdl_trigger();
@@ -520,7 +530,7 @@ partition_rows_kernel(const int64_t* __restrict__ ids, int n_ids, int rows, int3
       lo[row - high] = row;
     }
   }
-  if (tid == 0) { result[0] = warp_sum[31]; result[1] = bad; }
+  if (tid == 0 && warp_sum[31] != n_ids) hi[n_ids - 1] = bad_list_mark(warp_sum[31], bad);
 }
 
 template <typename T, bool FP4, bool SILU, int MATH>
@@ -581,8 +591,7 @@ static void split_rows(const int64_t* ids, int n_ids, int rows, int32_t* lo, int
   if (rows <= 0 || n_ids < 0 || n_ids > rows || (n_ids && (!ids || !hi)) || (n_ids < rows && !lo)) throw std::runtime_error("Invalid split-rows arguments");
   const size_t shared = size_t((rows + 31) / 32) * 8;
   if (shared > 47 * 1024) throw std::runtime_error("Too many rows for one split");
-  // the verdict goes straight to the host's buffer, over the bus: no copy afterwards
-  check(launch_kernel(partition_rows_kernel, dim3(1), dim3(kPartitionThreads), shared, s, ids, n_ids, rows, lo, hi, static_cast<int*>(host_result().host)), "partition launch");
+  check(launch_kernel(partition_rows_kernel, dim3(1), dim3(kPartitionThreads), shared, s, ids, n_ids, rows, lo, hi), "partition launch");
 }
 
 static void split_pack(const void* weight, int n_ids, int rows, int k, const int32_t* lo, const int32_t* hi, void* w4, void* sf4, void* w8,
@@ -592,9 +601,9 @@ static void split_pack(const void* weight, int n_ids, int rows, int k, const int
   if (reinterpret_cast<uintptr_t>(weight) & 31) throw std::runtime_error("Split-pack weights must be 32-byte aligned");
   if (!aligned16(w4) || !aligned16(sf4) || !aligned16(w8) || !aligned16(sf8)) throw std::runtime_error("MX pack pointers must be 16-byte aligned");
   const QuantPart low{lo, static_cast<uint8_t*>(w4), static_cast<uint8_t*>(sf4), rows - n_ids, rows}, high{hi, static_cast<uint8_t*>(w8), static_cast<uint8_t*>(sf8), n_ids, rows};
-  check(dtype == HG_DTYPE_BF16 ? launch_rows<__nv_bfloat16>(weight, low, high, k, s) : launch_rows<__half>(weight, low, high, k, s), "split-pack launch");
+  int* const result = static_cast<int*>(host_result().host);   // written over the bus: no copy afterwards
+  check(dtype == HG_DTYPE_BF16 ? launch_rows<__nv_bfloat16>(weight, low, high, k, s, result) : launch_rows<__half>(weight, low, high, k, s, result), "split-pack launch");
   check(cudaStreamSynchronize(s), "split-pack");
-  const int* result = static_cast<const int*>(host_result().host);
   verdict[0] = result[0];
   verdict[1] = result[1];
 }

@@ -80,11 +80,12 @@ int hg_pack_bf16(const void* in, void* out, void* sf, int rows, int k, int fp4, 
 int hg_pack_mode_bf16(const void* in, void* out, void* sf, int rows, int k, int fp4, void* stream, int mode);
 
 /* Load-time packing of a [rows,k] 16-bit weight matrix (HG_DTYPE_*) into both partitions of a hybrid linear, in two calls on one
- * stream by one thread.  hg_split_rows: `ids` holds the output channels kept in MXFP8 (n_ids distinct values in [0,rows), any
- * order); enqueues the sorted channel maps `hi` [n_ids] and `lo` [rows-n_ids]; at most 192512 rows.  hg_split_pack: what
+ * stream.  hg_split_rows: `ids` holds the output channels kept in MXFP8 (n_ids distinct values in [0,rows), any
+ * order); enqueues the sorted channel maps `hi` [n_ids] and `lo` [rows-n_ids]; at most 192512 rows.  Maps of ids that are not
+ * distinct or out of range are marked (a negative last entry of `hi`) and not complete.  hg_split_pack: what
  * hg_pack writes for the rows the maps name, w4 [rows-n_ids,k/2] and sf4, w8 [n_ids,k] and sf8; waits for the stream.
- * verdict[2] = {distinct ids, 1 if an id was out of range}: with anything but {n_ids, 0} the outputs are not complete and must
- * not be used.  `weight` is 32-byte aligned.  (The reference gathers and packs per partition,
+ * verdict[2] = {distinct ids, 1 if an id was out of range} of these maps: with anything but {n_ids, 0} the outputs are not
+ * complete and must not be used.  `weight` is 32-byte aligned.  (The reference gathers and packs per partition,
  * integrations/vllm/hygemm_vllm/native.py:53-68.) */
 int hg_split_rows(const int64_t* ids, int n_ids, int rows, int32_t* lo, int32_t* hi, void* stream);
 int hg_split_pack(const void* weight, int n_ids, int rows, int k, const int32_t* lo, const int32_t* hi, void* w4, void* sf4,

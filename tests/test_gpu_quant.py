@@ -1,10 +1,12 @@
 """Quantiser and SwiGLU producer through the C ABI vs the CPU oracle (bit-exact)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
 
 import oracle
-from helpers import bits
+from helpers import SEED, bits
 from hygemm_vllm import native, producer
 
 pytestmark = pytest.mark.gpu
@@ -134,3 +136,38 @@ def test_silu_pack_vs_vllm_op():
             q, sf, dbg = producer.silu_pack(x, 0, debug=True)
             assert torch.equal(dbg.view(torch.int16), out.view(torch.int16)), (dtype, rows, k)
             assert torch.equal(q, q_ref) and torch.equal(sf, sf_ref)
+
+
+def test_split_verdict_belongs_to_the_maps_that_are_packed():
+    """Maps made in one order and packed in another, and maps that are never packed: every packing reports on its own maps."""
+    lib, stream = native.library(), torch.cuda.current_stream().cuda_stream
+    rows, k = 300, 256
+    weight = torch.randn(rows, k, generator=torch.Generator().manual_seed(SEED)).bfloat16().cuda()
+    lists = {"repeated": [7, 7, 9, 250], "out of range": [3, 300, 5, -1], "good": [299, 0, 31, 32], "none": [], "all": list(range(rows))[::-1],
+             "last one repeated": [5, 6, 299, 299], "all but one": [0, *range(rows - 1)]}
+    distinct = {"repeated": (3, 0), "out of range": (2, 1), "good": (4, 0), "none": (0, 0), "all": (rows, 0), "last one repeated": (3, 0),
+                "all but one": (rows - 1, 0)}
+
+    def maps(name):
+        ids = torch.tensor(lists[name], dtype=torch.int64).cuda()
+        hi = torch.full((len(lists[name]),), 1 << 30, dtype=torch.int32, device="cuda")
+        lo = torch.full((rows - len(lists[name]),), 1 << 30, dtype=torch.int32, device="cuda")
+        native.check(lib.hg_split_rows(ids.data_ptr(), ids.numel(), rows, lo.data_ptr(), hi.data_ptr(), stream))
+        torch.cuda.synchronize()
+        return lo, hi
+
+    made = {name: maps(name) for name in lists}
+    for name in reversed(lists):
+        lo, hi = made[name]
+        n = hi.numel()
+        w4, w8 = (torch.empty(s, dtype=torch.uint8, device="cuda") for s in ((rows - n, k // 2), (n, k)))
+        sf4, sf8 = (torch.empty(native.scale_size(r, k), dtype=torch.uint8, device="cuda") for r in (rows - n, n))
+        verdict = (C.c_int * 2)()
+        native.check(lib.hg_split_pack(weight.data_ptr(), n, rows, k, lo.data_ptr(), hi.data_ptr(), w4.data_ptr(), sf4.data_ptr(), w8.data_ptr(),
+                                       sf8.data_ptr(), verdict, 1, stream))
+        assert tuple(verdict) == distinct[name], name
+        if verdict[0] == n and not verdict[1]:
+            assert hi.tolist() == sorted(lists[name]) and lo.tolist() == sorted(set(range(rows)) - set(lists[name]))
+            for part, codes, sf, fp4 in ((lo, w4, sf4, True), (hi, w8, sf8, False)):
+                want, want_sf = native.pack(weight[part.long()].contiguous(), fp4)
+                assert torch.equal(codes, want) and torch.equal(sf, want_sf)
