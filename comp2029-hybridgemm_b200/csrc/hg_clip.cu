@@ -226,9 +226,9 @@ extern "C" int hg_clip_pack_stats(const void* in, const float* importance, void*
   HG_TRY
   if (!host_stats) throw std::runtime_error("Invalid MX clip-pack arguments");
   const auto s = static_cast<cudaStream_t>(stream);
-  const hg::HostResult result = hg::host_result();
+  hg::HostResult result(s);
   hg::clip_pack(in, importance, q4, scales, rows, k, offsets, n_offsets, dtype, static_cast<double*>(result.device), static_cast<double*>(result.host), s);
-  hg::check(cudaStreamSynchronize(s), "clip-pack");
+  result.wait("clip-pack");
   std::copy(static_cast<double*>(result.host), static_cast<double*>(result.host) + hg::kClipStats, host_stats);
   HG_CATCH
 }

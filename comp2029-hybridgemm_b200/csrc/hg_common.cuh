@@ -39,12 +39,26 @@ __host__ __device__ inline int64_t scale_word_offset(int row, int kb, int k) {
   return (int64_t(row / 128) * (k / 128) + kb) * 512 + (row % 32) * 16 + ((row % 128) / 32) * 4;
 }
 
-// For calls that end with a host-side result, 256 bytes each of pinned memory that kernels can write (a copy from device
-// memory, through a pageable buffer above all, costs more than the wait itself) and of zeroed device memory that a kernel
-// leaves zeroed.  They belong to the calling thread and device and are given back with the thread; such a call waits for
-// its stream, so one at a time uses them.
-struct HostResult { void* host; void* device; };
-HostResult host_result();
+// For calls that end with a host-side result: 256 bytes each of pinned memory that kernels can write (a copy from device
+// memory, through a pageable buffer above all, costs more than the wait itself) and of device memory, zeroed in the order
+// of the stream, that a kernel leaves zeroed.  A call holds a pair of its own for its duration.  Pairs go back to a pool, as many
+// as calls were ever under way at once on a device (at most kHostResultsKept wait there), once the stream has been
+// waited for; one whose stream cannot be waited for stays out of use.  They are allocated and freed in relaxed capture mode, so
+// that another thread's capture is not disturbed.
+constexpr size_t kHostResultsKept = 16;
+class HostResult {
+ public:
+  explicit HostResult(cudaStream_t stream);
+  ~HostResult();
+  HostResult(const HostResult&) = delete;
+  void wait(const char* what);   // for the stream; `host` is complete then
+  void* host = nullptr;
+  void* device = nullptr;
+ private:
+  cudaStream_t stream_;
+  int ordinal_ = 0;
+  bool waited_ = false;
+};
 
 #ifdef __CUDACC__
 // Programmatic dependent launch.  Every kernel of the library is launched with the

@@ -11,7 +11,9 @@
 // the kernel and every byte of the scale buffer is rewritten on every call.
 #include <algorithm>
 #include <cstdlib>
+#include <mutex>
 #include <type_traits>
+#include <vector>
 
 #include "hg_common.cuh"
 
@@ -22,32 +24,69 @@ std::string& last_error() {
   return message;
 }
 
-HostResult host_result() {
-  constexpr size_t kBytes = 256;
-  constexpr int kDevices = 64;
-  struct Buffers {
-    HostResult of[kDevices] = {};
-    ~Buffers() {
-      for (HostResult& r : of) {
-        if (r.host) cudaFreeHost(r.host);
-        if (r.device) cudaFree(r.device);
-      }
+namespace {
+
+struct HostPair { void* host; void* device; };
+
+struct HostPool {
+  std::mutex mutex;
+  std::vector<HostPair> idle[64];
+};
+HostPool& host_pool() {
+  static HostPool* const pool = new HostPool;   // not destroyed: at exit the driver may be gone before it
+  return *pool;
+}
+
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+constexpr size_t kHostResultBytes = 256;
+
+}  // namespace
+
+HostResult::HostResult(cudaStream_t stream) : stream_(stream) {
+  check(cudaGetDevice(&ordinal_), "cudaGetDevice");
+  if (ordinal_ < 0 || ordinal_ >= 64) throw std::runtime_error("Device ordinals 0..63 are supported");
+  HostPool& pool = host_pool();
+  {
+    std::lock_guard<std::mutex> lock(pool.mutex);
+    std::vector<HostPair>& idle = pool.idle[ordinal_];
+    if (!idle.empty()) {
+      host = idle.back().host;
+      device = idle.back().device;
+      idle.pop_back();
+      return;
     }
-  };
-  static thread_local Buffers buffers;
-  int device = 0;
-  check(cudaGetDevice(&device), "cudaGetDevice");
-  if (device < 0 || device >= kDevices) throw std::runtime_error("Device ordinals 0..63 are supported");
-  HostResult& r = buffers.of[device];
-  if (!r.host) check(cudaHostAlloc(&r.host, kBytes, cudaHostAllocPortable | cudaHostAllocMapped), "pinned buffer");
-  if (!r.device) {
-    void* fresh = nullptr;
-    check(cudaMalloc(&fresh, kBytes), "result buffer");
-    check(cudaMemset(fresh, 0, kBytes), "result buffer");
-    check(cudaDeviceSynchronize(), "result buffer");
-    r.device = fresh;
   }
-  return r;
+  const RelaxedCapture relaxed;
+  check(cudaHostAlloc(&host, kHostResultBytes, cudaHostAllocPortable | cudaHostAllocMapped), "pinned buffer");
+  cudaError_t e = cudaMalloc(&device, kHostResultBytes);
+  if (e != cudaSuccess) cudaFreeHost(host);
+  check(e, "result buffer");
+  check(cudaMemsetAsync(device, 0, kHostResultBytes, stream), "result buffer");
+}
+
+void HostResult::wait(const char* what) {
+  check(cudaStreamSynchronize(stream_), what);
+  waited_ = true;
+}
+
+HostResult::~HostResult() {
+  if (!waited_ && cudaStreamSynchronize(stream_) != cudaSuccess) return;   // an error before the wait: work may be in flight
+  HostPool& pool = host_pool();
+  {
+    std::lock_guard<std::mutex> lock(pool.mutex);
+    std::vector<HostPair>& idle = pool.idle[ordinal_];
+    if (idle.size() < kHostResultsKept) {
+      idle.push_back({host, device});
+      return;
+    }
+  }
+  const RelaxedCapture relaxed;
+  cudaFreeHost(host);
+  cudaFree(device);
 }
 
 bool pdl_enabled() {
@@ -601,9 +640,10 @@ static void split_pack(const void* weight, int n_ids, int rows, int k, const int
   if (reinterpret_cast<uintptr_t>(weight) & 31) throw std::runtime_error("Split-pack weights must be 32-byte aligned");
   if (!aligned16(w4) || !aligned16(sf4) || !aligned16(w8) || !aligned16(sf8)) throw std::runtime_error("MX pack pointers must be 16-byte aligned");
   const QuantPart low{lo, static_cast<uint8_t*>(w4), static_cast<uint8_t*>(sf4), rows - n_ids, rows}, high{hi, static_cast<uint8_t*>(w8), static_cast<uint8_t*>(sf8), n_ids, rows};
-  int* const result = static_cast<int*>(host_result().host);   // written over the bus: no copy afterwards
+  HostResult buffers(s);
+  int* const result = static_cast<int*>(buffers.host);   // written over the bus: no copy afterwards
   check(dtype == HG_DTYPE_BF16 ? launch_rows<__nv_bfloat16>(weight, low, high, k, s, result) : launch_rows<__half>(weight, low, high, k, s, result), "split-pack launch");
-  check(cudaStreamSynchronize(s), "split-pack");
+  buffers.wait("split-pack");
   verdict[0] = result[0];
   verdict[1] = result[1];
 }

@@ -1,5 +1,7 @@
 """Quantiser and SwiGLU producer through the C ABI vs the CPU oracle (bit-exact)."""
 import ctypes as C
+import threading
+import time
 
 import numpy as np
 import pytest
@@ -7,7 +9,7 @@ import torch
 
 import oracle
 from helpers import SEED, bits
-from hygemm_vllm import native, producer
+from hygemm_vllm import fp4_quant, native, producer
 
 pytestmark = pytest.mark.gpu
 
@@ -171,3 +173,50 @@ def test_split_verdict_belongs_to_the_maps_that_are_packed():
             for part, codes, sf, fp4 in ((lo, w4, sf4, True), (hi, w8, sf8, False)):
                 want, want_sf = native.pack(weight[part.long()].contiguous(), fp4)
                 assert torch.equal(codes, want) and torch.equal(sf, want_sf)
+
+
+def test_calls_with_a_host_result_beside_a_capture_and_from_many_threads():
+    """Packing and offline search end with numbers for the host.  A thread that made such calls and ends, or makes its first ones, does
+    not disturb a capture on another thread; calls of many threads at once each get their own numbers."""
+    w = (torch.randn(256, 256, generator=torch.Generator().manual_seed(SEED)) * 0.03).bfloat16().cuda()
+    ids = torch.arange(0, 256, 5).cuda()
+    _, _, want = fp4_quant.quantize(w)
+    may_end, made, failures = threading.Event(), threading.Barrier(9), []
+
+    def worker(index):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                scale = 2.0 ** index                         # an exact factor of the weights: its square in the errors
+                mine = w * scale
+                torch.cuda.current_stream().synchronize()
+                for _ in range(20):
+                    _, _, stats = fp4_quant.quantize(mine)
+                    assert stats["shift_groups"] == want["shift_groups"]
+                    for name in ("weight_error_before", "weight_error_after"):
+                        # the same terms, in another order: 8192 of them in fp64
+                        assert abs(stats[name] / (scale * scale * want[name]) - 1) < 1e-11
+                layer = native.DualLinear(mine, ids)
+                assert torch.equal(layer.hi.long(), ids)
+                layer.close()
+        except Exception as e:   # noqa: BLE001
+            failures.append(e)
+        made.wait()
+        may_end.wait()
+
+    threads = [threading.Thread(target=worker, args=(i,)) for i in range(8)]
+    for t in threads:
+        t.start()
+    made.wait()
+    assert not failures, failures
+    x = torch.ones(16, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = x + 1
+        may_end.set()
+        for t in threads:
+            t.join()
+        time.sleep(0.5)                                      # the threads themselves end a little after their joins
+        y = y + 1
+    graph.replay()
+    assert torch.equal(y, x + 2)
