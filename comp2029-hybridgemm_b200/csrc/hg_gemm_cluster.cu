@@ -24,6 +24,7 @@
 // hides it: loops here carry no divisions, addresses are independent of each other, and descriptors are sums.
 // Every mbarrier wait is bounded; on expiry the CTA records a code, drains and leaves.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -59,7 +60,6 @@ struct ClusterParams {
   uint32_t tmem_cols;
   const uint16_t* x;
   int x_bf16;
-  int audit_tokens;
   int* status;
 #ifdef HG_TRACE
   unsigned long long* trace;
@@ -190,7 +190,7 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // n / d with inverse = ceil(2^40 / d), exact while n d < 2^40; the host passes 0 where that or the product does not fit.
-__device__ __forceinline__ int fast_div(int64_t n, int d, uint64_t inverse) {
+__host__ __device__ __forceinline__ int fast_div(int64_t n, int d, uint64_t inverse) {
   return inverse ? int((uint64_t(n) * inverse) >> 40) : int(n / d);
 }
 
@@ -201,7 +201,7 @@ __device__ __forceinline__ int fast_div(int64_t n, int d, uint64_t inverse) {
 struct Unit {
   int part, atom, first, last, token0, n;   // rows first .. last - 1 of the 128-row atom (PAIR: of atoms 2 atom and 2 atom + 1)
 };
-__device__ __forceinline__ Unit unit_at(const ClusterParams& p, int u) {
+__host__ __device__ __forceinline__ Unit unit_at(const ClusterParams& p, int u) {
   Unit w;
   int tile;
   if (p.token_tiles == 1) {
@@ -225,10 +225,9 @@ __device__ __forceinline__ Unit unit_at(const ClusterParams& p, int u) {
   return w;
 }
 
-// 128-row atoms a unit starts: what the audit counters count.
-template <int PAIR>
-__device__ __forceinline__ int atoms_started(const ClusterParams& p, const Unit& w) {
-  return w.first ? 0 : min(PAIR, ((p.rows[w.part] + kTileRows - 1) >> 7) - w.atom * PAIR);
+// First K256 step of a slice of K (of the slice behind the last one: the end).
+__host__ __device__ __forceinline__ int first_step(const ClusterParams& p, int slice) {
+  return (((p.kblocks + 1) >> 1) * slice) >> p.split_log;
 }
 
 template <typename T, int PAIR, bool FUSED>
@@ -293,8 +292,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
 
   const uint32_t sf_cols = tmem_base + p.tmem_cols - 2u * kScaleStride;
   const int units = (p.tiles[0] + p.tiles[1]) * p.token_tiles;
-  const int steps = (p.kblocks + 1) >> 1;                        // K256 steps of a tile ...
-  const int step_begin = (steps * slice) >> p.split_log, step_end = (steps * (slice + 1)) >> p.split_log;   // ... and of this slice
+  const int step_begin = first_step(p, slice), step_end = first_step(p, slice + 1);   // K256 steps of this slice
   int error = 0;
 
   if (warp == 0) {
@@ -484,6 +482,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
           }
           __syncwarp();
           accumulate = 1;
+          issued += nkb;
           if (++stage == p.stages) { stage = 0; phase ^= 1u; }
         }
         if (error) break;
@@ -492,14 +491,12 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
 #ifdef HG_TRACE
         if (lane == 0 && it < 4) HG_STAMP(4 + it);
 #endif
-        issued += atoms_started<PAIR>(p, w) * (min(2 * step_end, p.kblocks) - 2 * step_begin) *
-                  ((min(w.n, p.tokens - w.token0) + p.audit_tokens - 1) / p.audit_tokens);
       }
       // Every MMA of this CTA (pair) retires before TMEM is released.
       if (elect_one()) cg_commit<PAIR>(drain_bar, pair_mask);
       __syncwarp();
       if (!warp_wait(drain_bar, 0, abort_flag) && !error) error = kErrDrain;
-      if (lane == 0 && issued) atomicAdd(p.status + 1, issued);
+      if (lane == 0 && issued) atomicAdd(p.status + 1, issued * PAIR);   // a pair's MMA works on a tile of each CTA
     } else if (PAIR == 2) {
       // ---------------------------------------------------------------- second CTA of a pair: wait for the last MMA
       if (!warp_wait(drain_bar, 0, abort_flag) && !error) error = kErrDrain;
@@ -631,8 +628,10 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
         if (!p.overlap) release(acc);
       }
       if (threadIdx.x == 64 && it < 3) HG_STAMP(9 + 2 * it);
-      if (slice == 0 && half == 0 && threadIdx.x == 64) stored += atoms_started<PAIR>(p, w) * ((valid + p.audit_tokens - 1) / p.audit_tokens);
+      ++stored;
     }
+    // One warp speaks for the CTA's: an accumulator is only free for the next unit once all of them have arrived.  (Counted over all
+    // warps in shared memory, a block took 1 % longer at 16 tokens, 2 % at 37.)
     if (threadIdx.x == 64 && stored) atomicAdd(p.status + 2, stored);
   }
 
@@ -833,6 +832,23 @@ const int* cluster_capacity() {
   return capacity[device];
 }
 
+// Clusters of 1, 2, 4 and 8 CTAs on a device with `sms` SMs: what the current device holds if it has as many, else as many
+// as fit if no SM were out of reach of a cluster.
+static std::array<int, 4> capacity_for(int sms) {
+  int devices = 0, device = 0, count = 0;
+  if (cudaGetDeviceCount(&devices) == cudaSuccess && devices > 0 && cudaGetDevice(&device) == cudaSuccess &&
+      cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && count == sms) {
+    const int* held = cluster_capacity();
+    return {held[0], held[1], held[2], held[3]};
+  }
+  cudaGetLastError();   // no GPU: not this call's error
+  return {sms, sms >> 1, sms >> 2, sms >> 3};
+}
+
+ClusterPlan make_cluster_plan_for(int lo, int hi, int tokens, int k, int sms) {
+  return make_cluster_plan(lo, hi, tokens, k, capacity_for(sms).data());
+}
+
 template <typename T, int PAIR, bool FUSED>
 static cudaError_t launch(const ClusterPlan& plan, const ClusterParams& p, const ClusterMaps& maps, cudaStream_t stream, bool pdl) {
   cudaLaunchConfig_t config{};
@@ -855,19 +871,13 @@ static cudaError_t launch(const ClusterPlan& plan, const ClusterParams& p, const
   return cudaLaunchKernelEx(&config, cluster_gemm_kernel<T, PAIR, FUSED>, p, maps);
 }
 
-void launch_cluster(const ClusterPlan& plan, const ClusterCall& call, const ClusterMaps& maps, cudaStream_t stream, bool pdl) {
-  const hg_problem &l = *call.low, &h = *call.high, &any = l.rows ? l : h;
+// What follows from the plan and the shape alone.
+static ClusterParams shape_params(const ClusterPlan& plan, int rows_low, int rows_high, int tokens, int k) {
   ClusterParams p{};
-  const hg_problem* parts[2] = {&l, &h};
-  for (int i = 0; i < 2; ++i) {
-    p.rows[i] = parts[i]->rows; p.cut_log[i] = plan.cut_log[i]; p.tiles[i] = plan.tiles[i];
-    p.sfa[i] = static_cast<const uint8_t*>(parts[i]->weight_scales);
-    p.ids[i] = static_cast<const int32_t*>(parts[i]->ids);
-  }
+  const int rows[2] = {rows_low, rows_high};
+  for (int i = 0; i < 2; ++i) { p.rows[i] = rows[i]; p.cut_log[i] = plan.cut_log[i]; p.tiles[i] = plan.tiles[i]; }
   p.slot_rows = plan.slot_rows; p.least_rows = plan.least_rows;
-  p.sfb = static_cast<const uint8_t*>(any.activation_scales);
-  p.out = call.out;
-  p.outputs = any.outputs; p.tokens = any.tokens; p.k = any.k; p.kblocks = any.k / kTileK;
+  p.tokens = tokens; p.k = k; p.kblocks = k / kTileK;
   p.n_tile = plan.n_tile; p.n_tail = plan.n_tail; p.token_tiles = plan.token_tiles; p.stages = plan.stages;
   p.async_push = plan.n_tile <= 32;
   p.ring_exchange = plan.ring_exchange; p.split = plan.split; p.clusters = plan.clusters;
@@ -882,9 +892,46 @@ void launch_cluster(const ClusterPlan& plan, const ClusterCall& call, const Clus
   p.by_tiles = inverse((tiles + 1) * uint64_t(plan.tiles[1]), tiles);
   p.acc_shift = plan.acc_shift; p.overlap = plan.overlap;
   p.tmem_cols = uint32_t(plan.tmem_cols);
+  return p;
+}
+
+std::vector<ClusterPart> cluster_parts(const ClusterPlan& plan, int rows_low, int rows_high, int tokens, int k) {
+  const ClusterParams p = shape_params(plan, rows_low, rows_high, tokens, k);
+  const int units = (p.tiles[0] + p.tiles[1]) * p.token_tiles, cluster_ctas = plan.pair * plan.split;
+  std::vector<ClusterPart> parts;
+  parts.reserve(size_t(units) * cluster_ctas);
+  for (int cluster = 0; cluster < plan.clusters; ++cluster)
+    for (int rank = 0; rank < cluster_ctas; ++rank)
+      for (int u = cluster; u < units; u += plan.clusters) {
+        const Unit w = unit_at(p, u);
+        const int half = rank % plan.pair, slice = rank / plan.pair, atom = w.atom * plan.pair + half, log = p.cut_log[w.part];
+        ClusterPart part;
+        part.cta = cluster * cluster_ctas + rank;
+        part.tile = (w.part ? plan.pair * p.tiles[0] : 0) + (atom << log) + (w.first >> (7 - log));
+        part.token_tile = w.token0 / p.n_tile;
+        part.kb_begin = 2 * first_step(p, slice);
+        part.kb_end = std::min(2 * first_step(p, slice + 1), p.kblocks);
+        part.slice = slice;
+        part.first_row = atom * kTileRows + w.first;
+        part.rows = std::max(0, std::min(kTileRows >> log, p.rows[w.part] - part.first_row));
+        parts.push_back(part);
+      }
+  return parts;
+}
+
+void launch_cluster(const ClusterPlan& plan, const ClusterCall& call, const ClusterMaps& maps, cudaStream_t stream, bool pdl) {
+  const hg_problem &l = *call.low, &h = *call.high, &any = l.rows ? l : h;
+  ClusterParams p = shape_params(plan, l.rows, h.rows, any.tokens, any.k);
+  const hg_problem* parts[2] = {&l, &h};
+  for (int i = 0; i < 2; ++i) {
+    p.sfa[i] = static_cast<const uint8_t*>(parts[i]->weight_scales);
+    p.ids[i] = static_cast<const int32_t*>(parts[i]->ids);
+  }
+  p.sfb = static_cast<const uint8_t*>(any.activation_scales);
+  p.out = call.out;
+  p.outputs = any.outputs;
   p.x = static_cast<const uint16_t*>(call.x);
   p.x_bf16 = call.x_dtype == HG_DTYPE_BF16;
-  p.audit_tokens = call.audit_tokens;
   p.status = call.status;
 #ifdef HG_TRACE
   p.trace = call.trace;

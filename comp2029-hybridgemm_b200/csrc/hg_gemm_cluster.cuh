@@ -28,6 +28,15 @@ struct ClusterPlan {
 // Plan for one shape; `max_clusters[i]` is the number of clusters of 2^i CTAs the device holds at once.
 ClusterPlan make_cluster_plan(int rows_low, int rows_high, int tokens, int k, const int max_clusters[4]);
 
+// The same for a device with `sms` SMs; asks the current device if it has as many.
+ClusterPlan make_cluster_plan_for(int rows_low, int rows_high, int tokens, int k, int sms);
+
+// What one CTA does for one unit, CTA by CTA and in the order of its units.  The kernel's counters add kb_end - kb_begin and
+// one per part.  Tiles are numbered through the partitions; `rows` is what is left of the tile's height at the end of one
+// (0 in the second CTA of a pair whose atom is not there).
+struct ClusterPart { int cta, tile, token_tile, kb_begin, kb_end, slice, first_row, rows; };
+std::vector<ClusterPart> cluster_parts(const ClusterPlan& plan, int rows_low, int rows_high, int tokens, int k);
+
 // What the device holds of clusters of 1, 2, 4 and 8 CTAs (one CTA per SM); queried once per device.
 const int* cluster_capacity();
 
@@ -38,7 +47,6 @@ struct ClusterCall {
   int x_dtype;
   OutTargets out;
   int dtype;              // output type
-  int audit_tokens;       // tokens per tile of the schedule whose units the audit counters count
   int* status;
   unsigned long long* trace;
 };

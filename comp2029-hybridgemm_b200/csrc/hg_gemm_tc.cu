@@ -1221,7 +1221,7 @@ void tc_run(TcGemm* g, const hg_problem& l, const hg_problem& h, cudaStream_t st
       hit->codes = any.activation;
       hit->scales = any.activation_scales;
     }
-    ClusterCall call{&l, &h, x, x_dtype, out, g->dtype, plan.n_tile, g->d_status, nullptr};
+    ClusterCall call{&l, &h, x, x_dtype, out, g->dtype, g->d_status, nullptr};
 #ifdef HG_TRACE
     call.trace = g->d_trace;
 #endif
@@ -1426,7 +1426,7 @@ void tc_run_static(int schedule, const hg_problem& l, const hg_problem& h, int d
   if (entry->clustered) {
     // The cluster kernel keeps its partial sums on chip: of the array it needs the status words only.
     const ClusterPlan& cluster = entry->cluster;
-    ClusterCall call{&l, &h, nullptr, HG_DTYPE_BF16, OutTargets{}, dtype, plan.n_tile, reinterpret_cast<int*>(base + kStaticStatusOffset), nullptr};
+    ClusterCall call{&l, &h, nullptr, HG_DTYPE_BF16, OutTargets{}, dtype, reinterpret_cast<int*>(base + kStaticStatusOffset), nullptr};
     call.out.ptr = any.output;
     ClusterMaps maps{};
     if (l.rows) set_weight_maps(maps, cluster, l, 0);

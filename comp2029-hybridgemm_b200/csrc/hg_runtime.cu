@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <memory>
 
+#include "hg_gemm_cluster.cuh"
 #include "hg_gemm_tc.cuh"
 
 namespace hg {
@@ -188,6 +189,20 @@ int hg_plan(int rows_low, int rows_high, int tokens, int k, int sms, int schedul
   HG_TRY
   if (!header || rows_low < 0 || rows_high < 0 || rows_low + rows_high == 0 || tokens <= 0 || k <= 0 || k % 128 || sms <= 0)
     throw std::runtime_error("Invalid hg_plan arguments");
+  if (schedule == HG_SCHEDULE_AUTO) {
+    const hg::ClusterPlan plan = hg::make_cluster_plan_for(rows_low, rows_high, tokens, k, sms);
+    const std::vector<hg::ClusterPart> parts = hg::cluster_parts(plan, rows_low, rows_high, tokens, k);
+    const int values[12] = {schedule, plan.clusters * plan.pair * plan.split, plan.n_tile, plan.token_tiles, plan.stages,
+                            plan.smem_bytes, plan.tmem_cols, 0, 0, int(parts.size()), 0, 1};
+    std::copy(values, values + 12, header);
+    if (units && int(parts.size()) > max_units) throw std::runtime_error("hg_plan: unit buffer too small");
+    for (size_t i = 0; units && i < parts.size(); ++i) {
+      const hg::ClusterPart& w = parts[i];
+      const int row[9] = {w.cta, w.tile, w.token_tile, w.kb_begin, w.kb_end, w.slice, plan.split, w.first_row, w.rows};
+      std::copy(row, row + 9, units + 9 * i);
+    }
+    return 0;
+  }
   const hg::Plan plan = hg::make_plan(rows_low, rows_high, tokens, k, sms, schedule);
   const int values[12] = {plan.schedule, plan.grid, plan.n_tile, plan.token_tiles, plan.stages, plan.smem_bytes,
                           plan.tmem_cols, plan.ws_slots, plan.counters, int(plan.units.size()),

@@ -130,8 +130,8 @@ int hg_info(void* handle, int* out20);
 void hg_destroy(void* handle);
 /* Device-side status of the last launches of this handle: 0 = ok, otherwise the
  * code a bounded in-kernel wait recorded before giving up.  status[3] = {error,
- * K128 blocks issued, work units stored} since the last call; clears them and
- * synchronises `stream`.
+ * K128 blocks issued, work units stored} since the last call, counted as they are issued and stored: a launch
+ * adds the sum of kb_end - kb_begin over the units of hg_plan, and their number.  Clears them and synchronises `stream`.
  * (The reference has no counterpart; its kernels cannot report a stuck wait.) */
 int hg_status(void* handle, void* stream, int* status);
 /* Host-only view of the tile schedule hg_create would build for a shape on a
@@ -139,7 +139,9 @@ int hg_status(void* handle, void* stream, int* status);
  * schedules live inside CUTLASS).  header[12] = schedule, grid, n_tile,
  * token_tiles, stages, shared bytes, TMEM columns, workspace slots, counters,
  * units, separate reduce launch (0/1), MMA-issuing threads; units (optional) receives 9 ints per unit: cta, tile, token_tile,
- * kb_begin, kb_end, split, nsplit, ws_slot, counter. */
+ * kb_begin, kb_end, split, nsplit, ws_slot, counter.  Under HG_SCHEDULE_AUTO the units are what each CTA of a cluster does (the
+ * CTAs of a pair have a tile each, slices of K a unit each), no workspace is used, and the last two are the tile's first row
+ * in its partition and its rows.  Where the current device has `sms` SMs it is asked how many clusters it holds. */
 int hg_plan(int rows_low, int rows_high, int tokens, int k, int sms, int schedule, int* header, int* units,
             int max_units);
 /* Diagnostic, only in a library built with -DHG_TRACE (build.py --trace; ordinary builds return -1 with an

@@ -69,6 +69,22 @@ def run_gemm(case: dict, dtype=torch.bfloat16, schedule=0, policy=0, fill=0xFF, 
     return host[guard:-guard].reshape(tokens, outputs).copy(), guards_ok, tuple(status)
 
 
+def expected_work(case, schedule):
+    """Totals that the units of the schedule add up to: the kernel's counters, which count as it issues and stores, must too."""
+    lib = native.library()
+    header = (C.c_int * 12)()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    shape = (case["lo"].size, case["hi"].size, case["tokens"], case["k"], sms, schedule)
+    native.check(lib.hg_plan(*shape, header, None, 0))
+    units = (C.c_int * (9 * header[9]))()
+    native.check(lib.hg_plan(*shape, header, units, header[9]))
+    units = np.array(units[:]).reshape(-1, 9)
+    if schedule:
+        tiles = -(-case["lo"].size // 128) + -(-case["hi"].size // 128)
+        assert (units[:, 4] - units[:, 3]).sum() == tiles * header[3] * (case["k"] // 128)
+    return int((units[:, 4] - units[:, 3]).sum()), header[9]
+
+
 def quantised_case(tokens, k, outputs, high, dtype=torch.bfloat16, seed=SEED):
     """Operands quantised by the CPU oracle plus the oracle's fp32 and 16-bit outputs."""
     x, w, ids = make_inputs(tokens, k, outputs, high, dtype, seed)

@@ -11,7 +11,7 @@ import pytest
 import torch
 
 import oracle
-from helpers import run_gemm
+from helpers import expected_work, run_gemm
 from hygemm_vllm import native, producer
 
 pytestmark = pytest.mark.gpu
@@ -23,6 +23,7 @@ def test_exact_at_the_edges_of_the_plan(tokens):
         case = oracle.exact_case(outputs, tokens, k, high, "random")
         got, guards, status = run_gemm(case, torch.bfloat16, 0)
         assert status[0] == 0 and guards, (outputs, k, high, status)
+        assert (status[1], status[2]) == expected_work(case, 0), (outputs, k, high, status)
         assert np.array_equal(got, case["expected"]), (outputs, k, high, int((got != case["expected"]).sum()))
 
 

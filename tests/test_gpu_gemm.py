@@ -7,7 +7,7 @@ import pytest
 import torch
 
 import oracle
-from helpers import bits, dev, make_inputs, quantised_case, rel_frobenius, run_gemm, to_float
+from helpers import bits, dev, expected_work, make_inputs, quantised_case, rel_frobenius, run_gemm, to_float
 from hygemm_vllm import native
 
 pytestmark = pytest.mark.gpu
@@ -19,17 +19,6 @@ EXACT = [(257, 7, 256, 0, "random"), (257, 7, 256, 1, "random"), (257, 7, 256, 2
          (511, 33, 384, 73, "interleaved"), (129, 1, 128, 17, "random"), (255, 17, 128, 51, "contiguous"),
          (4096, 128, 1024, 2048, "random"), (2049, 130, 384, 300, "interleaved")]
 SCHEDULES = {"auto": 0, "data_parallel": 1, "split_k": 2, "stream_k": 3}
-
-
-def expected_work(case, schedule):
-    """Closed-form totals the kernel's audit counters must reproduce."""
-    lib = native.library()
-    header = (C.c_int * 12)()
-    props = torch.cuda.get_device_properties(0)
-    native.check(lib.hg_plan(case["lo"].size, case["hi"].size, case["tokens"], case["k"],
-                             props.multi_processor_count, schedule, header, None, 0))
-    tiles = -(-case["lo"].size // 128) + -(-case["hi"].size // 128)
-    return tiles * header[3] * (case["k"] // 128), header[9]
 
 
 @pytest.mark.parametrize("schedule", list(SCHEDULES))

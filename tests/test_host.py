@@ -90,7 +90,40 @@ def test_data_parallel_ctas_run_their_mxfp8_tiles_first():
             assert flags == sorted(flags, reverse=True)     # every MXFP8 unit precedes every MXFP4 unit
 
 
-@pytest.mark.parametrize("schedule", [0, 1, 2, 3])
+@pytest.mark.parametrize("tokens", [1, 8, 16, 17, 32, 33, 37, 64, 65, 96, 128, 129, 130, 200, 257, 300, 777, 2048, 2049])
+def test_the_cluster_plan_covers_each_row_token_and_k_block_exactly_once(tokens):
+    """What AUTO launches: the units of `hg_plan` are computed by the function with which a CTA finds its work."""
+    for lo, hi, k in SHAPES + [(7003 - 701, 701, 2432), (1, 0, 128), (0, 33, 384)]:
+        for sms in (148, 7):
+            header, units = plan(lo, hi, tokens, k, 0, sms)
+            sched, grid, n_tile, token_tiles, stages, smem, tmem, slots, counters, n_units, reduce2, issuers = header
+            assert (sched, slots, counters, reduce2, issuers) == (0, 0, 0, 0, 1)
+            assert 1 <= grid <= sms and n_tile % 16 == 0 and 16 <= n_tile <= 256 and token_tiles == -(-tokens // n_tile)
+            assert 2 <= stages <= 12 and smem <= 232448 and tmem in (64, 128, 256, 512)
+            cta, tile, tt, begin, end, slice_, split, first, rows = units.T
+            assert set(cta) == set(range(grid)) and np.all(np.diff(cta) >= 0) and np.all((0 <= tt) & (tt < token_tiles))
+            assert split.min() == split.max() and np.all((0 <= slice_) & (slice_ < split))
+            assert np.all(begin % 2 == 0) and np.all(begin < end)
+            kblocks, parts = k // 128, split[0]
+            # every slice does the same tiles, and the slices of a tile are its K blocks in order
+            for s in range(parts):
+                of_slice = units[slice_ == s]
+                assert len({(int(b), int(e)) for b, e in of_slice[:, 3:5]}) == 1
+                assert of_slice[0, 3] == (0 if s == 0 else units[slice_ == s - 1][0, 4])
+            assert units[slice_ == parts - 1][0, 4] == kblocks
+            # rows of both partitions, once per token tile and slice
+            keys = units[:, [1, 2, 5]]
+            assert len(np.unique(keys, axis=0)) == len(units)
+            here = units[(slice_ == 0) & (rows > 0)]
+            spans = np.unique(here[:, [1, 7, 8]], axis=0)                     # tile, first row, rows
+            starts = np.flatnonzero(spans[:, 1] == 0)
+            assert len(starts) == (lo > 0) + (hi > 0)
+            for group, total in zip(np.split(spans, starts[1:]), [n for n in (lo, hi) if n]):
+                assert np.all(group[1:, 1] == group[:-1, 1] + group[:-1, 2]) and group[-1, 1] + group[-1, 2] == total
+            assert len(here) == len(spans) * token_tiles
+
+
+@pytest.mark.parametrize("schedule", [1, 2, 3])
 @pytest.mark.parametrize("tokens", [1, 16, 17, 128, 130, 300])
 def test_every_schedule_covers_each_tile_and_k_block_exactly_once(schedule, tokens):
     for lo, hi, k in SHAPES:
