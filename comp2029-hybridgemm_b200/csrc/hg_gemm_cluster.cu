@@ -803,6 +803,19 @@ void configure_cluster_kernels() {
   set_limits<__half, 1, false>(); set_limits<__half, 1, true>(); set_limits<__half, 2, false>();
 }
 
+void cluster_kernel_attributes(const ClusterPlan& plan, int dtype, int* registers, int* local_bytes, int* stage_bytes) {
+  cudaFuncAttributes attr{};
+  const bool bf16 = dtype == HG_DTYPE_BF16;
+  check(plan.pair == 2 ? (bf16 ? cudaFuncGetAttributes(&attr, cluster_gemm_kernel<__nv_bfloat16, 2, false>)
+                               : cudaFuncGetAttributes(&attr, cluster_gemm_kernel<__half, 2, false>))
+                       : (bf16 ? cudaFuncGetAttributes(&attr, cluster_gemm_kernel<__nv_bfloat16, 1, false>)
+                               : cudaFuncGetAttributes(&attr, cluster_gemm_kernel<__half, 1, false>)), "cudaFuncGetAttributes");
+  *registers = attr.numRegs;
+  *local_bytes = int(attr.localSizeBytes);
+  const ClusterSmem lay = cluster_smem(plan.stages, plan.n_tile, plan.pair, plan.split, plan.slot_rows, plan.least_rows, plan.ring_exchange);
+  *stage_bytes = int(2 * lay.b_tile + 1024 + lay.sfb_stage);
+}
+
 const int* cluster_capacity() {
   static int capacity[64][4];
   static std::once_flag once[64];

@@ -56,5 +56,8 @@ struct ClusterCall {
 struct ClusterMaps { CUtensorMap low, high, act, tail, low_scales, high_scales, act_scales; };
 void launch_cluster(const ClusterPlan& plan, const ClusterCall& call, const ClusterMaps& maps, cudaStream_t stream, bool pdl);
 void configure_cluster_kernels();
+// Registers and local memory of the instance a plan launches on prepacked activations; bytes of activations and of all
+// scales that a CTA brings in per K256 stage.
+void cluster_kernel_attributes(const ClusterPlan& plan, int dtype, int* registers, int* local_bytes, int* stage_bytes);
 
 }  // namespace hg

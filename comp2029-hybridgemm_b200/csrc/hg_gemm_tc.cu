@@ -1284,8 +1284,6 @@ void tc_destroy(TcGemm* g) {
   delete g;
 }
 
-const Plan& tc_plan(const TcGemm* g) { return g->plan; }
-
 int tc_trace(TcGemm* g, cudaStream_t stream, unsigned long long* out, int max_values) {
 #ifdef HG_TRACE
   const int values = std::min(max_values, 16 * g->plan.grid);
@@ -1298,11 +1296,18 @@ int tc_trace(TcGemm* g, cudaStream_t stream, unsigned long long* out, int max_va
 #endif
 }
 
-void tc_kernel_attributes(int* registers, int* local_bytes) {
+TcInfo tc_info(const TcGemm* g) {
+  TcInfo info{};
+  if (g->clustered) {
+    info = {HG_SCHEDULE_AUTO, g->cluster.n_tile, g->cluster.stages, g->cluster.smem_bytes, 0, 0, 0};
+    cluster_kernel_attributes(g->cluster, g->dtype, &info.registers, &info.local_bytes, &info.stage_bytes);
+    return info;
+  }
   cudaFuncAttributes attr{};
-  check(cudaFuncGetAttributes(&attr, hybrid_gemm_tc_kernel<__nv_bfloat16, false>), "cudaFuncGetAttributes");
-  *registers = attr.numRegs;
-  *local_bytes = int(attr.localSizeBytes);
+  check(g->dtype == HG_DTYPE_BF16 ? cudaFuncGetAttributes(&attr, hybrid_gemm_tc_kernel<__nv_bfloat16, false>)
+                                  : cudaFuncGetAttributes(&attr, hybrid_gemm_tc_kernel<__half, false>), "cudaFuncGetAttributes");
+  return {g->plan.schedule, g->plan.n_tile, g->plan.stages, g->plan.smem_bytes, attr.numRegs, int(attr.localSizeBytes),
+          2 * (g->plan.n_tile * 128 + 1024)};
 }
 
 void tc_status(TcGemm* g, cudaStream_t stream, int out[3]) {

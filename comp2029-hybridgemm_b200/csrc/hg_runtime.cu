@@ -154,13 +154,11 @@ int hg_info(void* handle, int* out) {
   if (!handle || !out) throw std::runtime_error("Null argument to hg_info");
   auto* r = static_cast<hg::Runner*>(handle);
   std::fill(out, out + 20, -1);
-  int regs = 0, local = 0;
-  hg::tc_kernel_attributes(&regs, &local);
-  const hg::Plan& plan = hg::tc_plan(r->tc);
+  const hg::TcInfo info = hg::tc_info(r->tc);
   for (int part = 0; part < 2; ++part) {
     if (!(part ? r->high.rows : r->low.rows)) continue;
-    const int values[10] = {plan.schedule, hg::kTileRows, plan.n_tile, 2 * hg::kTileK, plan.stages,
-                            regs, plan.smem_bytes, local, part, 0};
+    const int values[10] = {info.schedule, hg::kTileRows, info.n_tile, 2 * hg::kTileK, info.stages,
+                            info.registers, info.smem_bytes, info.local_bytes, part, 0};
     std::copy(values, values + 10, out + part * 10);
   }
   HG_CATCH
@@ -264,14 +262,11 @@ int hg_fused_info(void* handle, int* data) {
   HG_FUSED_TRY
   auto* f = static_cast<hg::FusedRunner*>(handle);
   if (!f || !data) throw std::runtime_error("Null argument to hg_fused_info");
-  int regs = 0, local = 0;
-  hg::tc_kernel_attributes(&regs, &local);
-  const hg::Plan& plan = hg::tc_plan(f->runner->tc);
-  // Bytes per K256 stage: MXFP4 weights arrive by cp.async (16 KiB packed), MXFP8 by TMA (32 KiB).
-  const int common = 2 * (plan.n_tile * 128 + 1024);
+  const hg::TcInfo info = hg::tc_info(f->runner->tc);
+  // Bytes per K256 stage and 128 weight rows: packed MXFP4 16 KiB, MXFP8 32 KiB, the rest is common.
   const int tiles = (f->low.rows + 127) / 128 + (f->high.rows + 127) / 128;
-  const int values[11] = {plan.schedule, hg::kTileRows, plan.n_tile, 2 * hg::kTileK, plan.stages, regs,
-                          plan.smem_bytes, local, 16384 + common, 32768 + common, tiles * 128};
+  const int values[11] = {info.schedule, hg::kTileRows, info.n_tile, 2 * hg::kTileK, info.stages, info.registers,
+                          info.smem_bytes, info.local_bytes, 16384 + info.stage_bytes, 32768 + info.stage_bytes, tiles * 128};
   std::copy(values, values + 11, data);
   HG_FUSED_CATCH
 }

@@ -124,7 +124,9 @@ int hg_linear(void* handle, const hg_problem* low, const hg_problem* high, const
 int hg_linear_silu(void* handle, const hg_problem* low, const hg_problem* high, const void* x, int x_dtype, int math,
                    void* workspace, void* output, void* stream);
 /* integrations/vllm/native/runtime.cu:151-161 — 10 ints per partition: id, tile_m,
- * tile_n, tile_k, stages, registers, shared bytes, local bytes, fp8, pingpong (-1 if absent). */
+ * tile_n, tile_k, stages, registers, shared bytes, local bytes, fp8, pingpong (-1 if absent).  They describe the kernel the
+ * handle launches on prepacked activations; id 0 (HG_SCHEDULE_AUTO) is the cluster kernel, whose tile_m is the height of a
+ * CTA's MMA (its tiles may cover half or a quarter of it). */
 int hg_info(void* handle, int* out20);
 /* integrations/vllm/native/runtime.cu:162 */
 void hg_destroy(void* handle);

@@ -7,7 +7,7 @@ import pytest
 import torch
 
 import oracle
-from helpers import bits, dev, expected_work, make_inputs, quantised_case, rel_frobenius, run_gemm, to_float
+from helpers import SEED, bits, dev, expected_work, make_inputs, quantised_case, rel_frobenius, run_gemm, to_float
 from hygemm_vllm import native
 
 pytestmark = pytest.mark.gpu
@@ -130,6 +130,23 @@ def test_rebind_to_other_shape_is_rejected():
     lib.hg_destroy(handle)
     bad = native.Problem(0, 7, 256, 257, None, None, None, None, None, None)
     assert lib.hg_create_dtype(0, 0, C.byref(bad), C.byref(bad), None, 1, C.byref(handle)) == -1
+
+
+@pytest.mark.parametrize("schedule", [0, 1, 2, 3])
+@pytest.mark.parametrize("outputs,tokens,k,high", [(3584, 128, 2432, 384), (640, 290, 896, 128), (257, 7, 256, 26)])
+def test_info_describes_the_plan_that_runs(outputs, tokens, k, high, schedule):
+    """`hg_info` of a handle against `hg_plan` of its shape: token tile, stages and shared memory (a handle of an explicit
+    schedule and one of AUTO run different kernels)."""
+    lib = native.library()
+    w = torch.randn(outputs, k, generator=torch.Generator().manual_seed(SEED)).bfloat16().cuda()
+    layer = native.DualLinear(w, torch.arange(high).cuda(), low_id=schedule, high_id=schedule)
+    layer(torch.ones(tokens, k, dtype=torch.bfloat16, device="cuda"))
+    info, header = layer.info(tokens), (C.c_int * 12)()
+    native.check(lib.hg_plan(outputs - high, high, tokens, k, torch.cuda.get_device_properties(0).multi_processor_count, schedule, header, None, 0))
+    for part in (info[:10], info[10:]):
+        assert (part[0], part[2], part[4], part[6]) == (header[0], header[2], header[4], header[5])
+        assert part[1] == 128 and part[3] == 256 and 32 <= part[5] <= 255 and part[7] >= 0
+    layer.close()
 
 
 SHAPES_7B = {"qkv": (3584, 4608, 512), "o_proj": (3584, 3584, 384), "gate_up": (3584, 37888, 3840),
