@@ -899,9 +899,6 @@ Plan make_plan(int rows_low, int rows_high, int tokens, int k, int sms, int sche
     plan.counters = counters;
   };
 
-  // AUTO runs the cluster kernel (hg_gemm_cluster.cu), which never cuts a tile over units: its unit list is the
-  // data-parallel one.
-  if (schedule == HG_SCHEDULE_AUTO) schedule = HG_SCHEDULE_DATA_PARALLEL;
   plan.ws_slots = 0;
   plan.counters = 0;
   if (schedule == HG_SCHEDULE_DATA_PARALLEL) {
@@ -1024,7 +1021,7 @@ static CtaHeads make_heads(const Plan& plan) {
 }
 
 struct TcGemm {
-  Plan plan;
+  Plan plan;                   // of an explicit schedule
   bool clustered = false;      // HG_SCHEDULE_AUTO: hg_gemm_cluster.cu
   ClusterPlan cluster;
   CtaHeads heads{};
@@ -1037,6 +1034,7 @@ struct TcGemm {
   int* d_cut = nullptr;
 #ifdef HG_TRACE
   unsigned long long* d_trace = nullptr;
+  int trace_ctas = 0;
 #endif
   // Tensor maps of recent operand pointers (the shape is fixed per handle): a serving loop alternates among
   // a few activation buffers and one weight pointer, so the driver call is paid once per pointer.
@@ -1088,22 +1086,22 @@ TcGemm* tc_create(const hg_problem& l, const hg_problem& h, int schedule, int dt
   auto g = std::make_unique<TcGemm>();
   g->rows[0] = l.rows; g->rows[1] = h.rows;
   g->tokens = any.tokens; g->k = any.k; g->outputs = any.outputs; g->dtype = dtype;
-  g->plan = make_plan(l.rows, h.rows, any.tokens, any.k, sms, schedule);
-  const Plan& plan = g->plan;
   if (schedule == HG_SCHEDULE_AUTO) {
     g->clustered = true;
     g->cluster = make_cluster_plan(l.rows, h.rows, any.tokens, any.k, cluster_capacity());
     check(cudaMalloc(&g->d_status, sizeof(int) * 4), "cudaMalloc status");
     check(cudaMemsetAsync(g->d_status, 0, sizeof(int) * 4, stream), "clear status");
 #ifdef HG_TRACE
-    g->plan.grid = g->cluster.clusters * g->cluster.pair * g->cluster.split;
-    check(cudaMalloc(&g->d_trace, sizeof(unsigned long long) * 16 * size_t(g->plan.grid)), "trace buffer");
-    check(cudaMemsetAsync(g->d_trace, 0, sizeof(unsigned long long) * 16 * size_t(g->plan.grid), stream), "trace buffer");
+    g->trace_ctas = g->cluster.clusters * g->cluster.pair * g->cluster.split;
+    check(cudaMalloc(&g->d_trace, sizeof(unsigned long long) * 16 * size_t(g->trace_ctas)), "trace buffer");
+    check(cudaMemsetAsync(g->d_trace, 0, sizeof(unsigned long long) * 16 * size_t(g->trace_ctas), stream), "trace buffer");
 #endif
     check(cudaStreamSynchronize(stream), "clear status");   // the first launch may be on another stream
     return g.release();
   }
-  g->heads = make_heads(g->plan);
+  g->plan = make_plan(l.rows, h.rows, any.tokens, any.k, sms, schedule);
+  const Plan& plan = g->plan;
+  g->heads = make_heads(plan);
   check(cudaMalloc(&g->d_units, sizeof(WorkUnit) * std::max<size_t>(1, plan.units.size())), "cudaMalloc units");
   check(cudaMalloc(&g->d_cta_begin, sizeof(int) * plan.cta_begin.size()), "cudaMalloc schedule");
   check(cudaMalloc(&g->d_workspace, sizeof(float) * std::max<int64_t>(1, int64_t(plan.ws_slots) * plan.n_tile * kTileRows)), "cudaMalloc workspace");
@@ -1111,6 +1109,7 @@ TcGemm* tc_create(const hg_problem& l, const hg_problem& h, int schedule, int dt
   check(cudaMalloc(&g->d_status, sizeof(int) * 4), "cudaMalloc status");
   check(cudaMalloc(&g->d_cut, sizeof(int) * std::max<size_t>(4, plan.cut_tiles.size())), "cudaMalloc cut list");
 #ifdef HG_TRACE
+  g->trace_ctas = plan.grid;
   check(cudaMalloc(&g->d_trace, sizeof(unsigned long long) * 16 * size_t(plan.grid)), "trace buffer");
   check(cudaMemsetAsync(g->d_trace, 0, sizeof(unsigned long long) * 16 * size_t(plan.grid), stream), "trace buffer");
 #endif
@@ -1172,7 +1171,7 @@ void tc_run(TcGemm* g, const hg_problem& l, const hg_problem& h, cudaStream_t st
   const bool fused = x != nullptr;
   validate(l, h, fused);
   if (fused) {
-    if (g->plan.n_tile != 16) throw std::runtime_error("Fused activation quantisation serves at most 16 tokens");
+    if ((g->clustered ? g->cluster.n_tile : g->plan.n_tile) != 16) throw std::runtime_error("Fused activation quantisation serves at most 16 tokens");
     if (x_dtype != HG_DTYPE_F16 && x_dtype != HG_DTYPE_BF16) throw std::runtime_error("Unknown activation dtype");
     if (reinterpret_cast<uintptr_t>(x) & 15) throw std::runtime_error("Activations must be 16-byte aligned");
   }
@@ -1286,7 +1285,7 @@ void tc_destroy(TcGemm* g) {
 
 int tc_trace(TcGemm* g, cudaStream_t stream, unsigned long long* out, int max_values) {
 #ifdef HG_TRACE
-  const int values = std::min(max_values, 16 * g->plan.grid);
+  const int values = std::min(max_values, 16 * g->trace_ctas);
   check(cudaMemcpyAsync(out, g->d_trace, sizeof(unsigned long long) * size_t(values), cudaMemcpyDeviceToHost, stream), "trace read");
   check(cudaStreamSynchronize(stream), "trace read");
   return values;
@@ -1420,10 +1419,13 @@ void tc_run_static(int schedule, const hg_problem& l, const hg_problem& h, int d
     entry = oldest;
     for (auto& resident : st.resident)
       if (resident == entry) resident = nullptr;   // the array of that device holds a schedule that is going away
-    entry->plan = make_plan(l.rows, h.rows, any.tokens, any.k, st.sms[device], schedule);
     entry->clustered = schedule == HG_SCHEDULE_AUTO;
-    if (entry->clustered) entry->cluster = make_cluster_plan(l.rows, h.rows, any.tokens, any.k, cluster_capacity());
-    else entry->heads = make_heads(entry->plan);
+    if (entry->clustered) {
+      entry->cluster = make_cluster_plan(l.rows, h.rows, any.tokens, any.k, cluster_capacity());
+    } else {
+      entry->plan = make_plan(l.rows, h.rows, any.tokens, any.k, st.sms[device], schedule);
+      entry->heads = make_heads(entry->plan);
+    }
     std::memcpy(entry->key, key, sizeof(key));
   }
   entry->used = ++st.clock;

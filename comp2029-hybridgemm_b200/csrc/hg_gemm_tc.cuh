@@ -42,7 +42,7 @@ struct Plan {
 };
 
 // Builds the tile schedule for one shape.  `sms` is the SM count of the device,
-// `schedule` one of HG_SCHEDULE_{AUTO,DATA_PARALLEL,SPLIT_K,STREAM_K}.
+// `schedule` one of HG_SCHEDULE_{DATA_PARALLEL,SPLIT_K,STREAM_K} (AUTO is hg_gemm_cluster.cu's).
 Plan make_plan(int rows_low, int rows_high, int tokens, int k, int sms, int schedule);
 
 struct TcGemm;  // opaque device-side state (plan buffers, workspace, counters, status)
