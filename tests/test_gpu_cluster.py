@@ -27,6 +27,22 @@ def test_exact_at_the_edges_of_the_plan(tokens):
         assert np.array_equal(got, case["expected"]), (outputs, k, high, int((got != case["expected"]).sum()))
 
 
+@pytest.mark.parametrize("tokens,k,forced", [(2048, 384, False), (1990, 896, False), (1825, 128, False), (777, 384, True), (290, 256, True)])
+def test_exact_with_several_wide_tiles_per_cluster(tokens, k, forced, monkeypatch):
+    """256-token tiles: their two accumulators share 32 TMEM columns, which are handed from one to the other early.  That happens from a
+    cluster's second unit on, so every cluster has at least two here, with tails of every kind of width."""
+    if forced:
+        monkeypatch.setenv("HYGEMM_CL_N", "256")
+    outputs, high = (8269, 800) if tokens > 512 else (18944, 1900)
+    case = oracle.exact_case(outputs, tokens, k, high, "random")
+    header = (C.c_int * 12)()
+    native.check(native.library().hg_plan(outputs - high, high, tokens, k, torch.cuda.get_device_properties(0).multi_processor_count, 0, header, None, 0))
+    assert header[2] == 256 and header[9] >= 1.9 * header[1], list(header)   # units per CTA
+    got, guards, status = run_gemm(case, torch.bfloat16, 0)
+    assert status[0] == 0 and guards and (status[1], status[2]) == expected_work(case, 0)
+    assert np.array_equal(got, case["expected"]), int((got != case["expected"]).sum())
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_swiglu_layer_call_equals_producer_then_gemm(dtype):
     """One foreign call for SwiGLU and down_proj: the same bytes as the producer followed by the GEMM on its codes."""

@@ -140,6 +140,59 @@ def test_silu_pack_vs_vllm_op():
             assert torch.equal(q, q_ref) and torch.equal(sf, sf_ref)
 
 
+def _specials(x, seed):
+    """The same matrix with infinities, NaNs, whole groups of them, zeros and the smallest values, about one group in fifty."""
+    g = torch.Generator().manual_seed(seed)
+    x = x.clone()
+    groups = x.view(-1, 32)
+    picked = torch.randperm(groups.shape[0], generator=g)[: max(8, groups.shape[0] // 50)].split(max(1, groups.shape[0] // 400))
+    for rows, value in zip(picked, (float("inf"), float("-inf"), float("nan"), 0.0, -0.0, torch.finfo(x.dtype).tiny, torch.finfo(x.dtype).smallest_normal / 4,
+                                    torch.finfo(x.dtype).max)):
+        half = rows[: rows.numel() // 2]
+        groups[half] = value
+        groups[rows, torch.randint(0, 32, (rows.numel(),), generator=g)] = value
+    return x
+
+
+# 4 M elements and more (SwiGLU: 8 M products) take the kernels with four rows a warp; K that is no multiple of their 512 columns, and
+# rows that end inside a 128-row scale block, in each of its quarters.
+MANY_ROWS = [(777, 18944), (4128 - 31, 2176), (65600, 128), (33000, 256), (4096, 2048)]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,k", MANY_ROWS)
+def test_many_rows_equal_few_rows_and_the_oracle(rows, k, dtype):
+    """`pack` and the SwiGLU producer on a large matrix against the oracle, and against the kernels for few rows on its
+    128-row blocks (infinities and NaNs too, which the oracle does not define)."""
+    assert rows * k >= 8 << 20
+    bf16 = dtype == torch.bfloat16
+    x = _random(rows, k, dtype, 1.0, rows + k)
+    for fp4 in (False, True):
+        q, sf = native.pack(x.cuda(), fp4)
+        want_q, want_sf = oracle.pack(x, fp4=fp4, bf16=bf16)
+        assert np.array_equal(q.cpu().numpy(), want_q) and np.array_equal(sf.cpu().numpy(), want_sf), fp4
+        special = _specials(x, rows).cuda()
+        chunks = [native.pack(c.contiguous(), fp4) for c in special.split(128)]
+        q, sf = native.pack(special, fp4)
+        assert torch.equal(q, torch.cat([c[0] for c in chunks])) and torch.equal(sf, torch.cat([c[1] for c in chunks])), fp4
+        if rows * k < 16 << 20:
+            shifted = torch.empty(rows * k + 8, dtype=dtype, device="cuda")[8:].view(rows, k).copy_(special)   # 16 bytes off: no 32-byte loads
+            other = native.pack(shifted, fp4)
+            assert torch.equal(q, other[0]) and torch.equal(sf, other[1]), fp4
+    gate = _random(rows, k, dtype, 2.0, rows + k + 1)
+    pair = torch.cat([gate, x], 1).cuda()
+    q, sf, product = producer.silu_pack(pair, 0, debug=True)
+    want_q, want_sf = oracle.pack(product.cpu(), bf16=bf16)
+    assert np.array_equal(q.cpu().numpy(), want_q) and np.array_equal(sf.cpu().numpy(), want_sf)
+    fast = producer.silu_pack(pair, 0)
+    assert torch.equal(fast[0], q) and torch.equal(fast[1], sf)
+    for math in (0, 1, 2):
+        pair = torch.cat([_specials(gate, rows + 1), _specials(x, rows + 2)], 1).cuda()
+        chunks = [producer.silu_pack(c.contiguous(), math) for c in pair.split(128)]
+        q, sf = producer.silu_pack(pair, math)
+        assert torch.equal(q, torch.cat([c[0] for c in chunks])) and torch.equal(sf, torch.cat([c[1] for c in chunks])), math
+
+
 def test_split_verdict_belongs_to_the_maps_that_are_packed():
     """Maps made in one order and packed in another, and maps that are never packed: every packing reports on its own maps."""
     lib, stream = native.library(), torch.cuda.current_stream().cuda_stream
