@@ -1,5 +1,5 @@
-// Hybrid MXFP4xMXFP8 + MXFP8xMXFP8 output-channel GEMM for sm_100a: the explicit schedules and hg_run_static, and the
-// handles of every schedule (AUTO launches the kernel of hg_gemm_cluster.cu).
+// Hybrid MXFP4xMXFP8 + MXFP8xMXFP8 output-channel GEMM for sm_100a: the kernel of the explicit schedules, and the
+// handles and hg_run_static of every schedule (AUTO launches the kernel of hg_gemm_cluster.cu).
 //
 // One persistent launch covers BOTH precision partitions of a hybrid linear
 // (the reference runs two CUTLASS SM120 kernels on two streams,

@@ -161,7 +161,8 @@ int hg_trace(void* handle, void* stream, unsigned long long* out, int max_values
  * where a layer runs: an engine whose memory pool owns the whole device, a latency-critical loop that
  * cannot afford the device-wide synchronisation an allocation implies, or code that meets a shape only
  * when it has to run it and so cannot warm a handle.  The tile schedule, split-K partial sums, arrival
- * counters and status words live in one array of HG_STATIC_SCRATCH_BYTES inside the library image.
+ * counters and status words live in one array of HG_STATIC_SCRATCH_BYTES inside the library image
+ * (HG_SCHEDULE_AUTO keeps its partial sums on chip and needs the status words only).
  *   - `schedule` is an HG_SCHEDULE_* id 0..3, `dtype` an HG_DTYPE_*; inputs and outputs as for hg_run.
  *   - The first call on a device looks up the array's device address and raises the kernel's
  *     shared-memory limit.
