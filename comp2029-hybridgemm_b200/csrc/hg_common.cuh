@@ -93,19 +93,15 @@ inline cudaError_t launch_kernel(void (*kernel)(KernelArgs...), dim3 grid, dim3 
 // exhaustively by the CPU tests) without a transcendental.
 template <bool FP4>
 __device__ __forceinline__ int mx_exponent(float amax) {
-  uint32_t b = __float_as_uint(amax);
+  const uint32_t b = __float_as_uint(amax);
   if (b == 0) return 0;
-  int ef = int(b >> 23);
-  if (ef == 0) return -127;
-  uint32_t man = b & 0x7fffffu;
-  int x = ef - 127;
-  int e = FP4 ? (man <= 0x400000u ? x - 2 : x - 1) : (man <= 0x600000u ? x - 8 : x - 7);
-  return max(-127, min(127, e));
+  // The mantissa carries into the exponent when it lies above that of MAX (1.5 x 2^2, 1.75 x 2^8).
+  return max(-127, FP4 ? int((b + 0x3fffffu) >> 23) - 129 : int((b + 0x1fffffu) >> 23) - 135);
 }
 
 // 2^-e as an fp32 factor (e in [-127,127]; 2^-127 is a subnormal constant).
 __device__ __forceinline__ float mx_inverse_scale(int e) {
-  return e == 127 ? __uint_as_float(0x00400000u) : __uint_as_float(uint32_t(127 - e) << 23);
+  return __uint_as_float(max(uint32_t(127 - e) << 23, 0x00400000u));
 }
 
 // Two floats -> two E4M3 bytes (lo in bits 0-7), round-to-nearest-even, saturating.
@@ -144,6 +140,51 @@ template <> __device__ __forceinline__ uint16_t from_float<__half>(float v) {
 }
 template <> __device__ __forceinline__ uint16_t from_float<__nv_bfloat16>(float v) {
   return __bfloat16_as_ushort(__float2bfloat16_rn(v));
+}
+
+// Pairs of 16-bit values in a word.
+template <typename T> struct Packed;
+template <> struct Packed<__half> {
+  static __device__ __forceinline__ uint32_t max_abs(uint32_t a, uint32_t b) {   // a is a maximum already
+    const __half2 m = __hmax2(*reinterpret_cast<const __half2*>(&a), __habs2(*reinterpret_cast<const __half2*>(&b)));
+    return *reinterpret_cast<const uint32_t*>(&m);
+  }
+  static __device__ __forceinline__ float2 widen(uint32_t v) { return __half22float2(*reinterpret_cast<const __half2*>(&v)); }
+  static __device__ __forceinline__ uint32_t swiglu(float2 act, uint32_t up) {   // (up + 0) as in silu8
+    const __half2 p = __hmul2(__floats2half2_rn(act.x, act.y), __hadd2(*reinterpret_cast<const __half2*>(&up), __float2half2_rn(0.f)));
+    return *reinterpret_cast<const uint32_t*>(&p);
+  }
+};
+template <> struct Packed<__nv_bfloat16> {
+  static __device__ __forceinline__ uint32_t max_abs(uint32_t a, uint32_t b) {
+    const __nv_bfloat162 m = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a), __habs2(*reinterpret_cast<const __nv_bfloat162*>(&b)));
+    return *reinterpret_cast<const uint32_t*>(&m);
+  }
+  static __device__ __forceinline__ float2 widen(uint32_t v) { return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
+  static __device__ __forceinline__ uint32_t swiglu(float2 act, uint32_t up) {
+    const __nv_bfloat162 p = __hmul2(__floats2bfloat162_rn(act.x, act.y), __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&up), __float2bfloat162_rn(0.f)));
+    return *reinterpret_cast<const uint32_t*>(&p);
+  }
+};
+
+// Two fp32 operations per instruction.
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mul.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{\n .reg .b64 x, y, z, w;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mov.b64 z, {%6, %7};\n fma.rn.f32x2 w, x, y, z;\n mov.b64 {%0, %1}, w;\n}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
 }
 #endif  // __CUDACC__
 

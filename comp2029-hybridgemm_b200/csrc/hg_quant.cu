@@ -131,43 +131,6 @@ __device__ __forceinline__ void silu8(const uint4& g4, const uint4& u4, float (&
   product = make_uint4(dw[0], dw[1], dw[2], dw[3]);
 }
 
-template <typename T> struct Packed;
-template <> struct Packed<__half> {
-  static __device__ __forceinline__ uint32_t max_abs(uint32_t a, uint32_t b) {   // a is a maximum already
-    const __half2 m = __hmax2(*reinterpret_cast<const __half2*>(&a), __habs2(*reinterpret_cast<const __half2*>(&b)));
-    return *reinterpret_cast<const uint32_t*>(&m);
-  }
-  static __device__ __forceinline__ float2 widen(uint32_t v) { return __half22float2(*reinterpret_cast<const __half2*>(&v)); }
-  static __device__ __forceinline__ uint32_t swiglu(float2 act, uint32_t up) {   // (up + 0) as in silu8
-    const __half2 p = __hmul2(__floats2half2_rn(act.x, act.y), __hadd2(*reinterpret_cast<const __half2*>(&up), __float2half2_rn(0.f)));
-    return *reinterpret_cast<const uint32_t*>(&p);
-  }
-};
-template <> struct Packed<__nv_bfloat16> {
-  static __device__ __forceinline__ uint32_t max_abs(uint32_t a, uint32_t b) {
-    const __nv_bfloat162 m = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a), __habs2(*reinterpret_cast<const __nv_bfloat162*>(&b)));
-    return *reinterpret_cast<const uint32_t*>(&m);
-  }
-  static __device__ __forceinline__ float2 widen(uint32_t v) { return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
-  static __device__ __forceinline__ uint32_t swiglu(float2 act, uint32_t up) {
-    const __nv_bfloat162 p = __hmul2(__floats2bfloat162_rn(act.x, act.y), __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&up), __float2bfloat162_rn(0.f)));
-    return *reinterpret_cast<const uint32_t*>(&p);
-  }
-};
-
-// Two fp32 operations per instruction.
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  float2 r;
-  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mul.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}"
-      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return r;
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  float2 r;
-  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}"
-      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return r;
-}
 __device__ __forceinline__ float exp2_fast(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 __device__ __forceinline__ float reciprocal_fast(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 

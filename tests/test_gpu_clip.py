@@ -75,3 +75,29 @@ def test_no_offsets_is_round_to_nearest_and_feeds_a_layer():
     dense = x.float() @ w.float().t()
     assert (y.float() - dense).norm() / dense.norm() < 0.12
     assert stats["weight_error_after"] <= stats["weight_error_before"]
+
+
+@pytest.mark.parametrize("rows,k", [(1, 128), (7, 640), (9, 256), (1300, 3584)])
+@pytest.mark.parametrize("kind", ["outstanding", "hidden", "signed", "missing"])
+def test_candidates_ruled_out_by_one_term_never_win(rows, k, kind):
+    """The plain entry point against the oracle, bit for bit, where the bound on a clipped candidate is tight, useless or not a bound:
+    columns of outstanding importance, columns whose importance is zero (there the clipped candidate wins), negative and NaN importance."""
+    g = torch.Generator().manual_seed(SEED + rows + k)
+    w = torch.randn(rows, k, generator=g) * 0.03
+    w[torch.rand(rows, k, generator=g) < 0.02] *= 8
+    w = w.to(torch.bfloat16)
+    importance = torch.rand(k, generator=g) + 0.1
+    special = torch.rand(k, generator=g) < 0.05
+    importance[special] = {"outstanding": 400.0, "hidden": 0.0, "signed": -2.0, "missing": float("nan")}[kind]
+    if kind == "hidden":
+        w[:, special] *= 8
+    x, weight = w.cuda(), importance.cuda()
+    for offsets in [(0, -1, -2), (-2, -1, 0), (-3, -2, -2, 1), (-1,), (-4, -8, 2, -2, 0, -1, 3, -3)]:
+        q4 = torch.empty(rows, k // 2, dtype=torch.uint8, device="cuda")
+        scales = torch.empty(rows, k // 32, dtype=torch.uint8, device="cuda")
+        native.check(native.library().hg_clip_pack(x.data_ptr(), weight.data_ptr(), q4.data_ptr(), scales.data_ptr(), rows, k,
+                                                   (native.C.c_int * len(offsets))(*offsets), len(offsets), 1,
+                                                   native._stream(x.device)))
+        want_q4, want_scales = oracle.clip_pack(w, importance.numpy(), offsets, bf16=True)
+        assert (scales.cpu().numpy() == want_scales).all(), offsets
+        assert (q4.cpu().numpy() == want_q4).all(), offsets
