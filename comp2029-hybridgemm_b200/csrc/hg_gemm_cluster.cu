@@ -453,6 +453,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
         const uint32_t b_block = uint32_t(w.n / PAIR) * 8u;   // descriptor units (16 bytes) between the stage's activation tiles
         const uint32_t idesc = (w.part ? 0u : 5u << 7) | (uint32_t(w.n >> 3) << 17) | (1u << 23) | (uint32_t(PAIR * kTileRows >> 4) << 24);
         const bool two_atoms = w.n > 128;
+        const uint32_t sfb_col = 4u + (uint32_t(w.token0 & 127) >> 5);   // a second tile of 64 tokens starts in the middle of its scale atom
         uint32_t accumulate = 0;
         int step = step_begin;
         for (; step < step_end; ++step) {
@@ -477,7 +478,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
 #pragma unroll
               for (uint32_t j = 0; j < 4; ++j)
                 cg_mma<PAIR>(tmem_d, desc_of(a_lo + i * a_block + 2 * j, kDescTile), desc_of(b_lo + i * b_block + 2 * j, kDescTile),
-                             idesc | (j << 29) | (j << 4), i + j > 0 ? 1u : accumulate, sf, sf + 4);
+                             idesc | (j << 29) | (j << 4), i + j > 0 ? 1u : accumulate, sf, sf + sfb_col);
             }
             cg_commit<PAIR>(empty_bar(stage), pair_mask);
           }
@@ -673,10 +674,12 @@ static int tuning(const char* name, int value) {
 // launch takes the busiest cluster's time or its weights' time from HBM, whichever is longer, plus a little per CTA and the
 // exchange of partials.
 //
-// The constants are a fit to the order of 5500 measured launches: 425 shapes drawn from 640 to 37888 channels, K 512 to 18944
-// and 1 to 2048 tokens, each with every plan it can have.  The plan it prefers is 1.4 % slower than the best one of the shape
-// on average up to 128 tokens (5.7 % with the constants of fewer and longer shapes before; 7003 x 2432 at 77 tokens 8.8 -> 7.0
-// us, 1920 x 1280 at 66 tokens 6.5 -> 4.4 us) and 0.6 % above (1.7 % before).
+// The constants are a fit to the order of measured launches, every plan a shape can have, for shapes drawn from 640 to 38000
+// channels and K 512 to 18944.  Prefill: 1700 launches of the GEMM alone; the plan preferred is 0.6 % slower than the best one of
+// the shape on average.  Up to 128 tokens: layer calls (quantiser and GEMM), 2400 shapes, of which every fourth or so was fitted
+// to and the rest checked: 0.9 % slower than the best up to 64 tokens (1.9 % with constants fitted to the GEMM alone: between
+// quantisers a plan of few CTAs gains, as the launch behind it finds free SMs) and 1.1 % from 65 on (1.5 %; 10 % when two tiles of
+// 64 tokens were no choice).
 struct PlanFit {
   double mma_floor;                                  // cycles of a single CTA's narrow MMA with its operand reads
   double turn, l2, l2_wide, to_one;                  // us per turn of the ring; bytes per ns from L2 to all SMs, tiles of 129 tokens and more, to one
@@ -685,13 +688,16 @@ struct PlanFit {
   double hops, exchange, part, part_token;           // exchange: per doubling of the cluster, constant, per part, per part and token
   double cta, pair, cut, finer, hbm;                 // per CTA of the grid, paired CTAs, cut of all tiles, further cut of MXFP8 tiles; bytes per ns
 };
-constexpr PlanFit kDecodeFit{234, 1.34, 13100, 13100, 250, 0.147, 0.579, 0.0147, 0.374, 0.0146, 0.0221, 0.866, -0.379, 0.238, 0.0614, 0.00225,
-                             0.0199, 0.587, -0.0142, 0.268, 7200};
+constexpr PlanFit kDecodeFit{234.0, 1.313, 12213, 11174, 189.6, 0.09482, 0.5133, 0.0314, 1.07, 0.01755, 0.02057, 0.9327, -0.657, 0.1007, 0.0143, 0.005931,
+                             0.008127, 0.5955, -0.0378, 0.268, 16351};
+constexpr PlanFit kWideDecodeFit{236.7, 1.328, 12840, 13981, 250.0, 0.2656, 0.7058, 0.02462, 0.3386, 0.01767, 0.01224, 0.9089, -0.538, 0.1856, 0.06477, 0.003302,
+                                 0.01379, 0.5441, -0.02387, 0.2337, 8705};
 constexpr PlanFit kPrefillFit{234, 1.28, 18800, 12300, 380, 0.397, 1.75, 0.0159, 0.632, 0.0142, 0.0146, 0.648, -0.67, 0.09, 0.0186, 0.00254,
                               0.00225, 2.55, 0.0711, -0.221, 3120};
 
 static double plan_cost(const ClusterPlan& plan, int64_t units, int kblocks, double weight_kilobytes) {
-  const PlanFit& fit = plan.token_tiles == 1 && plan.n_tile <= 128 ? kDecodeFit : kPrefillFit;
+  const int columns = (plan.token_tiles - 1) * plan.n_tile + plan.n_tail;
+  const PlanFit& fit = columns <= 64 ? kDecodeFit : plan.token_tiles * plan.n_tile <= 128 ? kWideDecodeFit : kPrefillFit;
   const double steps = double((kblocks + 1) / 2) / plan.split;
   const int cluster_ctas = plan.pair * plan.split, ctas = plan.clusters * cluster_ctas;
   auto main_loop = [&](int n, bool high) {
@@ -758,7 +764,7 @@ ClusterPlan make_cluster_plan(int lo, int hi, int tokens, int k, const int max_c
     for (int log = pair - 1; log < 4; ++log)
       for (int cut = 0; cut < 3; ++cut)
         for (int more = 0; more < 3; ++more)
-          for (int n : {0, 128, 256}) {
+          for (int n : {0, 64, 128, 256}) {
               ClusterPlan plan;
               plan.pair = pair;
               plan.split = (1 << log) / pair;
@@ -766,11 +772,15 @@ ClusterPlan make_cluster_plan(int lo, int hi, int tokens, int k, const int max_c
               plan.cut_log[1] = cut + more;
               if (plan.split > steps || cut + more > 2 || max_clusters[log] < 1) continue;
               if (tokens <= 128) {
-                if (n || (tokens > 64 && pair == 1) || (tokens <= 32 && pair == 2)) continue;   // (fused quantisation: single CTAs)
-                plan.n_tile = plan.n_tail = (tokens + 16 * pair - 1) / (16 * pair) * (16 * pair);
-                plan.token_tiles = 1;
+                // From 65 tokens on also two tiles of 64: twice the CTAs with half the accumulators each, for a second read of the
+                // weights from L2.  Layers with few row tiles gain (128 tokens: 4608 x 3584 8.8 -> 7.7 us, 4096 x 1024 5.8 -> 4.2, 7003 x 2432
+                // at 77 tokens 7.3 -> 6.7), wide and long ones do not (37888 x 3584 23.7 -> 27.0, 3584 x 18944 16.1 -> 17.1).
+                if (n > 64 || (n && tokens <= 64) || (!n && tokens > 64 && pair == 1) || (tokens <= 32 && pair == 2)) continue;   // (fused quantisation: single CTAs)
+                plan.token_tiles = n ? 2 : 1;
+                plan.n_tail = (tokens - (n ? 64 : 0) + 16 * pair - 1) / (16 * pair) * (16 * pair);
+                plan.n_tile = n ? 64 : plan.n_tail;
               } else {
-                if (!n || pair == 1 || cut || (n == 256 && plan.split > 1)) continue;
+                if (n < 128 || pair == 1 || cut || (n == 256 && plan.split > 1)) continue;
                 plan.n_tile = n;
                 plan.token_tiles = (tokens + n - 1) / n;
                 plan.n_tail = (tokens - (plan.token_tiles - 1) * n + 31) / 32 * 32;

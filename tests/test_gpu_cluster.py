@@ -43,6 +43,24 @@ def test_exact_with_several_wide_tiles_per_cluster(tokens, k, forced, monkeypatc
     assert np.array_equal(got, case["expected"]), int((got != case["expected"]).sum())
 
 
+@pytest.mark.parametrize("pair", [1, 2])
+@pytest.mark.parametrize("split", [1, 2, 4])
+@pytest.mark.parametrize("tokens", [65, 80, 97, 128])
+def test_exact_in_two_tiles_of_64_tokens(tokens, split, pair, monkeypatch):
+    """65 to 128 tokens as two tiles, the second of which starts in the middle of its scale atom: single and paired CTAs, whole and cut
+    along K, one unit per cluster and (the last shape, uncut) several."""
+    for name, value in (("N", 64), ("PAIR", pair), ("SPLIT", split)):
+        monkeypatch.setenv("HYGEMM_CL_" + name, str(value))
+    for outputs, k, high in [(129, 1152, 1), (640, 896, 128)] + [(18944, 384, 1000)] * (split == 1):
+        case = oracle.exact_case(outputs, tokens, k, high, "random")
+        header = (C.c_int * 12)()
+        native.check(native.library().hg_plan(outputs - high, high, tokens, k, torch.cuda.get_device_properties(0).multi_processor_count, 0, header, None, 0))
+        assert (header[2], header[3]) == (64, 2), list(header)
+        got, guards, status = run_gemm(case, torch.bfloat16, 0)
+        assert status[0] == 0 and guards and (status[1], status[2]) == expected_work(case, 0), (outputs, k, high, status)
+        assert np.array_equal(got, case["expected"]), (outputs, k, high, int((got != case["expected"]).sum()))
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_swiglu_layer_call_equals_producer_then_gemm(dtype):
     """One foreign call for SwiGLU and down_proj: the same bytes as the producer followed by the GEMM on its codes."""
