@@ -331,8 +331,9 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
     // ------------------------------------------------------------------ activations and their scales (TMA)
     // One copy brings both K128 blocks (the map's third dimension counts them).
     if (!FUSED) {
-      pdl_wait();   // they are the previous kernel's output; the weight stream is not and already runs
-      if (lane == 0) HG_STAMP(2);
+      // They are the previous kernel's output; the weight stream is not and already runs.  Everything up to the first copy is
+      // done before the wait.
+      bool waiting = true;
       const uint32_t smem0 = __shfl_sync(0xffffffffu, base, 0);
       const uint32_t bars0 = PAIR == 1 ? smem0 + lay.bars : __shfl_sync(0xffffffffu, map_to_rank(bars, uint32_t(rank & ~1)), 0);
       const int atoms = (p.tokens + 127) >> 7;
@@ -347,6 +348,11 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
         for (int step = step_begin; step < step_end; ++step) {
           const int kb = 2 * step, nkb = min(2, p.kblocks - kb);
           if (!warp_wait(empty_bar(stage), phase, abort_flag)) { error = kErrProducer; break; }
+          if (waiting) {
+            pdl_wait();
+            waiting = false;
+            if (lane == 0) HG_STAMP(2);
+          }
           if (elect_one()) {
             const uint32_t bar = bars0 + uint32_t(stage) * 8u, dst = smem0 + lay.b + uint32_t(2 * stage) * lay.b_tile;
             if (PAIR == 1) mbar_expect_tx(bar, uint32_t(w.n) * 256u + uint32_t(n_atoms * nkb) * 512u);   // a block beyond K arrives as zeros

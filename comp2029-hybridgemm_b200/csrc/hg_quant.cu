@@ -168,7 +168,8 @@ __global__ void __launch_bounds__(256)
 mx_quant_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint8_t* __restrict__ sf,
                 uint16_t* __restrict__ debug, int rows, int k) {
   pdl_trigger();
-  pdl_wait();   // the input is usually the previous kernel's output
+  // All that does not depend on the input comes before the wait: the kernel is resident while the one in front still runs, and what
+  // follows the wait is the chain that a decode step is made of.
   const int kblocks = k >> 7;
   const int64_t real = int64_t(rows) * kblocks * 16;
   const int64_t tid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -177,21 +178,27 @@ mx_quant_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint
     const int pad_rows = ((rows + 127) & ~127) - rows;
     const int64_t p = tid - real;
     if (pad_rows == 0 || p >= int64_t(pad_rows) * kblocks) return;
-    const int row = rows + int(p % pad_rows), kb = int(p / pad_rows);
-    *reinterpret_cast<uint32_t*>(sf + scale_word_offset(row, kb, k)) = 0x7f7f7f7fu;
+    const int kb = int(uint32_t(p) / uint32_t(pad_rows)), row = rows + int(p) - kb * pad_rows;   // p is below k
+    uint32_t* const word = reinterpret_cast<uint32_t*>(sf + scale_word_offset(row, kb, k));
+    pdl_wait();
+    *word = 0x7f7f7f7fu;
     return;
   }
   const int lane = threadIdx.x & 31;
   const unsigned mask = 0xffffu << (lane & 16);        // the 16 threads of this (row, K128 block)
   const int sub = int(tid & 15);
   const int64_t item = tid >> 4;
-  const int row = int(item / kblocks), kb = int(item % kblocks);
+  const int row = item < (int64_t(1) << 31) ? int(uint32_t(item) / uint32_t(kblocks)) : int(item / kblocks), kb = int(item - int64_t(row) * kblocks);
   const int col = kb * 128 + sub * 8;
+  const uint16_t* const src = in + int64_t(row) * (SILU ? 2 * k : k) + col;
+  void* const to = out + (int64_t(row) * k + col) / (FP4 ? 2 : 1);
+  uint32_t* const scale_word = reinterpret_cast<uint32_t*>(sf + scale_word_offset(row, kb, k));
+  pdl_wait();   // the input is usually the previous kernel's output
 
   float v[8];
   if constexpr (SILU) {
-    const uint4 g4 = *reinterpret_cast<const uint4*>(in + int64_t(row) * 2 * k + col);
-    const uint4 u4 = *reinterpret_cast<const uint4*>(in + int64_t(row) * 2 * k + k + col);
+    const uint4 g4 = *reinterpret_cast<const uint4*>(src);
+    const uint4 u4 = *reinterpret_cast<const uint4*>(src + k);
     bool exact = MATH != 0 || debug;
     if (!exact) {
       const uint32_t g[4] = {g4.x, g4.y, g4.z, g4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w};
@@ -213,7 +220,7 @@ mx_quant_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint
     }
     __syncwarp(mask);
   } else {
-    const uint4 x4 = *reinterpret_cast<const uint4*>(in + int64_t(row) * k + col);
+    const uint4 x4 = *reinterpret_cast<const uint4*>(src);
     const uint32_t xw[4] = {x4.x, x4.y, x4.z, x4.w};
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = to_float<T>(uint16_t(xw[i >> 1] >> ((i & 1) * 16)));
@@ -230,12 +237,12 @@ mx_quant_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint
   for (int i = 0; i < 8; ++i) v[i] *= inv;
 
   if constexpr (FP4) {
-    *reinterpret_cast<uint32_t*>(out + (int64_t(row) * k + col) / 2) = cvt_e2m1x8(v);
+    *static_cast<uint32_t*>(to) = cvt_e2m1x8(v);
   } else {
     uint2 codes;
     codes.x = cvt_e4m3x2(v[0], v[1]) | (cvt_e4m3x2(v[2], v[3]) << 16);
     codes.y = cvt_e4m3x2(v[4], v[5]) | (cvt_e4m3x2(v[6], v[7]) << 16);
-    *reinterpret_cast<uint2*>(out + int64_t(row) * k + col) = codes;
+    *static_cast<uint2*>(to) = codes;
   }
 
   // Gather the four K32 exponents of this K128 block into one scale word.
@@ -243,7 +250,7 @@ mx_quant_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint
   const uint32_t byte = uint32_t(e + 127);
   const uint32_t word = __shfl_sync(mask, byte, base) | (__shfl_sync(mask, byte, base + 4) << 8) |
                         (__shfl_sync(mask, byte, base + 8) << 16) | (__shfl_sync(mask, byte, base + 12) << 24);
-  if (sub == 0) *reinterpret_cast<uint32_t*>(sf + scale_word_offset(row, kb, k)) = word;
+  if (sub == 0) *scale_word = word;
 }
 
 // ---- Many rows: weights at load time, prefill activations -----------------------------------------------------------
@@ -359,13 +366,13 @@ template <typename T>
 __global__ void __launch_bounds__(256, kRowsBlocks)
 mx_rows_kernel(const uint16_t* __restrict__ in, const QuantPart low, const QuantPart high, int k, int* __restrict__ verdict) {
   pdl_trigger();
-  pdl_wait();   // input and row lists come from the kernels before
-  if (verdict && blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<int2*>(verdict) = list_verdict(high.ids, high.rows);
   const int lane = threadIdx.x & 31, chunks = (k + 511) >> 9;
   const int low_groups = ((low.rows + 127) & ~127) >> 2, groups = low_groups + (((high.rows + 127) & ~127) >> 2);
   const int stride = gridDim.x * 8;
   int item = blockIdx.x * 8 + (threadIdx.x >> 5);
   int group = item / chunks, col = ((item - group * chunks) << 9) + 16 * lane;
+  pdl_wait();   // input and row lists come from the kernels before
+  if (verdict && blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<int2*>(verdict) = list_verdict(high.ids, high.rows);
   Raw16 raw[4], next[4];
   auto load = [&](Raw16 (&to)[4]) {
     int source[4];
@@ -405,12 +412,12 @@ template <typename T, int MATH>
 __global__ void __launch_bounds__(256, 4)
 mx_silu_rows_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint8_t* __restrict__ sf, uint16_t* __restrict__ debug, int rows, int k) {
   pdl_trigger();
-  pdl_wait();
   const int lane = threadIdx.x & 31, chunks = (k + 511) >> 9;
   const int item = blockIdx.x * 8 + (threadIdx.x >> 5);
   const int group = item / chunks, col = ((item - group * chunks) << 9) + 16 * lane;
   if (group >= ((rows + 127) & ~127) >> 2) return;
   const int row0 = (group >> 5) * 128 + (group & 31);
+  pdl_wait();
   struct Pair { Raw16 gate, up; };
   auto load = [&](Pair& to, int row) {
     to.gate = to.up = Raw16{};
@@ -483,11 +490,11 @@ partition_rows_kernel(const int64_t* __restrict__ ids, int n_ids, int rows, int3
   extern __shared__ uint32_t bitmap[];   // words of the bitmap, then the MXFP8 rows before each word
   __shared__ int warp_sum[32];
   pdl_trigger();
-  pdl_wait();
   const int words = (rows + 31) >> 5, tid = threadIdx.x, lane = tid & 31;
   int* const before = reinterpret_cast<int*>(bitmap + words);
   for (int w = tid; w < words; w += kPartitionThreads) bitmap[w] = 0;
   __syncthreads();
+  pdl_wait();
   int bad = 0;
   for (int i = tid; i < n_ids; i += kPartitionThreads) {
     const int64_t id = ids[i];
