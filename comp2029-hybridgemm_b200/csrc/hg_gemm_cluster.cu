@@ -444,15 +444,18 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
       // low words of the shared-memory descriptors of stage 0; a stage is a constant number of 16-byte units further on
       const uint32_t a_desc = (smem0 + lay.a) >> 4, a_stage = lay.a_tile >> 3, b_desc = smem0 >> 4, b_stage = lay.b_tile >> 3;
       const uint32_t sfa_desc = (smem0 + lay.sfa) >> 4, sfb_desc = (smem0 + lay.sfb) >> 4, sfb_stage = lay.sfb_stage >> 4;
+      // Waits until the accumulator of the n-th unit is free.  Overlapping accumulators: one becomes free when the epilogue of the
+      // OTHER one has drained the shared columns, so accumulator 1 waits for an arrival on its first use as well.
+      auto acc_free = [&](int n) {
+        const uint32_t parity = (uint32_t(n >> 1) & 1u) ^ (p.overlap && (n & 1) ? 0u : 1u);
+        return PAIR == 2 ? warp_wait_cluster(acc_empty_bar(n & 1), parity, abort_flag) : warp_wait(acc_empty_bar(n & 1), parity, abort_flag);
+      };
       int stage = 0, it = 0, issued = 0;
       uint32_t phase = 0;
       for (int u = cluster; u < units && !error; u += p.clusters, ++it) {
         const Unit w = unit_at(p, u);
         const int acc = it & 1;
-        // Overlapping accumulators: an accumulator becomes free when the epilogue of the OTHER one has drained the
-        // shared columns, so accumulator 1 waits for an arrival on its first use as well.
-        const uint32_t acc_parity = (uint32_t(it >> 1) & 1u) ^ (p.overlap && acc ? 0u : 1u);
-        if (!(PAIR == 2 ? warp_wait_cluster(acc_empty_bar(acc), acc_parity, abort_flag) : warp_wait(acc_empty_bar(acc), acc_parity, abort_flag))) { error = kErrMmaAcc; break; }
+        if (!acc_free(it)) { error = kErrMmaAcc; break; }
         tc_fence_after();
         const uint32_t tmem_d = tmem0 + uint32_t(acc * p.acc_shift);
         const uint32_t a_block = uint32_t(w.last - w.first) * 8u;
@@ -506,6 +509,10 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
       if (elect_one()) cg_commit<PAIR>(drain_bar, pair_mask);
       __syncwarp();
       if (!warp_wait(drain_bar, 0, abort_flag) && !error) error = kErrDrain;
+      // The other CTA's epilogues arrive here also for units that do not follow: this CTA stays until they have.
+      if (PAIR == 2)
+        for (int n = it; n <= it + (p.overlap ? 0 : 1) && !error; ++n)
+          if (!acc_free(n)) error = kErrDrain;
     } else if (PAIR == 2) {
       // ---------------------------------------------------------------- second CTA of a pair: wait for the last MMA
       if (!warp_wait(drain_bar, 0, abort_flag) && !error) error = kErrDrain;
@@ -653,8 +660,16 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
   }
   tc_fence_before();
   __syncwarp();
-  if (cluster_ctas > 1) cluster_sync();   // no CTA leaves while another may still write its shared memory or arrive on its barriers
-  else __syncthreads();
+  // No CTA leaves while another may still write its shared memory or arrive on its barriers.  All that was sent has been waited for
+  // where it arrives (an error aside), so the barrier needs no release, which would wait for the stores to global memory; the end
+  // of the grid does.
+  if (cluster_ctas > 1) {
+    if (error) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    else asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  } else {
+    __syncthreads();
+  }
   if (warp == 1) {
     tc_fence_after();
     cg_dealloc<PAIR>(tmem_base, p.tmem_cols);

@@ -193,7 +193,10 @@ mx_quant_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint
   const uint16_t* const src = in + int64_t(row) * (SILU ? 2 * k : k) + col;
   void* const to = out + (int64_t(row) * k + col) / (FP4 ? 2 : 1);
   uint32_t* const scale_word = reinterpret_cast<uint32_t*>(sf + scale_word_offset(row, kb, k));
-  pdl_wait();   // the input is usually the previous kernel's output
+  // Usually the previous kernel's output, and in L2; where it is older it comes in during the wait.
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(src) : "memory");
+  if constexpr (SILU) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + k) : "memory");
+  pdl_wait();
 
   float v[8];
   if constexpr (SILU) {
