@@ -177,6 +177,10 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void arrive_remote(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// The same where nothing in memory is handed over, and the release would wait for the thread's stores.
+__device__ __forceinline__ void arrive_remote_relaxed(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
 __device__ __forceinline__ void store_remote(uint32_t cluster_addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
   asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
@@ -511,7 +515,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
       if (!warp_wait(drain_bar, 0, abort_flag) && !error) error = kErrDrain;
       // The other CTA's epilogues arrive here also for units that do not follow: this CTA stays until they have.
       if (PAIR == 2)
-        for (int n = it; n <= it + (p.overlap ? 0 : 1) && !error; ++n)
+        for (int n = it; p.split == 1 && n <= it + (p.overlap ? 0 : 1) && !error; ++n)
           if (!acc_free(n)) error = kErrDrain;
     } else if (PAIR == 2) {
       // ---------------------------------------------------------------- second CTA of a pair: wait for the last MMA
@@ -546,7 +550,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
         __syncwarp();
         if (lane == 0) {
           if (PAIR == 1) mbar_arrive(acc_empty_bar(which));
-          else arrive_remote(map_to_rank(acc_empty_bar(which), leader));
+          else arrive_remote_relaxed(map_to_rank(acc_empty_bar(which), leader));
         }
       };
       // N columns of this thread's row from column c on.
@@ -597,7 +601,8 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
               store_async(to, map_to_rank(red_full, owner), tc_loaded(r[4 * i]), tc_loaded(r[4 * i + 1]), tc_loaded(r[4 * i + 2]), tc_loaded(r[4 * i + 3]));
           }
         }
-        release(acc);
+        // A cluster that splits K has one unit, and nobody waits for the accumulator.  (Single CTAs measure 0.1 us faster with it.)
+        if constexpr (PAIR == 1) release(acc);
         if (!p.async_push && lane < p.split) arrive_remote(map_to_rank(red_full, uint32_t(lane * PAIR + half)));
         if (!warp_wait_cluster(red_full, 0, abort_flag)) { error = kErrEpilogue; break; }
         const uint32_t pieces = base + lay.red + uint32_t(row_in_tile) * 16u;
