@@ -127,6 +127,13 @@ template <int PAIR> __device__ __forceinline__ void cg_commit(uint32_t bar, uint
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                  ::"r"(bar), "h"(cta_mask) : "memory");
 }
+// The same, in every CTA of the mask whatever the tile.
+template <int PAIR> __device__ __forceinline__ void cg_commit_to(uint32_t bar, uint16_t cta_mask) {
+  if constexpr (PAIR == 1)
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(bar), "h"(cta_mask) : "memory");
+  else cg_commit<PAIR>(bar, cta_mask);
+}
 template <int PAIR> __device__ __forceinline__ void cg_cp_scales(uint32_t tmem, uint64_t desc) {
   if constexpr (PAIR == 1) tc_cp_scales(tmem, desc);
   else asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem), "l"(desc) : "memory");
@@ -278,7 +285,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
       mbar_init(acc_empty_bar(s), 4 * kSides * PAIR);
     }
     mbar_init(red_full, p.async_push ? 1u : uint32_t(4 * kSides * p.split));   // one thread, with the bytes to come; or every warp
-    mbar_init(red_empty, uint32_t(4 * kSides * p.split));
+    mbar_init(red_empty, uint32_t(p.split));
     mbar_init(drain_bar, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -501,6 +508,8 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
         }
         if (error) break;
         issued += min(2 * step, p.kblocks) - 2 * step_begin;   // as far as the loop came
+        if (p.ring_exchange && elect_one()) cg_commit_to<PAIR>(red_empty, uint16_t((1u << cluster_ctas) - 1u));
+        __syncwarp();
         if (elect_one()) cg_commit<PAIR>(acc_full_bar(acc), pair_mask);
         __syncwarp();
 #ifdef HG_TRACE
@@ -576,8 +585,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
       if (p.split > 1) {
         // Every slice owns 2^share_log groups of four columns.  A partial goes straight to the shared memory of the slice
         // that owns its group (lanes write 512 contiguous bytes), one hop; the owner adds the pieces in K order.
-        // In the ring: every slice first tells the others that its own MMAs, and with them its ring, are done.
-        if (p.ring_exchange && lane < p.split) arrive_remote(map_to_rank(red_empty, uint32_t(lane * PAIR + half)));
+        // In the ring: every slice's last commit tells all the others that its MMAs, and with them its ring, are done.
         if (p.ring_exchange && !warp_wait_cluster(red_empty, 0, abort_flag)) { error = kErrEpilogue; break; }
         const uint32_t share = 1u << p.share_log;
         const uint32_t my_piece = base + lay.red + (uint32_t(slice) << (p.share_log + 11)) + uint32_t(row_in_tile) * 16u;
