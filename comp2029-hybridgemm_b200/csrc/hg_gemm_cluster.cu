@@ -611,6 +611,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
         }
         // A cluster that splits K has one unit, and nobody waits for the accumulator.  (Single CTAs measure 0.1 us faster with it.)
         if constexpr (PAIR == 1) release(acc);
+        else __syncwarp();   // an arrival releases what the whole warp stored
         if (!p.async_push && lane < p.split) arrive_remote(map_to_rank(red_full, uint32_t(lane * PAIR + half)));
         if (!warp_wait_cluster(red_full, 0, abort_flag)) { error = kErrEpilogue; break; }
         const uint32_t pieces = base + lay.red + uint32_t(row_in_tile) * 16u;

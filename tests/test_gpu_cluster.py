@@ -61,6 +61,23 @@ def test_exact_in_two_tiles_of_64_tokens(tokens, split, pair, monkeypatch):
         assert np.array_equal(got, case["expected"]), (outputs, k, high, int((got != case["expected"]).sum()))
 
 
+@pytest.mark.parametrize("tokens,pair,split", [(t, p, s) for t, p in [(17, 1), (33, 1), (36, 2), (50, 1), (64, 2), (100, 2), (128, 2)]
+                                               for s in (2, 4, 8) if p * s <= 8])
+def test_exact_cut_along_k_at_every_way_of_the_exchange(tokens, pair, split, monkeypatch):
+    """Partial sums of one token tile on all their ways through a cluster: asynchronous stores up to 32 tokens, above that through the ring,
+    with slices of one K128 block and of unequal length, partitions that end inside a tile and tiles of 128, 64 and 32 rows."""
+    width = -(-tokens // (16 * pair)) * 16 * pair
+    for name, value in (("N", width), ("PAIR", pair), ("SPLIT", split)):
+        monkeypatch.setenv("HYGEMM_CL_" + name, str(value))
+    for (outputs, k, high), cut in [((129, 128 * (2 * split - 1), 1), 0), ((640, 2432, 128), 1), ((257, 3200, 1), 2)]:
+        monkeypatch.setenv("HYGEMM_CL_CUT", str(cut))
+        case = oracle.exact_case(outputs, tokens, k, high, "random")
+        for _ in range(3):
+            got, guards, status = run_gemm(case, torch.bfloat16, 0)
+            assert status[0] == 0 and guards and (status[1], status[2]) == expected_work(case, 0), (outputs, k, high, status)
+            assert np.array_equal(got, case["expected"]), (outputs, k, high, int((got != case["expected"]).sum()))
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_swiglu_layer_call_equals_producer_then_gemm(dtype):
     """One foreign call for SwiGLU and down_proj: the same bytes as the producer followed by the GEMM on its codes."""
