@@ -730,7 +730,8 @@ constexpr PlanFit kWideDecodeFit{236.7, 1.328, 12840, 13981, 250.0, 0.2656, 0.70
 constexpr PlanFit kPrefillFit{234, 1.28, 18800, 12300, 380, 0.397, 1.75, 0.0159, 0.632, 0.0142, 0.0146, 0.648, -0.67, 0.09, 0.0186, 0.00254,
                               0.00225, 2.55, 0.0711, -0.221, 3120};
 
-static double plan_cost(const ClusterPlan& plan, int64_t units, int kblocks, double weight_kilobytes) {
+// `reject`: a plan that costs this much or more may be given any cost from there on.
+static double plan_cost(const ClusterPlan& plan, int units, int kblocks, double weight_kilobytes, double reject) {
   const int columns = (plan.token_tiles - 1) * plan.n_tile + plan.n_tail;
   const PlanFit& fit = columns <= 64 ? kDecodeFit : plan.token_tiles * plan.n_tile <= 128 ? kWideDecodeFit : kPrefillFit;
   const double steps = double((kblocks + 1) / 2) / plan.split;
@@ -750,28 +751,55 @@ static double plan_cost(const ClusterPlan& plan, int64_t units, int kblocks, dou
   const double main_of[2][2] = {{main_loop(plan.n_tile, false), main_loop(plan.n_tail, false)},
                                 {plan.tiles[1] ? main_loop(plan.n_tile, true) : 0, plan.tiles[1] ? main_loop(plan.n_tail, true) : 0}};
   const double store_of[2][2] = {{stores(plan.n_tile, false), stores(plan.n_tail, false)}, {stores(plan.n_tile, true), stores(plan.n_tail, true)}};
-  std::vector<double> load(size_t(plan.clusters), 0.0), storing(size_t(plan.clusters), 0.0);   // end of a cluster's main loops, of its stores
-  const int64_t tiles = int64_t(plan.tiles[0]) + plan.tiles[1];
-  for (int64_t u = 0; u < units; ++u) {
-    const int64_t t = u / plan.token_tiles;
-    const bool tail = u % plan.token_tiles == plan.token_tiles - 1;
-    const bool high = plan.token_tiles == 1 ? t < plan.tiles[1] : (t + 1) * plan.tiles[1] / tiles > t * plan.tiles[1] / tiles;
-    double &main_end = load[size_t(u % plan.clusters)], &store_end = storing[size_t(u % plan.clusters)];
-    // two accumulators: a main loop starts once the stores before the last ones are done
-    main_end = std::max(main_end + main_of[high][tail], store_end);
-    store_end = main_end + store_of[high][tail];
-  }
-  const double busiest = *std::max_element(storing.begin(), storing.end());
   double exchange = 0;
   if (plan.split > 1)
     exchange = fit.hops * std::log2(double(cluster_ctas)) + fit.exchange + (fit.part + fit.part_token * plan.n_tile) * plan.split;
   const double least = weight_kilobytes / fit.hbm + store_of[0][1];
-  return fit.cta * ctas + (plan.pair == 2 ? fit.pair : 0) + fit.cut * plan.cut_log[0] + fit.finer * (plan.cut_log[1] - plan.cut_log[0]) +
-         std::max(busiest, least) + exchange;
+  auto total = [&](double busiest) {
+    return fit.cta * ctas + (plan.pair == 2 ? fit.pair : 0) + fit.cut * plan.cut_log[0] + fit.finer * (plan.cut_log[1] - plan.cut_log[0]) +
+           std::max(busiest, least) + exchange;
+  };
+  // Cluster 0 has the most units.  (The margin is far above the rounding of the sums below.)
+  const int most = (units + plan.clusters - 1) / plan.clusters;
+  double shortest = 1e30;
+  for (int part = 0; part < 2; ++part)
+    if (plan.tiles[part]) shortest = std::min({shortest, main_of[part][0], main_of[part][1]});
+  if (const double bound = total(most * shortest * (1 - 1e-9)); bound >= reject) return bound;
+
+  // End of a cluster's main loops and of its stores.  Two accumulators: a main loop starts once the stores before the last ones are done.
+  struct Ends { double main = 0, stores = 0; };
+  auto add = [&](Ends& ends, bool high, bool tail) {
+    ends.main = std::max(ends.main + main_of[high][tail], ends.stores);
+    ends.stores = ends.main + store_of[high][tail];
+  };
+  double busiest = 0;
+  if (plan.token_tiles == 1) {
+    // MXFP8 tiles come first, so clusters differ only in how many units of each kind they have: the first ones may have one more.
+    for (const int cluster : {0, plan.tiles[1] % plan.clusters, units % plan.clusters}) {
+      Ends ends;
+      for (int u = cluster; u < units; u += plan.clusters) add(ends, u < plan.tiles[1], true);
+      busiest = std::max(busiest, ends.stores);
+    }
+  } else {
+    std::vector<Ends> ends(size_t(plan.clusters));
+    const int tiles = plan.tiles[0] + plan.tiles[1];
+    int cluster = 0, spread = 0;   // spread: how far the running share of MXFP8 tiles is beyond the last whole one (see unit_at)
+    for (int t = 0; t < tiles; ++t) {
+      spread += plan.tiles[1];
+      const bool high = spread >= tiles;
+      if (high) spread -= tiles;
+      for (int tt = 0; tt < plan.token_tiles; ++tt) {
+        add(ends[size_t(cluster)], high, tt == plan.token_tiles - 1);
+        if (++cluster == plan.clusters) cluster = 0;
+      }
+    }
+    for (const Ends& e : ends) busiest = std::max(busiest, e.stores);
+  }
+  return total(busiest);
 }
 
 // Ring, TMEM and shared-memory figures that follow from the other choices.  False when the ring would be too shallow.
-static bool finish_plan(ClusterPlan& plan) {
+static bool finish_plan(ClusterPlan& plan, int most_stages) {
   const int n_cols = (plan.n_tile + 31) & ~31;
   plan.overlap = plan.n_tile > 224 ? 1 : 0;
   plan.acc_shift = plan.overlap ? 224 : n_cols;
@@ -780,8 +808,7 @@ static bool finish_plan(ClusterPlan& plan) {
   while (plan.tmem_cols < cols) plan.tmem_cols *= 2;
   plan.slot_rows = kTileRows >> std::min(plan.cut_log[0], plan.cut_log[1]);
   plan.least_rows = kTileRows >> std::max(plan.cut_log[0], plan.cut_log[1]);
-  const int most = std::min(kClusterMaxStages, tuning("HYGEMM_CL_STAGES", kClusterMaxStages));
-  for (plan.stages = most; plan.stages >= 2; --plan.stages) {
+  for (plan.stages = most_stages; plan.stages >= 2; --plan.stages) {
     plan.smem_bytes = 1024 + int(cluster_smem(plan.stages, plan.n_tile, plan.pair, plan.split, plan.slot_rows, plan.least_rows, plan.ring_exchange).end);
     if (plan.smem_bytes <= kMaxSmem) return true;
   }
@@ -795,6 +822,7 @@ ClusterPlan make_cluster_plan(int lo, int hi, int tokens, int k, const int max_c
   best.cost = 1e30;
   const int force_split = tuning("HYGEMM_CL_SPLIT", 0), force_pair = tuning("HYGEMM_CL_PAIR", 0), force_n = tuning("HYGEMM_CL_N", 0);
   const int force_cut = tuning("HYGEMM_CL_CUT", -1), force_cut_high = tuning("HYGEMM_CL_CUT_HIGH", -1);
+  const int most_stages = std::min(kClusterMaxStages, tuning("HYGEMM_CL_STAGES", kClusterMaxStages));
   for (int pair = 1; pair <= 2; ++pair)
     for (int log = pair - 1; log < 4; ++log)
       for (int cut = 0; cut < 3; ++cut)
@@ -832,8 +860,8 @@ ClusterPlan make_cluster_plan(int lo, int hi, int tokens, int k, const int max_c
               // Worth its extra hop (about 0.4 us) where the exchange buffer would take a stage from the ring (down_proj at 128
               // tokens 17.1 -> 16.0 us).
               plan.ring_exchange = plan.split > 1 && plan.n_tile > 32;
-              if (!finish_plan(plan)) continue;
-              plan.cost = plan_cost(plan, units, kblocks, (lo * 0.53125 + hi * 1.03125) * k * 1e-3);
+              if (!finish_plan(plan, most_stages)) continue;
+              plan.cost = plan_cost(plan, int(units), kblocks, (lo * 0.53125 + hi * 1.03125) * k * 1e-3, best.cost);
               if (plan.cost < best.cost) best = plan;
             }
   if (best.cost >= 1e30) throw std::runtime_error("No cluster schedule for this shape");

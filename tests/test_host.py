@@ -8,6 +8,7 @@ import re
 import shutil
 import subprocess
 import sys
+import time
 from pathlib import Path
 
 import numpy as np
@@ -121,6 +122,26 @@ def test_the_cluster_plan_covers_each_row_token_and_k_block_exactly_once(tokens)
             for group, total in zip(np.split(spans, starts[1:]), [n for n in (lo, hi) if n]):
                 assert np.all(group[1:, 1] == group[:-1, 1] + group[:-1, 2]) and group[-1, 1] + group[-1, 2] == total
             assert len(here) == len(spans) * token_tiles
+
+
+@pytest.mark.parametrize("lo,hi,k", [(34048, 3840, 3584), (25856, 2816, 4096), (10800, 1200, 6144), (6302, 701, 2432)])
+def test_the_plan_search_costs_at_65_to_128_tokens_about_what_it_costs_at_64(lo, hi, k):
+    """The first call of a token count of a layer pays for the search.  From 65 tokens on it has several times the units to look at, and took
+    3 to 6 times as long when it walked every unit of every plan (159 us for the first shape; 1.5 to 1.9 times and 9 us now).  Best of
+    many, so that a busy machine does not decide."""
+    lib, header = native.library(), (C.c_int * 12)()
+
+    def cost(tokens):
+        best = float("inf")
+        for _ in range(100):
+            start = time.perf_counter()
+            lib.hg_plan(lo, hi, tokens, k, 148, 0, header, None, 0)
+            best = min(best, time.perf_counter() - start)
+        return best
+
+    at_64 = cost(64)
+    for tokens in (65, 77, 128):
+        assert cost(tokens) <= 2.5 * at_64, (tokens, at_64)
 
 
 @pytest.mark.parametrize("schedule", [1, 2, 3])
