@@ -665,22 +665,26 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
     if (threadIdx.x == 64 && stored) atomicAdd(p.status + 2, stored);
   }
 
+  auto settle = [] {   // time for everything in flight to land
+    const long long start = clock64();
+    while (clock64() - start < 400000ll) __nanosleep(1000);
+  };
   if (error) {
     *abort_flag = 1;
     atomicCAS(p.status, 0, error * 1000000 + int(blockIdx.x));
-    // Copies and MMAs in flight get time to land before shared memory and TMEM are released.
-    const long long start = clock64();
-    while (clock64() - start < 400000ll) __nanosleep(1000);
+    settle();   // copies and MMAs, before shared memory and TMEM are released
   }
   tc_fence_before();
   __syncwarp();
   // No CTA leaves while another may still write its shared memory or arrive on its barriers.  All that was sent has been waited for
-  // where it arrives (an error aside), so the barrier needs no release, which would wait for the stores to global memory; the end
-  // of the grid does.
+  // where it arrives, so the barrier needs no release, which would wait for the stores to global memory; the end of the grid does.
+  // Not so where a wait ran out: what this CTA sent is covered by its release, and what the others still sent to it, whose
+  // arrival says nothing about their stores, gets time to land once they have all arrived.
   if (cluster_ctas > 1) {
     if (error) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     else asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (error) settle();
   } else {
     __syncthreads();
   }
