@@ -710,27 +710,33 @@ static int tuning(const char* name, int value) {
 // delivers, over all SMs and to one.  An SM stores 1.4 sectors per cycle: 128 rows of an MXFP4 tile touch 13 sectors per token,
 // 128 rows of an MXFP8 tile 128, so an MXFP8 tile of 256 tokens is stored for 13 us.  Finer MXFP8 tiles spread that over more
 // CTAs (qkv of Qwen2.5-7B: 24.8 -> 17.5 us at 777 tokens, 46.7 -> 37.5 us at 2048).  Stores run under the next main loop.  The
-// launch takes the busiest cluster's time or its weights' time from HBM, whichever is longer, plus a little per CTA and the
-// exchange of partials.
+// launch takes the busiest cluster's time, plus a little per CTA and the exchange of partials; prefill also no less than its
+// weights' time from HBM.  (In decode the busiest cluster's L2 reads hold the weights already; a bound there decided none of 24000
+// shapes.)
 //
-// The constants are a fit to the order of measured launches, every plan a shape can have, for shapes drawn from 640 to 38000
-// channels and K 512 to 18944.  Prefill: 1700 launches of the GEMM alone; the plan preferred is 0.6 % slower than the best one of
-// the shape on average.  Up to 128 tokens: layer calls (quantiser and GEMM), 2400 shapes, of which every fourth or so was fitted
-// to and the rest checked: 0.9 % slower than the best up to 64 tokens (1.9 % with constants fitted to the GEMM alone: between
-// quantisers a plan of few CTAs gains, as the launch behind it finds free SMs) and 1.1 % from 65 on (1.5 %; 10 % when two tiles of
-// 64 tokens were no choice).
+// The constants are weights of a fit to the order of measured launches, every plan a shape can have, for shapes drawn from 640 to
+// 38000 channels and K 512 to 18944; a rate among them need not be one that a unit of the chip has.  Prefill: 1700 launches of the
+// GEMM alone; the plan preferred is 0.6 % slower than the best one of the shape on average.  Up to 128 tokens: layer calls
+// (quantiser and GEMM) back to back, 2400 shapes, of which every fourth or so was fitted to and the rest checked: 0.9 % slower than the
+// best up to 64 tokens (1.9 % with constants fitted to the GEMM alone) and 1.1 % from 65 on (1.5 %; 10 % when two tiles of 64
+// tokens were no choice).  Up to twelve layers took turns there, so weights of less than about 10 MB stayed in L2.  Checked since on
+// 905 other layers of up to 12000 channels with all their weights cold: 1.8 % and 2.3 % (the same layers with weights in L2 1.6 %
+// and 1.9 %).  Behind a kernel that has just written the activations and does not release its dependents early (an elementwise
+// kernel of torch was measured) small layers at few tokens want fewer CTAs than back to back: 2009 x 640 at 14 tokens takes 5.98
+// us with 34 CTAs, that kernel included, and took 5.82 with 19 (back to back 3.77 and 4.28).  Over 110 layers such calls took
+// 5.4 % less than with the constants and kernels before.
 struct PlanFit {
   double mma_floor;                                  // cycles of a single CTA's narrow MMA with its operand reads
   double turn, l2, l2_wide, to_one;                  // us per turn of the ring; bytes per ns from L2 to all SMs, tiles of 129 tokens and more, to one
   double unit, split_unit, split_token;              // after a unit's main loop, whole or one of several parts of K; per token
   double store, store_token, low_row, high_row;      // stores: start; per token; cycles per token and row
   double hops, exchange, part, part_token;           // exchange: per doubling of the cluster, constant, per part, per part and token
-  double cta, pair, cut, finer, hbm;                 // per CTA of the grid, paired CTAs, cut of all tiles, further cut of MXFP8 tiles; bytes per ns
+  double cta, pair, cut, finer, hbm;                 // per CTA of the grid, paired CTAs, cut of all tiles, further cut of MXFP8 tiles; bytes per ns (0: no bound)
 };
-constexpr PlanFit kDecodeFit{234.0, 1.313, 12213, 11174, 189.6, 0.09482, 0.5133, 0.0314, 1.07, 0.01755, 0.02057, 0.9327, -0.657, 0.1007, 0.0143, 0.005931,
-                             0.008127, 0.5955, -0.0378, 0.268, 16351};
-constexpr PlanFit kWideDecodeFit{236.7, 1.328, 12840, 13981, 250.0, 0.2656, 0.7058, 0.02462, 0.3386, 0.01767, 0.01224, 0.9089, -0.538, 0.1856, 0.06477, 0.003302,
-                                 0.01379, 0.5441, -0.02387, 0.2337, 8705};
+constexpr PlanFit kDecodeFit{234.0, 1.313, 12213, 12213, 189.6, 0.09482, 0.5133, 0.0314, 1.07, 0.01755, 0.02057, 0.9327, -0.657, 0.1007, 0.0143, 0.005931,
+                             0.008127, 0.5955, -0.0378, 0.268, 0};
+constexpr PlanFit kWideDecodeFit{236.7, 1.328, 12840, 12840, 250.0, 0.2656, 0.7058, 0.02462, 0.3386, 0.01767, 0.01224, 0.9089, -0.538, 0.1856, 0.06477, 0.003302,
+                                 0.01379, 0.5441, -0.02387, 0.2337, 0};
 constexpr PlanFit kPrefillFit{234, 1.28, 18800, 12300, 380, 0.397, 1.75, 0.0159, 0.632, 0.0142, 0.0146, 0.648, -0.67, 0.09, 0.0186, 0.00254,
                               0.00225, 2.55, 0.0711, -0.221, 3120};
 
@@ -758,7 +764,7 @@ static double plan_cost(const ClusterPlan& plan, int units, int kblocks, double 
   double exchange = 0;
   if (plan.split > 1)
     exchange = fit.hops * std::log2(double(cluster_ctas)) + fit.exchange + (fit.part + fit.part_token * plan.n_tile) * plan.split;
-  const double least = weight_kilobytes / fit.hbm + store_of[0][1];
+  const double least = fit.hbm ? weight_kilobytes / fit.hbm + store_of[0][1] : 0;
   auto total = [&](double busiest) {
     return fit.cta * ctas + (plan.pair == 2 ? fit.pair : 0) + fit.cut * plan.cut_log[0] + fit.finer * (plan.cut_log[1] - plan.cut_log[0]) +
            std::max(busiest, least) + exchange;
