@@ -89,8 +89,9 @@ inline cudaError_t launch_kernel(void (*kernel)(KernelArgs...), dim3 grid, dim3 
 
 // Smallest e with amax * 2^-e <= MAX (448 for E4M3, 6 for E2M1), clamped to
 // [-127,127]; e = 0 for an all-zero block.  Equals ceil(log2(amax/MAX)) of
-// integrations/vllm/native/runtime.cu:71-72 for every 16-bit input (proved
-// exhaustively by the CPU tests) without a transcendental.
+// integrations/vllm/native/runtime.cu:71-72 for every 16-bit input without a
+// transcendental (the CPU tests compare this formula, restated in the oracle,
+// for all of them; the GPU tests quantise every one as the maximum of a group).
 template <bool FP4>
 __device__ __forceinline__ int mx_exponent(float amax) {
   const uint32_t b = __float_as_uint(amax);

@@ -56,6 +56,7 @@ def lib():
             ("hgo_e2m1_from_float", C.c_uint8, [C.c_float]), ("hgo_e2m1_to_float", C.c_float, [C.c_uint8]),
             ("hgo_exponent_literal", C.c_int, [C.c_float, C.c_int]),
             ("hgo_exponent_exact", C.c_int, [C.c_float, C.c_int]),
+            ("hgo_exponent_carry", C.c_int, [C.c_float, C.c_int]),
             ("hgo_exact_reference", C.c_float, [C.c_int] * 4),
             ("hgo_threads", C.c_int, []), ("hgo_set_threads", None, [C.c_int]),
         ]:

@@ -11,7 +11,7 @@
  * decode_logical, scale_indices) stored under tests/golden/; the E4M3
  * conversion is checked against the CPU float8_e4m3fn cast of PyTorch and
  * against the host conversion of the CUTLASS headers for every 16-bit input;
- * the exponent rule is checked exhaustively against its closed form.  The
+ * the exponent rule is checked exhaustively against its closed forms.  The
  * reference's CUDA quantiser itself cannot execute off an SM120 GPU.
  *
  * Each function cites the reference file:line it follows (paths are relative
@@ -214,8 +214,8 @@ int hgo_exponent_literal(float amax, int fp4) {
   return (int)l;
 }
 
-/* Closed form used by the CUDA kernels: the smallest e with amax*2^-e <= max,
- * computed from the fp32 bit pattern (no transcendental). */
+/* Closed form: the smallest e with amax*2^-e <= max, by cases on the fp32 bit
+ * pattern (no transcendental). */
 int hgo_exponent_exact(float amax, int fp4) {
   if (!(amax > 0)) return 0;
   uint32_t b = float_to_bits(amax);
@@ -228,6 +228,15 @@ int hgo_exponent_exact(float amax, int fp4) {
   if (e < -127) e = -127;
   if (e > 127) e = 127;
   return e;
+}
+
+/* The same as the CUDA kernels compute it: a mantissa above that of max carries
+ * into the exponent when the distance to the end of the binade is added. */
+int hgo_exponent_carry(float amax, int fp4) {
+  const uint32_t b = float_to_bits(amax);
+  if (b == 0) return 0;
+  const int e = fp4 ? (int)((b + 0x3fffffu) >> 23) - 129 : (int)((b + 0x1fffffu) >> 23) - 135;
+  return e < -127 ? -127 : e;
 }
 
 /* ------------------------------------------------------------------------- */

@@ -70,6 +70,27 @@ def test_pack_every_finite_16bit_value(dtype):
     assert np.array_equal(sf.cpu().numpy(), want_sf)
 
 
+@pytest.mark.parametrize("fp4", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_every_16bit_value_as_the_maximum_of_a_group(dtype, fp4):
+    """Codes and scale bytes of both formats, so the values just below and above each 1.5 x 2^n and 1.75 x 2^n are among them; the exponent
+    search without offsets starts from the same exponents."""
+    everything = torch.arange(1, 1 << 15, dtype=torch.int32).to(torch.int16).view(dtype)
+    values = everything[torch.isfinite(everything.float())]
+    values = torch.cat([values, values.new_zeros(-values.numel() % 4)])
+    groups = torch.zeros(values.numel(), 32, dtype=dtype)
+    for column, factor in ((0, 1.0), (7, -0.5), (13, 0.37), (31, -0.08)):
+        groups[:, column] = (values.float() * factor).to(dtype)
+    x = groups.view(-1, 128)
+    q, sf = native.pack(x.cuda(), fp4)
+    want_q, want_sf = oracle.pack(x, fp4=fp4, bf16=dtype == torch.bfloat16)
+    assert np.array_equal(sf.cpu().numpy(), want_sf) and np.array_equal(q.cpu().numpy(), want_q)
+    if fp4:
+        codes, scales, _ = fp4_quant.quantize(x.cuda(), offsets=())
+        assert np.array_equal(codes.cpu().numpy(), want_q)
+        assert np.array_equal(scales.cpu().numpy(), want_sf[oracle.scale_indices(*x.shape)])
+
+
 def test_fp4_tie_table():
     """allocation/check_components.py:14 of the reference: exact ties and signed zeros."""
     ties = [0., -0., .25, .75, 1.25, 1.75, 2.5, 3.5, 5., 6., -.25, -.75, -1.25, -1.75, -2.5, -3.5, -5., -6.]

@@ -65,6 +65,18 @@ def test_exponent_rule_literal_equals_closed_form_exhaustively(fp4):
             assert a == b, (float(v), a, b)
 
 
+@pytest.mark.parametrize("fp4", [0, 1])
+def test_exponent_by_carry_equals_the_other_forms_exhaustively(fp4):
+    """The form the kernels compute, for zero, every positive fp16 and bf16 value (subnormal in fp32 too) and infinity."""
+    L = oracle.lib()
+    for vals in (ALL16.view(np.float16).astype(np.float32), (ALL16.astype(np.uint32) << 16).view(np.float32)):
+        for v in vals[(vals >= 0) & ~np.signbit(vals)]:
+            value = C.c_float(float(v))
+            got = L.hgo_exponent_carry(value, fp4)
+            assert got == L.hgo_exponent_exact(value, fp4), float(v)
+            assert not np.isfinite(v) or got == L.hgo_exponent_literal(value, fp4), float(v)
+
+
 def test_decode_matches_reference_decode_mx(golden):
     g = golden("decode_mx.npz")
     for rows, k in [(3, 128), (130, 256), (33, 896)]:
