@@ -101,3 +101,41 @@ def test_candidates_ruled_out_by_one_term_never_win(rows, k, kind):
         want_q4, want_scales = oracle.clip_pack(w, importance.numpy(), offsets, bf16=True)
         assert (scales.cpu().numpy() == want_scales).all(), offsets
         assert (q4.cpu().numpy() == want_q4).all(), offsets
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("kind", ["plain", "outstanding", "hidden"])
+@pytest.mark.parametrize("rows,k", [(5, 128), (300, 640)])
+def test_statistics_against_independent_sums(rows, k, kind, dtype):
+    """How many groups moved by each offset, and the four error sums, against the oracle's codes.  All terms are non-negative; each is
+    rounded three times in fp32 and eight are added in fp32 before fp64 takes over, so a sum is off by at most about 11 x 2^-24 = 7e-7."""
+    g = torch.Generator().manual_seed(SEED + rows)
+    w = torch.randn(rows, k, generator=g) * 0.03
+    w[torch.rand(rows, k, generator=g) < 0.02] *= 8
+    importance = torch.rand(k, generator=g) + 0.1
+    special = torch.rand(k, generator=g) < 0.05
+    if kind == "hidden":
+        w[:, special] *= 8
+    importance[special] = {"plain": 1.0, "outstanding": 400.0, "hidden": 0.0}[kind]
+    w[0], w[1, :32], w[2, 32:64] = 0, 0, 1e-7
+    w, weight = w.to(dtype), None if kind == "plain" else importance
+    bf16, scale = dtype == torch.bfloat16, (torch.ones(k) if weight is None else weight).double()
+    x = w.double()
+
+    def error(packed, scale_bytes, per_column):
+        values = fp4_quant.decode_logical(torch.from_numpy(packed), torch.from_numpy(scale_bytes), k).double()
+        return float(((values - x).square() * per_column).sum())
+
+    nearest = oracle.clip_pack(w, None, (), bf16=bf16)
+    moves = set()
+    for offsets in [(0, -1, -2), (-2, 3, -1, 0, 1), (2, -3, -4, -1, 0, 1, -2, -8), (-1,), ()]:
+        q4, scales, stats = fp4_quant.quantize(w.cuda(), None if weight is None else weight.cuda(), offsets)
+        want = oracle.clip_pack(w, None if weight is None else weight.numpy(), offsets, bf16=bf16)
+        assert (scales.cpu().numpy() == want[1]).all() and (q4.cpu().numpy() == want[0]).all(), offsets
+        moved = want[1].astype(np.int64) - nearest[1].astype(np.int64)
+        assert stats["shift_groups"] == {str(-o): int((moved == o).sum()) for o in offsets}, offsets
+        moves |= set(moved.ravel().tolist())
+        for name, value in (("weighted_error_before", error(*nearest, scale)), ("weighted_error_after", error(*want, scale)),
+                            ("weight_error_before", error(*nearest, 1.0)), ("weight_error_after", error(*want, 1.0))):
+            np.testing.assert_allclose(stats[name], value, rtol=1e-6, err_msg=f"{name} {offsets}")
+    assert moves >= ({0, -1} if kind != "hidden" else {0, -1, -2, -3})
