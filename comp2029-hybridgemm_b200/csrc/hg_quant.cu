@@ -168,8 +168,10 @@ __global__ void __launch_bounds__(256)
 mx_quant_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint8_t* __restrict__ sf,
                 uint16_t* __restrict__ debug, int rows, int k) {
   pdl_trigger();
-  // All that does not depend on the input comes before the wait: the kernel is resident while the one in front still runs, and what
-  // follows the wait is the chain that a decode step is made of.
+  // All that does not depend on the input comes before the wait: behind a kernel that releases its dependents early, as this
+  // library's do, this one is resident while that one still runs, and what follows the wait is the chain that a decode step is made
+  // of.  Behind one that does not (an engine's norm or attention) there is no wait to hide work in: over 110 layers of up to 128
+  // tokens calls became 13 % faster back to back with all changes of that time, and 5 % behind an elementwise kernel of torch.
   const int kblocks = k >> 7;
   const int64_t real = int64_t(rows) * kblocks * 16;
   const int64_t tid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -193,7 +195,8 @@ mx_quant_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint
   const uint16_t* const src = in + int64_t(row) * (SILU ? 2 * k : k) + col;
   void* const to = out + (int64_t(row) * k + col) / (FP4 ? 2 : 1);
   uint32_t* const scale_word = reinterpret_cast<uint32_t*>(sf + scale_word_offset(row, kb, k));
-  // Usually the previous kernel's output, and in L2; where it is older it comes in during the wait.
+  // The previous kernel's output is in L2, and the prefetch does nothing; an older input comes in during the wait.  Layer calls on old
+  // inputs take 0.2 % longer without it on average (23 shapes), behind a kernel that writes the input the same.
   asm volatile("prefetch.global.L2 [%0];" ::"l"(src) : "memory");
   if constexpr (SILU) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + k) : "memory");
   pdl_wait();
