@@ -204,15 +204,6 @@ class Sweep:
             self.host[m] = {"x_qkv": x[0].contiguous().pin_memory(), "x_gate": x[2].contiguous().pin_memory(),
                             "x_o": x[1][:, :k_o].contiguous().pin_memory()}
             self.dev[m] = {n: t.to(device) for n, t in self.host[m].items()}
-        # quantiser launches per M (one SwiGLU-quantiser; three activation quantisers unless they are fused
-        # into the GEMM launch) plus the GEMM launches (a GEMM whose cut tiles are summed by the separate
-        # reduce kernel counts two)
-        def quantisers(i, m):
-            separate = [name for name in ("qkv", "o_proj", "gate_up")
-                        if m > native.FUSED_QUANT_TOKENS or self.layer_for(i)[name].outputs > native.FUSED_QUANT_MAX_OUTPUTS]
-            return 1 + len(separate)
-        self.launches_per_step = sum(quantisers(i, m) + sum(launches_of(self.layer_for(i)[name], m) for name in SHAPES)
-                                     for i, m in enumerate(M_SWEEP))
         self.event_factory = lambda: torch.cuda.Event(enable_timing=True)
         # Row-parallel layers under tensor parallelism: the GEMM writes its partial sums into a peer-mapped
         # buffer and a second launch pulls every rank's partials over NVLink and sums them
@@ -222,11 +213,26 @@ class Sweep:
             try:
                 from hygemm_vllm import tp
                 self.exchange = tp.PeerExchange(group, max(M_SWEEP) * HIDDEN, torch.bfloat16, device)
-                self.launches_per_step += 2 * len(M_SWEEP)
                 self.exchange_note = self.verify_exchange()
             except Exception as exc:     # no peer access between these GPUs, or symmetric memory unavailable
                 self.exchange = None
                 self.exchange_note = f"NCCL all-reduce ({type(exc).__name__}: {exc})"[:200]
+
+    def launches_per_step(self, captured):
+        """This library's launches in one step: a SwiGLU-quantiser per M, an activation quantiser wherever it does not run inside the
+        GEMM launch (`layer(x)` quantises there up to 16 tokens, in a captured call for one token only; the exchange up to 16
+        always), the GEMMs (two where cut tiles are summed by the reduce kernel) and two all-reduces per M under the exchange."""
+        most = min(self.native.FUSED_QUANT_TOKENS, 1) if captured else self.native.FUSED_QUANT_TOKENS
+        total = 0
+        for i, m in enumerate(M_SWEEP):
+            layer = self.layer_for(i)
+            total += 1 + sum(launches_of(layer[name], m) for name in SHAPES)
+            for name in ("qkv", "o_proj", "gate_up"):
+                exchanged = name == "o_proj" and self.exchange is not None
+                total += m > (self.native.FUSED_QUANT_TOKENS if exchanged else most) or (
+                    not exchanged and layer[name].outputs > self.native.FUSED_QUANT_MAX_OUTPUTS)
+            total += 2 * (self.exchange is not None)
+        return total
 
     def verify_exchange(self):
         """The fused exchange against GEMM + NCCL all-reduce on the same inputs, once, before timing."""
@@ -263,8 +269,9 @@ class Sweep:
             events.append((name, m, a, b))
             return y
 
-        # What `layer(x)` (the plugin-facing call) does: up to 16 tokens the activations are quantised inside
-        # the GEMM launch (hg_run_x); above that the quantiser is its own launch.  Events bracket the GEMM launch.
+        # What `layer(x)` (the plugin-facing call) does: the activations are quantised inside the GEMM launch (hg_run_x) up to
+        # 16 tokens in eager calls and for one token in captured ones; else the quantiser is its own launch.  Events bracket
+        # the GEMM launch, from 2 to 16 captured tokens with the quantiser in front of it.
         def linear(name, xin, row_parallel=False):
             rt = layer[name]
             if row_parallel and self.exchange is not None:
@@ -891,7 +898,7 @@ def main():
             "config": {"workload": "Qwen2.5-7B layer-shape hybrid GEMM sweep: qkv 3584->4608, o_proj 3584->3584, "
                                    "gate_up 3584->37888, down 18944->3584; M in 1,2,4,8,16,32,64,128; 10% MXFP8 channels",
                        "step": "per M: quantise+qkv, quantise+o_proj, quantise+gate_up, SwiGLU-quantise+down "
-                               "(M<=16: the three activation quantisers run inside their GEMM launch)",
+                               "(M=1, captured: the quantisers of qkv and o_proj run inside their GEMM launch)",
                        "parallelism": f"tp{world}" if world > 1 else "single GPU",
                        **({"row_parallel_sum": sweep.exchange_note} if world > 1 else {}),
                        "l2": "inputs larger than L2: two weight sets (272 MB) alternate between consecutive M",
@@ -900,7 +907,7 @@ def main():
                     "ms_per_step": e2e_ms / e2e_steps, "steps": e2e_steps, "api": e2e_api,
                     "eager_value": flops_step * e2e_steps / (e2e_eager_ms * 1e-3) / 1e12,
                     "eager_ms_per_step": e2e_eager_ms / e2e_steps},
-            "gpu_launches": sweep.launches_per_step * args.steps,
+            "gpu_launches": sweep.launches_per_step(graph is not None) * args.steps,
             "clocks": clocks,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                          "frac": achieved / hbm_peak,
