@@ -146,6 +146,10 @@ template <> __device__ __forceinline__ uint16_t from_float<__nv_bfloat16>(float 
 // Pairs of 16-bit values in a word.
 template <typename T> struct Packed;
 template <> struct Packed<__half> {
+  static __device__ __forceinline__ uint32_t min(uint32_t a, uint32_t b) {   // skips NaNs
+    const __half2 m = __hmin2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&m);
+  }
   static __device__ __forceinline__ uint32_t max_abs(uint32_t a, uint32_t b) {   // a is a maximum already
     const __half2 m = __hmax2(*reinterpret_cast<const __half2*>(&a), __habs2(*reinterpret_cast<const __half2*>(&b)));
     return *reinterpret_cast<const uint32_t*>(&m);
@@ -157,6 +161,10 @@ template <> struct Packed<__half> {
   }
 };
 template <> struct Packed<__nv_bfloat16> {
+  static __device__ __forceinline__ uint32_t min(uint32_t a, uint32_t b) {   // skips NaNs
+    const __nv_bfloat162 m = __hmin2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&m);
+  }
   static __device__ __forceinline__ uint32_t max_abs(uint32_t a, uint32_t b) {
     const __nv_bfloat162 m = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a), __habs2(*reinterpret_cast<const __nv_bfloat162*>(&b)));
     return *reinterpret_cast<const uint32_t*>(&m);

@@ -137,29 +137,63 @@ __device__ __forceinline__ float reciprocal_fast(float x) { float r; asm("rcp.ap
 // 2 N SwiGLU products by approximate exponentials and reciprocals, bit for bit silu8's.
 //
 // The gate's activation is rounded to 16 bits, so an fp32 value that is only nearly silu8's gives the same bits unless a
-// rounding boundary lies in between.  Pairs with a value within kDoubt fp32 units of one are computed as in silu8: over all
-// gates of both types down to -16 the two differ by at most 13 units.  So are gates below -16, where the error of the
-// exponent's argument grows, and fp16 activations below the normal range, whose boundaries lie elsewhere.  up + 0 and the
-// product are rounded once in the 16-bit type, as they are in fp32: a product of two fp16 values is exact in fp32, one of two
-// bf16 values down to 2^-126 (the caller leaves values near that to silu8).
-constexpr uint32_t kDoubt = 20;
+// rounding boundary lies in between.  Pairs with a value near one are computed as in silu8: over all gates of both types the two
+// differ by at most 8 fp32 units down to -6 and 13 down to -16 (the error of the exponent's argument grows with it), and lanes
+// whose gates all lie above -6 take a window of 10 units instead of 20.  So are gates below -16, and fp16 activations below the
+// normal range, whose boundaries lie elsewhere.  up + 0 and the product are rounded once in the 16-bit type, as they are in fp32: a
+// product of two fp16 values is exact in fp32, one of two bf16 values down to 2^-126 (the caller leaves values near that to silu8).
+//
+// Doubtful pairs are collected and computed one after the other at the end, all lanes' first ones together: a warp takes the exact
+// functions once or twice for its 32 x 2 N values, and not up to N times (fp16: of sixteen pairs of a warp four had a value in
+// doubt).
+constexpr uint32_t kDoubt = 20, kDoubtNear = 10;
+constexpr float kNearGate = -6.f;
 template <typename T, int N>
 __device__ __forceinline__ void silu_fast(const uint32_t (&gate)[N], const uint32_t (&up)[N], uint32_t (&product)[N]) {
   constexpr bool kHalf = std::is_same<T, __half>::value;
   constexpr int kShift = kHalf ? 19 : 16;                        // brings the bits below the 16-bit mantissa to the top
-  constexpr uint32_t kBoundary = 0x80000000u - (kDoubt << kShift), kWindow = 2 * kDoubt << kShift;
+  uint32_t least = gate[0];
+#pragma unroll
+  for (int i = 1; i < N; ++i) least = Packed<T>::min(least, gate[i]);
+  const float2 ends = Packed<T>::widen(least);
+  const float lowest = fminf(ends.x, ends.y);
+  const uint32_t window = (lowest < kNearGate ? kDoubt : kDoubtNear) << kShift, boundary = 0x80000000u - window;
+  uint32_t doubtful = 0;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     const float2 g = Packed<T>::widen(gate[i]);
     const float2 t = mul2(g, make_float2(-1.44269504f, -1.44269504f));
     const float2 s = add2(make_float2(exp2_fast(t.x), exp2_fast(t.y)), make_float2(1.f, 1.f));
-    float2 act = mul2(g, make_float2(reciprocal_fast(s.x), reciprocal_fast(s.y)));
-    const uint32_t x = __float_as_uint(act.x) * (1u << kShift) - kBoundary, y = __float_as_uint(act.y) * (1u << kShift) - kBoundary;
-    bool doubtful = min(x, y) <= kWindow || fminf(g.x, g.y) < -16.f;
-    if constexpr (kHalf)
-      doubtful |= (fabsf(act.x) < 6.103515625e-05f && g.x != 0.f) || (fabsf(act.y) < 6.103515625e-05f && g.y != 0.f);
-    if (__builtin_expect(doubtful, 0)) act = make_float2(g.x / (1.f + expf(-g.x)), g.y / (1.f + expf(-g.y)));
+    const float2 act = mul2(g, make_float2(reciprocal_fast(s.x), reciprocal_fast(s.y)));
+    const uint32_t x = __float_as_uint(act.x) * (1u << kShift) - boundary, y = __float_as_uint(act.y) * (1u << kShift) - boundary;
+    bool doubt = min(x, y) <= 2 * window;
+    if constexpr (kHalf)   // below 2^-14; zeros, which are exact, wrap round
+      doubt |= min((__float_as_uint(act.x) & 0x7fffffffu) - 1u, (__float_as_uint(act.y) & 0x7fffffffu) - 1u) < 0x38800000u - 1u;
+    if (doubt) doubtful |= 1u << i;
     product[i] = Packed<T>::swiglu(act, up[i]);
+  }
+  if (__builtin_expect(doubtful != 0 || lowest < -16.f, 0)) {
+    if (lowest < -16.f) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const float2 g = Packed<T>::widen(gate[i]);
+        if (fminf(g.x, g.y) < -16.f) doubtful |= 1u << i;
+      }
+    }
+#pragma unroll 1
+    while (doubtful) {
+      const int at = __ffs(int(doubtful)) - 1;
+      doubtful &= doubtful - 1;
+      uint32_t gate_at = gate[0], up_at = up[0];
+#pragma unroll
+      for (int i = 1; i < N; ++i)
+        if (i == at) { gate_at = gate[i]; up_at = up[i]; }
+      const float2 g = Packed<T>::widen(gate_at);
+      const uint32_t exact = Packed<T>::swiglu(make_float2(g.x / (1.f + expf(-g.x)), g.y / (1.f + expf(-g.y))), up_at);
+#pragma unroll
+      for (int i = 0; i < N; ++i)
+        if (i == at) product[i] = exact;
+    }
   }
 }
 
@@ -301,8 +335,9 @@ __device__ __forceinline__ uint32_t quantise16(const Raw16& x, uint8_t* codes, i
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const float2 pair = Packed<T>::widen(x.w[i]);
-      v[2 * i] = pair.x * inv;
-      v[2 * i + 1] = pair.y * inv;
+      const float2 scaled = mul2(pair, make_float2(inv, inv));
+      v[2 * i] = scaled.x;
+      v[2 * i + 1] = scaled.y;
     }
     if constexpr (FP4) {
       const float (&low)[8] = *reinterpret_cast<const float (*)[8]>(v), (&high)[8] = *reinterpret_cast<const float (*)[8]>(v + 8);
@@ -412,10 +447,10 @@ __device__ __forceinline__ void silu16(const Raw16& gate, const Raw16& up, Raw16
   }
 }
 
-// SwiGLU + MXFP8 for many rows; bound by instruction issue (27 per value, 39 with silu8 throughout), at 2048 x 18944 bf16 57 % of
-// the memory bandwidth: 60 -> 44 us, at 777 rows 23.4 -> 19.0 us.
+// SwiGLU + MXFP8 for many rows; bound by instruction issue.  2048 x 18944 bf16 44.8 us (62 % of the memory bandwidth; 46.2 with the
+// exact functions at every pair in doubt and four blocks to an SM), 777 rows 19.2 us (21.7), 60 with silu8 throughout at 2048.
 template <typename T, int MATH>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(256, 3)
 mx_silu_rows_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint8_t* __restrict__ sf, uint16_t* __restrict__ debug, int rows, int k) {
   pdl_trigger();
   const int lane = threadIdx.x & 31, chunks = (k + 511) >> 9;

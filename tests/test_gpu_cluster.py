@@ -261,3 +261,21 @@ def test_swiglu_of_every_gate_value(dtype):
         q, sf = producer.silu_pack(part, 0)
         exact_q, exact_sf, _ = producer.silu_pack(part, 0, debug=True)
         assert torch.equal(q, exact_q) and torch.equal(sf, exact_sf)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_swiglu_of_every_gate_from_minus_six_on(dtype):
+    """Lanes whose gates all lie above -6 take the narrower window around rounding boundaries: every such gate, infinity too, beside none
+    below, each with eight values of up, gives the bytes of the exact functions (whole values: tolerance 0)."""
+    k = 1024
+    every = torch.arange(65536, device="cuda").to(torch.int16).view(dtype)
+    gate = every[every >= -6].repeat(8)
+    gate = torch.cat([gate, gate[:-gate.numel() % k]])
+    g = torch.Generator(device="cuda").manual_seed(12)
+    gate = gate[torch.randperm(gate.numel(), device="cuda", generator=g)].view(-1, k)
+    x = torch.cat([gate, torch.randn(gate.shape, device="cuda", generator=g).to(dtype)], 1).contiguous()
+    many = x.repeat(-(-8200 // x.shape[0]), 1)   # the many-rows producer starts at 8 Mi elements
+    for part in (x[:256].contiguous(), x[256:].contiguous(), many):
+        q, sf = producer.silu_pack(part, 0)
+        exact_q, exact_sf, _ = producer.silu_pack(part, 0, debug=True)
+        assert torch.equal(q, exact_q) and torch.equal(sf, exact_sf)
