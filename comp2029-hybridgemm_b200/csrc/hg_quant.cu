@@ -354,29 +354,24 @@ __device__ __forceinline__ uint32_t quantise16(const Raw16& x, uint8_t* codes, i
   return word | __shfl_xor_sync(0xffffffffu, word, 4);
 }
 
-// Source rows of packed rows 128 (group / 32) + group % 32 + 32 r; -1: none.
-__device__ __forceinline__ void find_rows(int (&source)[4], const QuantPart& part, int group) {
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int row = (group >> 5) * 128 + (group & 31) + 32 * r;
-    source[r] = -1;
-    if (row < part.rows) {
-      const int s = part.ids ? __ldg(part.ids + row) : row;
-      // a list is incomplete, its entries undefined, when ids were repeated or out of range
-      if (uint32_t(s) < uint32_t(part.sources)) source[r] = s;
-    }
-  }
+// Source row of packed row 128 (group / 32) + group % 32 + 32 lane (lanes 0 to 3); -1: none.
+__device__ __forceinline__ int find_row(const QuantPart& part, int group, int lane) {
+  const int row = (group >> 5) * 128 + (group & 31) + 32 * lane;
+  if (lane >= 4 || row >= part.rows) return -1;
+  const int s = part.ids ? __ldg(part.ids + row) : row;
+  // a list is incomplete, its entries undefined, when ids were repeated or out of range
+  return uint32_t(s) < uint32_t(part.sources) ? s : -1;
 }
-// Columns col .. col + 15 of this lane.
-__device__ __forceinline__ void load_rows(Raw16 (&raw)[4], const int (&source)[4], const uint16_t* __restrict__ in, int col, int k) {
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    raw[r] = Raw16{};
-    if (source[r] >= 0 && col < k) raw[r] = load16(in + int64_t(source[r]) * k + col);
-  }
+// Columns col .. col + 15 of this lane in row r of the group whose source rows lanes 0 to 3 hold.
+__device__ __forceinline__ Raw16 load_row(int sources, int r, const uint16_t* __restrict__ in, int col, int k) {
+  const int source = __shfl_sync(0xffffffffu, sources, r);
+  Raw16 raw{};
+  if (source >= 0 && col < k) raw = load16(in + int64_t(source) * k + col);
+  return raw;
 }
+// Converts a group's four rows; each makes room for the same row of the next item.
 template <typename T, bool FP4>
-__device__ __forceinline__ void emit_rows(const Raw16 (&raw)[4], const QuantPart& part, int group, int col, int k, int lane) {
+__device__ __forceinline__ void emit_rows(Raw16 (&raw)[4], const QuantPart& part, int group, int col, int k, int lane, int sources, const uint16_t* __restrict__ in, int next_col) {
   const int row0 = (group >> 5) * 128 + (group & 31);
   uint32_t word[4];
 #pragma unroll
@@ -387,6 +382,7 @@ __device__ __forceinline__ void emit_rows(const Raw16 (&raw)[4], const QuantPart
       const int64_t at = int64_t(row) * k + col;
       word[r] = quantise16<T, FP4>(raw[r], col < k ? part.codes + (FP4 ? at >> 1 : at) : nullptr, lane);
     }
+    raw[r] = load_row(sources, r, in, next_col, k);
   }
   if (col < k && (lane & 7) == 0)
     *reinterpret_cast<uint4*>(part.sf + scale_word_offset(row0, col >> 7, k)) = make_uint4(word[0], word[1], word[2], word[3]);
@@ -400,38 +396,39 @@ __device__ __forceinline__ int2 list_verdict(const int32_t* hi, int n_ids) {
   return last >= 0 ? make_int2(n_ids, 0) : make_int2((-1 - last) >> 1, (-1 - last) & 1);
 }
 
-// Packs `low` to MXFP4 and `high` to MXFP8 (either may be empty).  Every warp walks items of one row group x 512 columns and has
-// the next item's loads in flight while it converts the current one (37888 x 3584 to MXFP4 56 us, 67 without).  Row numbers
-// another item ahead cost more in registers than their latency.  `verdict`: where to tell the host about the lists, or null.
+// Packs `low` to MXFP4 and `high` to MXFP8 (either may be empty).  Every warp walks items of one row group x 512 columns.  A row
+// that has been converted makes room for the same row of the next item, and the numbers of that item's rows have been under way
+// since the item before: a load that has to wait for a row number takes two latencies, and with those of the next item's rows
+// asked for together with the rows a layer of 37888 x 3584 took 105.9 us to pack instead of 93.4 (whole call; two sets of four
+// rows in registers).  A fourth block per SM gives nothing (94.5), a fifth spills (108).  `verdict`: where to tell the host about
+// the lists, or null.
 template <typename T>
 __global__ void __launch_bounds__(256, kRowsBlocks)
 mx_rows_kernel(const uint16_t* __restrict__ in, const QuantPart low, const QuantPart high, int k, int* __restrict__ verdict) {
   pdl_trigger();
   const int lane = threadIdx.x & 31, chunks = (k + 511) >> 9;
   const int low_groups = ((low.rows + 127) & ~127) >> 2, groups = low_groups + (((high.rows + 127) & ~127) >> 2);
-  const int stride = gridDim.x * 8;
-  int item = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int stride = gridDim.x * 8, item = blockIdx.x * 8 + (threadIdx.x >> 5);
   int group = item / chunks, col = ((item - group * chunks) << 9) + 16 * lane;
   pdl_wait();   // input and row lists come from the kernels before
   if (verdict && blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<int2*>(verdict) = list_verdict(high.ids, high.rows);
-  Raw16 raw[4], next[4];
-  auto load = [&](Raw16 (&to)[4]) {
-    int source[4];
-    if (group < low_groups) find_rows(source, low, group);
-    else find_rows(source, high, group - low_groups);
-    load_rows(to, source, in, col, k);
-  };
-  if (group < groups) load(raw);
-  while (group < groups) {
-    const int this_group = group, this_col = col;
-    item += stride;
-    group = item / chunks;
-    col = ((item - group * chunks) << 9) + 16 * lane;
-    if (group < groups) load(next);
-    if (this_group < low_groups) emit_rows<T, true>(raw, low, this_group, this_col, k, lane);
-    else emit_rows<T, false>(raw, high, this_group - low_groups, this_col, k, lane);
+  if (group >= groups) return;
+  auto rows_of = [&](int g) { return g < low_groups ? find_row(low, g, lane) : g < groups ? find_row(high, g - low_groups, lane) : -1; };
+  Raw16 raw[4];
+  int sources = rows_of(group);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) raw[r] = next[r];
+  for (int r = 0; r < 4; ++r) raw[r] = load_row(sources, r, in, col, k);
+  int ahead = item + stride;
+  sources = rows_of(ahead / chunks);
+  while (group < groups) {
+    const int next_group = ahead / chunks, next_col = ((ahead - next_group * chunks) << 9) + 16 * lane;
+    ahead += stride;
+    const int after = rows_of(ahead / chunks);
+    if (group < low_groups) emit_rows<T, true>(raw, low, group, col, k, lane, sources, in, next_col);
+    else emit_rows<T, false>(raw, high, group - low_groups, col, k, lane, sources, in, next_col);
+    group = next_group;
+    col = next_col;
+    sources = after;
   }
 }
 
@@ -537,10 +534,16 @@ partition_rows_kernel(const int64_t* __restrict__ ids, int n_ids, int rows, int3
   __syncthreads();
   pdl_wait();
   int bad = 0;
-  for (int i = tid; i < n_ids; i += kPartitionThreads) {
-    const int64_t id = ids[i];
-    if (id < 0 || id >= rows) bad = 1;
-    else atomicOr(bitmap + (id >> 5), 1u << (id & 31));
+  for (int first = tid; first < n_ids; first += 4 * kPartitionThreads) {   // four loads under way at once
+    int64_t id[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) id[j] = first + j * kPartitionThreads < n_ids ? ids[first + j * kPartitionThreads] : 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (first + j * kPartitionThreads >= n_ids) continue;
+      if (id[j] < 0 || id[j] >= rows) bad = 1;
+      else atomicOr(bitmap + (id[j] >> 5), 1u << (id[j] & 31));
+    }
   }
   bad = __syncthreads_or(bad);
   const int per = (words + kPartitionThreads - 1) / kPartitionThreads, begin = min(words, tid * per), end = min(words, begin + per);
@@ -570,10 +573,11 @@ partition_rows_kernel(const int64_t* __restrict__ ids, int n_ids, int rows, int3
     running += __popc(bitmap[w]);
   }
   __syncthreads();
+#pragma unroll 4
   for (int w = tid >> 5; w < words; w += kPartitionThreads / 32) {
     const uint32_t bits = bitmap[w];
     const int row = w * 32 + lane, high = before[w] + __popc(bits & ((1u << lane) - 1u));
-    if (row >= rows) break;
+    if (row >= rows) continue;
     if ((bits >> lane) & 1u) {
       if (high < n_ids) hi[high] = row;
     } else if (row - high < rows - n_ids) {
