@@ -218,19 +218,17 @@ class Sweep:
                 self.exchange = None
                 self.exchange_note = f"NCCL all-reduce ({type(exc).__name__}: {exc})"[:200]
 
-    def launches_per_step(self, captured):
+    def launches_per_step(self):
         """This library's launches in one step: a SwiGLU-quantiser per M, an activation quantiser wherever it does not run inside the
-        GEMM launch (`layer(x)` quantises there up to 16 tokens, in a captured call for one token only; the exchange up to 16
-        always), the GEMMs (two where cut tiles are summed by the reduce kernel) and two all-reduces per M under the exchange."""
-        most = min(self.native.FUSED_QUANT_TOKENS, 1) if captured else self.native.FUSED_QUANT_TOKENS
+        GEMM launch (see `native.quantises_in_gemm`; under the exchange o_proj does up to 16 tokens), the GEMMs (two where cut tiles
+        are summed by the reduce kernel) and two all-reduces per M under the exchange."""
         total = 0
         for i, m in enumerate(M_SWEEP):
             layer = self.layer_for(i)
             total += 1 + sum(launches_of(layer[name], m) for name in SHAPES)
             for name in ("qkv", "o_proj", "gate_up"):
                 exchanged = name == "o_proj" and self.exchange is not None
-                total += m > (self.native.FUSED_QUANT_TOKENS if exchanged else most) or (
-                    not exchanged and layer[name].outputs > self.native.FUSED_QUANT_MAX_OUTPUTS)
+                total += m > self.native.FUSED_QUANT_TOKENS if exchanged else not self.native.quantises_in_gemm(m, layer[name].outputs)
             total += 2 * (self.exchange is not None)
         return total
 
@@ -270,8 +268,7 @@ class Sweep:
             return y
 
         # What `layer(x)` (the plugin-facing call) does: the activations are quantised inside the GEMM launch (hg_run_x) up to
-        # 16 tokens in eager calls and for one token in captured ones; else the quantiser is its own launch.  Events bracket
-        # the GEMM launch, from 2 to 16 captured tokens with the quantiser in front of it.
+        # 16 tokens, in wide layers up to 8; else the quantiser is its own launch.  Events bracket the GEMM launch.
         def linear(name, xin, row_parallel=False):
             rt = layer[name]
             if row_parallel and self.exchange is not None:
@@ -279,7 +276,7 @@ class Sweep:
                     return timed(name, lambda: rt.run_exchange(self.exchange, x=xin))
                 q, sf = native.pack(xin)
                 return timed(name, lambda: rt.run_exchange(self.exchange, q=q, sf=sf))
-            if m <= native.FUSED_QUANT_TOKENS and rt.outputs <= native.FUSED_QUANT_MAX_OUTPUTS:
+            if native.quantises_in_gemm(m, rt.outputs):
                 return timed(name, lambda: rt(xin))
             q, sf = native.pack(xin)
             return timed(name, lambda: rt.run_packed(q, sf))
@@ -898,7 +895,7 @@ def main():
             "config": {"workload": "Qwen2.5-7B layer-shape hybrid GEMM sweep: qkv 3584->4608, o_proj 3584->3584, "
                                    "gate_up 3584->37888, down 18944->3584; M in 1,2,4,8,16,32,64,128; 10% MXFP8 channels",
                        "step": "per M: quantise+qkv, quantise+o_proj, quantise+gate_up, SwiGLU-quantise+down "
-                               "(M=1, captured: the quantisers of qkv and o_proj run inside their GEMM launch)",
+                               "(the quantisers run inside the GEMM launch up to M=16, gate_up's up to M=8)",
                        "parallelism": f"tp{world}" if world > 1 else "single GPU",
                        **({"row_parallel_sum": sweep.exchange_note} if world > 1 else {}),
                        "l2": "inputs larger than L2: two weight sets (272 MB) alternate between consecutive M",
@@ -907,7 +904,7 @@ def main():
                     "ms_per_step": e2e_ms / e2e_steps, "steps": e2e_steps, "api": e2e_api,
                     "eager_value": flops_step * e2e_steps / (e2e_eager_ms * 1e-3) / 1e12,
                     "eager_ms_per_step": e2e_eager_ms / e2e_steps},
-            "gpu_launches": sweep.launches_per_step(graph is not None) * args.steps,
+            "gpu_launches": sweep.launches_per_step() * args.steps,
             "clocks": clocks,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                          "frac": achieved / hbm_peak,

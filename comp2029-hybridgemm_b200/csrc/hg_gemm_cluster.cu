@@ -19,7 +19,7 @@
 // Roles per CTA: warp 0 weights and their scales (TMA), warp 1 MMA issue (idle in the second CTA of a pair, whose copies
 // complete on the first CTA's barriers: reporting every stage with a remote arrive cost 750 cycles each), then epilogue warps
 // (four; in pairs eight, two per TMEM quarter on alternate groups of sixteen columns), then one warp for the activations and
-// their scales (TMA) or, FUSED, four warps that quantise the activations.
+// their scales (TMA) or, FUSED, eight warps that quantise the activations.
 // One warp per scheduler runs most of these roles alone, so a dependent instruction costs about five cycles and nothing
 // hides it: loops here carry no divisions, addresses are independent of each other, and descriptors are sums.
 // Every mbarrier wait is bounded; on expiry the CTA records a code, drains and leaves.
@@ -37,9 +37,11 @@ namespace hg {
 
 namespace {
 
+constexpr int kClusterQuantThreads = 256;   // activation quantisers: sixteen per token and K256 step
+constexpr int kQuantAhead = 4;              // steps whose activations a quantiser has in registers or on the way
 __host__ __device__ constexpr int epilogue_sides(int pair) { return pair == 2 ? 2 : 1; }
 __host__ __device__ constexpr int first_act_warp(int pair) { return 2 + 4 * epilogue_sides(pair); }
-__host__ __device__ constexpr int cluster_threads(int pair, bool fused) { return first_act_warp(pair) * 32 + (fused ? kQuantThreads : 32); }
+__host__ __device__ constexpr int cluster_threads(int pair, bool fused) { return first_act_warp(pair) * 32 + (fused ? kClusterQuantThreads : 32); }
 constexpr int kClusterMaxStages = 12;
 constexpr int kMaxSmem = 232448;
 constexpr uint32_t kScaleStride = 16;                           // TMEM columns per scale set: weights 4, activations up to 8
@@ -277,7 +279,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.tail)) : "memory");
     }
     for (int s = 0; s < p.stages; ++s) {
-      mbar_init(full_bar(s), 1 + (FUSED ? kQuantThreads / 32 : 1));   // weights; activations or the quantiser warps
+      mbar_init(full_bar(s), 1 + (FUSED ? kClusterQuantThreads / 32 : 1));   // weights; activations or the quantiser warps
       mbar_init(empty_bar(s), 1);
     }
     for (int s = 0; s < 2; ++s) {
@@ -384,65 +386,71 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
     }
   } else if (FUSED && warp >= kActWarp) {
     // ------------------------------------------------------------------ activation quantisers
-    // Thread tq owns one K32 group (tq % 8) of token tq / 8 in each K256 step, with the arithmetic of mx_quant_kernel:
-    // codes and scales are the bytes hg_pack would have produced.  The next step's 64 bytes are requested before the
-    // current ones are converted.
+    // Two neighbouring threads own one K32 group of one token in each K256 step, with the arithmetic of mx_quant_kernel: codes and
+    // scales are the bytes hg_pack would have produced.  What bounds this is latency, of the loads above all, so a thread has
+    // the next kQuantAhead steps' values on the way.  With 128 threads of 32 values each and one step ahead a block of
+    // Qwen2.5-7B took longer in captured calls than with a quantiser in front from two tokens on; now it does not up to sixteen
+    // (8 tokens 40.7 us with separate quantisers, 40.4 with qkv and o_proj quantised here, 39.1 with gate_up too).
     if constexpr (FUSED) {
       const int tq = threadIdx.x - kActWarp * 32;
-      const int token = tq >> 3, blk = (tq & 7) >> 2, g = tq & 3;
-      const uint16_t* x_row = p.x + int64_t(token) * p.k + blk * 128 + g * 32;
-      auto load_x = [&](int kb, uint4 (&r)[4]) {
-        if (kb + blk < p.kblocks && token < p.tokens) {
-          const uint4* src = reinterpret_cast<const uint4*>(x_row + int64_t(kb) * 128);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) r[c] = src[c];
-        } else {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) r[c] = make_uint4(0u, 0u, 0u, 0u);
+      const int token = tq >> 4, blk = (tq >> 3) & 1, g = (tq >> 1) & 3, part = tq & 1;
+      const int steps = cluster < units ? step_end - step_begin : 0;
+      const int mine = token < p.tokens ? min(steps, ((p.kblocks - blk + 1) >> 1) - step_begin) : 0;   // steps that have this block
+      const char* const x_at = reinterpret_cast<const char*>(p.x + int64_t(token) * p.k + int64_t(step_begin) * 256 + (tq & 15) * 16);
+      const uint32_t codes_at = base + lay.b + uint32_t(blk) * lay.b_tile + uint32_t(token) * 128u + ((uint32_t(2 * g + part) ^ uint32_t(token & 7)) << 4);
+      const uint32_t scale_at = base + lay.sfb + uint32_t(blk) * 512u + uint32_t(token) * 16u + uint32_t(g);
+      struct Values { uint4 low, high; } ahead[kQuantAhead];
+      auto load_x = [&](int step, Values& to) {
+        to.low = to.high = make_uint4(0u, 0u, 0u, 0u);
+        if (step < mine) {
+          const uint4* const src = reinterpret_cast<const uint4*>(x_at + step * 512);
+          to.low = src[0];
+          to.high = src[1];
         }
       };
-      uint4 cur[4], nxt[4];
+      auto quantise = [&](const Values& x, uint32_t (&codes)[4], auto type) {   // returns the scale byte
+        using X = decltype(type);
+        const uint32_t word[8] = {x.low.x, x.low.y, x.low.z, x.low.w, x.high.x, x.high.y, x.high.z, x.high.w};
+        uint32_t top = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) top = Packed<X>::max_abs(top, word[i]);
+        top = Packed<X>::max_abs(top, __shfl_xor_sync(0xffffffffu, top, 1));
+        const float2 ends = Packed<X>::widen(top);
+        const int e = mx_exponent<false>(fmaxf(fmaxf(0.f, ends.x), ends.y));
+        const float inv = mx_inverse_scale(e);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 a = Packed<X>::widen(word[2 * i]), b = Packed<X>::widen(word[2 * i + 1]);
+          codes[i] = cvt_e4m3x2(a.x * inv, a.y * inv) | (cvt_e4m3x2(b.x * inv, b.y * inv) << 16);
+        }
+        return uint32_t(e + 127);
+      };
+      // An input that no kernel has just written comes into L2 during the wait.
+      for (int i = 0; i < mine; ++i) asm volatile("prefetch.global.L2 [%0];" ::"l"(x_at + i * 512) : "memory");
       int stage = 0;
       uint32_t phase = 1;
       pdl_wait();   // x is the previous kernel's output
-      if (cluster < units) load_x(2 * step_begin, cur);
       for (int u = cluster; u < units && !error; u += p.clusters) {
-        for (int step = step_begin; step < step_end; ++step) {
-          load_x(step + 1 < step_end ? 2 * step + 2 : 2 * step_begin, nxt);
-          if (!warp_wait(empty_bar(stage), phase, abort_flag)) { error = kErrLoader; break; }
-          if (2 * step + blk < p.kblocks && token < p.tokens) {   // columns of tokens that are not there are never stored
-            const uint32_t row_base = base + lay.b + uint32_t(2 * stage + blk) * lay.b_tile + uint32_t(token) * 128u;
-            const uint32_t sw = uint32_t(token & 7);
-            float v[32];
-            float amax = 0.f;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const uint32_t word[4] = {cur[c].x, cur[c].y, cur[c].z, cur[c].w};
+        for (int i = 0; i < kQuantAhead; ++i) load_x(i, ahead[i]);
+        for (int first = 0; first < steps && !error; first += kQuantAhead) {
 #pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                const uint16_t bits = uint16_t(word[i >> 1] >> ((i & 1) * 16));
-                v[c * 8 + i] = p.x_bf16 ? to_float<__nv_bfloat16>(bits) : to_float<__half>(bits);
-                amax = fmaxf(amax, fabsf(v[c * 8 + i]));
-              }
+          for (int i = 0; i < kQuantAhead; ++i) {
+            const int step = first + i;
+            if (step >= steps || error) break;
+            uint32_t codes[4];
+            const uint32_t scale = p.x_bf16 ? quantise(ahead[i], codes, __nv_bfloat16()) : quantise(ahead[i], codes, __half());
+            load_x(step + kQuantAhead, ahead[i]);
+            if (!warp_wait(empty_bar(stage), phase, abort_flag)) { error = kErrLoader; break; }
+            if (step < mine) {   // columns of tokens that are not there are never stored
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(codes_at + uint32_t(2 * stage) * lay.b_tile),
+                           "r"(codes[0]), "r"(codes[1]), "r"(codes[2]), "r"(codes[3]) : "memory");
+              if (part == 0) asm volatile("st.shared.u8 [%0], %1;" ::"r"(scale_at + uint32_t(stage) * lay.sfb_stage), "r"(scale) : "memory");
             }
-            const int e = mx_exponent<false>(amax);
-            const float inv = mx_inverse_scale(e);
-            uint32_t codes[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-              codes[i] = cvt_e4m3x2(v[4 * i] * inv, v[4 * i + 1] * inv) | (cvt_e4m3x2(v[4 * i + 2] * inv, v[4 * i + 3] * inv) << 16);
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_base + ((uint32_t(2 * g) ^ sw) << 4)),
-                         "r"(codes[0]), "r"(codes[1]), "r"(codes[2]), "r"(codes[3]) : "memory");
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_base + ((uint32_t(2 * g + 1) ^ sw) << 4)),
-                         "r"(codes[4]), "r"(codes[5]), "r"(codes[6]), "r"(codes[7]) : "memory");
-            asm volatile("st.shared.u8 [%0], %1;" ::"r"(base + lay.sfb + uint32_t(stage) * lay.sfb_stage + uint32_t(blk) * 512u + uint32_t(token & 31) * 16u + uint32_t(g)),
-                         "r"(uint32_t(e + 127)) : "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full_bar(stage));
+            if (++stage == p.stages) { stage = 0; phase ^= 1u; }
           }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(full_bar(stage));
-#pragma unroll
-          for (int c = 0; c < 4; ++c) cur[c] = nxt[c];
-          if (++stage == p.stages) { stage = 0; phase ^= 1u; }
         }
       }
     }

@@ -12,7 +12,6 @@
 
 #include <ATen/core/Tensor.h>
 #include <ATen/ops/empty.h>
-#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -38,7 +37,7 @@ struct Ready {
   void* handle;
   const hg_problem *low, *high;                       // inside `problems`
   int64_t tokens, k, outputs, packed;                 // packed: bytes of the quantised activations
-  bool fused;                                         // eager calls quantise inside the GEMM launch
+  bool fused;                                         // calls quantise inside the GEMM launch
   at::TensorOptions output, bytes;
   c10::Device device = c10::Device(c10::kCPU);
 };
@@ -188,11 +187,7 @@ PyObject* forward_checked(PyObject* self, const at::Tensor& x, long math) {
     const Unlocked unlocked;
     // Fresh tensors per call: under CUDA-graph capture the graph's pool owns them.
     y = at::empty({r->tokens, r->outputs}, r->output);
-    // Quantising inside the GEMM saves an eager call 2.5 us of host time for the second launch.  A replayed graph does not pay
-    // that, and there the separate quantiser runs under the end of the kernel in front: a decoder block of Qwen2.5-7B takes 43.2
-    // against 44.8 us at 8 tokens, 44.6 against 45.2 us at 16; one token is level or better in one launch.
-    const bool in_gemm = !swiglu && r->fused &&
-                         (tokens == 1 || c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None);
+    const bool in_gemm = !swiglu && r->fused;
     const int64_t bytes = in_gemm ? 0 : r->packed;
     if (bytes) workspace = at::empty({bytes}, r->bytes);
     const void* in = x.const_data_ptr();

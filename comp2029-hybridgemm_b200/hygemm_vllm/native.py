@@ -32,13 +32,16 @@ class Problem(C.Structure):
 
 
 PACK_MODE = int(os.environ.get("HYGEMM_PACK_MODE", "0"))
-# Eager calls at decode sizes (at most FUSED_QUANT_TOKENS tokens; one token in captured calls) quantise the activations inside
-# the GEMM kernel (`hg_run_x`: one launch instead of two, identical bytes); HYGEMM_FUSED_QUANT=0 turns it off.
+# Calls of at most FUSED_QUANT_TOKENS tokens quantise the activations inside the GEMM kernel (`hg_run_x`: one launch instead of
+# two, identical bytes); HYGEMM_FUSED_QUANT=0 turns it off.
 FUSED_QUANT_TOKENS = 16 if os.environ.get("HYGEMM_FUSED_QUANT", "1") != "0" else 0
-# Every CTA quantises the K slice it multiplies, so the work repeats once per row tile; layers wider than this
-# many output channels keep the separate quantiser launch (a decoder block with gate_up, 37888 wide, measured 45.2 us with its
-# own quantiser launch against 51.0 us fused at 16 tokens; narrow eager layers gain the host time of the launch).
-FUSED_QUANT_MAX_OUTPUTS = int(os.environ.get("HYGEMM_FUSED_QUANT_MAX_OUTPUTS", "8192"))
+# Every CTA quantises the K slice it multiplies, so the work repeats once per row tile.  Layers wider than this many output
+# channels keep the separate quantiser launch from FUSED_QUANT_WIDE_TOKENS + 1 tokens on: a captured decoder block with gate_up,
+# 37888 wide, takes 39.1 us against 40.4 with gate_up's own quantiser launch at 8 tokens, and 41.0 either way at 16.  A width
+# that is asked for holds at every token count.
+_max_outputs = os.environ.get("HYGEMM_FUSED_QUANT_MAX_OUTPUTS")
+FUSED_QUANT_MAX_OUTPUTS = int(_max_outputs or "8192")
+FUSED_QUANT_WIDE_TOKENS = 0 if _max_outputs else min(8, FUSED_QUANT_TOKENS)
 # Row-parallel exchange: up to this many tokens the partial sums cross NVLink as fp32 (rounded once after the sum).
 FUSED_QUANT_TOKENS_F32 = 16
 # Launch policies of hg_run (reference: native.py:14-15).
@@ -125,6 +128,11 @@ def check(status: int) -> None:
 def scale_size(rows: int, k: int) -> int:
     """Bytes of the padded scale buffer; the closed form of `hg_scale_size` (no foreign call on the hot path)."""
     return ((rows + 127) // 128) * (k // 128) * 512 if rows > 0 and k > 0 else 0
+
+
+def quantises_in_gemm(tokens: int, outputs: int) -> bool:
+    """Whether a plain call of a layer quantises its activations inside the GEMM launch."""
+    return tokens <= (FUSED_QUANT_TOKENS if outputs <= FUSED_QUANT_MAX_OUTPUTS else FUSED_QUANT_WIDE_TOKENS)
 
 
 def _stream(device) -> int:
@@ -258,7 +266,7 @@ class DualLinear:
         y = torch.empty((tokens, self.outputs), dtype=self.dtype, device=x.device)
         low, high = self.problems(x, x, y)
         handle = self._handle(tokens, self.low_id, self.high_id, C.byref(low), C.byref(high), _stream(x.device))
-        fused = tokens <= FUSED_QUANT_TOKENS and self.outputs <= FUSED_QUANT_MAX_OUTPUTS
+        fused = quantises_in_gemm(tokens, self.outputs)
         self._ready[tokens] = _host.prepare(self, tokens, handle.value, C.addressof(low), C.addressof(high), (low, high), y,
                                             tokens * self.k + scale_size(tokens, self.k), fused)
         result = _host.forward(self, x, math)

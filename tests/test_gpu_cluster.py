@@ -279,3 +279,31 @@ def test_swiglu_of_every_gate_from_minus_six_on(dtype):
         q, sf = producer.silu_pack(part, 0)
         exact_q, exact_sf, _ = producer.silu_pack(part, 0, debug=True)
         assert torch.equal(q, exact_q) and torch.equal(sf, exact_sf)
+
+
+@pytest.mark.parametrize("tokens", [1, 2, 7, 8, 9, 16])
+@pytest.mark.parametrize("outputs,k,high", [(19900, 384, 1900), (20000, 1408, 1), (640, 3712, 64), (300, 128, 30)])
+def test_quantisation_in_the_gemm_over_several_units(outputs, k, high, tokens):
+    """Several units to a CTA, K of fewer and of more steps than a quantiser has on the way and no multiple of them, eager and captured:
+    the bytes of the quantiser followed by the GEMM (the same arithmetic: tolerance 0)."""
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    for dtype in (torch.bfloat16, torch.float16):
+        w = torch.randn(outputs, k, device="cuda", generator=g, dtype=dtype) * 0.04
+        layer = native.DualLinear(w, torch.randperm(outputs, device="cuda", generator=g)[:high])
+        x = torch.randn(tokens, k, device="cuda", generator=g).to(dtype)
+        x[:, ::97] *= 20
+        want = layer.run_packed(*native.pack(x))
+        y = torch.empty_like(want)
+        low, hi = layer.problems(x, x, y)   # in the GEMM at every token count
+        handle = layer.handles[next(iter(layer.handles))]
+        stream = torch.cuda.current_stream().cuda_stream
+        native.check(native.library().hg_run_x(handle, C.byref(low), C.byref(hi), x.data_ptr(), native.DTYPES[dtype], stream))
+        assert torch.equal(y.view(torch.int16), want.view(torch.int16)) and torch.equal(layer(x).view(torch.int16), want.view(torch.int16))
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            captured = layer(x)
+        x.mul_(2)
+        graph.replay()
+        assert torch.equal(captured.view(torch.int16), layer.run_packed(*native.pack(x)).view(torch.int16))
+        assert layer.status()[0] == 0
+        layer.close()
