@@ -29,6 +29,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <numeric>
 #include <vector>
 
 #include "hg_gemm_cluster.cuh"
@@ -44,7 +45,7 @@ __host__ __device__ constexpr int first_act_warp(int pair) { return 2 + 4 * epil
 __host__ __device__ constexpr int cluster_threads(int pair, bool fused) { return first_act_warp(pair) * 32 + (fused ? kClusterQuantThreads : 32); }
 constexpr int kClusterMaxStages = 12;
 constexpr int kMaxSmem = 232448;
-constexpr uint32_t kScaleStride = 16;                           // TMEM columns per scale set: weights 4, activations up to 8
+constexpr uint32_t kScaleStride = 16;                           // TMEM columns per scale set: weights 4, activations up to 12
 
 struct ClusterParams {
   int rows[2], cut_log[2], tiles[2];   // a 128-row atom (PAIR: two) is cut into 2^cut_log tiles
@@ -55,6 +56,7 @@ struct ClusterParams {
   OutTargets out;
   int outputs, tokens, k, kblocks;
   int n_tile, n_tail, token_tiles, stages, split, split_log, share_log, clusters;
+  int n_step, sf_atoms, turned;   // see ClusterPlan
   int async_push;      // partials travel by st.async
   int ring_exchange;   // partials are exchanged in the ring, which is idle by then (a cluster that splits K has one unit)
   int acc_shift, overlap;
@@ -80,13 +82,13 @@ __host__ __device__ inline int share_log_of(int n_tile, int split) {
 struct ClusterSmem {
   uint32_t b, sfa, sfb, a, red, bars, end;  // byte offsets from the 1024-aligned base; activations start at 0
   uint32_t a_tile, b_tile;                  // bytes of one K128 block
-  uint32_t sfb_stage;                       // bytes of the activation scales of a stage: per 128 tokens two atoms
+  uint32_t sfb_stage;                       // bytes of the activation scales of a stage: two atoms for every 128 tokens a tile touches
 };
-__host__ __device__ inline ClusterSmem cluster_smem(int stages, int n_tile, int pair, int split, int slot_rows, int least_rows, int ring_exchange) {
+__host__ __device__ inline ClusterSmem cluster_smem(int stages, int n_tile, int sf_atoms, int pair, int split, int slot_rows, int least_rows, int ring_exchange) {
   ClusterSmem s;
   s.a_tile = uint32_t(slot_rows) * 128u;
   s.b_tile = uint32_t(n_tile / pair) * 128u;
-  s.sfb_stage = uint32_t((n_tile + 127) / 128) * 1024u;
+  s.sfb_stage = uint32_t(sf_atoms) * 1024u;
   s.b = 0;
   s.sfa = uint32_t(stages) * 2u * s.b_tile;
   s.sfb = s.sfa + uint32_t(stages) * 1024u;
@@ -211,10 +213,19 @@ __host__ __device__ __forceinline__ int fast_div(int64_t n, int d, uint64_t inve
 // scatter over the whole output row, and all but the last epilogue of a CTA run under the next main loop.  With several
 // token tiles they are spread evenly among the MXFP4 tiles, so that the two partitions of a channel range (both sorted)
 // are stored at about the same time and meet in L2: an MXFP8 tile writes one or two channels of nearly every sector.
+// Where the number of clusters and that of the token tiles have a common factor, a cluster with several units would meet some of the
+// token tiles only, and some clusters all the short ones (777 tokens in steps of 256: eight whole tiles beside four whole and four
+// short ones).  There a row tile starts with the token tile that its round over the clusters has come to (`turned`).
 struct Unit {
   int part, atom, first, last, token0, n;   // rows first .. last - 1 of the 128-row atom (PAIR: of atoms 2 atom and 2 atom + 1)
 };
-__host__ __device__ __forceinline__ Unit unit_at(const ClusterParams& p, int u) {
+// A cluster's units: u = cluster, cluster + clusters, ...; `turn` counts them modulo the token tiles.
+__host__ __device__ __forceinline__ void next_unit(const ClusterParams& p, int& u, int& turn) {
+  u += p.clusters;
+  if (++turn == p.token_tiles) turn = 0;
+}
+template <bool WIDE>
+__host__ __device__ __forceinline__ Unit unit_at(const ClusterParams& p, int u, int cluster, int turn) {
   Unit w;
   int tile;
   if (p.token_tiles == 1) {
@@ -223,13 +234,20 @@ __host__ __device__ __forceinline__ Unit unit_at(const ClusterParams& p, int u) 
     w.token0 = 0;
     w.n = p.n_tail;
   } else {
-    const int t = fast_div(u, p.token_tiles, p.by_token_tiles), tt = u - t * p.token_tiles, total = p.tiles[0] + p.tiles[1];
+    const int t = fast_div(u, p.token_tiles, p.by_token_tiles), total = p.tiles[0] + p.tiles[1];
+    int tt = u - t * p.token_tiles;
+    if (WIDE && p.turned) {   // the row tile's first unit is of this round over the clusters, or of the one before
+      tt += turn - (tt > cluster);
+      if (tt < 0) tt += p.token_tiles;
+      if (tt >= p.token_tiles) tt -= p.token_tiles;
+    }
     const int high_before = fast_div(int64_t(t) * p.tiles[1], total, p.by_tiles);
     const int high_after = fast_div(int64_t(t + 1) * p.tiles[1], total, p.by_tiles);
     w.part = high_after > high_before;
     tile = w.part ? high_before : t - high_before;
-    w.token0 = tt * p.n_tile;
-    w.n = tt == p.token_tiles - 1 ? p.n_tail : p.n_tile;
+    const int step = WIDE ? p.n_step : p.n_tile;
+    w.token0 = tt * step;
+    w.n = tt == p.token_tiles - 1 ? p.n_tail : step;
   }
   const int log = p.cut_log[w.part], height = kTileRows >> log;
   w.atom = tile >> log;
@@ -243,14 +261,17 @@ __host__ __device__ __forceinline__ int first_step(const ClusterParams& p, int s
   return (((p.kblocks + 1) >> 1) * slice) >> p.split_log;
 }
 
-template <typename T, int PAIR, bool FUSED>
+// WIDE: token tiles that start in the middle of a scale atom, a last tile wider than the others, units in turn (see ClusterPlan).  An
+// instance by itself: behind a quantiser, where its code is new to the instruction caches, a launch of it takes 0.3 us more (1536 x
+// 1536 at 887 tokens, quantiser included, 8.5 us against 8.8; behind another launch of its own both take 6.5).
+template <typename T, int PAIR, bool FUSED, bool WIDE>
 __global__ void __launch_bounds__(cluster_threads(PAIR, FUSED), 1)
 cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_constant__ ClusterMaps maps) {
   if (threadIdx.x == 0) HG_STAMP(0);
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
-  const ClusterSmem lay = cluster_smem(p.stages, p.n_tile, PAIR, p.split, p.slot_rows, p.least_rows, p.ring_exchange);
+  const ClusterSmem lay = cluster_smem(p.stages, p.n_tile, WIDE ? p.sf_atoms : (p.n_tile + 127) / 128, PAIR, p.split, p.slot_rows, p.least_rows, p.ring_exchange);
   const uint32_t bars = base + lay.bars;
   auto full_bar = [&](int s) { return bars + uint32_t(s) * 8u; };
   auto empty_bar = [&](int s) { return bars + uint32_t(kClusterMaxStages + s) * 8u; };
@@ -316,8 +337,8 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
     const uint32_t bars0 = PAIR == 1 ? smem0 + lay.bars : __shfl_sync(0xffffffffu, map_to_rank(bars, uint32_t(rank & ~1)), 0);
     int stage = 0;
     uint32_t phase = 1;
-    for (int u = cluster; u < units && !error; u += p.clusters) {
-      const Unit w = unit_at(p, u);
+    for (int u = cluster, turn = 0; u < units && !error; next_unit(p, u, turn)) {
+      const Unit w = unit_at<WIDE>(p, u, cluster, turn);
       const int atom = w.atom * PAIR + half;
       const uint8_t* sfa_src = p.sfa[w.part] + int64_t(atom) * p.kblocks * 512;
       const int row = atom * kTileRows + w.first;
@@ -352,11 +373,11 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
       const int atoms = (p.tokens + 127) >> 7;
       int stage = 0;
       uint32_t phase = 1;
-      for (int u = cluster; u < units && !error; u += p.clusters) {
-        const Unit w = unit_at(p, u);
-        const int first_atom = w.token0 >> 7, n_atoms = min((w.n + 127) >> 7, atoms - first_atom);
+      for (int u = cluster, turn = 0; u < units && !error; next_unit(p, u, turn)) {
+        const Unit w = unit_at<WIDE>(p, u, cluster, turn);
+        const int first_atom = w.token0 >> 7, n_atoms = min(((WIDE ? w.token0 & 127 : 0) + w.n + 127) >> 7, atoms - first_atom);
         const int row = w.token0 + half * (w.n / PAIR);
-        const bool whole = w.n == p.n_tile;
+        const bool whole = w.n == (WIDE ? p.n_step : p.n_tile);
         const uint8_t* sfb_src = p.sfb + int64_t(first_atom) * p.kblocks * 512;
         for (int step = step_begin; step < step_end; ++step) {
           const int kb = 2 * step, nkb = min(2, p.kblocks - kb);
@@ -370,7 +391,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
             const uint32_t bar = bars0 + uint32_t(stage) * 8u, dst = smem0 + lay.b + uint32_t(2 * stage) * lay.b_tile;
             if (PAIR == 1) mbar_expect_tx(bar, uint32_t(w.n) * 256u + uint32_t(n_atoms * nkb) * 512u);   // a block beyond K arrives as zeros
             else if (half == 0) mbar_expect_tx(full_bar(stage), 2u * (uint32_t(w.n / 2) * 256u + uint32_t(n_atoms) * 1024u));
-            // a short last token tile has a box of its own: its second block follows the first directly
+            // a last token tile of another width has a box of its own: its second block follows the first directly
             if (whole) cg_load_3d<PAIR>(dst, &maps.act, bar, 0, row, kb);
             else cg_load_3d<PAIR>(dst, &maps.tail, bar, 0, row, kb);
             for (int a = 0; a < n_atoms; ++a) {
@@ -471,8 +492,8 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
       };
       int stage = 0, it = 0, issued = 0;
       uint32_t phase = 0;
-      for (int u = cluster; u < units && !error; u += p.clusters, ++it) {
-        const Unit w = unit_at(p, u);
+      for (int u = cluster, turn = 0; u < units && !error; next_unit(p, u, turn), ++it) {
+        const Unit w = unit_at<WIDE>(p, u, cluster, turn);
         const int acc = it & 1;
         if (!acc_free(it)) { error = kErrMmaAcc; break; }
         tc_fence_after();
@@ -480,8 +501,9 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
         const uint32_t a_block = uint32_t(w.last - w.first) * 8u;
         const uint32_t b_block = uint32_t(w.n / PAIR) * 8u;   // descriptor units (16 bytes) between the stage's activation tiles
         const uint32_t idesc = (w.part ? 0u : 5u << 7) | (uint32_t(w.n >> 3) << 17) | (1u << 23) | (uint32_t(PAIR * kTileRows >> 4) << 24);
-        const bool two_atoms = w.n > 128;
-        const uint32_t sfb_col = 4u + (uint32_t(w.token0 & 127) >> 5);   // a second tile of 64 tokens starts in the middle of its scale atom
+        // After an odd multiple of 64 tokens a tile starts in the middle of a scale atom.
+        const uint32_t sfb_col = 4u + (uint32_t(w.token0 & 127) >> 5), sf_end = (uint32_t(w.token0) & 127u) + uint32_t(w.n);
+        const bool two_atoms = WIDE ? sf_end > 128 : w.n > 128;
         uint32_t accumulate = 0;
         int step = step_begin;
         for (; step < step_end; ++step) {
@@ -502,7 +524,10 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
               const uint32_t sf = sf0 + i * kScaleStride;
               cg_cp_scales<PAIR>(sf, desc_of(sfa_lo + i * 32u, kDescScales));
               cg_cp_scales<PAIR>(sf + 4, desc_of(sfb_lo + i * 32u, kDescScales));
-              if (two_atoms) cg_cp_scales<PAIR>(sf + 8, desc_of(sfb_lo + i * 32u + 64u, kDescScales));
+              if (two_atoms) {
+                cg_cp_scales<PAIR>(sf + 8, desc_of(sfb_lo + i * 32u + 64u, kDescScales));
+                if (WIDE && sf_end > 256) cg_cp_scales<PAIR>(sf + 12, desc_of(sfb_lo + i * 32u + 128u, kDescScales));
+              }
 #pragma unroll
               for (uint32_t j = 0; j < 4; ++j)
                 cg_mma<PAIR>(tmem_d, desc_of(a_lo + i * a_block + 2 * j, kDescTile), desc_of(b_lo + i * b_block + 2 * j, kDescTile),
@@ -549,8 +574,8 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
     const bool out_f32 = p.out.f32 != 0;
     const int row_bytes = p.outputs * (out_f32 ? 4 : 2);
     const uint32_t leader = uint32_t(rank & ~(PAIR - 1));
-    for (int u = cluster; u < units; u += p.clusters, ++it) {
-      const Unit w = unit_at(p, u);
+    for (int u = cluster, turn = 0; u < units; next_unit(p, u, turn), ++it) {
+      const Unit w = unit_at<WIDE>(p, u, cluster, turn);
       const int acc = it & 1;
       const int row = (w.atom * PAIR + half) * kTileRows + row_in_tile;
       const bool active = quarter * 32 >= w.first && quarter * 32 < w.last;   // this quarter's rows belong to the tile
@@ -725,8 +750,9 @@ static int tuning(const char* name, int value) {
 // shapes.)
 //
 // The constants are weights of a fit to the order of measured launches, every plan a shape can have, for shapes drawn from 640 to
-// 38000 channels and K 512 to 18944; a rate among them need not be one that a unit of the chip has.  Prefill: 1700 launches of the
-// GEMM alone; the plan preferred is 0.6 % slower than the best one of the shape on average.  Up to 128 tokens: layer calls
+// 38000 channels and K 512 to 18944; a rate among them need not be one that a unit of the chip has.  Prefill: the GEMM alone, 2338
+// shapes, half of them layers of 7B models, 13 plans of each; the plan preferred is 0.9 % slower than the best one of the
+// shape on average (0.6 % up to 512 tokens, 1.3 % from 1025 on; 2.0 % with the constants for steps of 128 and 256 tokens).  Up to 128 tokens: layer calls
 // (quantiser and GEMM) back to back, 2400 shapes, of which every fourth or so was fitted to and the rest checked: 0.9 % slower than the
 // best up to 64 tokens (1.9 % with constants fitted to the GEMM alone) and 1.1 % from 65 on (1.5 %; 10 % when two tiles of 64
 // tokens were no choice).  Up to twelve layers took turns there, so weights of less than about 10 MB stayed in L2.  Checked since on
@@ -736,29 +762,29 @@ static int tuning(const char* name, int value) {
 // us with 34 CTAs, that kernel included, and took 5.82 with 19 (back to back 3.77 and 4.28).  Over 110 layers such calls took
 // 5.4 % less than with the constants and kernels before.
 struct PlanFit {
-  double mma_floor;                                  // cycles of a single CTA's narrow MMA with its operand reads
+  double mma_floor, mma;                             // cycles of a single CTA's narrow MMA with its operand reads; factor on the time of every MMA
   double turn, l2, l2_wide, to_one;                  // us per turn of the ring; bytes per ns from L2 to all SMs, tiles of 129 tokens and more, to one
   double unit, split_unit, split_token;              // after a unit's main loop, whole or one of several parts of K; per token
   double store, store_token, low_row, high_row;      // stores: start; per token; cycles per token and row
   double hops, exchange, part, part_token;           // exchange: per doubling of the cluster, constant, per part, per part and token
   double cta, pair, cut, finer, hbm;                 // per CTA of the grid, paired CTAs, cut of all tiles, further cut of MXFP8 tiles; bytes per ns (0: no bound)
 };
-constexpr PlanFit kDecodeFit{234.0, 1.313, 12213, 12213, 189.6, 0.09482, 0.5133, 0.0314, 1.07, 0.01755, 0.02057, 0.9327, -0.657, 0.1007, 0.0143, 0.005931,
+constexpr PlanFit kDecodeFit{234.0, 1, 1.313, 12213, 12213, 189.6, 0.09482, 0.5133, 0.0314, 1.07, 0.01755, 0.02057, 0.9327, -0.657, 0.1007, 0.0143, 0.005931,
                              0.008127, 0.5955, -0.0378, 0.268, 0};
-constexpr PlanFit kWideDecodeFit{236.7, 1.328, 12840, 12840, 250.0, 0.2656, 0.7058, 0.02462, 0.3386, 0.01767, 0.01224, 0.9089, -0.538, 0.1856, 0.06477, 0.003302,
+constexpr PlanFit kWideDecodeFit{236.7, 1, 1.328, 12840, 12840, 250.0, 0.2656, 0.7058, 0.02462, 0.3386, 0.01767, 0.01224, 0.9089, -0.538, 0.1856, 0.06477, 0.003302,
                                  0.01379, 0.5441, -0.02387, 0.2337, 0};
-constexpr PlanFit kPrefillFit{234, 1.28, 18800, 12300, 380, 0.397, 1.75, 0.0159, 0.632, 0.0142, 0.0146, 0.648, -0.67, 0.09, 0.0186, 0.00254,
-                              0.00225, 2.55, 0.0711, -0.221, 3120};
+constexpr PlanFit kPrefillFit{234, 1.349, 1.355, 13290, 11130, 243.2, 0.7072, 0.718, 0.01597, 0.6543, 0.01595, 0.009445, 0.759, -0.5018, 0.06879, 0.02652, 0.007437,
+                              0.009874, 2.55, 0.0711, -0.0974, 4600};
 
 // `reject`: a plan that costs this much or more may be given any cost from there on.
 static double plan_cost(const ClusterPlan& plan, int units, int kblocks, double weight_kilobytes, double reject) {
-  const int columns = (plan.token_tiles - 1) * plan.n_tile + plan.n_tail;
-  const PlanFit& fit = columns <= 64 ? kDecodeFit : plan.token_tiles * plan.n_tile <= 128 ? kWideDecodeFit : kPrefillFit;
+  const int columns = (plan.token_tiles - 1) * plan.n_step + plan.n_tail;
+  const PlanFit& fit = columns <= 64 ? kDecodeFit : columns <= 128 ? kWideDecodeFit : kPrefillFit;
   const double steps = double((kblocks + 1) / 2) / plan.split;
   const int cluster_ctas = plan.pair * plan.split, ctas = plan.clusters * cluster_ctas;
   auto main_loop = [&](int n, bool high) {
     const double b = double(n) / plan.pair;
-    const double mma = 2 * (plan.pair == 2 ? std::max(2.0 * n, 200.0 + b) : std::max(171.0, fit.mma_floor + 1.3 * b)) / 1900;
+    const double mma = 2 * (plan.pair == 2 ? std::max(2.0 * n, 200.0 + b) : std::max(171.0, fit.mma_floor + 1.3 * b)) / 1900 * fit.mma;
     auto bytes = [&](int part) { return 1000 * (double(kTileRows >> plan.cut_log[part]) * (part ? 0.25 : 0.125) + b * 0.25 + 2); };
     const double average = (bytes(0) * plan.tiles[0] + bytes(1) * plan.tiles[1]) / (double(plan.tiles[0]) + plan.tiles[1]);
     const double step = std::max({mma, fit.turn / plan.stages, average * ctas / (1000 * (n > 128 ? fit.l2_wide : fit.l2)), bytes(high) / (1000 * fit.to_one)});
@@ -768,9 +794,9 @@ static double plan_cost(const ClusterPlan& plan, int units, int kblocks, double 
     const double rows = double(kTileRows >> plan.cut_log[high]);
     return fit.store + std::max(fit.store_token * n, n * rows * (high ? fit.high_row : fit.low_row) / 1900) / plan.split;
   };
-  const double main_of[2][2] = {{main_loop(plan.n_tile, false), main_loop(plan.n_tail, false)},
-                                {plan.tiles[1] ? main_loop(plan.n_tile, true) : 0, plan.tiles[1] ? main_loop(plan.n_tail, true) : 0}};
-  const double store_of[2][2] = {{stores(plan.n_tile, false), stores(plan.n_tail, false)}, {stores(plan.n_tile, true), stores(plan.n_tail, true)}};
+  const double main_of[2][2] = {{main_loop(plan.n_step, false), main_loop(plan.n_tail, false)},
+                                {plan.tiles[1] ? main_loop(plan.n_step, true) : 0, plan.tiles[1] ? main_loop(plan.n_tail, true) : 0}};
+  const double store_of[2][2] = {{stores(plan.n_step, false), stores(plan.n_tail, false)}, {stores(plan.n_step, true), stores(plan.n_tail, true)}};
   double exchange = 0;
   if (plan.split > 1)
     exchange = fit.hops * std::log2(double(cluster_ctas)) + fit.exchange + (fit.part + fit.part_token * plan.n_tile) * plan.split;
@@ -803,14 +829,16 @@ static double plan_cost(const ClusterPlan& plan, int units, int kblocks, double 
   } else {
     std::vector<Ends> ends(size_t(plan.clusters));
     const int tiles = plan.tiles[0] + plan.tiles[1];
-    int cluster = 0, spread = 0;   // spread: how far the running share of MXFP8 tiles is beyond the last whole one (see unit_at)
+    int cluster = 0, round = 0;   // of the next unit; see unit_at
+    int spread = 0;               // how far the running share of MXFP8 tiles is beyond the last whole one
     for (int t = 0; t < tiles; ++t) {
       spread += plan.tiles[1];
       const bool high = spread >= tiles;
       if (high) spread -= tiles;
+      const int last = plan.token_tiles - 1 - (plan.turned ? round % plan.token_tiles : 0);
       for (int tt = 0; tt < plan.token_tiles; ++tt) {
-        add(ends[size_t(cluster)], high, tt == plan.token_tiles - 1);
-        if (++cluster == plan.clusters) cluster = 0;
+        add(ends[size_t(cluster)], high, tt == last);
+        if (++cluster == plan.clusters) { cluster = 0; ++round; }
       }
     }
     for (const Ends& e : ends) busiest = std::max(busiest, e.stores);
@@ -829,7 +857,7 @@ static bool finish_plan(ClusterPlan& plan, int most_stages) {
   plan.slot_rows = kTileRows >> std::min(plan.cut_log[0], plan.cut_log[1]);
   plan.least_rows = kTileRows >> std::max(plan.cut_log[0], plan.cut_log[1]);
   for (plan.stages = most_stages; plan.stages >= 2; --plan.stages) {
-    plan.smem_bytes = 1024 + int(cluster_smem(plan.stages, plan.n_tile, plan.pair, plan.split, plan.slot_rows, plan.least_rows, plan.ring_exchange).end);
+    plan.smem_bytes = 1024 + int(cluster_smem(plan.stages, plan.n_tile, plan.sf_atoms, plan.pair, plan.split, plan.slot_rows, plan.least_rows, plan.ring_exchange).end);
     if (plan.smem_bytes <= kMaxSmem) return true;
   }
   return false;
@@ -842,12 +870,17 @@ ClusterPlan make_cluster_plan(int lo, int hi, int tokens, int k, const int max_c
   best.cost = 1e30;
   const int force_split = tuning("HYGEMM_CL_SPLIT", 0), force_pair = tuning("HYGEMM_CL_PAIR", 0), force_n = tuning("HYGEMM_CL_N", 0);
   const int force_cut = tuning("HYGEMM_CL_CUT", -1), force_cut_high = tuning("HYGEMM_CL_CUT_HIGH", -1);
+  // Token tiles of `way` tokens (0: one tile), the last one holding what is left; -way: with what is left joined to the one before.
+  const std::array<int, 5> decode_ways{0, 64}, prefill_ways{128, 256, 192, -128, -192};
+  const std::array<int, 5>& all_ways = tokens <= 128 ? decode_ways : prefill_ways;
+  const int* const ways_end = all_ways.data() + (tokens <= 128 ? 2 : 5);
   const int most_stages = std::min(kClusterMaxStages, tuning("HYGEMM_CL_STAGES", kClusterMaxStages));
   for (int pair = 1; pair <= 2; ++pair)
     for (int log = pair - 1; log < 4; ++log)
       for (int cut = 0; cut < 3; ++cut)
         for (int more = 0; more < 3; ++more)
-          for (int n : {0, 64, 128, 256}) {
+          for (const int* way_at = all_ways.data(); way_at < ways_end; ++way_at) {
+              const int way = *way_at;
               ClusterPlan plan;
               plan.pair = pair;
               plan.split = (1 << log) / pair;
@@ -858,16 +891,27 @@ ClusterPlan make_cluster_plan(int lo, int hi, int tokens, int k, const int max_c
                 // From 65 tokens on also two tiles of 64: twice the CTAs with half the accumulators each, for a second read of the
                 // weights from L2.  Layers with few row tiles gain (128 tokens: 4608 x 3584 8.8 -> 7.7 us, 4096 x 1024 5.8 -> 4.2, 7003 x 2432
                 // at 77 tokens 7.3 -> 6.7), wide and long ones do not (37888 x 3584 23.7 -> 27.0, 3584 x 18944 16.1 -> 17.1).
-                if (n > 64 || (n && tokens <= 64) || (!n && tokens > 64 && pair == 1) || (tokens <= 32 && pair == 2)) continue;   // (fused quantisation: single CTAs)
-                plan.token_tiles = n ? 2 : 1;
-                plan.n_tail = (tokens - (n ? 64 : 0) + 16 * pair - 1) / (16 * pair) * (16 * pair);
-                plan.n_tile = n ? 64 : plan.n_tail;
+                if ((way && tokens <= 64) || (!way && tokens > 64 && pair == 1) || (tokens <= 32 && pair == 2)) continue;   // (fused quantisation: single CTAs)
+                plan.token_tiles = way ? 2 : 1;
+                plan.n_tail = (tokens - way + 16 * pair - 1) / (16 * pair) * (16 * pair);
+                plan.n_step = way ? way : plan.n_tail;
               } else {
-                if (n < 128 || pair == 1 || cut || (n == 256 && plan.split > 1)) continue;
-                plan.n_tile = n;
-                plan.token_tiles = (tokens + n - 1) / n;
-                plan.n_tail = (tokens - (plan.token_tiles - 1) * n + 31) / 32 * 32;
+                // Steps of 192 beside those of 128 and 256, and a short last tile joined to the one before it, so that the tiles of a ragged
+                // prompt fit the clusters: 37888 x 3584 at 160 tokens in one tile 31.5 -> 25.0 us, at 300 in 192 + 108 48.9 -> 45.0, 3584 x 18944
+                // at 777 in 3 x 192 + 201 54.4 -> 49.4, 4608 x 3584 at 2048 by steps of 192 36.1 -> 31.8.
+                if (pair == 1 || cut) continue;
+                plan.n_step = std::abs(way);
+                plan.token_tiles = way < 0 ? tokens / plan.n_step : (tokens + plan.n_step - 1) / plan.n_step;
+                if (plan.token_tiles < 1) continue;
+                plan.n_tail = (tokens - (plan.token_tiles - 1) * plan.n_step + 31) / 32 * 32;
+                if (plan.n_tail > 256) continue;
+                if (plan.token_tiles == 1) plan.n_step = plan.n_tail;
               }
+              plan.n_tile = std::max(plan.n_step, plan.n_tail);
+              if (tokens > 128 && ((tokens + plan.n_tile - 1) / plan.n_tile != plan.token_tiles || (plan.n_tile > 224 && plan.split > 1))) continue;
+              // Atoms that the last tile and the first ones touch; a second one may start in the middle of its first.
+              const int last_start = (plan.token_tiles - 1) * plan.n_step % 128, odd_start = plan.token_tiles > 2 ? plan.n_step % 128 : 0;
+              plan.sf_atoms = std::max(last_start + plan.n_tail + 127, plan.token_tiles > 1 ? odd_start + plan.n_step + 127 : 0) / 128;
               if ((force_split && plan.split != force_split) || (force_pair && pair != force_pair) || (force_n && plan.n_tile != force_n) ||
                   (force_cut >= 0 && cut != force_cut) || (force_cut_high >= 0 && cut + more != force_cut_high))
                 continue;
@@ -877,37 +921,43 @@ ClusterPlan make_cluster_plan(int lo, int hi, int tokens, int k, const int max_c
               // With several units to a cluster every exchange would stall the next main loop (gate_up at 16 tokens, K in
               // two: 19.8 us against 15.4).
               if (plan.split > 1 && units > plan.clusters) continue;
+              plan.turned = tokens > 128 && 4 * plan.n_tail <= 3 * plan.n_step && units > plan.clusters && plan.clusters >= plan.token_tiles &&
+                            std::gcd(plan.clusters, plan.token_tiles) > 1;
               // Worth its extra hop (about 0.4 us) where the exchange buffer would take a stage from the ring (down_proj at 128
               // tokens 17.1 -> 16.0 us).
               plan.ring_exchange = plan.split > 1 && plan.n_tile > 32;
               if (!finish_plan(plan, most_stages)) continue;
-              plan.cost = plan_cost(plan, int(units), kblocks, (lo * 0.53125 + hi * 1.03125) * k * 1e-3, best.cost);
+              plan.wide = plan.turned || (tokens > 128 && plan.token_tiles > 1 && (plan.n_step % 128 || plan.n_tail > plan.n_step));
+              // The instance for them has to be better by more than the estimate's error.
+              const double margin = plan.wide ? 1.03 : 1, start = plan.wide ? 0.3 : 0;
+              plan.cost = margin * plan_cost(plan, int(units), kblocks, (lo * 0.53125 + hi * 1.03125) * k * 1e-3, (best.cost - start) / margin) + start;
               if (plan.cost < best.cost) best = plan;
             }
   if (best.cost >= 1e30) throw std::runtime_error("No cluster schedule for this shape");
   return best;
 }
 
-template <typename T, int PAIR, bool FUSED>
+template <typename T, int PAIR, bool FUSED, bool WIDE = false>
 static void set_limits() {
-  check(cudaFuncSetAttribute(cluster_gemm_kernel<T, PAIR, FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem), "cudaFuncSetAttribute");
+  check(cudaFuncSetAttribute(cluster_gemm_kernel<T, PAIR, FUSED, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem), "cudaFuncSetAttribute");
 }
 
 void configure_cluster_kernels() {
-  set_limits<__nv_bfloat16, 1, false>(); set_limits<__nv_bfloat16, 1, true>(); set_limits<__nv_bfloat16, 2, false>();
-  set_limits<__half, 1, false>(); set_limits<__half, 1, true>(); set_limits<__half, 2, false>();
+  set_limits<__nv_bfloat16, 1, false>(); set_limits<__nv_bfloat16, 1, true>(); set_limits<__nv_bfloat16, 2, false>(); set_limits<__nv_bfloat16, 2, false, true>();
+  set_limits<__half, 1, false>(); set_limits<__half, 1, true>(); set_limits<__half, 2, false>(); set_limits<__half, 2, false, true>();
 }
 
 void cluster_kernel_attributes(const ClusterPlan& plan, int dtype, int* registers, int* local_bytes, int* stage_bytes) {
   cudaFuncAttributes attr{};
   const bool bf16 = dtype == HG_DTYPE_BF16;
-  check(plan.pair == 2 ? (bf16 ? cudaFuncGetAttributes(&attr, cluster_gemm_kernel<__nv_bfloat16, 2, false>)
-                               : cudaFuncGetAttributes(&attr, cluster_gemm_kernel<__half, 2, false>))
-                       : (bf16 ? cudaFuncGetAttributes(&attr, cluster_gemm_kernel<__nv_bfloat16, 1, false>)
-                               : cudaFuncGetAttributes(&attr, cluster_gemm_kernel<__half, 1, false>)), "cudaFuncGetAttributes");
+  auto get = [&](auto wide_kernel, auto pair_kernel, auto kernel) {
+    check(cudaFuncGetAttributes(&attr, plan.wide ? wide_kernel : plan.pair == 2 ? pair_kernel : kernel), "cudaFuncGetAttributes");
+  };
+  if (bf16) get(cluster_gemm_kernel<__nv_bfloat16, 2, false, true>, cluster_gemm_kernel<__nv_bfloat16, 2, false, false>, cluster_gemm_kernel<__nv_bfloat16, 1, false, false>);
+  else get(cluster_gemm_kernel<__half, 2, false, true>, cluster_gemm_kernel<__half, 2, false, false>, cluster_gemm_kernel<__half, 1, false, false>);
   *registers = attr.numRegs;
   *local_bytes = int(attr.localSizeBytes);
-  const ClusterSmem lay = cluster_smem(plan.stages, plan.n_tile, plan.pair, plan.split, plan.slot_rows, plan.least_rows, plan.ring_exchange);
+  const ClusterSmem lay = cluster_smem(plan.stages, plan.n_tile, plan.sf_atoms, plan.pair, plan.split, plan.slot_rows, plan.least_rows, plan.ring_exchange);
   *stage_bytes = int(2 * lay.b_tile + 1024 + lay.sfb_stage);
 }
 
@@ -933,7 +983,7 @@ const int* cluster_capacity() {
       config.attrs = attribute;
       config.numAttrs = 1;
       int clusters = 0;
-      check(cudaOccupancyMaxActiveClusters(&clusters, cluster_gemm_kernel<__nv_bfloat16, 2, false>, &config), "cluster occupancy");
+      check(cudaOccupancyMaxActiveClusters(&clusters, cluster_gemm_kernel<__nv_bfloat16, 2, false, false>, &config), "cluster occupancy");
       capacity[device][log] = std::min(clusters, sms >> log);
     }
   });
@@ -957,7 +1007,7 @@ ClusterPlan make_cluster_plan_for(int lo, int hi, int tokens, int k, int sms) {
   return make_cluster_plan(lo, hi, tokens, k, capacity_for(sms).data());
 }
 
-template <typename T, int PAIR, bool FUSED>
+template <typename T, int PAIR, bool FUSED, bool WIDE = false>
 static cudaError_t launch(const ClusterPlan& plan, const ClusterParams& p, const ClusterMaps& maps, cudaStream_t stream, bool pdl) {
   cudaLaunchConfig_t config{};
   config.gridDim = dim3(unsigned(plan.clusters * plan.pair * plan.split));
@@ -976,7 +1026,7 @@ static cudaError_t launch(const ClusterPlan& plan, const ClusterParams& p, const
   }
   config.attrs = attribute;
   config.numAttrs = unsigned(count);
-  return cudaLaunchKernelEx(&config, cluster_gemm_kernel<T, PAIR, FUSED>, p, maps);
+  return cudaLaunchKernelEx(&config, cluster_gemm_kernel<T, PAIR, FUSED, WIDE>, p, maps);
 }
 
 // What follows from the plan and the shape alone.
@@ -986,6 +1036,7 @@ static ClusterParams shape_params(const ClusterPlan& plan, int rows_low, int row
   for (int i = 0; i < 2; ++i) { p.rows[i] = rows[i]; p.cut_log[i] = plan.cut_log[i]; p.tiles[i] = plan.tiles[i]; }
   p.slot_rows = plan.slot_rows; p.least_rows = plan.least_rows;
   p.tokens = tokens; p.k = k; p.kblocks = k / kTileK;
+  p.n_step = plan.n_step; p.sf_atoms = plan.sf_atoms; p.turned = plan.turned;
   p.n_tile = plan.n_tile; p.n_tail = plan.n_tail; p.token_tiles = plan.token_tiles; p.stages = plan.stages;
   p.async_push = plan.n_tile <= 32;
   p.ring_exchange = plan.ring_exchange; p.split = plan.split; p.clusters = plan.clusters;
@@ -1010,13 +1061,13 @@ std::vector<ClusterPart> cluster_parts(const ClusterPlan& plan, int rows_low, in
   parts.reserve(size_t(units) * cluster_ctas);
   for (int cluster = 0; cluster < plan.clusters; ++cluster)
     for (int rank = 0; rank < cluster_ctas; ++rank)
-      for (int u = cluster; u < units; u += plan.clusters) {
-        const Unit w = unit_at(p, u);
+      for (int u = cluster, turn = 0; u < units; next_unit(p, u, turn)) {
+        const Unit w = plan.wide ? unit_at<true>(p, u, cluster, turn) : unit_at<false>(p, u, cluster, turn);
         const int half = rank % plan.pair, slice = rank / plan.pair, atom = w.atom * plan.pair + half, log = p.cut_log[w.part];
         ClusterPart part;
         part.cta = cluster * cluster_ctas + rank;
         part.tile = (w.part ? plan.pair * p.tiles[0] : 0) + (atom << log) + (w.first >> (7 - log));
-        part.token_tile = w.token0 / p.n_tile;
+        part.token_tile = w.token0 / p.n_step;
         part.kb_begin = 2 * first_step(p, slice);
         part.kb_end = std::min(2 * first_step(p, slice + 1), p.kblocks);
         part.slice = slice;
@@ -1048,6 +1099,7 @@ void launch_cluster(const ClusterPlan& plan, const ClusterCall& call, const Clus
   cudaError_t e;
   if (call.x) e = bf16 ? launch<__nv_bfloat16, 1, true>(plan, p, maps, stream, pdl) : launch<__half, 1, true>(plan, p, maps, stream, pdl);
   else if (plan.pair == 1) e = bf16 ? launch<__nv_bfloat16, 1, false>(plan, p, maps, stream, pdl) : launch<__half, 1, false>(plan, p, maps, stream, pdl);
+  else if (plan.wide) e = bf16 ? launch<__nv_bfloat16, 2, false, true>(plan, p, maps, stream, pdl) : launch<__half, 2, false, true>(plan, p, maps, stream, pdl);
   else e = bf16 ? launch<__nv_bfloat16, 2, false>(plan, p, maps, stream, pdl) : launch<__half, 2, false>(plan, p, maps, stream, pdl);
   check(e, "hybrid GEMM launch");
 }

@@ -10,8 +10,12 @@ struct ClusterPlan {
   int pair = 1;            // CTAs that share one MMA tile: 1, or 2 (cta_group::2)
   int split = 1;           // slices of K per tile, one CTA (pair) of the cluster each
   int clusters = 0;        // persistent clusters of pair * split CTAs
-  int n_tile = 0;          // tokens per tile
-  int n_tail = 0;          // MMA columns of the last token tile
+  int wide = 0;            // token tiles that only the kernel's WIDE instance takes
+  int n_tile = 0;          // MMA columns of the widest token tile
+  int n_step = 0;          // tokens of every token tile but the last
+  int n_tail = 0;          // MMA columns of the last token tile; may be more than n_step
+  int sf_atoms = 0;        // 128-token scale atoms that a token tile touches at most
+  int turned = 0;          // rows of units start with another token tile each round over the clusters
   int token_tiles = 0;
   int cut_log[2] = {0, 0};     // each partition's 128-row atoms (pairs of atoms) are cut into 2^cut_log tiles
   int tiles[2] = {0, 0};       // tiles of each partition
@@ -50,7 +54,7 @@ struct ClusterCall {
   int* status;
   unsigned long long* trace;
 };
-// Boxes: weights 128 >> cut_log rows x 2 K128 blocks; activations n_tile / pair and, for the last token tile, n_tail / pair rows;
+// Boxes: weights 128 >> cut_log rows x 2 K128 blocks; activations n_step / pair and, for the last token tile, n_tail / pair rows;
 // scales (pairs only) 2 atoms.  Maps a launch does not use (an absent partition; activations quantised in the kernel) may
 // be zeros.
 struct ClusterMaps { CUtensorMap low, high, act, tail, low_scales, high_scales, act_scales; };

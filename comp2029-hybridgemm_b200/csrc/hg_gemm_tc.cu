@@ -1004,8 +1004,8 @@ static void set_weight_maps(ClusterMaps& maps, const ClusterPlan& plan, const hg
   if (plan.pair == 2) (part ? maps.high_scales : maps.low_scales) = make_scale_map(q.weight_scales, scale_size(q.rows, q.k) / 512);
 }
 static void set_activation_maps(ClusterMaps& maps, const ClusterPlan& plan, const hg_problem& q) {
-  maps.act = make_block_map(q.activation, q.tokens, q.k, plan.n_tile / plan.pair);
-  maps.tail = plan.n_tail == plan.n_tile ? maps.act : make_block_map(q.activation, q.tokens, q.k, plan.n_tail / plan.pair);
+  maps.act = make_block_map(q.activation, q.tokens, q.k, plan.n_step / plan.pair);
+  maps.tail = plan.n_tail == plan.n_step ? maps.act : make_block_map(q.activation, q.tokens, q.k, plan.n_tail / plan.pair);
   if (plan.pair == 2) maps.act_scales = make_scale_map(q.activation_scales, scale_size(q.tokens, q.k) / 512);
 }
 

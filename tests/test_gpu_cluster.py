@@ -43,6 +43,21 @@ def test_exact_with_several_wide_tiles_per_cluster(tokens, k, forced, monkeypatc
     assert np.array_equal(got, case["expected"]), int((got != case["expected"]).sum())
 
 
+@pytest.mark.parametrize("tokens,width", [(129, 160), (160, 160), (193, 224), (300, 192), (310, 256), (450, 192), (577, 224), (641, 192), (777, 224), (1000, 192)])
+def test_exact_in_tiles_that_fit_a_ragged_prompt(tokens, width, monkeypatch):
+    """One tile of up to 256 tokens, steps of 192 whose every second tile starts in the middle of a scale atom, a last tile joined to the one
+    before it (wider than the others, over three scale atoms): one and several units to a cluster, whole and cut along K."""
+    monkeypatch.setenv("HYGEMM_CL_N", str(width))
+    for (outputs, k, high), split in [((8269, 384, 800), 1), ((640, 896, 128), 1), ((640, 896, 128), 2), ((18944, 128, 1000), 1)]:
+        if split > 1 and width > 224:
+            continue   # 256 tokens are never cut along K
+        monkeypatch.setenv("HYGEMM_CL_SPLIT", str(split))
+        case = oracle.exact_case(outputs, tokens, k, high, "random")
+        got, guards, status = run_gemm(case, torch.bfloat16, 0)
+        assert status[0] == 0 and guards and (status[1], status[2]) == expected_work(case, 0), (outputs, k, high, split, status)
+        assert np.array_equal(got, case["expected"]), (outputs, k, high, split, int((got != case["expected"]).sum()))
+
+
 @pytest.mark.parametrize("pair", [1, 2])
 @pytest.mark.parametrize("split", [1, 2, 4])
 @pytest.mark.parametrize("tokens", [65, 80, 97, 128])
