@@ -12,6 +12,8 @@
 
 #include <ATen/core/Tensor.h>
 #include <ATen/ops/empty.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -38,7 +40,7 @@ struct Ready {
   const hg_problem *low, *high;                       // inside `problems`
   int64_t tokens, k, outputs, packed;                 // packed: bytes of the quantised activations
   bool fused;                                         // calls quantise inside the GEMM launch
-  at::TensorOptions output, bytes;
+  at::TensorOptions output;
   c10::Device device = c10::Device(c10::kCPU);
 };
 
@@ -179,7 +181,7 @@ PyObject* forward_checked(PyObject* self, const at::Tensor& x, long math) {
       !operands_unchanged(layer, *r->low, *r->high))
     Py_RETURN_NONE;
   const int dtype = type == at::kBFloat16 ? HG_DTYPE_BF16 : HG_DTYPE_F16;
-  at::Tensor y, workspace;
+  at::Tensor y;
   int status;
   {
     // Without the interpreter lock, as torch's own bindings: an allocator may wait for a thread that wants it (one whose
@@ -189,10 +191,16 @@ PyObject* forward_checked(PyObject* self, const at::Tensor& x, long math) {
     y = at::empty({r->tokens, r->outputs}, r->output);
     const bool in_gemm = !swiglu && r->fused;
     const int64_t bytes = in_gemm ? 0 : r->packed;
-    if (bytes) workspace = at::empty({bytes}, r->bytes);
+    // Scratch that nobody else sees: the allocator itself, for the same stream and with the same lifetime, without a tensor round it
+    // (0.45 us of a call of two launches, of which the host then needs 6.7 us).
+    c10::DataPtr workspace;
+    if (bytes) {
+      const c10::cuda::CUDAGuard guard(r->device);
+      workspace = c10::cuda::CUDACachingAllocator::get()->allocate(size_t(bytes));
+    }
     const void* in = x.const_data_ptr();
     void* out = y.mutable_data_ptr();
-    void* scratch = bytes ? workspace.mutable_data_ptr() : nullptr;
+    void* scratch = workspace.get();
     void* stream = c10::cuda::getCurrentCUDAStream(r->device.index()).stream();
     status = swiglu ? run_linear_silu(r->handle, r->low, r->high, in, dtype, int(math), scratch, out, stream)
                     : run_linear(r->handle, r->low, r->high, in, dtype, scratch, out, stream);
@@ -245,7 +253,6 @@ PyObject* prepare(PyObject*, PyObject* args) {
   r->fused = fused;
   r->device = like.device();
   r->output = at::TensorOptions().dtype(like.scalar_type()).device(like.device());
-  r->bytes = r->output.dtype(at::kByte);
   return capsule;
 }
 
