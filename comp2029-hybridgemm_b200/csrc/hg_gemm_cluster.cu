@@ -19,7 +19,7 @@
 // Roles per CTA: warp 0 weights and their scales (TMA), warp 1 MMA issue (idle in the second CTA of a pair, whose copies
 // complete on the first CTA's barriers: reporting every stage with a remote arrive cost 750 cycles each), then epilogue warps
 // (four; in pairs eight, two per TMEM quarter on alternate groups of sixteen columns), then one warp for the activations and
-// their scales (TMA) or, FUSED, eight warps that quantise the activations.
+// their scales (TMA) or, FUSED, up to eight warps that quantise the activations.
 // One warp per scheduler runs most of these roles alone, so a dependent instruction costs about five cycles and nothing
 // hides it: loops here carry no divisions, addresses are independent of each other, and descriptors are sums.
 // Every mbarrier wait is bounded; on expiry the CTA records a code, drains and leaves.
@@ -38,7 +38,7 @@ namespace hg {
 
 namespace {
 
-constexpr int kClusterQuantThreads = 256;   // activation quantisers: sixteen per token and K256 step
+constexpr int kClusterQuantThreads = 256;   // activation quantisers at most: sixteen per token and K256 step, and no warp without a token
 constexpr int kQuantAhead = 4;              // steps whose activations a quantiser has in registers or on the way
 __host__ __device__ constexpr int epilogue_sides(int pair) { return pair == 2 ? 2 : 1; }
 __host__ __device__ constexpr int first_act_warp(int pair) { return 2 + 4 * epilogue_sides(pair); }
@@ -300,7 +300,7 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.tail)) : "memory");
     }
     for (int s = 0; s < p.stages; ++s) {
-      mbar_init(full_bar(s), 1 + (FUSED ? kClusterQuantThreads / 32 : 1));   // weights; activations or the quantiser warps
+      mbar_init(full_bar(s), 1 + (FUSED ? (blockDim.x >> 5) - kActWarp : 1));   // weights; activations or the quantiser warps
       mbar_init(empty_bar(s), 1);
     }
     for (int s = 0; s < 2; ++s) {
@@ -411,7 +411,9 @@ cluster_gemm_kernel(const __grid_constant__ ClusterParams p, const __grid_consta
     // scales are the bytes hg_pack would have produced.  What bounds this is latency, of the loads above all, so a thread has
     // the next kQuantAhead steps' values on the way.  With 128 threads of 32 values each and one step ahead a block of
     // Qwen2.5-7B took longer in captured calls than with a quantiser in front from two tokens on; now it does not up to sixteen
-    // (8 tokens 40.7 us with separate quantisers, 40.4 with qkv and o_proj quantised here, 39.1 with gate_up too).
+    // (8 tokens 40.7 us with separate quantisers, 40.4 with qkv and o_proj quantised here, 39.1 with gate_up too).  A launch has two
+    // tokens to a warp and no more warps than that: seven idle ones made a block at one token take 38.8 us instead of 37.1, at four
+    // 38.9 instead of 38.0.
     if constexpr (FUSED) {
       const int tq = threadIdx.x - kActWarp * 32;
       const int token = tq >> 4, blk = (tq >> 3) & 1, g = (tq >> 1) & 3, part = tq & 1;
@@ -1011,7 +1013,7 @@ template <typename T, int PAIR, bool FUSED, bool WIDE = false>
 static cudaError_t launch(const ClusterPlan& plan, const ClusterParams& p, const ClusterMaps& maps, cudaStream_t stream, bool pdl) {
   cudaLaunchConfig_t config{};
   config.gridDim = dim3(unsigned(plan.clusters * plan.pair * plan.split));
-  config.blockDim = dim3(cluster_threads(PAIR, FUSED));
+  config.blockDim = dim3(FUSED ? first_act_warp(PAIR) * 32 + (p.tokens + 1) / 2 * 32 : cluster_threads(PAIR, false));
   config.dynamicSmemBytes = size_t(plan.smem_bytes);
   config.stream = stream;
   cudaLaunchAttribute attribute[2];

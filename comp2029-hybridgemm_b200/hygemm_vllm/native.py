@@ -37,7 +37,7 @@ PACK_MODE = int(os.environ.get("HYGEMM_PACK_MODE", "0"))
 FUSED_QUANT_TOKENS = 16 if os.environ.get("HYGEMM_FUSED_QUANT", "1") != "0" else 0
 # Every CTA quantises the K slice it multiplies, so the work repeats once per row tile.  Layers wider than this many output
 # channels keep the separate quantiser launch from FUSED_QUANT_WIDE_TOKENS + 1 tokens on: a captured decoder block with gate_up,
-# 37888 wide, takes 39.1 us against 40.4 with gate_up's own quantiser launch at 8 tokens, and 41.0 either way at 16.  A width
+# 37888 wide, takes 39.0 us against 40.4 with gate_up's own quantiser launch at 8 tokens, and 41.0 either way at 16.  A width
 # that is asked for holds at every token count.
 _max_outputs = os.environ.get("HYGEMM_FUSED_QUANT_MAX_OUTPUTS")
 FUSED_QUANT_MAX_OUTPUTS = int(_max_outputs or "8192")
