@@ -296,7 +296,7 @@ mx_quant_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint
 // ---- Many rows: weights at load time, prefill activations -----------------------------------------------------------
 //
 // A warp owns rows r, r+32, r+64, r+96 of a 128-row scale block x 512 columns, sixteen consecutive values per lane and row,
-// and keeps their four 32-byte loads in flight (SwiGLU: rows r and r+32, four loads).  Sixteen values per lane halve the
+// and has its four 32-byte loads (SwiGLU: eight) in flight before it converts the first.  Sixteen values per lane halve the
 // instructions per value against eight (one shuffle, one exponent and one scale byte per sixteen, maxima in packed 16-bit
 // form): the kernel above is bound by them, 3.8 TB/s on a 272 MB weight matrix.  The four rows share the 16-byte
 // entries of the scale atoms, so scales leave as whole entries instead of single words, each a partial write of a
@@ -444,20 +444,17 @@ __device__ __forceinline__ void silu16(const Raw16& gate, const Raw16& up, Raw16
   }
 }
 
-// SwiGLU + MXFP8 for many rows; bound by instruction issue.  A warp owns rows r and r + 32 of half a 128-row scale block x 512 columns, has
-// both rows' loads under way and writes eight bytes of scales at a time.  With four rows to a warp (three blocks to an SM then) a
-// launch had half as many warps and ended with a nearly empty last wave more often: over seven shapes of 500 to 2048 rows, fp16 and
-// bf16, 2.5 % more time on average (1500 x 8192 18.1 against 17.1 us, 777 x 18944 19.7 and 19.7, 2048 x 18944 48.1 and 48.1 bf16, 47.1
-// and 46.1 fp16); one row to a warp 8 % more, warps that take items a grid apart 8 % more.
+// SwiGLU + MXFP8 for many rows; bound by instruction issue.  2048 x 18944 bf16 44.8 us (62 % of the memory bandwidth; 46.2 with the
+// exact functions at every pair in doubt and four blocks to an SM), 777 rows 19.2 us (21.7), 60 with silu8 throughout at 2048.
 template <typename T, int MATH>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(256, 3)
 mx_silu_rows_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint8_t* __restrict__ sf, uint16_t* __restrict__ debug, int rows, int k) {
   pdl_trigger();
   const int lane = threadIdx.x & 31, chunks = (k + 511) >> 9;
   const int item = blockIdx.x * 8 + (threadIdx.x >> 5);
   const int group = item / chunks, col = ((item - group * chunks) << 9) + 16 * lane;
-  if (group >= ((rows + 127) & ~127) >> 1) return;
-  const int row0 = (group >> 6) * 128 + (group & 32) * 2 + (group & 31);
+  if (group >= ((rows + 127) & ~127) >> 2) return;
+  const int row0 = (group >> 5) * 128 + (group & 31);
   pdl_wait();
   struct Pair { Raw16 gate, up; };
   auto load = [&](Pair& to, int row) {
@@ -491,14 +488,20 @@ mx_silu_rows_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, 
     __syncwarp();
     return quantise16<T, false>(product, col < k ? out + int64_t(row) * k + col : nullptr, lane);
   };
+  uint32_t word[4] = {};
   Pair a, b;
   load(a, row0);
-  load(b, row0 + 32);
-  uint32_t word[2];
-  word[0] = convert(a, row0);
-  word[1] = convert(b, row0 + 32);
+#pragma unroll 1   // four copies of the body do not fit the instruction cache
+  for (int r = 0; r < 4; r += 2) {   // the next row's loads are in flight during a row's arithmetic
+    load(b, row0 + 32 * (r + 1));
+    word[0] = word[2];
+    word[1] = word[3];
+    word[2] = convert(a, row0 + 32 * r);
+    if (r == 0) load(a, row0 + 64);
+    word[3] = convert(b, row0 + 32 * (r + 1));
+  }
   if (col < k && (lane & 7) == 0)
-    *reinterpret_cast<uint2*>(sf + scale_word_offset(row0, col >> 7, k)) = make_uint2(word[0], word[1]);
+    *reinterpret_cast<uint4*>(sf + scale_word_offset(row0, col >> 7, k)) = make_uint4(word[0], word[1], word[2], word[3]);
 }
 
 // From this many elements on (SwiGLU: twice as many) the many-rows kernels are faster (K = 3584: 777 rows 3.2 us against 3.8,
@@ -588,7 +591,7 @@ template <typename T, bool FP4, bool SILU, int MATH>
 static cudaError_t launch_quant(const void* in, void* out, void* sf, void* debug, int rows, int k, cudaStream_t s) {
   if (int64_t(rows) * k >= (SILU ? 2 : 1) * kManyRowsElements && (reinterpret_cast<uintptr_t>(in) & 31) == 0) {   // 32-byte loads
     if constexpr (SILU) {
-      const int64_t groups = ((int64_t(rows) + 127) & ~int64_t(127)) / 2;
+      const int64_t groups = ((int64_t(rows) + 127) & ~int64_t(127)) / 4;
       return launch_kernel(mx_silu_rows_kernel<T, MATH>, dim3(row_blocks(groups, k)), dim3(256), 0, s, static_cast<const uint16_t*>(in),
                            static_cast<uint8_t*>(out), static_cast<uint8_t*>(sf), static_cast<uint16_t*>(debug), rows, k);
     } else {
