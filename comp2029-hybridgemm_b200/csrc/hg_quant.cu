@@ -296,7 +296,7 @@ mx_quant_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint
 // ---- Many rows: weights at load time, prefill activations -----------------------------------------------------------
 //
 // A warp owns rows r, r+32, r+64, r+96 of a 128-row scale block x 512 columns, sixteen consecutive values per lane and row,
-// and has its four 32-byte loads (SwiGLU: eight) in flight before it converts the first.  Sixteen values per lane halve the
+// and has their four 32-byte loads in flight (SwiGLU: those of the next row during a row's arithmetic).  Sixteen values per lane halve the
 // instructions per value against eight (one shuffle, one exponent and one scale byte per sixteen, maxima in packed 16-bit
 // form): the kernel above is bound by them, 3.8 TB/s on a 272 MB weight matrix.  The four rows share the 16-byte
 // entries of the scale atoms, so scales leave as whole entries instead of single words, each a partial write of a
