@@ -13,6 +13,7 @@
 #include <ATen/core/Tensor.h>
 #include <ATen/ops/empty.h>
 #include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -39,7 +40,7 @@ struct Ready {
   void* handle;
   const hg_problem *low, *high;                       // inside `problems`
   int64_t tokens, k, outputs, packed;                 // packed: bytes of the quantised activations
-  bool fused;                                         // calls quantise inside the GEMM launch
+  int fused;                                          // calls quantise inside the GEMM launch: 0 none, 1 all, 2 eager ones
   at::TensorOptions output;
   c10::Device device = c10::Device(c10::kCPU);
 };
@@ -189,7 +190,7 @@ PyObject* forward_checked(PyObject* self, const at::Tensor& x, long math) {
     const Unlocked unlocked;
     // Fresh tensors per call: under CUDA-graph capture the graph's pool owns them.
     y = at::empty({r->tokens, r->outputs}, r->output);
-    const bool in_gemm = !swiglu && r->fused;
+    const bool in_gemm = !swiglu && (r->fused == 1 || (r->fused == 2 && c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None));
     const int64_t bytes = in_gemm ? 0 : r->packed;
     // Scratch that nobody else sees: the allocator itself, for the same stream and with the same lifetime, without a tensor round it
     // (0.45 us of a call of two launches, of which the host then needs 6.7 us).
@@ -235,7 +236,7 @@ PyObject* prepare(PyObject*, PyObject* args) {
   long long tokens, packed;
   int fused;
   unsigned long long handle, low, high;
-  if (!PyArg_ParseTuple(args, "OLKKKOOLp", &layer, &tokens, &handle, &low, &high, &problems, &y, &packed, &fused)) return nullptr;
+  if (!PyArg_ParseTuple(args, "OLKKKOOLi", &layer, &tokens, &handle, &low, &high, &problems, &y, &packed, &fused)) return nullptr;
   if (!THPVariable_Check(y)) return PyErr_SetString(PyExc_TypeError, "prepare: y must be a tensor"), nullptr;
   auto* r = new Ready{};
   r->problems = Py_NewRef(problems);

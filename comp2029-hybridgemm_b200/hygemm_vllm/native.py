@@ -266,7 +266,9 @@ class DualLinear:
         y = torch.empty((tokens, self.outputs), dtype=self.dtype, device=x.device)
         low, high = self.problems(x, x, y)
         handle = self._handle(tokens, self.low_id, self.high_id, C.byref(low), C.byref(high), _stream(x.device))
-        fused = quantises_in_gemm(tokens, self.outputs)
+        fused = int(quantises_in_gemm(tokens, self.outputs))
+        if self.low_id or self.high_id:   # an explicit schedule: the kernel of hg_gemm_tc.cu, whose quantisers save a launch and no time on the GPU
+            fused = (1 if tokens == 1 else 2) if fused and self.outputs <= FUSED_QUANT_MAX_OUTPUTS else 0
         self._ready[tokens] = _host.prepare(self, tokens, handle.value, C.addressof(low), C.addressof(high), (low, high), y,
                                             tokens * self.k + scale_size(tokens, self.k), fused)
         result = _host.forward(self, x, math)
