@@ -812,12 +812,19 @@ static double plan_cost(const ClusterPlan& plan, int units, int kblocks, double 
     return fit.cta * ctas + (plan.pair == 2 ? fit.pair : 0) + fit.cut * plan.cut_log[0] + fit.finer * (plan.cut_log[1] - plan.cut_log[0]) +
            std::max(busiest, least) + exchange;
   };
-  // Cluster 0 has the most units.  (The margin is far above the rounding of the sums below.)
+  // Cluster 0 has the most units, and no plan is done before an average cluster's main loops and the last one's stores are, or before
+  // an average cluster's stores and the main loop of the first ones are.  (The margin is far above the rounding of the sums below.)
   const int most = (units + plan.clusters - 1) / plan.clusters;
-  double shortest = 1e30;
+  double main_least = 1e30, main_all = 0, store_least = 1e30, store_all = 0;
   for (int part = 0; part < 2; ++part)
-    if (plan.tiles[part]) shortest = std::min({shortest, main_of[part][0], main_of[part][1]});
-  if (const double bound = total(most * shortest * (1 - 1e-9)); bound >= reject) return bound;
+    if (plan.tiles[part]) {
+      main_least = std::min({main_least, main_of[part][0], main_of[part][1]});
+      store_least = std::min({store_least, store_of[part][0], store_of[part][1]});
+      main_all += plan.tiles[part] * ((plan.token_tiles - 1) * main_of[part][0] + main_of[part][1]);
+      store_all += plan.tiles[part] * ((plan.token_tiles - 1) * store_of[part][0] + store_of[part][1]);
+    }
+  const double soonest = std::max(std::max(most * main_least, main_all / plan.clusters) + store_least, main_least + store_all / plan.clusters);
+  if (const double bound = total(soonest * (1 - 1e-9)); bound >= reject) return bound;
 
   // End of a cluster's main loops and of its stores.  Two accumulators: a main loop starts once the stores before the last ones are done.
   struct Ends { double main = 0, stores = 0; };
@@ -836,6 +843,7 @@ static double plan_cost(const ClusterPlan& plan, int units, int kblocks, double 
   } else {
     std::vector<Ends> ends(size_t(plan.clusters));
     const int tiles = plan.tiles[0] + plan.tiles[1];
+    const double enough = (reject - total(0) + least) * (1 + 1e-9);   // a cluster that is busy for so long decides against the plan
     int cluster = 0, round = 0;   // of the next unit; see unit_at
     int spread = 0;               // how far the running share of MXFP8 tiles is beyond the last whole one
     for (int t = 0; t < tiles; ++t) {
@@ -844,11 +852,13 @@ static double plan_cost(const ClusterPlan& plan, int units, int kblocks, double 
       if (high) spread -= tiles;
       const int last = plan.token_tiles - 1 - (plan.turned ? round % plan.token_tiles : 0);
       for (int tt = 0; tt < plan.token_tiles; ++tt) {
-        add(ends[size_t(cluster)], high, tt == last);
+        Ends& e = ends[size_t(cluster)];
+        add(e, high, tt == last);
+        busiest = std::max(busiest, e.stores);
         if (++cluster == plan.clusters) { cluster = 0; ++round; }
       }
+      if (busiest >= enough) return total(busiest);
     }
-    for (const Ends& e : ends) busiest = std::max(busiest, e.stores);
   }
   return total(busiest);
 }
@@ -870,6 +880,37 @@ static bool finish_plan(ClusterPlan& plan, int most_stages) {
   return false;
 }
 
+// Token tiles of a prompt: `count` of them, `step` tokens each, the last one holding what is left (`tail`, in MMA columns).
+struct TokenTiles { int step, count, tail, sf_atoms; };
+
+// Steps of 128, 256 and 192 tokens, and those of 128 and 192 with a short last tile joined to the one before it, so that the tiles of a
+// ragged prompt fit the clusters: 37888 x 3584 at 160 tokens in one tile 31.5 -> 25.0 us, at 300 in 192 + 108 48.9 -> 45.0, 3584 x
+// 18944 at 777 in 3 x 192 + 201 54.4 -> 49.4, 4608 x 3584 at 2048 by steps of 192 36.1 -> 31.8.  hg_plan tells its callers the
+// widest tile, of which a prompt has ceil(tokens / widest): joined tails that would need a tile more are left out (beyond 1376 tokens
+// all of them).  Each split is listed once: a search walks it in up to 15 ways, and every new length of a prompt pays for one search per
+// layer.
+static int token_tiles_of(int tokens, TokenTiles (&ways)[5]) {
+  int n = 0;
+  for (const int way : {128, 256, 192, -128, -192}) {
+    TokenTiles t;
+    t.step = std::abs(way);
+    t.count = way < 0 ? tokens / t.step : (tokens + t.step - 1) / t.step;
+    if (t.count < 1) continue;
+    t.tail = (tokens - (t.count - 1) * t.step + 31) / 32 * 32;
+    if (t.tail > 256) continue;
+    if (t.count == 1) t.step = t.tail;
+    const int widest = std::max(t.step, t.tail);
+    if ((tokens + widest - 1) / widest != t.count) continue;
+    // Atoms that the last tile and the first ones touch; a second one may start in the middle of its first.
+    const int last_start = (t.count - 1) * t.step % 128, odd_start = t.count > 2 ? t.step % 128 : 0;
+    t.sf_atoms = std::max(last_start + t.tail + 127, t.count > 1 ? odd_start + t.step + 127 : 0) / 128;
+    bool listed = false;
+    for (int i = 0; i < n; ++i) listed |= ways[i].step == t.step && ways[i].count == t.count;
+    if (!listed) ways[n++] = t;
+  }
+  return n;
+}
+
 ClusterPlan make_cluster_plan(int lo, int hi, int tokens, int k, const int max_clusters[4]) {
   const int kblocks = k / kTileK, steps = (kblocks + 1) / 2;
   const int atoms[2] = {(lo + kTileRows - 1) / kTileRows, (hi + kTileRows - 1) / kTileRows};
@@ -877,17 +918,14 @@ ClusterPlan make_cluster_plan(int lo, int hi, int tokens, int k, const int max_c
   best.cost = 1e30;
   const int force_split = tuning("HYGEMM_CL_SPLIT", 0), force_pair = tuning("HYGEMM_CL_PAIR", 0), force_n = tuning("HYGEMM_CL_N", 0);
   const int force_cut = tuning("HYGEMM_CL_CUT", -1), force_cut_high = tuning("HYGEMM_CL_CUT_HIGH", -1);
-  // Token tiles of `way` tokens (0: one tile), the last one holding what is left; -way: with what is left joined to the one before.
-  const std::array<int, 5> decode_ways{0, 64}, prefill_ways{128, 256, 192, -128, -192};
-  const std::array<int, 5>& all_ways = tokens <= 128 ? decode_ways : prefill_ways;
-  const int* const ways_end = all_ways.data() + (tokens <= 128 ? 2 : 5);
+  TokenTiles ways[5];
+  const int n_ways = tokens <= 128 ? 2 : token_tiles_of(tokens, ways);
   const int most_stages = std::min(kClusterMaxStages, tuning("HYGEMM_CL_STAGES", kClusterMaxStages));
   for (int pair = 1; pair <= 2; ++pair)
     for (int log = pair - 1; log < 4; ++log)
       for (int cut = 0; cut < 3; ++cut)
         for (int more = 0; more < 3; ++more)
-          for (const int* way_at = all_ways.data(); way_at < ways_end; ++way_at) {
-              const int way = *way_at;
+          for (int way = 0; way < n_ways; ++way) {
               ClusterPlan plan;
               plan.pair = pair;
               plan.split = (1 << log) / pair;
@@ -900,25 +938,20 @@ ClusterPlan make_cluster_plan(int lo, int hi, int tokens, int k, const int max_c
                 // at 77 tokens 7.3 -> 6.7), wide and long ones do not (37888 x 3584 23.7 -> 27.0, 3584 x 18944 16.1 -> 17.1).
                 if ((way && tokens <= 64) || (!way && tokens > 64 && pair == 1) || (tokens <= 32 && pair == 2)) continue;   // (fused quantisation: single CTAs)
                 plan.token_tiles = way ? 2 : 1;
-                plan.n_tail = (tokens - way + 16 * pair - 1) / (16 * pair) * (16 * pair);
-                plan.n_step = way ? way : plan.n_tail;
+                plan.n_tail = (tokens - 64 * way + 16 * pair - 1) / (16 * pair) * (16 * pair);
+                plan.n_step = way ? 64 : plan.n_tail;
+                plan.n_tile = std::max(plan.n_step, plan.n_tail);
+                plan.sf_atoms = 1;
               } else {
-                // Steps of 192 beside those of 128 and 256, and a short last tile joined to the one before it, so that the tiles of a ragged
-                // prompt fit the clusters: 37888 x 3584 at 160 tokens in one tile 31.5 -> 25.0 us, at 300 in 192 + 108 48.9 -> 45.0, 3584 x 18944
-                // at 777 in 3 x 192 + 201 54.4 -> 49.4, 4608 x 3584 at 2048 by steps of 192 36.1 -> 31.8.
                 if (pair == 1 || cut) continue;
-                plan.n_step = std::abs(way);
-                plan.token_tiles = way < 0 ? tokens / plan.n_step : (tokens + plan.n_step - 1) / plan.n_step;
-                if (plan.token_tiles < 1) continue;
-                plan.n_tail = (tokens - (plan.token_tiles - 1) * plan.n_step + 31) / 32 * 32;
-                if (plan.n_tail > 256) continue;
-                if (plan.token_tiles == 1) plan.n_step = plan.n_tail;
+                const TokenTiles& t = ways[way];
+                plan.token_tiles = t.count;
+                plan.n_step = t.step;
+                plan.n_tail = t.tail;
+                plan.n_tile = std::max(t.step, t.tail);
+                plan.sf_atoms = t.sf_atoms;
+                if (plan.n_tile > 224 && plan.split > 1) continue;
               }
-              plan.n_tile = std::max(plan.n_step, plan.n_tail);
-              if (tokens > 128 && ((tokens + plan.n_tile - 1) / plan.n_tile != plan.token_tiles || (plan.n_tile > 224 && plan.split > 1))) continue;
-              // Atoms that the last tile and the first ones touch; a second one may start in the middle of its first.
-              const int last_start = (plan.token_tiles - 1) * plan.n_step % 128, odd_start = plan.token_tiles > 2 ? plan.n_step % 128 : 0;
-              plan.sf_atoms = std::max(last_start + plan.n_tail + 127, plan.token_tiles > 1 ? odd_start + plan.n_step + 127 : 0) / 128;
               if ((force_split && plan.split != force_split) || (force_pair && pair != force_pair) || (force_n && plan.n_tile != force_n) ||
                   (force_cut >= 0 && cut != force_cut) || (force_cut_high >= 0 && cut + more != force_cut_high))
                 continue;
