@@ -105,3 +105,38 @@ def to_float(bits16: np.ndarray, dtype) -> np.ndarray:
 
 def rel_frobenius(got: np.ndarray, ref: np.ndarray) -> float:
     return float(np.linalg.norm(got.astype(np.float64) - ref) / max(np.linalg.norm(ref), 1e-30))
+
+
+def swiglu_unit_probe(gate: torch.Tensor):
+    """`up` [gates, 32] such that one unit of a gate's 16-bit activation shows in the MXFP8 bytes of the K32 group of its 32 products, and
+    the activations' bits.
+
+    A gate fills a group by itself, so no larger product sets its scale.  `up` lies in one binade that brings the products near one;
+    its values are chosen where the activation, its neighbours and theirs fall on two sides of a rounding boundary of E4M3 (the
+    activation by fp64, so the kernels' may be a neighbour of it), the last one is the largest and fixes the scale."""
+    dtype, device = gate.dtype, gate.device
+    mantissas, bias, low, high = (1024, 15, -14, 15) if dtype == torch.float16 else (128, 127, -126, 127)
+    bits = (gate.double() / (1 + torch.exp(-gate.double()))).to(dtype).view(torch.int16)
+    sign, magnitude = bits < 0, bits.int() & 0x7FFF
+    top = int(torch.tensor(torch.finfo(dtype).max, dtype=dtype).view(torch.int16))
+    def value(m):
+        return torch.where(sign, -m, m)
+
+    def activation(step):
+        m = (magnitude + step).clamp(1, top).to(torch.int16).view(dtype).float()
+        return value(m)
+    exponent = torch.frexp(activation(0)).exponent - 1
+    scale = torch.exp2((-exponent).clamp(low, high).double())
+    candidates = 1 + torch.arange(mantissas, device=device, dtype=torch.float64) / mantissas
+    ups = (scale[:, None] * candidates).to(dtype)
+    def codes(step, e):
+        product = (activation(step)[:, None] * ups.float()).to(dtype).double()
+        return (product * torch.exp2(-e.double())[:, None]).float().clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8)
+    largest = (activation(0) * ups[:, -1].float()).to(dtype).double().abs()
+    mantissa, e = torch.frexp(largest)
+    e = e - 9 + (mantissa > 0.875).int()
+    at = {step: codes(step, e) for step in (-2, -1, 0, 1, 2)}
+    chosen = [torch.topk((at[step] != at[step + 1]).to(torch.float32), 8, dim=1).indices for step in (-2, -1, 0, 1)]
+    index = torch.cat(chosen, 1)
+    index[:, -1] = mantissas - 1
+    return ups.gather(1, index), bits

@@ -11,7 +11,7 @@ import pytest
 import torch
 
 import oracle
-from helpers import expected_work, run_gemm
+from helpers import expected_work, run_gemm, swiglu_unit_probe
 from hygemm_vllm import native, producer
 
 pytestmark = pytest.mark.gpu
@@ -279,21 +279,23 @@ def test_swiglu_of_every_gate_value(dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-def test_swiglu_of_every_gate_from_minus_six_on(dtype):
-    """Lanes whose gates all lie above -6 take the narrower window around rounding boundaries: every such gate, infinity too, beside none
-    below, each with eight values of up, gives the bytes of the exact functions (whole values: tolerance 0)."""
-    k = 1024
-    every = torch.arange(65536, device="cuda").to(torch.int16).view(dtype)
-    gate = every[every >= -6].repeat(8)
-    gate = torch.cat([gate, gate[:-gate.numel() % k]])
-    g = torch.Generator(device="cuda").manual_seed(12)
-    gate = gate[torch.randperm(gate.numel(), device="cuda", generator=g)].view(-1, k)
-    x = torch.cat([gate, torch.randn(gate.shape, device="cuda", generator=g).to(dtype)], 1).contiguous()
-    many = x.repeat(-(-8200 // x.shape[0]), 1)   # the many-rows producer starts at 8 Mi elements
-    for part in (x[:256].contiguous(), x[256:].contiguous(), many):
-        q, sf = producer.silu_pack(part, 0)
-        exact_q, exact_sf, _ = producer.silu_pack(part, 0, debug=True)
-        assert torch.equal(q, exact_q) and torch.equal(sf, exact_sf)
+def test_swiglu_of_every_gate_to_the_last_unit(dtype):
+    """The producers' activations of all finite gates, wide and narrow window around rounding boundaries, are the exact functions' to the last
+    of their 16 bits: a gate has a K32 group to itself and values of up with which one unit shows in its bytes (tolerance 0; the CPU test of
+    `swiglu_unit_probe` plants the unit).  One row, few rows, many rows (from 8 Mi elements)."""
+    gate = torch.arange(65536, device="cuda").to(torch.int16).view(dtype)
+    gate = gate[torch.isfinite(gate)].sort().values
+    gate = torch.cat([gate, gate[:-gate.numel() % 2304]])
+    up, _ = swiglu_unit_probe(gate)
+    pairs = torch.stack([gate[:, None].expand_as(up), up])
+    for k, rows in ((1024, 1), (1024, 300), (1024, 8208), (9216, 57)):
+        part = pairs.reshape(2, -1, k)
+        part = torch.cat([part[0], part[1]], 1)
+        part = part.repeat(-(-rows // part.shape[0]), 1)
+        for x in part[:8].split(1) if rows == 1 else part.split(rows):
+            q, sf = producer.silu_pack(x, 0)
+            exact_q, exact_sf, _ = producer.silu_pack(x, 0, debug=True)
+            assert torch.equal(q, exact_q) and torch.equal(sf, exact_sf), (k, rows)
 
 
 @pytest.mark.parametrize("tokens", [1, 2, 7, 8, 9, 16])

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 import oracle
+from helpers import swiglu_unit_probe
 
 ALL16 = np.arange(65536, dtype=np.uint16)
 
@@ -257,3 +258,28 @@ def test_clip_search_never_increases_the_weighted_error():
 
     after, before = error(q4, scales), error(base_q, base_sf[oracle.scale_indices(64, 384)])
     assert (after <= before * (1 + 1e-6) + 1e-25).all() and after.sum() < before.sum()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_swiglu_unit_probe_shows_one_unit_of_every_gate(dtype):
+    """The inputs of the GPU test that pins the SwiGLU activations to the last bit: with one unit more or less in a gate's activation the bytes
+    of its K32 group differ, for every finite gate with an activation that has such a neighbour."""
+    gate = torch.arange(65536).to(torch.int16).view(dtype)
+    gate = gate[torch.isfinite(gate)]
+    up, bits = swiglu_unit_probe(gate)
+
+    def pack(activation):
+        product = (activation.view(dtype).float()[:, None] * up.float()).to(dtype).reshape(-1, 128)
+        codes, scales = oracle.pack(product, bf16=dtype == torch.bfloat16)
+        return codes.reshape(-1, 32), scales[oracle.scale_indices(*product.shape)].reshape(-1)
+
+    codes, scales = pack(bits)
+    largest = int(torch.tensor(torch.finfo(dtype).max, dtype=dtype).view(torch.int16))
+    magnitude = bits.int() & 0x7FFF
+    for step in (-1, 1):
+        planted = magnitude + step
+        has_neighbour = ((magnitude > 0) & (planted > 0) & (planted <= largest)).numpy()
+        assert has_neighbour.sum() > 0.4 * len(gate)
+        wrong = pack(torch.where(bits < 0, planted - 32768, planted).to(torch.int16))
+        differs = (wrong[0] != codes).any(1) | (wrong[1] != scales)
+        assert differs[has_neighbour].all(), gate[torch.from_numpy(has_neighbour & ~differs)]
