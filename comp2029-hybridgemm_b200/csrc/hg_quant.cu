@@ -145,10 +145,10 @@ __device__ __forceinline__ float reciprocal_fast(float x) { float r; asm("rcp.ap
 //
 // Doubtful pairs are collected and computed one after the other at the end, all lanes' first ones together: a warp takes the exact
 // functions once or twice for its 32 x 2 N values, and not up to N times (fp16: of sixteen pairs of a warp four had a value in
-// doubt).
+// doubt).  IN_PLACE: each behind a branch of its own, which needs fewer registers (see in_place).
 constexpr uint32_t kDoubt = 20, kDoubtNear = 10;
 constexpr float kNearGate = -6.f;
-template <typename T, int N>
+template <typename T, bool IN_PLACE = false, int N>
 __device__ __forceinline__ void silu_fast(const uint32_t (&gate)[N], const uint32_t (&up)[N], uint32_t (&product)[N]) {
   constexpr bool kHalf = std::is_same<T, __half>::value;
   constexpr int kShift = kHalf ? 19 : 16;                        // brings the bits below the 16-bit mantissa to the top
@@ -164,15 +164,19 @@ __device__ __forceinline__ void silu_fast(const uint32_t (&gate)[N], const uint3
     const float2 g = Packed<T>::widen(gate[i]);
     const float2 t = mul2(g, make_float2(-1.44269504f, -1.44269504f));
     const float2 s = add2(make_float2(exp2_fast(t.x), exp2_fast(t.y)), make_float2(1.f, 1.f));
-    const float2 act = mul2(g, make_float2(reciprocal_fast(s.x), reciprocal_fast(s.y)));
+    float2 act = mul2(g, make_float2(reciprocal_fast(s.x), reciprocal_fast(s.y)));
     const uint32_t x = __float_as_uint(act.x) * (1u << kShift) - boundary, y = __float_as_uint(act.y) * (1u << kShift) - boundary;
     bool doubt = min(x, y) <= 2 * window;
     if constexpr (kHalf)   // below 2^-14; zeros, which are exact, wrap round
       doubt |= min((__float_as_uint(act.x) & 0x7fffffffu) - 1u, (__float_as_uint(act.y) & 0x7fffffffu) - 1u) < 0x38800000u - 1u;
-    if (doubt) doubtful |= 1u << i;
+    if constexpr (IN_PLACE) {
+      if (__builtin_expect(doubt || fminf(g.x, g.y) < -16.f, 0)) act = make_float2(g.x / (1.f + expf(-g.x)), g.y / (1.f + expf(-g.y)));
+    } else if (doubt) {
+      doubtful |= 1u << i;
+    }
     product[i] = Packed<T>::swiglu(act, up[i]);
   }
-  if (__builtin_expect(doubtful != 0 || lowest < -16.f, 0)) {
+  if (!IN_PLACE && __builtin_expect(doubtful != 0 || lowest < -16.f, 0)) {
     if (lowest < -16.f) {
 #pragma unroll
       for (int i = 0; i < N; ++i) {
@@ -197,8 +201,8 @@ __device__ __forceinline__ void silu_fast(const uint32_t (&gate)[N], const uint3
   }
 }
 
-template <typename T, bool FP4, bool SILU, int MATH>
-__global__ void __launch_bounds__(256)
+template <typename T, bool FP4, bool SILU, int MATH, bool IN_PLACE = false>
+__global__ void __launch_bounds__(256, IN_PLACE ? 8 : 0)
 mx_quant_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint8_t* __restrict__ sf,
                 uint16_t* __restrict__ debug, int rows, int k) {
   pdl_trigger();
@@ -243,7 +247,7 @@ mx_quant_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint
     if (!exact) {
       const uint32_t g[4] = {g4.x, g4.y, g4.z, g4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w};
       uint32_t p[4];
-      silu_fast<T>(g, u, p);
+      silu_fast<T, IN_PLACE>(g, u, p);
       widen8<T>(make_uint4(p[0], p[1], p[2], p[3]), v);
       if constexpr (!std::is_same<T, __half>::value) {
         uint32_t top = 0;
@@ -510,6 +514,14 @@ mx_silu_rows_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, 
 // 107 us against 56.
 constexpr int64_t kManyRowsElements = 4 << 20;
 
+// Where the few-rows SwiGLU takes doubtful pairs in place (fp16).  It runs beside the GEMM of gate_up, whose pairs of CTAs (from 33 tokens
+// on) leave 4096 registers in three of an SM's four parts: two blocks of 32 registers a thread, one of 40, which is what collecting the
+// pairs needs.  Where gate_up fills the chip (144 row tiles) and the blocks find room in twos, or nearly so, one in ones is a wave more:
+// gate_up and SwiGLU + down of 4096 x 14336 at 37 tokens (259 blocks) 28.5 us in place, 29.4 collected; of 4096 x 11008 at 40 25.1 and
+// 25.6, at 56 (301 blocks) 26.1 and 26.5; of 3584 x 9344 at 64 22.3 and 23.2.  Elsewhere collecting is 1 to 2 % better (8192
+// channels at 64 tokens 22.3 and 21.9; 14336 at 44, 308 blocks, 30.0 and 29.7; 18944 at 33, 305 blocks, 30.7 and 30.4).
+static bool in_place(int rows, int k) { return rows > 32 && 2 * k >= 144 * 128 && int64_t(rows) * k <= 302 * 2048; }
+
 static unsigned row_blocks(int64_t groups, int k) { return unsigned((groups * ((k + 511) / 512) + 7) / 8); }
 
 template <typename T>
@@ -603,6 +615,11 @@ static cudaError_t launch_quant(const void* in, void* out, void* sf, void* debug
   const int64_t pad_rows = ((rows + 127) & ~127) - rows;
   const int64_t threads = int64_t(rows) * kblocks * 16 + pad_rows * kblocks;
   const int64_t blocks = (threads + 255) / 256;
+  if constexpr (SILU && MATH == 0 && std::is_same<T, __half>::value)
+    if (in_place(rows, k))
+      return launch_kernel(mx_quant_kernel<T, FP4, SILU, MATH, true>, dim3(unsigned(blocks)), dim3(256), 0, s,
+                           static_cast<const uint16_t*>(in), static_cast<uint8_t*>(out), static_cast<uint8_t*>(sf),
+                           static_cast<uint16_t*>(debug), rows, k);
   return launch_kernel(mx_quant_kernel<T, FP4, SILU, MATH>, dim3(unsigned(blocks)), dim3(256), 0, s,
                        static_cast<const uint16_t*>(in), static_cast<uint8_t*>(out), static_cast<uint8_t*>(sf),
                        static_cast<uint16_t*>(debug), rows, k);

@@ -282,7 +282,7 @@ def test_swiglu_of_every_gate_value(dtype):
 def test_swiglu_of_every_gate_to_the_last_unit(dtype):
     """The producers' activations of all finite gates, wide and narrow window around rounding boundaries, are the exact functions' to the last
     of their 16 bits: a gate has a K32 group to itself and values of up with which one unit shows in its bytes (tolerance 0; the CPU test of
-    `swiglu_unit_probe` plants the unit).  One row, few rows, many rows (from 8 Mi elements)."""
+    `swiglu_unit_probe` plants the unit).  One row of 1024, few rows, many rows (from 8 Mi elements) and, wide and of 33 rows or more, in place."""
     gate = torch.arange(65536, device="cuda").to(torch.int16).view(dtype)
     gate = gate[torch.isfinite(gate)].sort().values
     gate = torch.cat([gate, gate[:-gate.numel() % 2304]])
@@ -296,6 +296,17 @@ def test_swiglu_of_every_gate_to_the_last_unit(dtype):
             q, sf = producer.silu_pack(x, 0)
             exact_q, exact_sf, _ = producer.silu_pack(x, 0, debug=True)
             assert torch.equal(q, exact_q) and torch.equal(sf, exact_sf), (k, rows)
+
+
+@pytest.mark.parametrize("rows,k", [(32, 9216), (33, 9088), (33, 9216), (67, 9216), (68, 9216), (33, 18688), (33, 18816)])
+def test_swiglu_where_doubtful_pairs_are_taken_in_place(rows, k):
+    """Around the edges of the rule (33 rows, 9216 channels, 302 blocks of 2048 elements), both types: the exact functions' bytes."""
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    for dtype in (torch.float16, torch.bfloat16):
+        x = (torch.randn(rows, 2 * k, device="cuda", generator=g) * 5).to(dtype)
+        q, sf = producer.silu_pack(x, 0)
+        exact_q, exact_sf, _ = producer.silu_pack(x, 0, debug=True)
+        assert torch.equal(q, exact_q) and torch.equal(sf, exact_sf)
 
 
 @pytest.mark.parametrize("tokens", [1, 2, 7, 8, 9, 16])
