@@ -58,6 +58,21 @@ def test_exact_in_tiles_that_fit_a_ragged_prompt(tokens, width, monkeypatch):
         assert np.array_equal(got, case["expected"]), (outputs, k, high, split, int((got != case["expected"]).sum()))
 
 
+@pytest.mark.parametrize("tokens", [801, 820, 832])
+@pytest.mark.parametrize("outputs,k,high", [(8269, 384, 800), (18944, 128, 1000), (18944, 1152, 2000)])
+def test_exact_with_a_last_tile_of_256_tokens_behind_tiles_of_192(outputs, k, high, tokens, monkeypatch):
+    """Steps of 192 with what is left joined to the last one: two accumulators that share columns serve tiles of unlike width, and 256
+    columns start in the middle of a scale atom and read three.  Every cluster has several units; steps of 256 would need two atoms."""
+    monkeypatch.setenv("HYGEMM_CL_N", "256")
+    case = oracle.exact_case(outputs, tokens, k, high, "random")
+    header = (C.c_int * 12)()
+    native.check(native.library().hg_plan(outputs - high, high, tokens, k, torch.cuda.get_device_properties(0).multi_processor_count, 0, header, None, 0))
+    assert list(header[2:6]) == [256, 4, 3, 210208] and header[9] >= 1.9 * header[1], list(header)
+    got, guards, status = run_gemm(case, torch.bfloat16, 0)
+    assert status[0] == 0 and guards and (status[1], status[2]) == expected_work(case, 0), status
+    assert np.array_equal(got, case["expected"]), int((got != case["expected"]).sum())
+
+
 @pytest.mark.parametrize("pair", [1, 2])
 @pytest.mark.parametrize("split", [1, 2, 4])
 @pytest.mark.parametrize("tokens", [65, 80, 97, 128])
