@@ -228,7 +228,7 @@ class Sweep:
             total += 1 + sum(launches_of(layer[name], m) for name in SHAPES)
             for name in ("qkv", "o_proj", "gate_up"):
                 exchanged = name == "o_proj" and self.exchange is not None
-                total += m > self.native.FUSED_QUANT_TOKENS if exchanged else not self.native.quantises_in_gemm(m, layer[name].outputs, layer[name].k)
+                total += m > self.native.FUSED_QUANT_TOKENS if exchanged else not self.native.quantises_in_gemm(m, layer[name].outputs)
             total += 2 * (self.exchange is not None)
         return total
 
@@ -267,8 +267,8 @@ class Sweep:
             events.append((name, m, a, b))
             return y
 
-        # What `layer(x)` (the plugin-facing call) does when captured: the activations are quantised inside the GEMM launch (hg_run_x)
-        # for few tokens; else the quantiser is its own launch.  Events bracket the GEMM launch.
+        # What `layer(x)` (the plugin-facing call) does: the activations are quantised inside the GEMM launch (hg_run_x) up to
+        # 16 tokens, in wide layers up to 8; else the quantiser is its own launch.  Events bracket the GEMM launch.
         def linear(name, xin, row_parallel=False):
             rt = layer[name]
             if row_parallel and self.exchange is not None:
@@ -276,7 +276,7 @@ class Sweep:
                     return timed(name, lambda: rt.run_exchange(self.exchange, x=xin))
                 q, sf = native.pack(xin)
                 return timed(name, lambda: rt.run_exchange(self.exchange, q=q, sf=sf))
-            if native.quantises_in_gemm(m, rt.outputs, rt.k):
+            if native.quantises_in_gemm(m, rt.outputs):
                 return timed(name, lambda: rt(xin))
             q, sf = native.pack(xin)
             return timed(name, lambda: rt.run_packed(q, sf))
@@ -895,7 +895,7 @@ def main():
             "config": {"workload": "Qwen2.5-7B layer-shape hybrid GEMM sweep: qkv 3584->4608, o_proj 3584->3584, "
                                    "gate_up 3584->37888, down 18944->3584; M in 1,2,4,8,16,32,64,128; 10% MXFP8 channels",
                        "step": "per M: quantise+qkv, quantise+o_proj, quantise+gate_up, SwiGLU-quantise+down "
-                               "(the quantisers run inside the GEMM launch up to M=8)",
+                               "(the quantisers run inside the GEMM launch up to M=16, gate_up's up to M=8)",
                        "parallelism": f"tp{world}" if world > 1 else "single GPU",
                        **({"row_parallel_sum": sweep.exchange_note} if world > 1 else {}),
                        "l2": "inputs larger than L2: two weight sets (272 MB) alternate between consecutive M",

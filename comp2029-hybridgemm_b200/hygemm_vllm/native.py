@@ -32,15 +32,16 @@ class Problem(C.Structure):
 
 
 PACK_MODE = int(os.environ.get("HYGEMM_PACK_MODE", "0"))
-# Calls of at most FUSED_QUANT_TOKENS tokens may quantise the activations inside the GEMM kernel (`hg_run_x`: one launch instead of
-# two, identical bytes); `quantises_in_gemm` has the rule, HYGEMM_FUSED_QUANT=0 turns it off.  A width that is asked for by
-# HYGEMM_FUSED_QUANT_MAX_OUTPUTS holds at every token count, and no wider layer does it.
+# Calls of at most FUSED_QUANT_TOKENS tokens quantise the activations inside the GEMM kernel (`hg_run_x`: one launch instead of
+# two, identical bytes); HYGEMM_FUSED_QUANT=0 turns it off.
 FUSED_QUANT_TOKENS = 16 if os.environ.get("HYGEMM_FUSED_QUANT", "1") != "0" else 0
+# Every CTA quantises the K slice it multiplies, so the work repeats once per row tile.  Layers wider than this many output
+# channels keep the separate quantiser launch from FUSED_QUANT_WIDE_TOKENS + 1 tokens on: a captured decoder block with gate_up,
+# 37888 wide, takes 39.0 us against 40.4 with gate_up's own quantiser launch at 8 tokens, and 41.0 either way at 16.  A width
+# that is asked for holds at every token count.
 _max_outputs = os.environ.get("HYGEMM_FUSED_QUANT_MAX_OUTPUTS")
 FUSED_QUANT_MAX_OUTPUTS = int(_max_outputs or "8192")
 FUSED_QUANT_WIDE_TOKENS = 0 if _max_outputs else min(8, FUSED_QUANT_TOKENS)
-FUSED_QUANT_CAPTURED_TOKENS = FUSED_QUANT_TOKENS if _max_outputs else min(12, FUSED_QUANT_TOKENS)
-FUSED_QUANT_SMALL_LAYER = 4 << 20
 # Row-parallel exchange: up to this many tokens the partial sums cross NVLink as fp32 (rounded once after the sum).
 FUSED_QUANT_TOKENS_F32 = 16
 # Launch policies of hg_run (reference: native.py:14-15).
@@ -129,21 +130,9 @@ def scale_size(rows: int, k: int) -> int:
     return ((rows + 127) // 128) * (k // 128) * 512 if rows > 0 and k > 0 else 0
 
 
-def quantises_in_gemm(tokens: int, outputs: int, k: int, captured: bool = True) -> bool:
-    """Whether a plain call of a layer quantises its activations inside the GEMM launch.
-
-    Every CTA quantises the K that it multiplies, so the work repeats once per row tile.  An eager call saves the host's time for a launch
-    (2.5 us) and does it up to 16 tokens.  A captured one does not pay that, and its separate quantiser may run under the GEMM
-    in front: up to 12 tokens the single launch is better or level (4608 x 3584 at 12: 5.44 -> 5.03 us back to back, 8.80 -> 8.19 behind a
-    kernel that writes the input, that one included; 3584 x 18944 10.15 -> 10.27 and 13.41 -> 12.68), above that only in layers of up to 4 Mi
-    weights (896 x 896 at 16 3.46 -> 2.70 and 5.89 -> 5.63; but 3584 x 3584 4.76 -> 4.92 and 7.39 -> 7.34, and a decode block of
-    that width at 14 tokens 25.3 -> 26.1).  Wider than 8192 channels CTAs have several row tiles: up to 8 tokens (37888 x 3584 at 8: 15.3 ->
-    14.3 and 17.7 -> 17.4; 28672 x 8192, the worst of those measured, 27.4 -> 26.4 and 30.2 -> 30.7; two launches from 9 on: 22016 x
-    4096 at 10 behind its writer 17.0 us, 17.3 in one)."""
-    if outputs > FUSED_QUANT_MAX_OUTPUTS:
-        return tokens <= FUSED_QUANT_WIDE_TOKENS
-    any_call = not captured or outputs * k <= FUSED_QUANT_SMALL_LAYER
-    return tokens <= (FUSED_QUANT_TOKENS if any_call else FUSED_QUANT_CAPTURED_TOKENS)
+def quantises_in_gemm(tokens: int, outputs: int) -> bool:
+    """Whether a plain call of a layer quantises its activations inside the GEMM launch."""
+    return tokens <= (FUSED_QUANT_TOKENS if outputs <= FUSED_QUANT_MAX_OUTPUTS else FUSED_QUANT_WIDE_TOKENS)
 
 
 def _stream(device) -> int:
@@ -277,10 +266,9 @@ class DualLinear:
         y = torch.empty((tokens, self.outputs), dtype=self.dtype, device=x.device)
         low, high = self.problems(x, x, y)
         handle = self._handle(tokens, self.low_id, self.high_id, C.byref(low), C.byref(high), _stream(x.device))
-        eager, captured = (quantises_in_gemm(tokens, self.outputs, self.k, c) for c in (False, True))
+        fused = int(quantises_in_gemm(tokens, self.outputs))
         if self.low_id or self.high_id:   # an explicit schedule: the kernel of hg_gemm_tc.cu, whose quantisers save a launch and no time on the GPU
-            eager, captured = eager and self.outputs <= FUSED_QUANT_MAX_OUTPUTS, captured and tokens == 1 and self.outputs <= FUSED_QUANT_MAX_OUTPUTS
-        fused = 1 if captured else 2 if eager else 0
+            fused = (1 if tokens == 1 else 2) if fused and self.outputs <= FUSED_QUANT_MAX_OUTPUTS else 0
         self._ready[tokens] = _host.prepare(self, tokens, handle.value, C.addressof(low), C.addressof(high), (low, high), y,
                                             tokens * self.k + scale_size(tokens, self.k), fused)
         result = _host.forward(self, x, math)
