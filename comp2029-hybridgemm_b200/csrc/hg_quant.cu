@@ -449,7 +449,8 @@ __device__ __forceinline__ void silu16(const Raw16& gate, const Raw16& up, Raw16
 }
 
 // SwiGLU + MXFP8 for many rows; bound by instruction issue.  2048 x 18944 bf16 44.8 us (62 % of the memory bandwidth; 46.2 with the
-// exact functions at every pair in doubt and four blocks to an SM), 777 rows 19.2 us (21.7), 60 with silu8 throughout at 2048.
+// exact functions at every pair in doubt and four blocks to an SM), 777 rows 19.2 us (21.7), 60 with silu8 throughout at 2048.  The
+// bf16 instance spills 32 bytes a thread (80 with four blocks).
 template <typename T, int MATH>
 __global__ void __launch_bounds__(256, 3)
 mx_silu_rows_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, uint8_t* __restrict__ sf, uint16_t* __restrict__ debug, int rows, int k) {
@@ -508,10 +509,11 @@ mx_silu_rows_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, 
     *reinterpret_cast<uint4*>(sf + scale_word_offset(row0, col >> 7, k)) = make_uint4(word[0], word[1], word[2], word[3]);
 }
 
-// From this many elements on (SwiGLU: twice as many) the many-rows kernels are faster (K = 3584: 777 rows 3.2 us against 3.8,
-// 2048 rows 6.5 against 5.4; SwiGLU: 512 x 8192 7.6 us against 11.7, 256 x 18944 8.8 against 9.3, 777 x 18944 23.3 against 21.0,
-// 2048 x 18944 57 against 45); below, one load per thread has the shorter chain.  gate_up's 37888 x 3584 weights to MXFP4:
-// 107 us against 56.
+// From this many elements on (SwiGLU: twice as many) the many-rows kernels are faster; below, one load per thread has the shorter chain.
+// Inputs in L2, few rows against many, bf16: 1171 x 3584 (4.0 Mi) 3.2 us against 3.6, 1400 x 3584 3.8 and 3.65, 2048 x 3584 5.25 and
+// 4.4, 777 x 18944 9.9 and 6.7; SwiGLU 300 x 14336 (4.1 Mi) 6.7 and 9.3, 500 x 14336 10.35 and 10.9, 585 x 14336 (8.0 Mi) 11.9
+// and 11.8, 1024 x 8192 11.9 and 12.1, 600 x 18944 15.7 and 13.7, 2048 x 18944 52 and 45; fp16 the same within 5 %.  In layer calls
+// around 8 Mi elements the many-rows SwiGLU is 3 % better on average.  gate_up's 37888 x 3584 weights to MXFP4: 107 us against 54.
 constexpr int64_t kManyRowsElements = 4 << 20;
 
 // Where the few-rows SwiGLU takes doubtful pairs in place (fp16).  It runs beside the GEMM of gate_up, whose pairs of CTAs (from 33 tokens

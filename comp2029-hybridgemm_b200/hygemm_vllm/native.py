@@ -35,10 +35,15 @@ PACK_MODE = int(os.environ.get("HYGEMM_PACK_MODE", "0"))
 # Calls of at most FUSED_QUANT_TOKENS tokens quantise the activations inside the GEMM kernel (`hg_run_x`: one launch instead of
 # two, identical bytes); HYGEMM_FUSED_QUANT=0 turns it off.
 FUSED_QUANT_TOKENS = 16 if os.environ.get("HYGEMM_FUSED_QUANT", "1") != "0" else 0
-# Every CTA quantises the K slice it multiplies, so the work repeats once per row tile.  Layers wider than this many output
-# channels keep the separate quantiser launch from FUSED_QUANT_WIDE_TOKENS + 1 tokens on: a captured decoder block with gate_up,
-# 37888 wide, takes 39.0 us against 40.4 with gate_up's own quantiser launch at 8 tokens, and 41.0 either way at 16.  A width
-# that is asked for holds at every token count.
+# Every CTA quantises the K slice it multiplies, so the work repeats once per row tile, and a separate quantiser of an older input may
+# run under the GEMM in front.  Up to 8192 output channels one launch is better or level at every token count on average: 27
+# captured decode blocks of 13 to 16 tokens took 1.5 % less than with quantisers in front (hidden sizes 1280 to 2048 3 to 12 % less, 3328 to
+# 3584 with as many qkv channels 2 to 4 % more); deciding it layer by layer there is worse than either (Qwen2.5-7B at 16 tokens 37.7 us with
+# qkv and o_proj in one launch or in two each, 38.9 with o_proj alone in two).  Wider layers have several row tiles to a CTA and do it up to
+# FUSED_QUANT_WIDE_TOKENS tokens: at 8, on an older input and behind a kernel that has just written it (that one included), 37888 x
+# 3584 takes 15.3 -> 14.3 us and 17.7 -> 17.4, 28672 x 8192 27.4 -> 26.4 and 30.2 -> 30.7, 16384 x 5120 10.9 -> 10.6 and 13.4 -> 14.1
+# (the worst of thirteen, which gain 6 % on average on older inputs and 1 % behind the writer); at 10 those of 12288 channels and
+# more lose up to 4 % behind the writer.  A width that is asked for holds at every token count.
 _max_outputs = os.environ.get("HYGEMM_FUSED_QUANT_MAX_OUTPUTS")
 FUSED_QUANT_MAX_OUTPUTS = int(_max_outputs or "8192")
 FUSED_QUANT_WIDE_TOKENS = 0 if _max_outputs else min(8, FUSED_QUANT_TOKENS)
